@@ -67,7 +67,7 @@ NORMALS_OFF, NORMALS_BYTES, NORMALS_FLOAT = 0, 1, 2
 # inside fill: +z ray parity (ClassifyInOutCPU / ClassifyInOutLevel2CPU) or the rasterised
 # stencil parity (ClassifyInOut2x / ClassifyInOut2xLevel2)
 FILL_RAY, FILL_STENCIL = 0, 1
-# Level2 SAT organisation (identical results): chosen per launch, queued records, or per lane
+# Level2 SAT organisation: one serves all, the values are accepted without effect
 LEVEL2_AUTO, LEVEL2_QUEUED, LEVEL2_INLINE = 0, 1, 2
 
 
@@ -313,7 +313,8 @@ class Context:
         self._check(lib().gpv_set_level2_chunk(self._h, int(max_voxels)), "set_level2_chunk")
 
     def set_level2_mode(self, mode):
-        """LEVEL2_AUTO (default), LEVEL2_QUEUED or LEVEL2_INLINE: the Level2 SAT organisation."""
+        """LEVEL2_AUTO (default), LEVEL2_QUEUED or LEVEL2_INLINE: accepted, without effect (the Level2
+        SAT has one organisation)."""
         self._check(lib().gpv_set_level2_mode(self._h, int(mode)), "set_level2_mode")
 
     def set_host_expand(self, threads=-1, slab_mask=0xff, share=45, min_level2_bytes=64 << 20):

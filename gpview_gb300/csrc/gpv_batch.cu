@@ -241,7 +241,8 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
       res_hier(n + 1, 0);
   std::vector<MeshDesc> md(n);
   int64_t tris = 0, tiles = 0, fwarps = 0, rows = 0, xchunks = 0, words = 0, togg = 0, stgw = 0;
-  int max_keybits = 1, warp_words = 0;
+  int max_keybits = 1;
+  Level2Words l2_words = {0, 0};
   int64_t max_T = 1;
   bool any_l2 = false;
   for (int m = 0; m < n; ++m) {
@@ -306,7 +307,7 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
   CK(ws.get(&stmp, (size_t)scan_temp_words(swords)));
   // the boundary-voxel total: past the boundary plane's words in the prefix when both are scanned
   const uint32_t *btot = kmark ? wpre + words : wtot;
-  CK(ws.get(&queue, 1 + kMaxSlabs));  // [0] Level1 tickets, [1 + k] Level2 tickets of slab k
+  CK(ws.get(&queue, 1 + 2 * kMaxSlabs));  // [0] Level1 tickets, then those of each slab's Level2 kernels
   // z slabs of the Level2 launch when the outputs go to the host (one mesh): the boundary ranks
   // at up to kMaxSlabs fine slab starts are read with the first phase's counts; the launch then
   // groups fine slabs into as many slabs as the Level2 output size calls for
@@ -361,8 +362,11 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
     d.has_l2 = g.level2 ? 1 : 0;
     d.fnorm = fnorm ? fnorm + d.tri_base : nullptr;
     d.l1n = nmode ? static_cast<uint8_t *>(set->l1n) + res_l1n[m] : nullptr;
-    if (g.level2)
-      warp_words = std::max(warp_words, level2_warp_words(d.g, ctx->l2_chunk_cap, stencil));
+    if (g.level2) {
+      const Level2Words w = level2_warp_words(d.g, ctx->l2_chunk_cap, stencil);
+      l2_words.sat = std::max(l2_words.sat, w.sat);
+      l2_words.fill = std::max(l2_words.fill, w.fill);
+    }
   }
   BatchDev bd;
   bd.md = d_md;
@@ -475,13 +479,6 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
                           d_slab, s);
     mark(4);
   };
-  // the ray fill's u/v-passing items queued before their per-voxel work: measured faster with
-  // Level2 grids of up to 8^3 cells (the Level2 kernel on torus262k 0.596 -> 0.550 ms, on a 16k
-  // sphere at 4^3 0.146 -> 0.129 ms, on 512 meshes of the batched workload 36.6 -> 36.0 ms) and
-  // slower at 16^3 (star1310k 3.94 -> 4.21 ms)
-  bool l2_fillq = !stencil && any_l2;
-  for (int m = 0; m < n; ++m)
-    if (gh[m].level2 && gh[m].cells > kFillQueueCells) l2_fillq = false;
   // per-stage event times of this call (timing on)
   auto take_stage_times = [&] {
     if (!ctx->timing) return;
@@ -571,6 +568,7 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
       CK(ws.get(&useg, (size_t)cap.U + 1));
       CK(ws.get(&sortmp, (size_t)scan_temp_words(cap.U + 1)));
       CK(ws.get(&l2tmp, (size_t)level2_temp_words(cap.U)));
+      CK(ws.get(&bd.smask, (size_t)level2_mask_words(cap.U, cap.l2bytes)));
     }
     CK(ctx_malloc_async(ctx, &set->bindex, 4 * std::max<int64_t>(cap.B, 4), s));
     CK(ctx_malloc_async(ctx, &set->l2, std::max<int64_t>(cap.l2bytes, 16), s));
@@ -584,14 +582,14 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
                        (uint64_t)(uintptr_t)sortmp, (uint64_t)(uintptr_t)l2tmp,
                        (uint64_t)(uintptr_t)set->l1, (uint64_t)(uintptr_t)set->prefix,
                        (uint64_t)(uintptr_t)set->bindex, (uint64_t)(uintptr_t)set->l2,
-                       (uint64_t)warp_words, (uint64_t)l2_fillq, (uint64_t)ctx->l2_mode,
-                       (uint64_t)any_l2})
+                       (uint64_t)l2_words.sat, (uint64_t)l2_words.fill, (uint64_t)any_l2,
+                       (uint64_t)(uintptr_t)bd.smask})
       sig2.push_back(x);
     CK(run_phase(ctx, 2, s, capturing, [&] {
       phase1_launches(cnt, any_l2 ? cap.U + 1 : 0);
       // the second half's bases and sizes, on the device
       launch_plan(bdp, d_md, static_cast<int32_t *>(set->bindex), static_cast<uint8_t *>(set->l2),
-                  cap, ctx->l2_mode, d_plan, s);
+                  cap, d_plan, s);
       mark(5);
       launch_expand(bdp, wpre, s);
       mark(6);
@@ -599,8 +597,8 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
         count_sort_pairs(bdp, nullptr, cap.tiles, keys, vals, wpre + words, cap.U, cap.P, cnt,
                          useg, kalt, valt, wtot + 1, sortmp, s);
         mark(7);
-        launch_level2(bdp, kalt, valt, useg, cap.U, l2tmp, warp_words, ctx->num_sms, s,
-                      [&] { mark(9); }, 0, 1, {}, 0, nullptr, true, l2_fillq);
+        launch_level2(bdp, kalt, valt, useg, cap.U, l2tmp, l2_words, ctx->num_sms, s,
+                      [&] { mark(9); });
       } else {
         mark(7);
         mark(9);
@@ -703,6 +701,7 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
     // every mesh when normals are on
     md[m].pair_base = P2;
     md[m].u_base = ub;
+    md[m].l2_base = l2off[m];
     if (gh[m].level2 || nmode) {
       P2 += (int64_t)st.pairs;
       ub += (int64_t)st.boundary;
@@ -793,6 +792,7 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
     CK(ws.get(&sortmp, (size_t)std::max({sort_seg_temp_words(ntiles), scan_temp_words(P2),
                                          scan_temp_words(ub)})));
     CK(ws.get(&l2tmp, (size_t)level2_temp_words(ub)));
+    if (any_l2) CK(ws.get(&bd.smask, (size_t)level2_mask_words(ub, l2bytes)));
     if (stencil && any_l2) {  // per boundary voxel: the column prefix of sample coverage
       for (int m = 0; m < n; ++m)
         if (gh[m].level2) bd.stp_words = std::max(bd.stp_words, (4 * gh[m].n2[0] * gh[m].n2[1] + 31) / 32);
@@ -838,14 +838,6 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
   }
   // host outputs: recorded too when only page-locked Level1 copies ride along (direct Level2)
   const bool phase1_graph = !sink || (l2_direct && sink->l1_pinned && !packed);
-  bool l2_queue = true;
-  {
-    std::unique_ptr<bool[]> has_l2(new bool[n]);
-    for (int m = 0; m < n; ++m) has_l2[m] = gh[m].level2;
-    l2_queue = ctx->l2_mode == GPV_LEVEL2_QUEUED   ? true
-               : ctx->l2_mode == GPV_LEVEL2_INLINE ? false
-                                                   : level2_queue_pays(ctx->h_stats, has_l2.get(), n);
-  }
   std::vector<uint64_t> sig1;
   bool any_hier = false;
   for (int m = 0; m < n; ++m) any_hier = any_hier || res_hier[m + 1] > res_hier[m];
@@ -856,14 +848,14 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
                      (uint64_t)P2, (uint64_t)max_keybits, (uint64_t)nmode, (uint64_t)val_bits,
                      (uint64_t)(uintptr_t)sortmp, (uint64_t)(uintptr_t)flags, (uint64_t)(uintptr_t)uidx,
                      (uint64_t)(uintptr_t)wtot, (uint64_t)(uintptr_t)useg, (uint64_t)any_l2,
-                     (uint64_t)ub, (uint64_t)(uintptr_t)l2tmp, (uint64_t)warp_words, (uint64_t)zslab,
+                     (uint64_t)ub, (uint64_t)(uintptr_t)l2tmp, (uint64_t)l2_words.sat, (uint64_t)l2_words.fill,
+                     (uint64_t)(uintptr_t)bd.smask, (uint64_t)zslab,
                      (uint64_t)nslab, (uint64_t)gh[0].n[2], (uint64_t)(sink != nullptr),
                      (uint64_t)(uintptr_t)(sink ? sink->l1 : nullptr),
                      (uint64_t)(uintptr_t)(sink ? sink->prefix : nullptr),
                      (uint64_t)(uintptr_t)(sink ? sink->bindex : nullptr), (uint64_t)gh[0].N1,
                      (uint64_t)Btot, (uint64_t)(uintptr_t)set->l1, (uint64_t)(uintptr_t)set->prefix,
-                     (uint64_t)(uintptr_t)set->bindex, (uint64_t)(uintptr_t)cs, (uint64_t)l2_queue,
-                     (uint64_t)l2_fillq,
+                     (uint64_t)(uintptr_t)set->bindex, (uint64_t)(uintptr_t)cs,
                      (uint64_t)n, (uint64_t)(uintptr_t)d_md, (uint64_t)(uintptr_t)ctx->h_md,
                      (uint64_t)(uintptr_t)ctx->h_tiles, (uint64_t)(uintptr_t)ctx->h_tb,
                      (uint64_t)(uintptr_t)stats, (uint64_t)(uintptr_t)ctx->h_stats,
@@ -915,7 +907,7 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
       }
       mark(7);
       if (any_l2)
-        launch_level2(bd, sk, sv, useg, ub, l2tmp, warp_words, ctx->num_sms, s, [&] { mark(9); },
+        launch_level2(bd, sk, sv, useg, ub, l2tmp, l2_words, ctx->num_sms, s, [&] { mark(9); },
                       zslab, nslab, [&](int k, cudaStream_t ls) {
                         if (packed) {  // the host expands this slab's codes once it is done
                           cudaEventRecord(ctx->cev[1 + k], ls);
@@ -929,7 +921,7 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
                         if (b > a)
                           cudaMemcpyAsync(sink->l2 + a, static_cast<uint8_t *>(set->l2) + a, b - a,
                                           cudaMemcpyDeviceToHost, cs);
-                      }, gh[0].n[2], sink ? &ctx->slab_aux : nullptr, l2_queue, l2_fillq);
+                      }, gh[0].n[2], sink ? &ctx->slab_aux : nullptr);
       else
         mark(9);
       if (nmode) {

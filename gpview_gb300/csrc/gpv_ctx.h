@@ -45,7 +45,7 @@ struct gpv_ctx {
   // it at 4 for 16^3 sub-grids).  torus262k at 8^3, Level2 kernel ms: 8 -> 0.626, 16 -> 0.596,
   // 32 -> 0.712 (fewer chunks per column repeat the fill's u/v work for the triangles above them)
   int l2_chunk_cap = 16;
-  int l2_mode = GPV_LEVEL2_AUTO;       // Level2 SAT organisation (GPV_LEVEL2_*)
+  int l2_mode = GPV_LEVEL2_AUTO;       // gpv_set_level2_mode (no effect)
   // failure-detection hooks (gpv_set_debug) and what they caused (gpv_get_debug)
   uint32_t wait_limit = 0;             // Level1 tile wait polls (0: built-in)
   int fail_wait = 0;                   // Level1's tile wait gives up at once

@@ -71,6 +71,7 @@ struct MeshDesc {
   int64_t pair_base;     // ... of pairs (dense layout after the sort)
   int64_t u_base;        // ... of boundary voxels
   int64_t stile_base;    // ... of pair-sort tiles (one-graph calls: set on the device by k_plan)
+  int64_t l2_base;       // ... of Level2 cells (output bytes)
   int32_t ch;            // Level2 chunk length
   int32_t has_l2;        // the mesh has a Level2 grid
   float4 *fnorm;         // normals on: normalised face normal per triangle
@@ -90,7 +91,6 @@ struct MeshDesc {
 // re-runs the call with the exact sizes.
 struct DevPlan {
   uint32_t ok;
-  uint32_t qsel;     // Level2 SAT organisation: 1 queued records, 0 per lane
   uint32_t ub;       // boundary voxels of the meshes with a Level2 grid (the sorted segments)
   uint32_t ntiles;   // pair-sort tiles of those meshes
   unsigned long long P2;       // pairs of those meshes
@@ -128,6 +128,8 @@ struct BatchDev {
   // packed Level2 host output: in z slab k of the Level2 launch, the boundary voxels whose output
   // index is below pk_end[k] write MeshDesc::l2codes instead of bytes (the slab's first share)
   uint32_t pk_end[kSlabsMax] = {};
+  // Level2 SAT masks (one bit per cell) between the two Level2 kernels, level2_mask_words() of them
+  uint32_t *smask = nullptr;
   // one-graph calls: the device-computed sizes of the second half (nullptr: sizes from the host)
   const DevPlan *plan = nullptr;
 };
@@ -179,11 +181,10 @@ void launch_slab_offsets(const uint32_t *wpre, const uint32_t *wtot, int64_t wor
                          int nz, int zslab, int nslab, uint32_t *out, cudaStream_t s);
 // One-graph calls: from the first half's per-mesh counts, the per-mesh bases of the second half
 // (u_base, pair_base, stile_base, and the bindex and l2 slices of the given result arenas) and
-// the DevPlan, checked against the capacities the second half was recorded with.  level2_mode is
-// GPV_LEVEL2_*; the automatic choice is the host's level2_queue_pays, evaluated on the device.
+// the DevPlan, checked against the capacities the second half was recorded with.
 struct PlanCaps { int64_t B, U, l2bytes, tiles, P; };  // boundary, sorted, Level2 bytes, tiles, pairs
 void launch_plan(const BatchDev &bd, MeshDesc *d_md, int32_t *bindex, uint8_t *l2,
-                 const PlanCaps &caps, int level2_mode, DevPlan *plan, cudaStream_t s);
+                 const PlanCaps &caps, DevPlan *plan, cudaStream_t s);
 // Device-side per-mesh pair segments (emit_base, pair_cap, keys, vals) from prep's sat1 counts.
 void launch_pair_bases(const BatchDev &bd, MeshDesc *d_md, uint32_t *keys, uint32_t *vals,
                        int64_t cap, cudaStream_t s);
@@ -224,8 +225,10 @@ bool sort_pairs_seg(const BatchDev &bd, const SortTile *tiles, const int64_t *ti
 constexpr int kSortTileItems = 2048;
 
 int level2_chunk(const GridDev &g, int cap = 32);
-int level2_warp_words(const GridDev &g, int cap = 32, bool stencil = false);
+struct Level2Words { int sat, fill; };  // shared-memory words per warp of the two Level2 kernels
+Level2Words level2_warp_words(const GridDev &g, int cap = 32, bool stencil = false);
 int64_t level2_temp_words(int64_t Btot);
+inline int64_t level2_mask_words(int64_t B, int64_t l2bytes) { return l2bytes / 32 + B + 1; }
 // before_kernel (optional) runs on the host between the work-item launches and the Level2
 // kernel's launch, e.g. to record an event that times the kernel alone.
 // With zslab > 0 and nslab > 1 the Level2 kernel runs once per slab of zslab Level1 layers (one
@@ -237,17 +240,10 @@ struct SlabStreams {  // two streams and their events for overlapping slab launc
   cudaEvent_t fork, join[2];
 };
 void launch_level2(const BatchDev &bd, const uint32_t *keys, const uint32_t *vals,
-                   const uint32_t *useg, int64_t Btot, uint32_t *tmp, int warp_words, int num_sms,
+                   const uint32_t *useg, int64_t Btot, uint32_t *tmp, Level2Words words, int num_sms,
                    cudaStream_t s, const std::function<void()> &before_kernel = {}, int zslab = 0,
                    int nslab = 1, const std::function<void(int, cudaStream_t)> &after_slab = {},
-                   int slab_nz = 0, const SlabStreams *aux = nullptr, bool queue = true,
-                   bool fillq = false);
-// Level2 SAT organisation for a batch (see k_level2c): queued records when most of the pair work
-// belongs to meshes whose pairs carry many (triangle, sub-column) items.
-bool level2_queue_pays(const MeshStats *stats, const bool *has_l2, int n);
-// Level2 ray-fill organisation: the u/v-passing items queued before their per-voxel work when
-// every Level2 grid of the launch has at most kFillQueueCells cells.
-constexpr int kFillQueueCells = 512;
+                   int slab_nz = 0, const SlabStreams *aux = nullptr);
 
 // ---- normals (gpv_normals.cu) ----------------------------------------------------------------
 void launch_face_normals(const BatchDev &bd, cudaStream_t s);

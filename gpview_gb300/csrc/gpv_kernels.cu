@@ -83,31 +83,29 @@ __device__ __forceinline__ void warp_add(unsigned long long *dst, unsigned long 
   }
 }
 
-// The four prep counters of a 256-thread block: one atomic each per block when every thread of
+// The prep counters of a 256-thread block: one atomic each per block when every thread of
 // the block works on the same mesh (the common case), else per warp.  Thousands of per-warp
 // atomics on one counter serialise at L2.
 __device__ __forceinline__ void block_add_prep(MeshStats *st, unsigned long long a,
                                                unsigned long long b, unsigned long long c,
-                                               unsigned long long d, unsigned long long e) {
-  __shared__ unsigned long long s_acc[5][8];
+                                               unsigned long long d) {
+  __shared__ unsigned long long s_acc[4][8];
   __shared__ MeshStats *s_first;
   if (threadIdx.x == 0) s_first = st;
   __syncthreads();
   if (__syncthreads_and(st == s_first)) {
-    a = warp_sum(a); b = warp_sum(b); c = warp_sum(c); d = warp_sum(d); e = warp_sum(e);
+    a = warp_sum(a); b = warp_sum(b); c = warp_sum(c); d = warp_sum(d);
     const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     if (lane == 0) {
       s_acc[0][warp] = a; s_acc[1][warp] = b; s_acc[2][warp] = c; s_acc[3][warp] = d;
-      s_acc[4][warp] = e;
     }
     __syncthreads();
-    if (threadIdx.x < 5) {
+    if (threadIdx.x < 4) {
       unsigned long long v = 0;
 #pragma unroll
       for (int w = 0; w < 8; ++w) v += s_acc[threadIdx.x][w];
       unsigned long long *dst = threadIdx.x == 0 ? &st->sat1 : threadIdx.x == 1 ? &st->sat_units
-                                : threadIdx.x == 2 ? &st->fill_units : threadIdx.x == 3 ? &st->ray1
-                                : &st->xycells;
+                                : threadIdx.x == 2 ? &st->fill_units : &st->ray1;
       if (v) atomicAdd(dst, v);
     }
   } else {
@@ -115,7 +113,6 @@ __device__ __forceinline__ void block_add_prep(MeshStats *st, unsigned long long
     warp_add(&st->sat_units, b);
     warp_add(&st->fill_units, c);
     warp_add(&st->ray1, d);
-    warp_add(&st->xycells, e);
   }
 }
 
@@ -158,7 +155,7 @@ __global__ void __launch_bounds__(256) k_prep(BatchDev bd) {
   const int m = find_mesh<&MeshDesc::tri_base>(bd.md, bd.nmesh, live ? gi : bd.total_tris - 1);
   const MeshDesc &d = bd.md[m];
   const GridDev &g = d.g;
-  unsigned long long sat1 = 0, su = 0, fu = 0, r1 = 0, xy = 0;
+  unsigned long long sat1 = 0, su = 0, fu = 0, r1 = 0;
   if (live) {
     const int64_t t = gi - d.tri_base;
     float V[9];
@@ -196,10 +193,6 @@ __global__ void __launch_bounds__(256) k_prep(BatchDev bd) {
       const int ay = last_le(g.c1[1], g.n[1], mxy, g.c1[1][0], g.g[1]) -
                      first_ge(g.c1[1], g.n[1], mny, g.c1[1][0], g.g[1]) + 1;
       if (ax > 0 && ay > 0) r1 = (unsigned long long)ax * ay * g.n[2];
-      if (g.n2[0] > 0) {  // x/y extent in Level2 cells (the density of the Level2 SAT items)
-        const float ex = fminf((mxx - mnx) * g.inv_g2[0], 1e6f), ey = fminf((mxy - mny) * g.inv_g2[1], 1e6f);
-        xy = (unsigned long long)((ex + 1.f) * (ey + 1.f) * 16.f);
-      }
     }
     const bool sat_ok = lo[0] <= hi[0] && lo[1] <= hi[1] && lo[2] <= hi[2];
     if (sat_ok) {
@@ -224,7 +217,7 @@ __global__ void __launch_bounds__(256) k_prep(BatchDev bd) {
                          (int)pack2(lo[2], hi[2]), 0);
     d.fbox[t] = fb;
   }
-  block_add_prep(d.stats, sat1, su, fu, r1, xy);
+  block_add_prep(d.stats, sat1, su, fu, r1);
 }
 
 // Per-mesh pair emission segments from the candidate counts prep just produced: exclusive prefix
@@ -273,14 +266,13 @@ __global__ void __launch_bounds__(1024) k_pair_bases(int nmesh, MeshDesc *md, ui
 }
 
 // One-graph calls: the second half's per-mesh bases and sizes from the first half's counts (one
-// block; meshes in rounds of 1024, seven running sums scanned together).  The sums, per mesh:
+// block; meshes in rounds of 1024, six running sums scanned together).  The sums, per mesh:
 // 0 boundary voxels (boundaryIndex slices), 1 the same for meshes with a Level2 grid (sorted
-// segments), 2 their Level2 bytes, 3 their pair-sort tiles, 4 their pairs, 5 the pairs of those
-// whose pairs carry many Level2 SAT items (the queued organisation's measure, as
-// level2_queue_pays computes it on the host), 6 meshes with a raised status.
-constexpr int kPlanSums = 7;
+// segments), 2 their Level2 bytes, 3 their pair-sort tiles, 4 their pairs, 5 meshes with a raised
+// status.
+constexpr int kPlanSums = 6;
 __global__ void __launch_bounds__(1024) k_plan(int nmesh, MeshDesc *md, int32_t *bindex,
-                                               uint8_t *l2, PlanCaps caps, int mode,
+                                               uint8_t *l2, PlanCaps caps,
                                                DevPlan *plan) {
   __shared__ unsigned long long s_w[32][kPlanSums];
   __shared__ unsigned long long s_carry[kPlanSums];
@@ -301,8 +293,7 @@ __global__ void __launch_bounds__(1024) k_plan(int nmesh, MeshDesc *md, int32_t 
       v[2] = has ? b * cells : 0ull;
       v[3] = has ? (p + kSortTileItems - 1) / kSortTileItems : 0ull;
       v[4] = has ? p : 0ull;
-      v[5] = (has && st.xycells >= 64ull * p) ? p : 0ull;
-      v[6] = st.status != 0u;
+      v[5] = st.status != 0u;
     }
     unsigned long long x[kPlanSums];
 #pragma unroll
@@ -337,6 +328,7 @@ __global__ void __launch_bounds__(1024) k_plan(int nmesh, MeshDesc *md, int32_t 
       md[m].u_base = (int64_t)e[1];
       md[m].pair_base = (int64_t)e[4];
       md[m].stile_base = (int64_t)e[3];
+      md[m].l2_base = (int64_t)e[2];
       md[m].bindex = bindex + min((long long)e[0], (long long)caps.B);
       md[m].l2 = l2 + min((long long)e[2], (long long)caps.l2bytes);
     }
@@ -349,12 +341,9 @@ __global__ void __launch_bounds__(1024) k_plan(int nmesh, MeshDesc *md, int32_t 
   if (threadIdx.x == 0) {
     const unsigned long long *t = s_carry;
     DevPlan p;
-    p.ok = t[6] == 0 && t[0] <= (unsigned long long)caps.B && t[1] <= (unsigned long long)caps.U &&
+    p.ok = t[5] == 0 && t[0] <= (unsigned long long)caps.B && t[1] <= (unsigned long long)caps.U &&
            t[2] <= (unsigned long long)caps.l2bytes && t[3] <= (unsigned long long)caps.tiles &&
            t[4] <= (unsigned long long)caps.P;
-    p.qsel = mode == GPV_LEVEL2_QUEUED   ? 1u
-             : mode == GPV_LEVEL2_INLINE ? 0u
-                                         : ((double)t[5] > 0.9 * (double)t[4] ? 1u : 0u);
     p.ub = (uint32_t)min(t[1], 0xffffffffull);
     p.ntiles = (uint32_t)min(t[3], 0xffffffffull);
     p.P2 = t[4];
@@ -903,8 +892,8 @@ void launch_pair_bases(const BatchDev &bd, MeshDesc *d_md, uint32_t *keys, uint3
 }
 
 void launch_plan(const BatchDev &bd, MeshDesc *d_md, int32_t *bindex, uint8_t *l2,
-                 const PlanCaps &caps, int level2_mode, DevPlan *plan, cudaStream_t s) {
-  k_plan<<<1, 1024, 0, s>>>(bd.nmesh, d_md, bindex, l2, caps, level2_mode, plan);
+                 const PlanCaps &caps, DevPlan *plan, cudaStream_t s) {
+  k_plan<<<1, 1024, 0, s>>>(bd.nmesh, d_md, bindex, l2, caps, plan);
   count_launch();
 }
 

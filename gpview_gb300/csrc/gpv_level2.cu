@@ -6,18 +6,21 @@
 // recorded in voxels (i,j,z) with z >= k; otherwise 0.
 //
 // Work unit: a chunk of up to CH consecutive boundary voxels of one Level1 column (one warp).
-//   SAT   -- (triangle, sub-column) items of each voxel, flattened over the 32 lanes; the cells
-//            of a sub-column are tested only inside the plane slab that can pass the SAT's own
-//            plane test (PlaneSlab), and one atomic per sub-column writes the z bits.
+//   SAT   -- each axis test of the SAT that crosses an edge with a box axis depends on two of the
+//            three coordinates, so the cells that pass the nine of them are the ones whose x/y, y/z
+//            and x/z squares pass three two-dimensional tests.  Those are solved a row at a time
+//            (row_span): the interval of cells that certainly pass and the one outside which every
+//            cell certainly fails, with the float tests' error bounds.  A sub-column's cells are the
+//            intersection of two such intervals with the plane test's, written with one atomic.
+//            Only sub-columns with a cell between the two intervals (about one in a hundred) run
+//            the exact float tests.
 //   fill  -- the column's triangle entries flagged as topmost occurrences are the union sets
 //            of all voxels of the chunk at once (voxel k sees the triangles whose topmost z is
-//            >= k).  The u/v part of each ray test depends only on the sub-column, so it runs
-//            once per (triangle, sub-column) for the whole chunk.  Voxels that lie certainly below
-//            the triangle (t at their top origin exceeds 1e-6 by twice a float error bound) are
-//            entirely hit: one "full hit" toggle marks the highest of them and a suffix XOR over
-//            the chunk's voxels expands it.  In the remaining voxels t at each origin follows
-//            from t at the top origin (exact t falls by the rise of the origin); only origins
-//            within the error band of the crossing evaluate their own t.
+//            >= k).  The sub-columns whose ray meets the triangle come from the same row solver;
+//            the height of the triangle's plane there gives the number of ray origins below it, so
+//            one toggle marks the highest voxel that is hit entirely (a suffix XOR over the chunk's
+//            voxels expands it) and one run of bits the voxel that holds the crossing.  Rays and
+//            crossings within the error bounds run the exact float tests.
 #include "gpv_internal.h"
 
 namespace gpv {
@@ -27,6 +30,7 @@ namespace {
 constexpr unsigned FULL = 0xffffffffu;
 constexpr float EPS24 = 5.9604644775390625e-08f;  // 2^-24
 constexpr int kWarps = 4;
+constexpr int kDirectCells = 4;  // a triangle whose box meets at most this many cells is tested exactly
 constexpr int kMaskWords = 512;  // words of one mask kind per warp (sets the chunk length)
 
 __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v) {
@@ -46,36 +50,93 @@ __device__ __forceinline__ T warp_sum(T v) {
   return v;
 }
 
-// Slab of cell centres the triangle's plane test can accept.  For a cell centre c the SAT's
-// plane test (planeBoxOverlap on the box-relative, rounded edges) can only pass when
-//   |n_f . (V0 - c)| <= |n_f| . h + E,
-// with n_f the float normal (V1-V0) x (V2-V1) and E a bound on the float deviations of both
-// sides from exact arithmetic.  With R the largest |V_i,q - c_q| over the voxel's centres and
-// h the largest half size, the deviations sum to less than 736 eps R^2 (h + R); E uses 1024.
-struct PlaneSlab { float nx, ny, nz, H; };
+// 1/x to about an ulp (range arithmetic only, never inside a predicate).
+__device__ __forceinline__ float rcp_fast(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float ff(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 
-__device__ __forceinline__ PlaneSlab plane_slab(const float *V, float cx0, float cx1, float cy0,
-                                                float cy1, float cz0, float cz1, const float h[3]) {
-  const float a0 = fs(V[3], V[0]), a1 = fs(V[4], V[1]), a2 = fs(V[5], V[2]);
-  const float b0 = fs(V[6], V[3]), b1 = fs(V[7], V[4]), b2 = fs(V[8], V[5]);
-  PlaneSlab ps;
-  ps.nx = fs(fm(a1, b2), fm(a2, b1));
-  ps.ny = fs(fm(a2, b0), fm(a0, b2));
-  ps.nz = fs(fm(a0, b1), fm(a1, b0));
-  const float lo[3] = {cx0 - h[0], cy0 - h[1], cz0 - h[2]};
-  const float hi[3] = {cx1 + h[0], cy1 + h[1], cz1 + h[2]};
-  float R = 0.f;
-#pragma unroll
-  for (int q = 0; q < 3; ++q) {
-    const float vmn = fminf(V[q], fminf(V[3 + q], V[6 + q]));
-    const float vmx = fmaxf(V[q], fmaxf(V[3 + q], V[6 + q]));
-    R = fmaxf(R, fmaxf(fabsf(vmx - lo[q]), fabsf(hi[q] - vmn)));
+__device__ __forceinline__ uint32_t cvt_pair_ceil(float lo, float hi) {
+  short a, b;  // (the conversion saturates)
+  asm("cvt.rpi.s16.f32 %0, %1;" : "=h"(a) : "f"(lo));
+  asm("cvt.rpi.s16.f32 %0, %1;" : "=h"(b) : "f"(hi));
+  return (uint32_t)(uint16_t)a | ((uint32_t)(uint16_t)b << 16);
+}
+__device__ __forceinline__ uint32_t cvt_pair_floor(float lo, float hi) {
+  short a, b;
+  asm("cvt.rmi.s16.f32 %0, %1;" : "=h"(a) : "f"(lo));
+  asm("cvt.rmi.s16.f32 %0, %1;" : "=h"(b) : "f"(hi));
+  return (uint32_t)(uint16_t)a | ((uint32_t)(uint16_t)b << 16);
+}
+
+// ---- rows of a two-dimensional triangle / square test ----------------------------------------
+// The squares of half sizes (ha, hb) centred at ((i - base) ga, k gb); the triangle (a[], b[]).
+// An edge (ea, eb) separates where eb * a - ea * b of the edge (t, at the square) and of the opposite
+// vertex (t + S) both exceed rad = |eb| ha + |ea| hb or both lie below -rad, so it passes for
+//   t0 + k ea gb - rad + min(S, 0)  <=  (i - base) eb ga  <=  t0 + k ea gb + rad + max(S, 0),
+// t0 being t at (0, 0).  `dl` bounds the roundings of those sides and of what the float test compares
+// (see the callers), ta and tb the distance of the centre tables from their affine form; a slope below
+// 1/512 of the bound is replaced by it, which moves a side by at most 1/16 of it over 32 cells.  kIdx
+// covers the rounding of the index arithmetic (values up to 64 with a relative error of a few 2^-23).
+// Row k passes the edge's float test for every i in [lo + w2, hi - w2] and for none outside [lo, hi],
+// with lo and hi moving by s per row.
+constexpr float kIdx = 1.f / 16384.f;
+struct EdgeRows { float lo, hi, w2, s; };
+
+__device__ __forceinline__ EdgeRows edge_rows(float ea, float eb, float a, float b, float ha, float hb,
+                                              float ga, float gb, float sn, float sp, float dl,
+                                              float ta, float tb, float base) {
+  const float t = ff(eb, a, -(ea * b));
+  const float rad = ff(fabsf(eb), ha, fabsf(ea) * hb);
+  const float d = ff(fabsf(eb), ta, ff(fabsf(ea), tb, dl));
+  const float s = eb * ga;
+  const float inv = rcp_fast(copysignf(fmaxf(fabsf(s), d * (1.f / 512.f)), s));
+  const float x1 = (t - rad + sn) * inv, x2 = (t + rad + sp) * inv;
+  const float w = ff(d, fabsf(inv), kIdx);
+  return {fminf(x1, x2) - w + base, fmaxf(x1, x2) + w + base, 2.f * w, ea * gb * inv};
+}
+
+// Solves rows 0 .. n-1 into out[]: [lo_o, end_o) holds every i of the row that can pass, [lo_i, end_i)
+// only ones that do; one byte each, lo_o | lo_i << 8 | end_i << 16 | end_o << 24.  bl and be are the
+// i that can and that certainly pass the a axis' own test (lo_o | lo_i << 16 and end_i | end_o << 16),
+// and rows outside [in_lo, in_end) may fail the b axis' own: they pass nothing for certain.
+__device__ __forceinline__ void solve_rows(uint32_t *out, int n, float a0, float a1, float a2, float b0,
+                                           float b1, float b2, float ha, float hb, float ga, float gb,
+                                           float dl, float ta, float tb, int base, uint32_t bl,
+                                           uint32_t be, int in_lo, int in_end) {
+  const float e0a = a1 - a0, e0b = b1 - b0, e1a = a2 - a1, e1b = b2 - b1, e2a = a0 - a2, e2b = b0 - b2;
+  const float S = ff(e0b, e1a, -(e0a * e1b));
+  const float sn = fminf(S, 0.f), sp = fmaxf(S, 0.f), fb = (float)base;
+  const EdgeRows r0 = edge_rows(e0a, e0b, a0, b0, ha, hb, ga, gb, sn, sp, dl, ta, tb, fb);
+  const EdgeRows r1 = edge_rows(e1a, e1b, a1, b1, ha, hb, ga, gb, sn, sp, dl, ta, tb, fb);
+  const EdgeRows r2 = edge_rows(e2a, e2b, a2, b2, ha, hb, ga, gb, sn, sp, dl, ta, tb, fb);
+  float k = 0.f;
+#pragma unroll 1
+  for (int i = 0; i < n; ++i, k += 1.f) {
+    const float l0 = ff(k, r0.s, r0.lo), l1 = ff(k, r1.s, r1.lo), l2 = ff(k, r2.s, r2.lo);
+    const float h0 = ff(k, r0.s, r0.hi), h1 = ff(k, r1.s, r1.hi), h2 = ff(k, r2.s, r2.hi);
+    const float lo_o = fmaxf(l0, fmaxf(l1, l2)), hi_o = fminf(h0, fminf(h1, h2));
+    const float lo_i = fmaxf(l0 + r0.w2, fmaxf(l1 + r1.w2, l2 + r2.w2));
+    const float hi_i = fminf(h0 - r0.w2, fminf(h1 - r1.w2, h2 - r2.w2));
+    const uint32_t L = __vmins2(__vmaxs2(cvt_pair_ceil(lo_o, lo_i), bl), 0x00400040u);
+    uint32_t E = __vmaxs2(__vmins2(cvt_pair_floor(hi_i + 1.f, hi_o + 1.f), be), 0u);
+    if (i < in_lo || i >= in_end) E &= 0xffff0000u;
+    out[i] = __byte_perm(L, E, 0x6420);
   }
-  R *= 1.0001f;
-  const float hm = fmaxf(h[0], fmaxf(h[1], h[2]));
-  const float E = 1024.f * EPS24 * R * R * (hm + R);
-  ps.H = fabsf(ps.nx) * h[0] + fabsf(ps.ny) * h[1] + fabsf(ps.nz) * h[2] + E;
-  return ps;
+}
+
+// Cells of one axis whose boxes can meet [tmin, tmax] ([lo, hi]) and those that certainly do
+// ([in_lo, in_end)), by the SAT's own box-axis test; `md` (cells) bounds the distance of the centre
+// table from c0 + k * g2 and the roundings.
+__device__ __forceinline__ void cell_ranges(float tmin, float tmax, float c0, float inv_g2, int n2,
+                                            float md, int &lo, int &hi, int &in_lo, int &in_end) {
+  const float f0 = ff(tmin - c0, inv_g2, 0.5f), f1 = ff(tmax - c0, inv_g2, 0.5f);
+  lo = max(__float2int_rd(f0 - md), 0);
+  hi = min(__float2int_rd(f1 + md), n2 - 1);
+  in_lo = min(max(__float2int_rd(f0 + md), 0), n2);
+  in_end = max(min(__float2int_rd(f1 - md), n2 - 1), -1) + 1;
 }
 
 // Bits of one Level2 column (n2z cells along z) start at bit (q*n2x + p)*n2z of a voxel's mask.
@@ -99,28 +160,6 @@ __device__ __forceinline__ float ray_tval(const RayTri &r, const RayCol &c, floa
   return fm(fa(fa(fm(r.e2x, q0), fm(r.e2y, q1)), fm(r.e2z, q2)), r.inv_det);
 }
 
-// First index i in [0, n] with tab[i] >= x, and last index in [-1, n-1] with tab[i] <= x, for an
-// increasing table of spacing ~1/inv: an arithmetic estimate corrected by table comparisons
-// (the result is exactly the table's, the estimate only saves the scan).
-__device__ __forceinline__ int tab_first_ge(const float *tab, int n, float x, float inv) {
-  const float t0 = __ldg(tab);
-  if (!(x > t0)) return 0;                       // also x = -inf
-  const float f = fminf((x - t0) * inv, (float)n);  // +inf and huge x clamp to n
-  int i = (int)ceilf(f);
-  while (i > 0 && __ldg(tab + i - 1) >= x) --i;
-  while (i < n && __ldg(tab + i) < x) ++i;
-  return i;
-}
-__device__ __forceinline__ int tab_last_le(const float *tab, int n, float x, float inv) {
-  const float t0 = __ldg(tab);
-  if (x < t0) return -1;
-  const float f = fminf((x - t0) * inv, (float)(n - 1));
-  int i = (int)floorf(f);
-  while (i < n - 1 && __ldg(tab + i + 1) <= x) ++i;
-  while (i >= 0 && __ldg(tab + i) > x) --i;
-  return i;
-}
-
 // Number of origins r in [0, n) with otop - oz[r] > dthr (float subtraction), for an increasing
 // table oz of spacing ~1/inv: the count is a prefix length because otop - oz[r] rounds
 // monotonically; an arithmetic estimate is corrected by table comparisons.
@@ -131,7 +170,9 @@ __device__ __forceinline__ int count_drop_above(const float *oz, int n, float ot
   if (!(f > 0.f)) i = 0;
   else if (f >= (float)n) i = n;
   else i = (int)ceilf(f);
+#pragma unroll 1
   while (i > 0 && !(otop - __ldg(oz + i - 1) > dthr)) --i;
+#pragma unroll 1
   while (i < n && otop - __ldg(oz + i) > dthr) ++i;
   return i;
 }
@@ -139,6 +180,7 @@ __device__ __forceinline__ int count_drop_above(const float *oz, int n, float ot
 // last index tl in [0,31] with pre[tl] <= it (pre nondecreasing, pre[0] = 0)
 __device__ __forceinline__ int batch_search(const uint32_t *pre, uint32_t it) {
   int lo = 0, hi = 31;
+#pragma unroll 1
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
     if (pre[mid] <= it) lo = mid; else hi = mid - 1;
@@ -146,27 +188,37 @@ __device__ __forceinline__ int batch_search(const uint32_t *pre, uint32_t it) {
   return lo;
 }
 
+constexpr int kSol = 640;    // solved rows of one batch (a triangle has at most 96)
+constexpr int kRows = kSol / 2 + 32 * kDirectCells;  // its rows of sub-columns, at most
+
 struct WarpScratch {
-  float v[32][9];     // triangle vertices of the current batch
-  float x[32][7];     // SAT: slab normal, H, 1/(sub-columns per row), 1/nz, slab bound; fill: 1/det,
-                      // well-conditioned flag, 1/(sub-columns per row).  Odd row stride: no bank conflicts
-  uint32_t rng[32];   // packed sub-cell ranges
-  uint32_t pre[33];   // exclusive prefix of item counts
-  int jm[32];         // SAT: the triangle's voxel in the chunk; fill: voxels of the chunk below
-                      // the triangle's topmost voxel
-  uint32_t zrec[32];  // SAT: (triangle slot, p, q) of a sub-column item
-  uint32_t seg[33];   // SAT: first pair of each voxel of the chunk, and the end
-  uint32_t zown[64];  // SAT: (record lane, cell) of each (triangle, cell) item of a window;
-                      // queued fill: Tx of each record
-  uint32_t brec[64];  // SAT: queued (triangle slot, p, q) records of sub-columns passing the
-                      // z-invariant axes; queued fill: (triangle slot, sub-column) records of
-                      // sub-columns passing u/v
-  float fty[64];      // queued fill: Ty of each record
+  float x[32][9];      // per-triangle constants (odd stride: no bank conflicts)
+  uint32_t rng[32][3]; // first sub-column, first row, cell range of exact-only triangles
+  uint32_t tri[32];    // triangle id
+  int jm[32];          // SAT: the triangle's voxel in the chunk; fill: voxels of the chunk up to the
+                       // triangle's topmost voxel; bit 8: exact tests only
+  uint32_t pre[33];    // exclusive prefix of the solved rows
+  uint32_t row[33];    // exclusive prefix of the rows of sub-columns
+  uint32_t seg[33];    // SAT: first pair of each voxel of the chunk, and the end
+  uint32_t sol[kSol];  // solved rows
+  uint32_t rtri[64];   // queued exact work: triangle id and
+  uint32_t rpos[64];   // voxel (or voxel count), sub-column and cell range
+  uint8_t own[kRows];  // triangle slot of each row of sub-columns
 };
+static_assert(sizeof(WarpScratch) % 4 == 0, "word layout");
+
+struct StScratch {    // stencil fill: the batch's triangles
+  float v[32][9];     // snapped vertices and heights
+  float rA[32];
+  uint32_t rng[32];   // packed sample ranges
+  uint32_t pre[33];   // exclusive prefix of sample counts
+};
+static_assert(sizeof(StScratch) <= sizeof(WarpScratch), "the stencil fill's scratch overlays the ray fill's");
 
 // ---- item construction -----------------------------------------------------------------------
 __device__ __forceinline__ int mesh_of_u(const MeshDesc *md, int nmesh, int64_t u) {
   int lo = 0, hi = nmesh - 1;
+#pragma unroll 1
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
     if (md[mid].u_base <= u) lo = mid; else hi = mid - 1;
@@ -234,25 +286,48 @@ __global__ void k_itemflags(BatchDev bd, const uint32_t *__restrict__ keys,
   iflag[u] = (d.has_l2 && start) ? 1u : 0u;
 }
 
-__global__ void k_itemstarts(BatchDev bd, const uint32_t *__restrict__ iflag,
-                             const uint32_t *__restrict__ iord, int64_t Bcap,
-                             uint32_t *__restrict__ istart, uint32_t *__restrict__ nitems) {
+// Work item of the Level2 kernels: a run of boundary voxels of one Level1 column.
+struct __align__(16) Item {
+  uint32_t ua;       // first boundary voxel
+  uint32_t m_mesh;   // voxels (1..32) | first of its column << 6 | mesh << 7
+  uint32_t col;      // column (y * nx + x)
+  uint32_t col_end;  // first boundary voxel of the next column
+};
+
+__global__ void k_itemstarts(BatchDev bd, const uint32_t *__restrict__ keys,
+                             const uint32_t *__restrict__ useg, const uint32_t *__restrict__ cflag,
+                             const uint32_t *__restrict__ cord, const uint32_t *__restrict__ colhead,
+                             const uint32_t *__restrict__ iflag, const uint32_t *__restrict__ iord,
+                             int64_t Bcap, Item *__restrict__ items, uint32_t *__restrict__ nitems) {
   const int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t B = sorted_voxels(bd, Bcap);
   if (u >= B) return;
-  if (iflag[u]) istart[iord[u]] = (uint32_t)u;
+  if (iflag[u]) {
+    const int mesh = mesh_of_u(bd.md, bd.nmesh, u);
+    const MeshDesc &d = bd.md[mesh];
+    Item it;
+    it.ua = (uint32_t)u;
+    it.col = keys[useg[u]] / (uint32_t)d.g.n[2];
+    it.col_end = colhead[cord[u] + cflag[u]];
+    // (an item ends where the next one of its column starts)
+    const uint32_t end = min(it.col_end, (uint32_t)u + (uint32_t)d.ch);
+    uint32_t e = (uint32_t)u + 1;
+    while (e < end && !iflag[e]) ++e;
+    it.m_mesh = (e - (uint32_t)u) | (cflag[u] << 6) | ((uint32_t)mesh << 7);
+    items[iord[u]] = it;
+  }
   if (u == B - 1) *nitems = iord[u] + iflag[u];
 }
 
 // Items of one mesh ordered by z slab (order within a slab is free): per-slab counts, their
 // exclusive prefix (ioff[0..nslab]), then each item placed in its slab's range.
-__global__ void k_item_slab_count(const uint32_t *__restrict__ istart,
+__global__ void k_item_slab_count(const Item *__restrict__ items,
                                   const uint32_t *__restrict__ nitems, const uint32_t *__restrict__ keys,
                                   const uint32_t *__restrict__ useg, int nz, int zslab,
                                   uint32_t *__restrict__ cnt) {
   const int64_t it = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (it >= (int64_t)*nitems) return;
-  atomicAdd(&cnt[(keys[useg[istart[it]]] % (uint32_t)nz) / (uint32_t)zslab], 1u);
+  atomicAdd(&cnt[(keys[useg[items[it].ua]] % (uint32_t)nz) / (uint32_t)zslab], 1u);
 }
 
 __global__ void k_item_slab_offsets(uint32_t *__restrict__ cnt, int nslab, uint32_t *__restrict__ ioff) {
@@ -266,13 +341,13 @@ __global__ void k_item_slab_offsets(uint32_t *__restrict__ cnt, int nslab, uint3
   ioff[nslab] = a;
 }
 
-__global__ void k_item_slab_place(const uint32_t *__restrict__ istart,
+__global__ void k_item_slab_place(const Item *__restrict__ items,
                                   const uint32_t *__restrict__ nitems, const uint32_t *__restrict__ keys,
                                   const uint32_t *__restrict__ useg, int nz, int zslab,
                                   uint32_t *__restrict__ cur, uint32_t *__restrict__ ilist) {
   const int64_t it = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (it >= (int64_t)*nitems) return;
-  const uint32_t sl = (keys[useg[istart[it]]] % (uint32_t)nz) / (uint32_t)zslab;
+  const uint32_t sl = (keys[useg[items[it].ua]] % (uint32_t)nz) / (uint32_t)zslab;
   ilist[atomicAdd(&cur[sl], 1u)] = (uint32_t)it;
 }
 
@@ -291,6 +366,7 @@ __device__ __forceinline__ void write_block_vec(uint8_t *out, uint32_t *codes,
                                                 const uint32_t *ftacc, int ncol2, unsigned lane,
                                                 unsigned long long &nbd, unsigned long long &nin) {
   const int chunks = NZ * ncol2 / 16;
+#pragma unroll 1
   for (int c = (int)lane; c < chunks; c += 32) {
     const int byte0 = c * 16;
     const int r = byte0 / ncol2, pq0 = byte0 - r * ncol2;
@@ -357,7 +433,7 @@ __global__ void __launch_bounds__(kPrefixWarps * 32) k_stencil_segment(
     BatchDev bd, const uint32_t *__restrict__ keys, const uint32_t *__restrict__ vals,
     const uint32_t *__restrict__ useg, const uint32_t *__restrict__ cflag,
     const uint32_t *__restrict__ cord, const uint32_t *__restrict__ colhead,
-    const uint32_t *__restrict__ istart, const uint32_t *__restrict__ nitems, int64_t B) {
+    const Item *__restrict__ items, const uint32_t *__restrict__ nitems, int64_t B) {
   __shared__ uint32_t s_mask[kPrefixWarps][kPrefixMaskWords];
   __shared__ StTri s_t[kPrefixWarps][32];
   __shared__ uint32_t s_pre[kPrefixWarps][32];
@@ -365,8 +441,8 @@ __global__ void __launch_bounds__(kPrefixWarps * 32) k_stencil_segment(
   const int64_t it = (int64_t)blockIdx.x * kPrefixWarps + warp;
   const int64_t NI = (int64_t)*nitems;
   if (it >= NI) return;
-  const uint32_t ua = istart[it];
-  const uint32_t ue = it + 1 < NI ? istart[it + 1] : (uint32_t)B;  // the item's voxels [ua, ue)
+  const uint32_t ua = items[it].ua;
+  const uint32_t ue = it + 1 < NI ? items[it + 1].ua : (uint32_t)B;  // the item's voxels [ua, ue)
   if (ue >= colhead[cord[ua] + cflag[ua]]) return;  // the column's last item: no item reads it
   const MeshDesc &d = bd.md[mesh_of_u(bd.md, bd.nmesh, ua)];
   if (!d.has_l2) return;
@@ -464,561 +540,89 @@ __global__ void __launch_bounds__(kPrefixWarps * 32) k_stencil_scan(
 }
 
 // ---- Level2 ------------------------------------------------------------------------------------
-// ST: the stencil fill (ClassifyInOut2xLevel2) instead of the ray fill.  QUEUE: the (triangle,
-// sub-column) items passing the z-invariant axes are queued and their slab work done 32 records
-// at a time (pays off when a pair has many items: triangles large against the Level2 cells);
-// otherwise each item lane does its own slab work.  FQ (ray fill): the (triangle, sub-column)
-// items passing u/v are queued the same way before their per-voxel work.
-template <bool ST, bool QUEUE, bool FQ>
-// Six blocks per SM for the queued organisation (80 registers); five with the queued fill (96
-// registers, no spills: torus262k 0.535 -> 0.526 ms, a 16k sphere at 4^3 0.136 -> 0.130 ms, while
-// five blocks made star1310k, which keeps the inline fill, 3.6% slower); seven for the per-lane
-// organisation (72), measured 1.5-3% faster there (the 4096-mesh batch, a 4^3 Level2 grid).
-__global__ void __launch_bounds__(kWarps * 32, QUEUE ? (FQ ? 5 : 6) : 7) k_level2c(
-    BatchDev bd, const uint32_t *__restrict__ keys, const uint32_t *__restrict__ vals,
-    const uint32_t *__restrict__ useg, const uint32_t *__restrict__ cflag,
-    const uint32_t *__restrict__ cord, const uint32_t *__restrict__ colhead,
-    const uint32_t *__restrict__ istart, const uint32_t *__restrict__ nitems, int per_warp,
-    int slab, int zslab, const uint32_t *__restrict__ ilist, const uint32_t *__restrict__ ioff) {
-  extern __shared__ uint32_t sm[];
-  // one-graph calls launch both SAT organisations; the device plan picks one
-  if (bd.plan && bd.plan->qsel != (QUEUE ? 1u : 0u)) return;
-  const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  uint32_t *base = sm + (size_t)warp * per_warp;
-  // all items, or (z slabs) this launch's slab of the slab-ordered item list
-  const int64_t i0 = ilist ? (int64_t)ioff[slab] : 0;
-  const int64_t NI = ilist ? (int64_t)ioff[slab + 1] - i0 : (int64_t)*nitems;
-  for (;;) {
-  // ---- pull the next chunk item from the queue (one ticket per warp)
-  uint32_t tk = 0;
-  if (lane == 0) tk = atomicAdd(&bd.queue[1 + slab], 1u);
-  const int64_t it = (int64_t)__shfl_sync(FULL, tk, 0);
-  if (it >= NI) return;
-  const uint32_t ua = ilist ? istart[ilist[i0 + it]] : istart[it];
-  const MeshDesc &d = bd.md[mesh_of_u(bd.md, bd.nmesh, ua)];
-  const GridDev &g = d.g;
-  const float4 *__restrict__ ptri = d.ptri;
-  const float4 *__restrict__ fbox = d.fbox;
-  const int CH = d.ch;
-  const int n2x = g.n2[0], n2y = g.n2[1], n2z = g.n2[2];
-  const int cells = n2x * n2y * n2z;
-  const int W = (cells + 31) >> 5;
-  const int ncol2 = n2x * n2y;
-  const int FW = (ncol2 + 31) >> 5;
-  uint32_t *sat = base;
-  uint32_t *par = sat + CH * W;
-  uint32_t *ft = par + CH * W;
-  int *kz = (int *)(ft + CH * FW);
-  uint32_t *ftacc = (uint32_t *)(kz + CH);
-  WarpScratch &ws = *reinterpret_cast<WarpScratch *>(ftacc + FW);
-  // stencil fill: per voxel, (2 n2x * 2 n2y) sample columns of n2z slice toggle bits; per voxel
-  // one bit per sample toggling every slice of that voxel and of the voxels above it
-  uint32_t *stg = reinterpret_cast<uint32_t *>(&ws + 1);
-  const int SWd = 4 * W;
-  const int FWS = (4 * ncol2 + 31) >> 5;
-  uint32_t *sft = stg + CH * SWd, *sftacc = sft + CH * FWS;
-
-  const uint32_t ucol_end = colhead[cord[ua] + cflag[ua]];  // first voxel of the next column
-  const int nx = g.n[0], ny = g.n[1], nz = g.n[2];
-  const uint32_t col = keys[useg[ua]] / (uint32_t)nz;
-  int m = (int)min((uint32_t)CH, ucol_end - ua);
-  if (zslab > 0) {
-    // this launch takes one slab of zslab Level1 layers; an item ends at the slab's edge and at
-    // the next CH-aligned item start of its column
-    const uint32_t chead = colhead[cord[ua] + cflag[ua] - 1u];
-    bool ok = false;
-    if ((int)lane < m) {
-      const int zl = (int)(keys[useg[ua + lane]] - col * (uint32_t)nz);
-      ok = zl / zslab == slab && (lane == 0 || (ua + lane - chead) % (uint32_t)CH != 0);
-    }
-    m = __ffs(~__ballot_sync(FULL, ok)) - 1;  // leading run of voxels of this item
-    if (m < 0) m = 32;
-  }
-  // clear the masks of the chunk's m voxels only (the arrays are sized for CH voxels)
-  for (int w = lane; w < m * W; w += 32) { sat[w] = 0; par[w] = 0; }
-  for (int w = lane; w < m * FW; w += 32) ft[w] = 0;
-  if (ST) {
-    for (int w = lane; w < m * SWd; w += 32) stg[w] = 0;
-    for (int w = lane; w < m * FWS; w += 32) sft[w] = 0;
-    // the coverage parity of the column's triangles recorded only below the chunk (none below a
-    // column's first voxel; the prefix pass writes the masks of the later chunk starts)
-    const bool first = colhead[cord[ua] + cflag[ua] - 1u] == ua;
-    for (int w = lane; w < FWS; w += 32) sftacc[w] = first ? 0u : bd.stp[(size_t)ua * bd.stp_words + w];
-  }
-  const int ci = (int)(col % (uint32_t)nx), cj = (int)(col / (uint32_t)nx);
-  if ((int)lane < m) kz[lane] = (int)(keys[useg[ua + lane]] - col * (uint32_t)nz);
+// The exact SAT of queued (triangle, voxel, sub-column, cell range) records, one per lane: cells
+// that another triangle has marked already are left out (the state is an OR).
+__device__ __noinline__ void sat_exact(const MeshDesc &d, WarpScratch &ws, uint32_t *sat,
+                                       const int *kz, int ci, int cj, uint32_t nr) {
+  const unsigned lane = threadIdx.x & 31u;
   __syncwarp();
-
-  const float *sx = g.c2s[0] + (size_t)ci * n2x, *sy = g.c2s[1] + (size_t)cj * n2y;
-  const float *ox = g.o2[0] + (size_t)ci * n2x, *oy = g.o2[1] + (size_t)cj * n2y;
-  const float sx0 = __ldg(sx), sx1 = __ldg(sx + n2x - 1), sy0 = __ldg(sy), sy1 = __ldg(sy + n2y - 1);
-
-  // ---------------- SAT of each voxel's own triangles: the chunk's (voxel, triangle) pairs are
-  // contiguous in the sorted lists and are taken 32 at a time across voxel boundaries.
-  if ((int)lane < m) ws.seg[lane] = useg[ua + lane];
-  if (lane == 0) ws.seg[m] = useg[ua + m];
-  __syncwarp();
-  {
-    const uint32_t S0 = ws.seg[0], S1 = ws.seg[m];
-    for (uint32_t b0 = S0; b0 < S1; b0 += 32) {
-      const uint32_t e = b0 + lane;
-      uint32_t cnt = 0;
-      if (e < S1) {
-        int jv = 0;  // last voxel whose segment starts at or before e
-#pragma unroll
-        for (int st = 16; st > 0; st >>= 1)
-          if (jv + st <= m - 1 && ws.seg[jv + st] <= e) jv += st;
+  if (lane < nr) {
+    const GridDev &g = d.g;
+    const int n2x = g.n2[0], n2z = g.n2[2];
+    const int W = (n2x * g.n2[1] * n2z + 31) >> 5;
+    const uint32_t t = ws.rtri[lane], pos = ws.rpos[lane];
+    const int jv = (int)(pos & 31u), p = (int)((pos >> 5) & 31u), q = (int)((pos >> 10) & 31u);
+    const int lo = (int)((pos >> 15) & 63u), end = (int)(pos >> 21);
+    uint32_t *m = sat + jv * W;
+    const int off = (q * n2x + p) * n2z, sh = off & 31;
+    uint32_t done = m[off >> 5] >> sh;
+    if (sh + n2z > 32) done |= m[(off >> 5) + 1] << (32 - sh);
+    uint32_t todo = ((0xffffffffu >> (32 - (end - lo))) << lo) & ~done;
+    if (todo) {
+      const float4 a0 = __ldg(d.ptri + 3 * (size_t)t), a1 = __ldg(d.ptri + 3 * (size_t)t + 1),
+                   a2 = __ldg(d.ptri + 3 * (size_t)t + 2);
+      const float V[9] = {a0.x, a0.y, a0.z, a1.x, a1.y, a1.z, a2.x, a2.y, a2.z};
+      const float h[3] = {g.e2[0], g.e2[1], g.e2[2]};
+      SatCol sc;
+      if (sat_col(V, __ldg(g.c2s[0] + (size_t)ci * n2x + p),
+                  __ldg(g.c2s[1] + (size_t)cj * g.n2[1] + q), h, sc)) {
         const float *sz = g.c2s[2] + (size_t)kz[jv] * n2z;
-        const float sz0 = __ldg(sz), sz1 = __ldg(sz + n2z - 1);
-        const uint32_t t = vals[e] & 0x7fffffffu;
-        const float4 a0 = __ldg(ptri + 3 * (size_t)t), a1 = __ldg(ptri + 3 * (size_t)t + 1),
-                     a2 = __ldg(ptri + 3 * (size_t)t + 2);
-        const float V[9] = {a0.x, a0.y, a0.z, a1.x, a1.y, a1.z, a2.x, a2.y, a2.z};
-        int p0, p1, q0, q1, r0, r1;
-        l2_cell_range(fminf(V[0], fminf(V[3], V[6])), fmaxf(V[0], fmaxf(V[3], V[6])), sx0, g.e2[0],
-                 g.inv_g2[0], n2x, p0, p1);
-        l2_cell_range(fminf(V[1], fminf(V[4], V[7])), fmaxf(V[1], fmaxf(V[4], V[7])), sy0, g.e2[1],
-                 g.inv_g2[1], n2y, q0, q1);
-        l2_cell_range(fminf(V[2], fminf(V[5], V[8])), fmaxf(V[2], fmaxf(V[5], V[8])), sz0, g.e2[2],
-                 g.inv_g2[2], n2z, r0, r1);
-        if (p0 <= p1 && q0 <= q1 && r0 <= r1) {
-          const PlaneSlab ps = plane_slab(V, sx0, sx1, sy0, sy1, sz0, sz1, g.e2);
-#pragma unroll
-          for (int q = 0; q < 9; ++q) ws.v[lane][q] = V[q];
-          ws.x[lane][0] = ps.nx; ws.x[lane][1] = ps.ny; ws.x[lane][2] = ps.nz; ws.x[lane][3] = ps.H;
-          const int np = p1 - p0 + 1;
-          // per-triangle factors of the (triangle, sub-column) items below
-          ws.x[lane][4] = __frcp_rn((float)np);
-          ws.x[lane][5] = fabsf(ps.nz) > 0.f ? __frcp_rn(ps.nz) : 0.f;
-          ws.x[lane][6] = ps.H + 8.f * EPS24 * fabsf(ps.nz) * (fabsf(V[2]) + fabsf(sz0) + fabsf(sz1));
-          ws.rng[lane] = (uint32_t)p0 | ((uint32_t)np << 6) | ((uint32_t)q0 << 12) |
-                         ((uint32_t)r0 << 18) | ((uint32_t)r1 << 24);
-          ws.jm[lane] = jv;
-          cnt = (uint32_t)(np * (q1 - q0 + 1));
+        uint32_t bits = 0;
+#pragma unroll 1
+        while (todo) {
+          const int r = __ffs(todo) - 1;
+          todo &= todo - 1u;
+          if (sat_z(sc, V, __ldg(sz + r), h)) bits |= 1u << r;
         }
-      }
-      const uint32_t inc = warp_incl_scan(cnt);
-      ws.pre[lane] = inc - cnt;
-      const uint32_t tot = __shfl_sync(FULL, inc, 31);
-      __syncwarp();
-      if constexpr (QUEUE) {
-      // (triangle, sub-column) items, 32 at a time (B1): the z-invariant SAT part; the items that
-      // pass are queued as records.  Every 32 records (B2): the plane slab selects the cells left
-      // for the full test, so that those lanes all work; then the (triangle, cell) tests run 32
-      // at a time whatever the per-column cell counts.  Each record lane lists its cells in a
-      // window of 64 slots (its lane and the cell's z), so a test lane reads its work from one
-      // slot.
-      uint32_t nrec = 0;
-      auto run_records = [&](uint32_t nr) {
-        uint32_t zm = 0, rec = 0;
-        if (lane < nr) {
-          rec = ws.brec[lane];
-          const int tl = (int)(rec & 31u), p = (int)((rec >> 5) & 63u), q = (int)((rec >> 11) & 63u);
-          const uint32_t rg = ws.rng[tl];
-          const int r0 = (int)((rg >> 18) & 63u), r1 = (int)((rg >> 24) & 63u);
-          const int jv = ws.jm[tl];
-          const uint32_t *satj = sat + jv * W;
-          const float *sz = g.c2s[2] + (size_t)kz[jv] * n2z;
-          const float sz0 = __ldg(sz);
-          // cells of this column already marked by another triangle need no test (OR only)
-          const int off = (q * n2x + p) * n2z, sh = off & 31;
-          uint32_t done = satj[off >> 5] >> sh;
-          if (sh + n2z > 32) done |= satj[(off >> 5) + 1] << (32 - sh);
-          const float V0 = ws.v[tl][0], V1 = ws.v[tl][1], V2 = ws.v[tl][2];
-          const float cx = __ldg(sx + p), cy = __ldg(sy + q);
-          const float nxs = ws.x[tl][0], nys = ws.x[tl][1], nzs = ws.x[tl][2], H = ws.x[tl][3];
-          const float sxy = fa(fm(nxs, fs(V0, cx)), fm(nys, fs(V1, cy)));
-          // The per-cell slab test |sxy + nz (V0z - cz)| <= H can only pass for cz within
-          // H/|nz| of V0z + sxy/nz; the interval is widened by the float error of that test
-          // (a few ulps of its terms, over |nz|) and one cell, and the exact per-cell test
-          // still runs.
-          int ra = r0, rb = r1;
-          const float rnz = ws.x[tl][5];
-          if (rnz != 0.f) {
-            const float zc = V2 + sxy * rnz;
-            const float ext = (ws.x[tl][6] + 8.f * EPS24 * fabsf(sxy)) * fabsf(rnz);
-            const float igz = g.inv_g2[2];
-            const float fa0 = (zc - ext - sz0) * igz - 1.f, fb0 = (zc + ext - sz0) * igz + 1.f;
-            if (fa0 > -2.f) ra = max(ra, (int)floorf(fminf(fa0, (float)n2z + 2.f)));
-            if (fb0 < (float)n2z + 2.f) rb = min(rb, (int)ceilf(fmaxf(fb0, -2.f)));
-          }
-          // The slab value is monotone in cz (each operation on cz is a monotone rounding:
-          // V0z - cz, then times nz, then plus sxy), so the cells passing |value| <= H are
-          // one interval of [ra, rb]; its ends are found by testing inwards from both ends.
-          while (ra <= rb && !(fabsf(fa(sxy, fm(nzs, fs(V2, __ldg(sz + ra))))) <= H)) ++ra;
-          while (rb > ra && !(fabsf(fa(sxy, fm(nzs, fs(V2, __ldg(sz + rb))))) <= H)) --rb;
-          if (ra <= rb)
-            zm = ((rb - ra + 1 >= 32) ? 0xffffffffu : ((1u << (rb - ra + 1)) - 1u)) << ra & ~done;
+        if (bits) {
+          atomicOr(&m[off >> 5], bits << sh);
+          if (sh + n2z > 32) atomicOr(&m[(off >> 5) + 1], bits >> (32 - sh));
         }
-        __syncwarp();  // records read: the queue may be refilled
-        const uint32_t zc = (uint32_t)__popc(zm);
-        const uint32_t zinc = warp_incl_scan(zc);
-        ws.zrec[lane] = rec;
-        const uint32_t ztot = __shfl_sync(FULL, zinc, 31);
-        for (uint32_t w0 = 0; w0 < ztot; w0 += 64) {
-          // each record lane lists its cells of this window: (record lane, cell r) per slot
-          {
-            uint32_t mm = zm, pos = zinc - zc;
-            while (mm && pos < w0) { mm &= mm - 1u; ++pos; }
-            while (mm && pos < w0 + 64u) {
-              ws.zown[pos - w0] = lane | ((uint32_t)(__ffs(mm) - 1) << 5);
-              mm &= mm - 1u;
-              ++pos;
-            }
-          }
-          __syncwarp();
-          const uint32_t wn = min(64u, ztot - w0);
-          for (uint32_t z = lane; z < wn; z += 32) {
-            const uint32_t own = ws.zown[z];
-            const uint32_t rc = ws.zrec[own & 31u];
-            const int r = (int)(own >> 5);
-            const int tl = (int)(rc & 31u), p = (int)((rc >> 5) & 63u), q = (int)((rc >> 11) & 63u);
-            const int jv = ws.jm[tl];
-            const float *sz = g.c2s[2] + (size_t)kz[jv] * n2z;
-            float V[9];
-#pragma unroll
-            for (int c = 0; c < 9; ++c) V[c] = ws.v[tl][c];
-            SatCol sc;
-            sat_col_values(V, __ldg(sx + p), __ldg(sy + q), sc);
-            if (sat_z(sc, V, __ldg(sz + r), g.e2)) {
-              const int bi = (q * n2x + p) * n2z + r;
-              atomicOr(&sat[jv * W + (bi >> 5)], 1u << (bi & 31));
-            }
-          }
-          __syncwarp();
-        }
-      };
-      // one call site for the record work (the last rounds only drain the queue)
-      for (uint32_t wb = 0; wb < tot || nrec > 0; wb += 32) {
-        const uint32_t w = wb + lane;
-        bool pass = false;
-        uint32_t rec = 0;
-        if (w < tot) {
-          const int tl = batch_search(ws.pre, w);
-          const uint32_t loc = w - ws.pre[tl];
-          const uint32_t rg = ws.rng[tl];
-          const int np = (int)((rg >> 6) & 63u);
-          // loc / np by a float reciprocal: exact here (loc < 1024, np <= 32, so the quotient of
-          // loc + 1/2 stays at least 1/64 away from an integer, far above the rounding)
-          const int qq = __float2int_rz(((float)loc + 0.5f) * ws.x[tl][4]);
-          const int p = (int)(rg & 63u) + (int)loc - qq * np;
-          const int q = (int)((rg >> 12) & 63u) + qq;
-          // No check for sub-columns whose cells are all marked already: it skipped ~2% of the
-          // items and cost more than it saved (the Level2 kernel: star1310k 3.96 -> 3.84 ms,
-          // torus262k 0.558 -> 0.540 ms); the record round still leaves marked cells out.
-          {
-            float V[9];
-#pragma unroll
-            for (int c = 0; c < 9; ++c) V[c] = ws.v[tl][c];
-            SatCol sc;
-            if (sat_col(V, __ldg(sx + p), __ldg(sy + q), g.e2, sc)) {
-              pass = true;
-              rec = (uint32_t)tl | ((uint32_t)p << 5) | ((uint32_t)q << 11);
-            }
-          }
-        }
-        const uint32_t bal = __ballot_sync(FULL, pass);
-        if (pass) ws.brec[nrec + __popc(bal & ((1u << lane) - 1u))] = rec;
-        nrec += (uint32_t)__popc(bal);
-        __syncwarp();
-        if (nrec >= 32 || (wb + 32 >= tot && nrec > 0)) {
-          const uint32_t nr = min(nrec, 32u);
-          run_records(nr);
-          // move the records beyond the first nr to the front
-          const uint32_t rest = (lane + nr < nrec) ? ws.brec[nr + lane] : 0u;
-          __syncwarp();
-          if (lane + nr < nrec) ws.brec[lane] = rest;
-          nrec -= nr;
-          __syncwarp();
-        }
-      }
-      } else {
-      // (triangle, sub-column) items, 32 at a time: z-invariant SAT part and the plane slab
-      // select the cells left for the full test; then those (triangle, cell) tests run 32 at a
-      // time so that the lanes stay busy whatever the per-column cell counts.  Each item lane
-      // lists its cells in a window of 64 slots (its lane and the cell's z), so a test lane
-      // reads its work from one slot.
-      for (uint32_t wb = 0; wb < tot; wb += 32) {
-        const uint32_t w = wb + lane;
-        uint32_t zm = 0, rec = 0;
-        if (w < tot) {
-          const int tl = batch_search(ws.pre, w);
-          const uint32_t loc = w - ws.pre[tl];
-          const uint32_t rg = ws.rng[tl];
-          const int np = (int)((rg >> 6) & 63u);
-          // loc / np by a float reciprocal: exact here (loc < 1024, np <= 32, so the quotient of
-          // loc + 1/2 stays at least 1/64 away from an integer, far above the rounding)
-          const int qq = __float2int_rz(((float)loc + 0.5f) * ws.x[tl][4]);
-          const int p = (int)(rg & 63u) + (int)loc - qq * np;
-          const int q = (int)((rg >> 12) & 63u) + qq;
-          const int r0 = (int)((rg >> 18) & 63u), r1 = (int)((rg >> 24) & 63u);
-          const int jv = ws.jm[tl];
-          const uint32_t *satj = sat + jv * W;
-          const float *sz = g.c2s[2] + (size_t)kz[jv] * n2z;
-          const float sz0 = __ldg(sz), sz1 = __ldg(sz + n2z - 1);
-          // cells of this column already marked by another triangle need no test (OR only); a
-          // gate for columns marked entirely cost more than it saved, as in the queued form
-          const int off = (q * n2x + p) * n2z, sh = off & 31;
-          uint32_t done = satj[off >> 5] >> sh;
-          if (sh + n2z > 32) done |= satj[(off >> 5) + 1] << (32 - sh);
-          {
-            float V[9];
-#pragma unroll
-            for (int c = 0; c < 9; ++c) V[c] = ws.v[tl][c];
-            const float cx = __ldg(sx + p), cy = __ldg(sy + q);
-            SatCol sc;
-            if (sat_col(V, cx, cy, g.e2, sc)) {
-              const float nxs = ws.x[tl][0], nys = ws.x[tl][1], nzs = ws.x[tl][2], H = ws.x[tl][3];
-              const float sxy = fa(fm(nxs, fs(V[0], cx)), fm(nys, fs(V[1], cy)));
-              // The per-cell slab test |sxy + nz (V0z - cz)| <= H can only pass for cz within
-              // H/|nz| of V0z + sxy/nz; the interval is widened by the float error of that test
-              // (a few ulps of its terms, over |nz|) and one cell, and the exact per-cell test
-              // still runs.
-              int ra = r0, rb = r1;
-              const float rnz = ws.x[tl][5];
-              if (rnz != 0.f) {
-                const float zc = V[2] + sxy * rnz;
-                const float ext = (ws.x[tl][6] + 8.f * EPS24 * fabsf(sxy)) * fabsf(rnz);
-                const float igz = g.inv_g2[2];
-                const float fa0 = (zc - ext - sz0) * igz - 1.f, fb0 = (zc + ext - sz0) * igz + 1.f;
-                if (fa0 > -2.f) ra = max(ra, (int)floorf(fminf(fa0, (float)n2z + 2.f)));
-                if (fb0 < (float)n2z + 2.f) rb = min(rb, (int)ceilf(fmaxf(fb0, -2.f)));
-              }
-              // The slab value is monotone in cz (each operation on cz is a monotone rounding:
-              // V0z - cz, then times nz, then plus sxy), so the cells passing |value| <= H are
-              // one interval of [ra, rb]; its ends are found by testing inwards from both ends.
-              while (ra <= rb && !(fabsf(fa(sxy, fm(nzs, fs(V[2], __ldg(sz + ra))))) <= H)) ++ra;
-              while (rb > ra && !(fabsf(fa(sxy, fm(nzs, fs(V[2], __ldg(sz + rb))))) <= H)) --rb;
-              if (ra <= rb)
-                zm = ((rb - ra + 1 >= 32) ? 0xffffffffu : ((1u << (rb - ra + 1)) - 1u)) << ra & ~done;
-              rec = (uint32_t)tl | ((uint32_t)p << 5) | ((uint32_t)q << 11);
-            }
-          }
-        }
-        const uint32_t zc = (uint32_t)__popc(zm);
-        const uint32_t zinc = warp_incl_scan(zc);
-        ws.zrec[lane] = rec;
-        const uint32_t ztot = __shfl_sync(FULL, zinc, 31);
-        for (uint32_t w0 = 0; w0 < ztot; w0 += 64) {
-          // each record lane lists its cells of this window: (record lane, cell r) per slot
-          {
-            uint32_t mm = zm, pos = zinc - zc;
-            while (mm && pos < w0) { mm &= mm - 1u; ++pos; }
-            while (mm && pos < w0 + 64u) {
-              ws.zown[pos - w0] = lane | ((uint32_t)(__ffs(mm) - 1) << 5);
-              mm &= mm - 1u;
-              ++pos;
-            }
-          }
-          __syncwarp();
-          const uint32_t wn = min(64u, ztot - w0);
-          for (uint32_t z = lane; z < wn; z += 32) {
-            const uint32_t own = ws.zown[z];
-            const uint32_t rc = ws.zrec[own & 31u];
-            const int r = (int)(own >> 5);
-            const int tl = (int)(rc & 31u), p = (int)((rc >> 5) & 63u), q = (int)((rc >> 11) & 63u);
-            const int jv = ws.jm[tl];
-            const float *sz = g.c2s[2] + (size_t)kz[jv] * n2z;
-            float V[9];
-#pragma unroll
-            for (int c = 0; c < 9; ++c) V[c] = ws.v[tl][c];
-            SatCol sc;
-            sat_col_values(V, __ldg(sx + p), __ldg(sy + q), sc);
-            if (sat_z(sc, V, __ldg(sz + r), g.e2)) {
-              const int bi = (q * n2x + p) * n2z + r;
-              atomicOr(&sat[jv * W + (bi >> 5)], 1u << (bi & 31));
-            }
-          }
-          __syncwarp();
-        }
-      }
       }
     }
   }
+  __syncwarp();
+}
 
-  uint64_t nun = 0;
-  if (ST) {
-    // ---------------- stencil fill: the triangles recorded anywhere in the Level1 column (the
-    // voxel strip of CreateVoxelStripDisplayLists, src/Object.cpp:605-633: each once, at its
-    // topmost record) are drawn into 2 n2x x 2 n2y samples over the Level1 voxel's x/y extent
-    // (glOrtho over [i*gridSizeX + bBoxMin, + gridSizeX], :1241-1266).  Slice s of voxel k clips
-    // at the Level2 ray-origin height o2z[k][s] (minZ + (s + 0.5)*gridSizeZ2, :1297), so a
-    // covered sample at height zs counts in every slice from the first with o2z >= zs: one
-    // toggle bit there, expanded by a prefix XOR below.
-    // triangles recorded from the chunk's first voxel up (those below are in the prefix)
-    const uint32_t g0 = useg[ua], g1 = useg[ucol_end];
-    const int SW = 2 * n2x, SH = 2 * n2y;
-    const float lx = fa(fm((float)ci, g.g[0]), g.bmin[0]), hx = fa(lx, g.g[0]);
-    const float ly = fa(fm((float)cj, g.g[1]), g.bmin[1]), hy = fa(ly, g.g[1]);
-    const float *ozt = g.o2[2];
-    // with increasing clip heights, the chunk's highest one is its top voxel's last slice
-    const float top_clip = __ldg(ozt + (size_t)kz[m - 1] * n2z + n2z - 1);
-    for (uint32_t b0 = g0; b0 < g1; b0 += 32) {
-      const uint32_t e = b0 + lane;
-      const uint32_t vv = e < g1 ? vals[e] : 0u;
-      uint32_t cnt = 0;
-      if (vv & 0x80000000u) {
-        const uint32_t t = vv & 0x7fffffffu;
-        const float4 a0 = __ldg(ptri + 3 * (size_t)t), a1 = __ldg(ptri + 3 * (size_t)t + 1),
-                     a2 = __ldg(ptri + 3 * (size_t)t + 2);
-        const float V[9] = {a0.x, a0.y, a0.z, a1.x, a1.y, a1.z, a2.x, a2.y, a2.z};
-        // The interpolated height of a covered sample is a convex combination of the vertex
-        // heights up to 7 eps max|z| of rounding, so a triangle whose lowest vertex lies more
-        // than 16 eps max|z| above the chunk's highest clip height counts in none of its slices.
-        const float zmn = fminf(V[2], fminf(V[5], V[8]));
-        const float zmag = fmaxf(fabsf(V[2]), fmaxf(fabsf(V[5]), fabsf(V[8])));
-        const bool above = g.oz_monotone && zmn - 16.f * EPS24 * zmag > top_clip;
-        StTri st;
-        if (!above && st_setup(V, lx, hx, ly, hy, SW, SH, st)) {
-#pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            ws.v[lane][2 * c] = __int_as_float(st.X[c]);
-            ws.v[lane][2 * c + 1] = __int_as_float(st.Y[c]);
-            ws.v[lane][6 + c] = st.z[c];
-          }
-          ws.x[lane][0] = st.rA;
-          const int nsx = st.sx1 - st.sx0 + 1;
-          ws.rng[lane] = (uint32_t)st.sx0 | ((uint32_t)nsx << 7) | ((uint32_t)st.sy0 << 14);
-          cnt = (uint32_t)(nsx * (st.sy1 - st.sy0 + 1));
-        }
+// The exact ray tests of queued (triangle, sub-column) records, one per lane: the toggles of the
+// chunk's voxels at or below the triangle's topmost voxel, top down.
+__device__ __noinline__ void fill_exact(const MeshDesc &d, WarpScratch &ws, uint32_t *par,
+                                        uint32_t *ft, const int *kz, int m, int ci, int cj,
+                                        uint32_t nr) {
+  const unsigned lane = threadIdx.x & 31u;
+  __syncwarp();
+  if (lane < nr) {
+    const GridDev &g = d.g;
+    const int n2x = g.n2[0], n2z = g.n2[2], ncol2 = n2x * g.n2[1];
+    const int W = (ncol2 * n2z + 31) >> 5, FW = (ncol2 + 31) >> 5;
+    const uint32_t t = ws.rtri[lane], pos = ws.rpos[lane];
+    const int p = (int)((pos >> 6) & 31u), q = (int)(pos >> 11), pq = q * n2x + p;
+    const float4 a0 = __ldg(d.ptri + 3 * (size_t)t), a1 = __ldg(d.ptri + 3 * (size_t)t + 1),
+                 a2 = __ldg(d.ptri + 3 * (size_t)t + 2);
+    const float4 fb = __ldg(d.fbox + t);
+    const float V[9] = {a0.x, a0.y, a0.z, a1.x, a1.y, a1.z, a2.x, a2.y, a2.z};
+    RayTri rt;
+    ray_tri_pre(V, a2.w, rt);
+    RayCol rc;
+    if (ray_col(rt, __ldg(g.o2[0] + (size_t)ci * n2x + p), __ldg(g.o2[1] + (size_t)cj * g.n2[1] + q), rc)) {
+      const float *ozt = g.o2[2];
+      // Certification bound E2, or 0 where there is none: an unbounded box marks an ill-conditioned
+      // x/y projection.  |t - t*| <= 8.2 eps M1 |1/det| for every origin of the chunk (t* exact,
+      // affine and decreasing in the origin height), with M1 taken at the largest |Tz| over the
+      // chunk's origins; 16 eps gives the float evaluation room.
+      float E2 = 0.f;
+      if (g.oz_monotone && !isinf(fb.x) && !isinf(fb.z)) {
+        const float Zm = fmaxf(fabsf(__ldg(ozt + (size_t)kz[0] * n2z) - rt.v1z),
+                               fabsf(__ldg(ozt + (size_t)kz[m - 1] * n2z + n2z - 1) - rt.v1z)) * 1.0001f;
+        const float atx = fabsf(rc.Tx), aty = fabsf(rc.Ty);
+        const float M1 = fabsf(rt.e2x) * (aty * fabsf(rt.e1z) + Zm * fabsf(rt.e1y)) +
+                         fabsf(rt.e2y) * (Zm * fabsf(rt.e1x) + atx * fabsf(rt.e1z)) +
+                         fabsf(rt.e2z) * (atx * fabsf(rt.e1y) + aty * fabsf(rt.e1x));
+        E2 = 2.f * 16.f * EPS24 * M1 * fabsf(rt.inv_det) * 1.0001f;
       }
-      const uint32_t inc = warp_incl_scan(cnt);
-      ws.pre[lane] = inc - cnt;
-      const uint32_t tot = __shfl_sync(FULL, inc, 31);
-      __syncwarp();
-      for (uint32_t w = lane; w < tot; w += 32) {
-        const int tl = batch_search(ws.pre, w);
-        const uint32_t loc = w - ws.pre[tl];
-        const uint32_t rg = ws.rng[tl];
-        const uint32_t nsx = (rg >> 7) & 127u;
-        const uint32_t row = loc / nsx;
-        StTri st;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          st.X[c] = __float_as_int(ws.v[tl][2 * c]);
-          st.Y[c] = __float_as_int(ws.v[tl][2 * c + 1]);
-          st.z[c] = ws.v[tl][6 + c];
-        }
-        st.rA = ws.x[tl][0];
-        const int sx = (int)(rg & 127u) + (int)(loc - row * nsx), sy = (int)((rg >> 14) & 127u) + (int)row;
-        float zs;
-        if (!st_cover(st, sx, sy, zs)) continue;
-        const int sidx = sy * SW + sx, sbit = sidx * n2z;
-        if (g.oz_monotone) {
-          // clip heights increase through the chunk: the lowest voxel whose top clip keeps zs
-          // gets its toggle at the first such slice, and every voxel above it keeps zs in all
-          // slices (one bit in its sample-toggle row, accumulated upwards)
-          int jv = 0;
-          while (jv < m && !(__ldg(ozt + (size_t)kz[jv] * n2z + n2z - 1) >= zs)) ++jv;
-          if (jv < m) {
-            const int b = sbit + st_first_slice(ozt + (size_t)kz[jv] * n2z, n2z, zs);
-            atomicXor(&stg[jv * SWd + (b >> 5)], 1u << (b & 31));
-            if (jv + 1 < m) atomicXor(&sft[(jv + 1) * FWS + (sidx >> 5)], 1u << (sidx & 31));
-          }
-        } else {
-          for (int jv = m - 1; jv >= 0; --jv) {
-            const int s0 = st_first_slice(ozt + (size_t)kz[jv] * n2z, n2z, zs);
-            if (s0 < n2z) {
-              const int b = sbit + s0;
-              atomicXor(&stg[jv * SWd + (b >> 5)], 1u << (b & 31));
-            }
-          }
-        }
-      }
-      __syncwarp();
-    }
-    // a cell is inside when at least 3 of its 4 samples are odd (ClassifyInOut2xLevel2,
-    // :1383-1401): parity per slice = prefix XOR of the sample column's toggles
-    const uint32_t zmask = n2z >= 32 ? 0xffffffffu : ((1u << n2z) - 1u);
-    for (int jv = 0; jv < m; ++jv) {
-      // samples toggled in every slice of this voxel: the XOR of the rows of it and below
-      for (int w = lane; w < FWS; w += 32) sftacc[w] ^= sft[jv * FWS + w];
-      __syncwarp();
-      const uint32_t *sj = stg + jv * SWd;
-      for (int pq = lane; pq < ncol2; pq += 32) {
-        const int q = pq / n2x, p = pq - q * n2x;
-        uint32_t x[4];
-#pragma unroll
-        for (int a = 0; a < 4; ++a) {
-          const int sidx = (2 * q + (a >> 1)) * SW + 2 * p + (a & 1);
-          uint32_t y = column_bits(sj, sidx * n2z, n2z);
-          y ^= y << 1; y ^= y << 2; y ^= y << 4; y ^= y << 8; y ^= y << 16;
-          if ((sftacc[sidx >> 5] >> (sidx & 31)) & 1u) y = ~y;
-          x[a] = y;
-        }
-        const uint32_t in = ((x[0] & x[1] & (x[2] | x[3])) | (x[2] & x[3] & (x[0] | x[1]))) & zmask;
-        if (in) or_column(par + jv * W, pq, n2z, in);
-      }
-    }
-    __syncwarp();
-  } else {
-  // ---------------- fill: u/v once per (triangle, sub-column) for the whole chunk
-  const uint32_t f0 = useg[ua], f1 = useg[ucol_end];
-  const float *ozt = g.o2[2];
-  const float oz_lo = __ldg(ozt + (size_t)kz[0] * n2z);
-  const float oz_hi = __ldg(ozt + (size_t)kz[m - 1] * n2z + n2z - 1);
-  for (uint32_t b0 = f0; b0 < f1; b0 += 32) {
-    const uint32_t e = b0 + lane;
-    const uint32_t vv = e < f1 ? vals[e] : 0u;
-    uint32_t cnt = 0;
-    if (vv & 0x80000000u) {
-      const uint32_t t = vv & 0x7fffffffu;
-      const int zt = (int)(keys[e] - col * (uint32_t)nz);
-      int jm = 0;
-      while (jm < m && kz[jm] <= zt) ++jm;
-      nun += (uint64_t)jm;
-      const float4 fb = __ldg(fbox + t);
-      if (jm > 0 && fb.x <= fb.z) {
-        // sub-columns whose origin lies in the box: first origin >= lo, last origin <= hi
-        const int p0 = tab_first_ge(ox, n2x, fb.x, g.inv_g2[0]);
-        const int p1 = tab_last_le(ox, n2x, fb.z, g.inv_g2[0]);
-        const int q0 = tab_first_ge(oy, n2y, fb.y, g.inv_g2[1]);
-        const int q1 = tab_last_le(oy, n2y, fb.w, g.inv_g2[1]);
-        if (p0 <= p1 && q0 <= q1) {
-          const float4 a0 = __ldg(ptri + 3 * (size_t)t), a1 = __ldg(ptri + 3 * (size_t)t + 1),
-                       a2 = __ldg(ptri + 3 * (size_t)t + 2);
-          const float V[9] = {a0.x, a0.y, a0.z, a1.x, a1.y, a1.z, a2.x, a2.y, a2.z};
-          RayTri rt;
-          ray_tri_pre(V, a2.w, rt);
-          ws.v[lane][0] = rt.v1x; ws.v[lane][1] = rt.v1y; ws.v[lane][2] = rt.v1z;
-          ws.v[lane][3] = rt.e1x; ws.v[lane][4] = rt.e1y; ws.v[lane][5] = rt.e1z;
-          ws.v[lane][6] = rt.e2x; ws.v[lane][7] = rt.e2y; ws.v[lane][8] = rt.e2z;
-          ws.x[lane][0] = rt.inv_det;
-          // Certification bound E2 (below), or 0 where there is none: an unbounded box marks an
-          // ill-conditioned x/y projection.  |t - t*| <= 8.2 eps M1 |1/det| for every origin of
-          // the chunk (t* exact, affine and decreasing in the origin height), with M1 taken at
-          // the largest |Tx|, |Ty| over the triangle's sub-columns (Tx = ox - v1x rounds
-          // monotonically in ox, so the extremes sit at the range ends) and the largest |Tz|
-          // over the chunk's origins; 16 eps gives the float evaluation room.
-          float E2 = 0.f;
-          if (g.oz_monotone && !isinf(fb.x) && !isinf(fb.z)) {
-            const float Zm = fmaxf(fabsf(oz_lo - rt.v1z), fabsf(oz_hi - rt.v1z)) * 1.0001f;
-            const float atx = fmaxf(fabsf(fs(__ldg(ox + p0), rt.v1x)), fabsf(fs(__ldg(ox + p1), rt.v1x)));
-            const float aty = fmaxf(fabsf(fs(__ldg(oy + q0), rt.v1y)), fabsf(fs(__ldg(oy + q1), rt.v1y)));
-            const float M1 = fabsf(rt.e2x) * (aty * fabsf(rt.e1z) + Zm * fabsf(rt.e1y)) +
-                             fabsf(rt.e2y) * (Zm * fabsf(rt.e1x) + atx * fabsf(rt.e1z)) +
-                             fabsf(rt.e2z) * (atx * fabsf(rt.e1y) + aty * fabsf(rt.e1x));
-            E2 = 2.f * 16.f * EPS24 * M1 * fabsf(rt.inv_det) * 1.0001f;
-          }
-          ws.x[lane][1] = E2;
-          const int np = p1 - p0 + 1;
-          ws.x[lane][2] = __frcp_rn((float)np);
-          ws.rng[lane] = (uint32_t)p0 | ((uint32_t)np << 6) | ((uint32_t)q0 << 12);
-          ws.jm[lane] = jm;
-          cnt = (uint32_t)(np * (q1 - q0 + 1));
-        }
-      }
-    }
-    const uint32_t inc = warp_incl_scan(cnt);
-    ws.pre[lane] = inc - cnt;
-    const uint32_t tot = __shfl_sync(FULL, inc, 31);
-    __syncwarp();
-    // The toggles of one (triangle slot, sub-column pq) item that passed u/v, in the voxels of the
-    // chunk at or below the triangle's topmost voxel, top down.
-    auto item_voxels = [&](const RayTri &rt, const RayCol &rc, int tl, int pq) {
-      const float E2 = ws.x[tl][1];
       const bool well = E2 > 0.f;
-      for (int jv = ws.jm[tl] - 1; jv >= 0; --jv) {
+#pragma unroll 1
+      for (int jv = (int)(pos & 63u) - 1; jv >= 0; --jv) {
         const float *oz = ozt + (size_t)kz[jv] * n2z;
         uint32_t bits = 0;
         if (well) {
@@ -1044,134 +648,708 @@ __global__ void __launch_bounds__(kWarps * 32, QUEUE ? (FQ ? 5 : 6) : 7) k_level
           const int rh = count_drop_above(oz, n2z, otop, dhit, g.inv_g2[2]);
           const int rm = count_drop_above(oz, n2z, otop, dmiss, g.inv_g2[2]);
           bits = rh >= 32 ? 0xffffffffu : ((1u << rh) - 1u);
+#pragma unroll 1
           for (int r = rh; r < rm; ++r)
             if (ray_t(rt, rc, __ldg(oz + r), g.thr)) bits |= 1u << r;
         } else {
+#pragma unroll 1
           for (int r = 0; r < n2z; ++r)
             if (ray_t(rt, rc, __ldg(oz + r), g.thr)) bits |= 1u << r;
         }
         if (bits) xor_column(par + jv * W, pq, n2z, bits);
       }
-    };
-    // (triangle slot, p, q) of item w of this batch
-    auto item_of = [&](uint32_t w, int &tl, int &p, int &q) {
-      tl = batch_search(ws.pre, w);
-      const uint32_t loc = w - ws.pre[tl];
-      const uint32_t rg = ws.rng[tl];
-      const int np = (int)((rg >> 6) & 63u);
-      const int qq = __float2int_rz(((float)loc + 0.5f) * ws.x[tl][2]);
-      p = (int)(rg & 63u) + (int)loc - qq * np;
-      q = (int)((rg >> 12) & 63u) + qq;
-    };
-    if constexpr (!FQ) {
-      // each item lane goes on to its own voxels
-      for (uint32_t w = lane; w < tot; w += 32) {
-        int tl, p, q;
-        item_of(w, tl, p, q);
-        RayTri rt;
-        rt.v1x = ws.v[tl][0]; rt.v1y = ws.v[tl][1]; rt.v1z = ws.v[tl][2];
-        rt.e1x = ws.v[tl][3]; rt.e1y = ws.v[tl][4]; rt.e1z = ws.v[tl][5];
-        rt.e2x = ws.v[tl][6]; rt.e2y = ws.v[tl][7]; rt.e2z = ws.v[tl][8];
-        rt.inv_det = ws.x[tl][0];
-        rt.ok = true;
-        RayCol rc;
-        if (!ray_col(rt, __ldg(ox + p), __ldg(oy + q), rc)) continue;
-        item_voxels(rt, rc, tl, q * n2x + p);
+    }
+  }
+  __syncwarp();
+}
+
+// Appends the records of the lanes with `push` to the exact-work queue and returns its length.
+__device__ __forceinline__ uint32_t queue_push(WarpScratch &ws, uint32_t nrec, bool push, uint32_t tri,
+                                               uint32_t pos) {
+  const uint32_t bal = __ballot_sync(FULL, push);
+  if (!bal) return nrec;
+  if (push) {
+    const uint32_t k = nrec + __popc(bal & ((1u << (threadIdx.x & 31u)) - 1u));
+    ws.rtri[k] = tri;
+    ws.rpos[k] = pos;
+  }
+  return nrec + (uint32_t)__popc(bal);
+}
+// Moves the records beyond the first 32 to the front (fewer than 32 of them).
+__device__ __forceinline__ uint32_t queue_shift(WarpScratch &ws, uint32_t nrec) {
+  const unsigned lane = threadIdx.x & 31u;
+  const bool more = lane + 32 < nrec;
+  const uint32_t a = more ? ws.rtri[lane + 32] : 0u, b = more ? ws.rpos[lane + 32] : 0u;
+  __syncwarp();
+  if (more) {
+    ws.rtri[lane] = a;
+    ws.rpos[lane] = b;
+  }
+  __syncwarp();
+  return nrec - 32;
+}
+
+// The next work item of a persistent launch (one ticket per warp): all items, or (z slabs) this
+// launch's slab of the slab-ordered item list.  False: none left.
+__device__ __forceinline__ bool next_item(uint32_t *ticket, const Item *__restrict__ items,
+                                          const uint32_t *__restrict__ nitems, int slab,
+                                          const uint32_t *__restrict__ ilist,
+                                          const uint32_t *__restrict__ ioff, Item &it) {
+  uint32_t tk = 0;
+  if ((threadIdx.x & 31u) == 0) tk = atomicAdd(ticket, 1u);
+  tk = __shfl_sync(FULL, tk, 0);
+  if (ilist) {
+    const uint32_t i0 = ioff[slab];
+    if (tk >= ioff[slab + 1] - i0) return false;
+    tk = ilist[i0 + tk];
+  } else if (tk >= *nitems) {
+    return false;
+  }
+  const uint4 v = __ldg(reinterpret_cast<const uint4 *>(items + tk));
+  it = {v.x, v.y, v.z, v.w};
+  return true;
+}
+
+// Words of a boundary voxel's SAT mask in BatchDev::smask: disjoint for every (mesh, voxel), since
+// the l2_base cells and u_base voxels of the meshes before fill fewer.
+__device__ __forceinline__ uint32_t *sat_words(const BatchDev &bd, const MeshDesc &d, uint32_t u, int W) {
+  return bd.smask + (d.l2_base >> 5) + d.u_base + ((int64_t)u - d.u_base) * W;
+}
+
+// The SAT and the fill are two kernels: one with both is 72 KB of code, and its warps, spread over
+// all of it, waited for instructions more than for anything else (4.9 of 12.5 cycles per issue on a
+// 262k-triangle torus, 128^3 / 8^3; 0.2 with two kernels).  The SAT masks go through device memory
+// (one bit per cell).  Both kernels are bound by instruction issue.  Measured against one kernel
+// testing every (triangle, sub-column) and listed cell exactly, both kernels together: the torus
+// 487 -> 275 us, a 1.3M-triangle star at 256^3 / 16^3 3.51 -> 1.76 ms, 256 mixed meshes in one call
+// 19.9 -> 11.7 ms, 7k large triangles at 150x170x130 / 6^3 279 -> 154 us.  A twentieth of the
+// instructions are exact tests (0.4-2.7% of the sub-columns); a lane per solved row instead of a lane
+// per triangle looping over its rows took 190 us for the torus' SAT against 134.
+//
+// k_level2c_sat: bd.smask gets every boundary voxel's mask of Level2 boundary cells.
+__global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_sat(
+    BatchDev bd, const uint32_t *__restrict__ keys, const uint32_t *__restrict__ vals,
+    const uint32_t *__restrict__ useg, const Item *__restrict__ items,
+    const uint32_t *__restrict__ nitems, int per_warp, int slab, const uint32_t *__restrict__ ilist,
+    const uint32_t *__restrict__ ioff) {
+  extern __shared__ uint32_t sm[];
+  const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  WarpScratch &ws = *reinterpret_cast<WarpScratch *>(sm + (size_t)warp * per_warp);
+  int *const kz = reinterpret_cast<int *>(&ws + 1);
+  uint32_t *const sat = reinterpret_cast<uint32_t *>(kz + 32);
+  Item it;
+  while (next_item(bd.queue + 1 + kSlabsMax + slab, items, nitems, slab, ilist, ioff, it)) {
+  const uint32_t ua = it.ua;
+  const MeshDesc &d = bd.md[it.m_mesh >> 7];
+  const GridDev &g = d.g;
+  const float4 *__restrict__ ptri = d.ptri;
+  const int n2x = g.n2[0], n2y = g.n2[1], n2z = g.n2[2];
+  const int W = (n2x * n2y * n2z + 31) >> 5;
+  const int nx = g.n[0], nz = g.n[2];
+  const int m = (int)(it.m_mesh & 63u);
+  const int ci = (int)(it.col % (uint32_t)nx), cj = (int)(it.col / (uint32_t)nx);
+#pragma unroll 1
+  for (int w = lane; w < m * W; w += 32) sat[w] = 0;
+  if ((int)lane < m) {
+    const uint32_t e = useg[ua + lane];
+    ws.seg[lane] = e;
+    kz[lane] = (int)(keys[e] - it.col * (uint32_t)nz);
+  }
+  if (lane == 0) ws.seg[m] = useg[ua + m];
+  __syncwarp();
+  const float *sx = g.c2s[0] + (size_t)ci * n2x, *sy = g.c2s[1] + (size_t)cj * n2y;
+  const float sx0 = __ldg(sx), sx1 = __ldg(sx + n2x - 1), sy0 = __ldg(sy), sy1 = __ldg(sy + n2y - 1);
+
+  // ---------------- SAT of each voxel's own triangles: the chunk's (voxel, triangle) pairs are
+  // contiguous in the sorted lists and are taken 32 at a time across voxel boundaries.
+  const float gx = g.g2[0], gy = g.g2[1], gz = g.g2[2];
+  // Distance of the centre tables from their affine form within a voxel: two roundings (eps times
+  // the coordinate) of the formulas' doubles.
+  const float tx = 2.02f * EPS24 * fmaxf(fabsf(sx0), fabsf(sx1)), ty = 2.02f * EPS24 * fmaxf(fabsf(sy0), fabsf(sy1));
+  uint32_t nrec = 0;
+  {
+    const float h0 = g.e2[0], h1 = g.e2[1], h2 = g.e2[2];
+    const uint32_t S0 = ws.seg[0], S1 = ws.seg[m];
+    uint32_t taken;  // pairs of a batch: 32, fewer where their rows would not fit
+#pragma unroll 1
+    for (uint32_t b0 = S0; b0 < S1; b0 += taken) {
+      // ---- one triangle per lane: its cell ranges, its plane and its rows
+      const uint32_t e = b0 + lane;
+      int p0 = 0, p1 = -1, pi = 0, pe = 0, q0 = 0, q1 = -1, qi = 0, qe = 0, r0 = 0, r1 = -1, ri = 0, re = 0;
+      bool direct = false;
+      uint32_t nsolve = 0, nrow = 0, t = 0;
+      int jv = 0;  // last voxel whose segment starts at or before e
+      float4 a0, a1, a2;
+      float R = 0.f, tz = 0.f;
+      const float *sz = nullptr;
+      if (e < S1) {
+#pragma unroll
+        for (int st = 16; st > 0; st >>= 1)
+          if (jv + st <= m - 1 && ws.seg[jv + st] <= e) jv += st;
+        sz = g.c2s[2] + (size_t)kz[jv] * n2z;
+        const float sz0 = __ldg(sz), sz1 = __ldg(sz + n2z - 1);
+        t = vals[e] & 0x7fffffffu;
+        a0 = __ldg(ptri + 3 * (size_t)t), a1 = __ldg(ptri + 3 * (size_t)t + 1),
+        a2 = __ldg(ptri + 3 * (size_t)t + 2);
+        const float xn = fminf(a0.x, fminf(a1.x, a2.x)), xx = fmaxf(a0.x, fmaxf(a1.x, a2.x));
+        const float yn = fminf(a0.y, fminf(a1.y, a2.y)), yx = fmaxf(a0.y, fmaxf(a1.y, a2.y));
+        const float zn = fminf(a0.z, fminf(a1.z, a2.z)), zx = fmaxf(a0.z, fmaxf(a1.z, a2.z));
+        tz = 2.02f * EPS24 * fmaxf(fabsf(sz0), fabsf(sz1));
+        cell_ranges(xn, xx, sx0, g.inv_g2[0], n2x, ff(tx, g.inv_g2[0], kIdx), p0, p1, pi, pe);
+        cell_ranges(yn, yx, sy0, g.inv_g2[1], n2y, ff(ty, g.inv_g2[1], kIdx), q0, q1, qi, qe);
+        cell_ranges(zn, zx, sz0, g.inv_g2[2], n2z, ff(tz, g.inv_g2[2], kIdx), r0, r1, ri, re);
+        // R bounds every vertex coordinate relative to a cell of the range, |V - c|, and with it
+        // every edge.  In units of eps R^2 (eps = 2^-24) the float sides of an edge test are off
+        // by less than 12 + 4 (position, radius), solve_rows' by less than 13 + 4 + 15 + 6 + 8
+        // (position, radius, S, sums, slope): 62, and 66 with the slope's 1/16.  In units of
+        // eps R^2 (R + h) the plane test's value is off by less than 78 and the one below by less
+        // than 90: 168, 179 with the slope's.
+        R = 1.0001f * fmaxf(xx - xn + 1.25f * gx + 2.f * tx,
+                            fmaxf(yx - yn + 1.25f * gy + 2.f * ty, zx - zn + 1.25f * gz + 2.f * tz));
+        if (p0 <= p1 && q0 <= q1 && r0 <= r1) {
+          const int np = p1 - p0 + 1, nq = q1 - q0 + 1;
+          // A few cells are tested as fast as they are solved; outside these magnitudes the
+          // bounds' own arithmetic could leave the normal range.
+          direct = np * nq * (r1 - r0 + 1) <= kDirectCells || !(R > 1e-9f && R < 1e9f);
+          nrow = (uint32_t)nq;
+          nsolve = direct ? 0u : (uint32_t)(2 * nq + np);
+          // (exact-only triangles outside the magnitudes have rows too, without solved ones)
+        }
       }
-    } else {
-      // the items passing u/v are queued as (triangle slot, sub-column) records with their Tx, Ty
-      // and their voxels done 32 records at a time, so that every lane of that loop works (most
-      // items fail u/v: 34% pass on torus262k)
-      uint32_t nfr = 0;
-      for (uint32_t wb = 0; wb < tot || nfr > 0; wb += 32) {
-        const uint32_t w = wb + lane;
-        bool pass = false;
-        uint32_t frec = 0;
-        RayCol rc0;
-        if (w < tot) {
-          int tl, p, q;
-          item_of(w, tl, p, q);
-          RayTri rt;  // the fields of the u/v test
-          rt.v1x = ws.v[tl][0]; rt.v1y = ws.v[tl][1];
-          rt.e1x = ws.v[tl][3]; rt.e1y = ws.v[tl][4];
-          rt.e2x = ws.v[tl][6]; rt.e2y = ws.v[tl][7];
-          rt.inv_det = ws.x[tl][0];
-          if (ray_col(rt, __ldg(ox + p), __ldg(oy + q), rc0)) {
-            pass = true;
-            frec = (uint32_t)tl | ((uint32_t)(q * n2x + p) << 5);
+      const uint32_t is = warp_incl_scan(nsolve), ir = warp_incl_scan(nrow);
+      taken = (uint32_t)__popc(__ballot_sync(FULL, is <= (uint32_t)kSol && ir <= (uint32_t)kRows));
+      if (lane == 0) ws.row[0] = 0;
+      ws.row[lane + 1] = ir;
+      if (lane < taken && nrow) {
+        ws.rng[lane][0] = (uint32_t)(p0 | ((p1 + 1) << 8));
+        ws.rng[lane][1] = (uint32_t)q0;
+        ws.rng[lane][2] = (uint32_t)(r0 | ((r1 + 1) << 8));
+        ws.tri[lane] = t;
+        ws.jm[lane] = jv | (direct ? 256 : 0);
+        ws.pre[lane] = is - nsolve;
+        uint8_t *own = ws.own + (ir - nrow);
+#pragma unroll 1
+        for (uint32_t k = 0; k < nrow; ++k) own[k] = (uint8_t)lane;
+        if (!direct) {
+          const int np = p1 - p0 + 1, nq = q1 - q0 + 1;
+          const float c0x = __ldg(sx + p0), c0y = __ldg(sy + q0), c0z = __ldg(sz + r0);
+          const float ux = a0.x - c0x, uy = a0.y - c0y, uz = a0.z - c0z;
+          const float vx = a1.x - c0x, vy = a1.y - c0y, vz = a1.z - c0z;
+          const float wx = a2.x - c0x, wy = a2.y - c0y, wz = a2.z - c0z;
+          // plane: a cell passes when |n . (V0 - c)| <= Hs; along z that is one interval
+          float nx = (vy - uy) * (wz - vz) - (vz - uz) * (wy - vy);
+          float ny = (vz - uz) * (wx - vx) - (vx - ux) * (wz - vz);
+          float nz_ = (vx - ux) * (wy - vy) - (vy - uy) * (wx - vx);
+          if (nz_ < 0.f) { nx = -nx; ny = -ny; nz_ = -nz_; }
+          const float E = 192.f * EPS24 * R * R * (R + fmaxf(h0, fmaxf(h1, h2))) +
+                          1.1f * (fabsf(nx) * tx + fabsf(ny) * ty + nz_ * tz);
+          const float inv = rcp_fast(fmaxf(nz_ * gz, E * (1.f / 512.f)));
+          const float w = ff(E, inv, kIdx);
+          ws.x[lane][0] = nx * ux + ny * uy + nz_ * uz;
+          ws.x[lane][1] = nx * gx;
+          ws.x[lane][2] = ny * gy;
+          ws.x[lane][3] = fabsf(nx) * h0 + fabsf(ny) * h1 + nz_ * h2;
+          ws.x[lane][4] = inv;
+          ws.x[lane][5] = (float)r0 - w;
+          ws.x[lane][6] = (float)r0 + w;
+          const float dl = 72.f * EPS24 * R * R, bx = 1.1f * tx, by = 1.1f * ty, bz = 1.1f * tz;
+          uint32_t *so = ws.sol + (is - nsolve);
+          const uint32_t xl = (uint32_t)(p0 | (pi << 16)), xe = (uint32_t)(pe | ((p1 + 1) << 16));
+          const uint32_t zl = (uint32_t)(r0 | (ri << 16)), ze = (uint32_t)(re | ((r1 + 1) << 16));
+          solve_rows(so, nq, ux, vx, wx, uy, vy, wy, h0, h1, gx, gy, dl, bx, by, p0, xl, xe, qi - q0, qe - q0);
+          solve_rows(so + nq, nq, uz, vz, wz, uy, vy, wy, h2, h1, gz, gy, dl, bz, by, r0, zl, ze, qi - q0, qe - q0);
+          solve_rows(so + 2 * nq, np, uz, vz, wz, ux, vx, wx, h2, h0, gz, gx, dl, bz, bx, r0, zl, ze, pi - p0, pe - p0);
+        }
+      }
+      __syncwarp();
+      // ---- one lane per row of sub-columns, a sub-column at a time
+      const uint32_t R1 = ws.row[taken];
+#pragma unroll 1
+      for (uint32_t rb0 = 0; rb0 < R1; rb0 += 32) {
+        const uint32_t rw = rb0 + lane;
+        int p = 0, pend = 0, pi_ = 0, pe_ = 0, q = 0, jv_ = 0, solz = 0, rlo = 0, rend = 0;
+        uint32_t YL = 0, YE = 0, tri = 0;
+        float num = 0.f, nxg = 0.f, Hs = 0.f, inv = 0.f, k1 = 0.f, k2 = 0.f;
+        bool dir = false;
+        if (rw < R1) {
+          const int tl = ws.own[rw];
+          const int dq = (int)(rw - ws.row[tl]), nq = (int)(ws.row[tl + 1] - ws.row[tl]);
+          const int jm = ws.jm[tl];
+          jv_ = jm & 255;
+          dir = (jm & 256) != 0;
+          tri = ws.tri[tl];
+          q = (int)ws.rng[tl][1] + dq;
+          const uint32_t rx = ws.rng[tl][0];
+          p = (int)(rx & 255u);
+          if (dir) {
+            const uint32_t rz = ws.rng[tl][2];
+            pend = (int)(rx >> 8);
+            rlo = (int)(rz & 255u);
+            rend = (int)(rz >> 8);
+          } else {
+            const uint32_t *so = ws.sol + ws.pre[tl];
+            const uint32_t sxy = so[dq], syz = so[nq + dq];
+            solz = (int)ws.pre[tl] + 2 * nq - p;
+            p = (int)(sxy & 255u);
+            pi_ = (int)((sxy >> 8) & 255u);
+            pe_ = (int)((sxy >> 16) & 255u);
+            pend = (int)(sxy >> 24);
+            YL = __byte_perm(syz, 0, 0x4140);
+            YE = __byte_perm(syz, 0, 0x4342);
+            nxg = ws.x[tl][1];
+            num = ff(-(float)(p - (int)(rx & 255u)), nxg, ff(-(float)dq, ws.x[tl][2], ws.x[tl][0]));
+            Hs = ws.x[tl][3];
+            inv = ws.x[tl][4];
+            k1 = ws.x[tl][5];
+            k2 = ws.x[tl][6];
           }
         }
-        const uint32_t fbal = __ballot_sync(FULL, pass);
-        if (pass) {
-          const uint32_t k = nfr + __popc(fbal & ((1u << lane) - 1u));
-          ws.brec[k] = frec;
-          ws.zown[k] = __float_as_uint(rc0.Tx);
-          ws.fty[k] = rc0.Ty;
+        uint32_t *satj = sat + jv_ * W;
+        float dp = 0.f;
+        const float k1e = k1 + 1.f, k2e = k2 + 1.f;
+#pragma unroll 1
+        while (__any_sync(FULL, p < pend)) {
+          bool amb = false;
+          int lo = rlo, end = rend;
+          if (p < pend) {
+            amb = dir;
+            if (!dir) {
+              const float nv = ff(-dp, nxg, num);
+              const float va = nv - Hs, vb = nv + Hs;
+              const uint32_t sxz = ws.sol[solz + p];
+              const uint32_t L = __vimax3_s16x2(cvt_pair_ceil(ff(va, inv, k1), ff(va, inv, k2)), YL,
+                                                __byte_perm(sxz, 0, 0x4140));
+              const uint32_t E = __vimin3_s16x2(cvt_pair_floor(ff(vb, inv, k1e), ff(vb, inv, k2e)), YE,
+                                                __byte_perm(sxz, 0, 0x4342));
+              const int lo_i = (int)L >> 16, end_i = (int)(short)(E & 0xffffu);
+              lo = (int)(short)(L & 0xffffu);
+              end = (int)E >> 16;
+              const bool sure = p >= pi_ && p < pe_;
+              if (sure && lo_i < end_i)
+                or_column(satj, q * n2x + p, n2z, (0xffffffffu >> (32 - (end_i - lo_i))) << lo_i);
+              amb = lo < end && !(sure && lo == lo_i && end == end_i);
+            }
+          }
+          nrec = queue_push(ws, nrec, amb, tri,
+                            (uint32_t)(jv_ | (p << 5) | (q << 10) | (lo << 15) | (end << 21)));
+          if (nrec >= 32) {
+            sat_exact(d, ws, sat, kz, ci, cj, 32);
+            nrec = queue_shift(ws, nrec);
+          }
+          ++p;
+          dp += 1.f;
         }
-        nfr += (uint32_t)__popc(fbal);
-        __syncwarp();
-        // every 32 records, and at the end of the batch (the records name its triangle slots)
-        if (nfr < 32 && !(wb + 32 >= tot && nfr > 0)) continue;
-        const uint32_t nr = min(nfr, 32u);
-        if (lane < nr) {
-          const uint32_t fr = ws.brec[lane];
-          const int tl = (int)(fr & 31u);
-          RayTri rt;
-          rt.v1x = ws.v[tl][0]; rt.v1y = ws.v[tl][1]; rt.v1z = ws.v[tl][2];
-          rt.e1x = ws.v[tl][3]; rt.e1y = ws.v[tl][4]; rt.e1z = ws.v[tl][5];
-          rt.e2x = ws.v[tl][6]; rt.e2y = ws.v[tl][7]; rt.e2z = ws.v[tl][8];
-          rt.inv_det = ws.x[tl][0];
-          rt.ok = true;
-          RayCol rc;
-          rc.Tx = __uint_as_float(ws.zown[lane]);
-          rc.Ty = ws.fty[lane];
-          item_voxels(rt, rc, tl, (int)(fr >> 5));
+      }
+      __syncwarp();
+    }
+    if (nrec) sat_exact(d, ws, sat, kz, ci, cj, nrec);
+    nrec = 0;
+  }
+  // the masks out
+  uint32_t *out = sat_words(bd, d, ua, W);
+#pragma unroll 1
+  for (int w = lane; w < m * W; w += 32) out[w] = sat[w];
+  __syncwarp();
+  }  // next item
+}
+
+// k_level2c_fill: the inside fill, and the Level2 states from it and the SAT masks.
+// ST: the stencil fill (ClassifyInOut2xLevel2) instead of the ray fill.
+template <bool ST>
+__global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_fill(
+    BatchDev bd, const uint32_t *__restrict__ keys, const uint32_t *__restrict__ vals,
+    const uint32_t *__restrict__ useg, const Item *__restrict__ items,
+    const uint32_t *__restrict__ nitems, int per_warp, int slab, const uint32_t *__restrict__ ilist,
+    const uint32_t *__restrict__ ioff) {
+  extern __shared__ uint32_t sm[];
+  const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  WarpScratch &ws = *reinterpret_cast<WarpScratch *>(sm + (size_t)warp * per_warp);
+  int *const kz = reinterpret_cast<int *>(&ws + 1);
+  uint32_t *const par = reinterpret_cast<uint32_t *>(kz + 32);
+  Item it;
+  while (next_item(bd.queue + 1 + slab, items, nitems, slab, ilist, ioff, it)) {
+  const uint32_t ua = it.ua;
+  const MeshDesc &d = bd.md[it.m_mesh >> 7];
+  const GridDev &g = d.g;
+  const float4 *__restrict__ ptri = d.ptri;
+  const float4 *__restrict__ fbox = d.fbox;
+  const int CH = d.ch;
+  const int n2x = g.n2[0], n2y = g.n2[1], n2z = g.n2[2];
+  const int cells = n2x * n2y * n2z;
+  const int W = (cells + 31) >> 5;
+  const int ncol2 = n2x * n2y;
+  const int FW = (ncol2 + 31) >> 5;
+  uint32_t *ft = par + CH * W, *ftacc = ft + CH * FW;
+  // stencil fill: per voxel, (2 n2x * 2 n2y) sample columns of n2z slice toggle bits; per voxel
+  // one bit per sample toggling every slice of that voxel and of the voxels above it
+  uint32_t *stg = ftacc + FW;
+  const int SWd = 4 * W;
+  const int FWS = (4 * ncol2 + 31) >> 5;
+  uint32_t *sft = stg + CH * SWd, *sftacc = sft + CH * FWS;
+
+  const uint32_t ucol_end = it.col_end;
+  const int nx = g.n[0], ny = g.n[1], nz = g.n[2];
+  const uint32_t col = it.col;
+  const int m = (int)(it.m_mesh & 63u);
+  const int ci = (int)(col % (uint32_t)nx), cj = (int)(col / (uint32_t)nx);
+  // clear the masks of the chunk's m voxels only (the arrays are sized for CH voxels)
+#pragma unroll 1
+  for (int w = lane; w < m * W; w += 32) par[w] = 0;
+#pragma unroll 1
+  for (int w = lane; w < m * FW; w += 32) ft[w] = 0;
+  if (ST) {
+#pragma unroll 1
+    for (int w = lane; w < m * SWd; w += 32) stg[w] = 0;
+#pragma unroll 1
+    for (int w = lane; w < m * FWS; w += 32) sft[w] = 0;
+    // the coverage parity of the column's triangles recorded only below the chunk (none below a
+    // column's first voxel; the prefix pass writes the masks of the later chunk starts)
+    const bool first = (it.m_mesh >> 6) & 1u;
+#pragma unroll 1
+    for (int w = lane; w < FWS; w += 32) sftacc[w] = first ? 0u : bd.stp[(size_t)ua * bd.stp_words + w];
+  }
+  if ((int)lane < m) kz[lane] = (int)(keys[useg[ua + lane]] - col * (uint32_t)nz);
+  __syncwarp();
+  const float *ox = g.o2[0] + (size_t)ci * n2x, *oy = g.o2[1] + (size_t)cj * n2y;
+  uint32_t *const satm = sat_words(bd, d, ua, W);
+
+  uint64_t nun = 0;
+  if (ST) {
+    // ---------------- stencil fill: the triangles recorded anywhere in the Level1 column (the
+    // voxel strip of CreateVoxelStripDisplayLists, src/Object.cpp:605-633: each once, at its
+    // topmost record) are drawn into 2 n2x x 2 n2y samples over the Level1 voxel's x/y extent
+    // (glOrtho over [i*gridSizeX + bBoxMin, + gridSizeX], :1241-1266).  Slice s of voxel k clips
+    // at the Level2 ray-origin height o2z[k][s] (minZ + (s + 0.5)*gridSizeZ2, :1297), so a
+    // covered sample at height zs counts in every slice from the first with o2z >= zs: one
+    // toggle bit there, expanded by a prefix XOR below.
+    StScratch &ss = *reinterpret_cast<StScratch *>(&ws);
+    // triangles recorded from the chunk's first voxel up (those below are in the prefix)
+    const uint32_t g0 = useg[ua], g1 = useg[ucol_end];
+    const int SW = 2 * n2x, SH = 2 * n2y;
+    const float lx = fa(fm((float)ci, g.g[0]), g.bmin[0]), hx = fa(lx, g.g[0]);
+    const float ly = fa(fm((float)cj, g.g[1]), g.bmin[1]), hy = fa(ly, g.g[1]);
+    const float *ozt = g.o2[2];
+    // with increasing clip heights, the chunk's highest one is its top voxel's last slice
+    const float top_clip = __ldg(ozt + (size_t)kz[m - 1] * n2z + n2z - 1);
+#pragma unroll 1
+    for (uint32_t b0 = g0; b0 < g1; b0 += 32) {
+      const uint32_t e = b0 + lane;
+      const uint32_t vv = e < g1 ? vals[e] : 0u;
+      uint32_t cnt = 0;
+      if (vv & 0x80000000u) {
+        const uint32_t t = vv & 0x7fffffffu;
+        const float4 a0 = __ldg(ptri + 3 * (size_t)t), a1 = __ldg(ptri + 3 * (size_t)t + 1),
+                     a2 = __ldg(ptri + 3 * (size_t)t + 2);
+        const float V[9] = {a0.x, a0.y, a0.z, a1.x, a1.y, a1.z, a2.x, a2.y, a2.z};
+        // The interpolated height of a covered sample is a convex combination of the vertex
+        // heights up to 7 eps max|z| of rounding, so a triangle whose lowest vertex lies more
+        // than 16 eps max|z| above the chunk's highest clip height counts in none of its slices.
+        const float zmn = fminf(V[2], fminf(V[5], V[8]));
+        const float zmag = fmaxf(fabsf(V[2]), fmaxf(fabsf(V[5]), fabsf(V[8])));
+        const bool above = g.oz_monotone && zmn - 16.f * EPS24 * zmag > top_clip;
+        StTri st;
+        if (!above && st_setup(V, lx, hx, ly, hy, SW, SH, st)) {
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            ss.v[lane][2 * c] = __int_as_float(st.X[c]);
+            ss.v[lane][2 * c + 1] = __int_as_float(st.Y[c]);
+            ss.v[lane][6 + c] = st.z[c];
+          }
+          ss.rA[lane] = st.rA;
+          const int nsx = st.sx1 - st.sx0 + 1;
+          ss.rng[lane] = (uint32_t)st.sx0 | ((uint32_t)nsx << 7) | ((uint32_t)st.sy0 << 14);
+          cnt = (uint32_t)(nsx * (st.sy1 - st.sy0 + 1));
         }
-        __syncwarp();
-        // move the records beyond the first nr to the front
-        uint32_t m0 = 0, m1 = 0;
-        float m2 = 0.f;
-        if (lane + nr < nfr) { m0 = ws.brec[nr + lane]; m1 = ws.zown[nr + lane]; m2 = ws.fty[nr + lane]; }
-        __syncwarp();
-        if (lane + nr < nfr) { ws.brec[lane] = m0; ws.zown[lane] = m1; ws.fty[lane] = m2; }
-        nfr -= nr;
-        __syncwarp();
+      }
+      const uint32_t inc = warp_incl_scan(cnt);
+      ss.pre[lane] = inc - cnt;
+      const uint32_t tot = __shfl_sync(FULL, inc, 31);
+      __syncwarp();
+#pragma unroll 1
+      for (uint32_t w = lane; w < tot; w += 32) {
+        const int tl = batch_search(ss.pre, w);
+        const uint32_t loc = w - ss.pre[tl];
+        const uint32_t rg = ss.rng[tl];
+        const uint32_t nsx = (rg >> 7) & 127u;
+        const uint32_t row = loc / nsx;
+        StTri st;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          st.X[c] = __float_as_int(ss.v[tl][2 * c]);
+          st.Y[c] = __float_as_int(ss.v[tl][2 * c + 1]);
+          st.z[c] = ss.v[tl][6 + c];
+        }
+        st.rA = ss.rA[tl];
+        const int sx = (int)(rg & 127u) + (int)(loc - row * nsx), sy = (int)((rg >> 14) & 127u) + (int)row;
+        float zs;
+        if (!st_cover(st, sx, sy, zs)) continue;
+        const int sidx = sy * SW + sx, sbit = sidx * n2z;
+        if (g.oz_monotone) {
+          // clip heights increase through the chunk: the lowest voxel whose top clip keeps zs
+          // gets its toggle at the first such slice, and every voxel above it keeps zs in all
+          // slices (one bit in its sample-toggle row, accumulated upwards)
+          int jv = 0;
+#pragma unroll 1
+          while (jv < m && !(__ldg(ozt + (size_t)kz[jv] * n2z + n2z - 1) >= zs)) ++jv;
+          if (jv < m) {
+            const int b = sbit + st_first_slice(ozt + (size_t)kz[jv] * n2z, n2z, zs);
+            atomicXor(&stg[jv * SWd + (b >> 5)], 1u << (b & 31));
+            if (jv + 1 < m) atomicXor(&sft[(jv + 1) * FWS + (sidx >> 5)], 1u << (sidx & 31));
+          }
+        } else {
+#pragma unroll 1
+          for (int jv = m - 1; jv >= 0; --jv) {
+            const int s0 = st_first_slice(ozt + (size_t)kz[jv] * n2z, n2z, zs);
+            if (s0 < n2z) {
+              const int b = sbit + s0;
+              atomicXor(&stg[jv * SWd + (b >> 5)], 1u << (b & 31));
+            }
+          }
+        }
+      }
+      __syncwarp();
+    }
+    // a cell is inside when at least 3 of its 4 samples are odd (ClassifyInOut2xLevel2,
+    // :1383-1401): parity per slice = prefix XOR of the sample column's toggles
+    const uint32_t zmask = n2z >= 32 ? 0xffffffffu : ((1u << n2z) - 1u);
+#pragma unroll 1
+    for (int jv = 0; jv < m; ++jv) {
+      // samples toggled in every slice of this voxel: the XOR of the rows of it and below
+#pragma unroll 1
+      for (int w = lane; w < FWS; w += 32) sftacc[w] ^= sft[jv * FWS + w];
+      __syncwarp();
+      const uint32_t *sj = stg + jv * SWd;
+#pragma unroll 1
+      for (int pq = lane; pq < ncol2; pq += 32) {
+        const int q = pq / n2x, p = pq - q * n2x;
+        uint32_t x[4];
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+          const int sidx = (2 * q + (a >> 1)) * SW + 2 * p + (a & 1);
+          uint32_t y = column_bits(sj, sidx * n2z, n2z);
+          y ^= y << 1; y ^= y << 2; y ^= y << 4; y ^= y << 8; y ^= y << 16;
+          if ((sftacc[sidx >> 5] >> (sidx & 31)) & 1u) y = ~y;
+          x[a] = y;
+        }
+        const uint32_t in = ((x[0] & x[1] & (x[2] | x[3])) | (x[2] & x[3] & (x[0] | x[1]))) & zmask;
+        if (in) or_column(par + jv * W, pq, n2z, in);
       }
     }
     __syncwarp();
+  } else {
+  // ---------------- fill: the sub-columns whose rays meet each triangle, for the whole chunk
+  const float gx = g.g2[0], gy = g.g2[1];
+  uint32_t nrec = 0;
+  const uint32_t f0 = useg[ua], f1 = useg[ucol_end];
+  const float *ozt = g.o2[2];
+  const int kz0 = kz[0];
+  const float ozb = __ldg(ozt + (size_t)kz0 * n2z), ozl = __ldg(ozt + (size_t)kz[m - 1] * n2z + n2z - 1);
+  const float ox0 = __ldg(ox), oy0 = __ldg(oy);
+  // distance of the origin tables from their affine form: within a voxel two roundings; over the
+  // chunk's heights the voxels' own corners (a float product and sum) too
+  const float tox = 2.02f * EPS24 * fmaxf(fabsf(ox0), fabsf(__ldg(ox + n2x - 1)));
+  const float toy = 2.02f * EPS24 * fmaxf(fabsf(oy0), fabsf(__ldg(oy + n2y - 1)));
+  const float toz = EPS24 * (6.1f * fmaxf(fabsf(ozb), fabsf(ozl)) + 4.1f * fabsf(g.bmin[2]));
+  const float mx = ff(tox, g.inv_g2[0], kIdx), my = ff(toy, g.inv_g2[1], kIdx);
+  const int span = (kz[m - 1] - kz0 + 1) * n2z;  // ray origins from the chunk's first voxel to its last
+  const float inv_n2z = rcp_fast((float)n2z);
+  // bit i: layer kz0 + i belongs to the chunk
+  const uint32_t layers = __reduce_or_sync(FULL, ((int)lane < m && kz[lane] - kz0 < 32) ? 1u << (kz[lane] - kz0) : 0u);
+  const bool near = kz[m - 1] - kz0 < 32;
+  uint32_t taken;  // records of a batch: 32, fewer where their rows would not fit
+#pragma unroll 1
+  for (uint32_t b0 = f0; b0 < f1; b0 += taken) {
+    const uint32_t e = b0 + lane;
+    const uint32_t vv = e < f1 ? vals[e] : 0u;
+    uint32_t nsolve = 0, nrow = 0;
+    int jmv = 0, p0 = 0, p1 = 0;
+    float ux = 0.f, uy = 0.f, vx = 0.f, vy = 0.f, wx = 0.f, wy = 0.f, dl = 0.f;
+    bool direct = false;
+    if (vv & 0x80000000u) {
+      const uint32_t t = vv & 0x7fffffffu;
+      const int zt = (int)(keys[e] - col * (uint32_t)nz);
+      int jm = 0;
+#pragma unroll 1
+      while (jm < m && kz[jm] <= zt) ++jm;
+      jmv = jm;
+      const float4 fb = __ldg(fbox + t);
+      if (jm > 0 && fb.x <= fb.z) {
+        // sub-columns whose origins can lie in the box
+        p0 = max(__float2int_ru((fb.x - ox0) * g.inv_g2[0] - mx), 0);
+        p1 = min(__float2int_rd((fb.z - ox0) * g.inv_g2[0] + mx), n2x - 1);
+        const int q0 = max(__float2int_ru((fb.y - oy0) * g.inv_g2[1] - my), 0);
+        const int q1 = min(__float2int_rd((fb.w - oy0) * g.inv_g2[1] + my), n2y - 1);
+        if (p0 <= p1 && q0 <= q1) {
+          const int np = p1 - p0 + 1, nq = q1 - q0 + 1;
+          const float4 a0 = __ldg(ptri + 3 * (size_t)t), a1 = __ldg(ptri + 3 * (size_t)t + 1),
+                       a2 = __ldg(ptri + 3 * (size_t)t + 2);
+          const float o0 = __ldg(ox + p0), o1 = __ldg(oy + q0);
+          ux = a0.x - o0, uy = a0.y - o1, vx = a1.x - o0, vy = a1.y - o1, wx = a2.x - o0, wy = a2.y - o1;
+          // Tx = ox - v1x and so on, over the triangle's sub-columns: at most atx, aty
+          const float atx = fmaxf(fabsf(ux), fmaxf(fabsf(vx), fabsf(wx))) + (float)(np - 1) * gx;
+          const float aty = fmaxf(fabsf(uy), fmaxf(fabsf(vy), fabsf(wy))) + (float)(nq - 1) * gy;
+          const float R = 1.0001f * fmaxf(fmaxf(atx, fmaxf(ux, fmaxf(vx, wx)) - fminf(ux, fminf(vx, wx))),
+                                          fmaxf(aty, fmaxf(uy, fmaxf(vy, wy)) - fminf(uy, fminf(vy, wy))));
+          // In units of eps R^2 the float u, v and u + v (times det) are off by less than 48 and
+          // solve_rows' sides by less than 42: 90, 96 with the slope's.  An unbounded box marks an
+          // ill-conditioned x/y projection, which has no bound on t: exact tests only.
+          direct = !g.oz_monotone || isinf(fb.x) || isinf(fb.z) || !(R > 1e-9f && R < 1e9f);
+          nrow = (uint32_t)nq;
+          if (!direct) {
+            nsolve = (uint32_t)nq;
+            // The plane's height over an origin is affine in (p, q): X = its height above the
+            // chunk's first origin, less 1e-6, in Level2 cells; the origins r < X are hit.  The
+            // float t of an origin differs from the exact t* by at most 8.2 eps M1 / |det| with
+            // M1 growing by at most 0.26 of |t*| away from the crossing (the box is bounded:
+            // rel <= 1/8), so it decides as t* does outside 1.35 (8.2 eps M0 / |det| + 1e-6)
+            // of the crossing, M0 being M1 at the triangle's own heights; X itself is off by
+            // less than 20 eps M0 / |det| and the roundings of the index arithmetic.
+            const float e1x = vx - ux, e1y = vy - uy, e1z = a1.z - a0.z, e2x = wx - ux, e2y = wy - uy, e2z = a2.z - a0.z;
+            const float Nx = e1y * e2z - e1z * e2y, Ny = e1z * e2x - e1x * e2z, Nz = e1x * e2y - e1y * e2x;
+            const float rn = rcp_fast(Nz), igz = g.inv_g2[2];
+            const float zt2 = 2.f * fmaxf(fabsf(e1z), fmaxf(fabsf(e2z), fabsf(e2z - e1z)));
+            const float M0 = fabsf(e2x) * (aty * fabsf(e1z) + zt2 * fabsf(e1y)) +
+                             fabsf(e2y) * (zt2 * fabsf(e1x) + atx * fabsf(e1z)) +
+                             fabsf(e2z) * (atx * fabsf(e1y) + aty * fabsf(e1x));
+            const float Kx = -(Nx * rn) * igz, Ky = -(Ny * rn) * igz;  // per unit of x, y
+            const float w = igz * (EPS24 * (40.f * M0 * fabsf(rn) + 8.f * zt2) + toz + 0.35f * g.thr) +
+                            fabsf(Kx) * tox + fabsf(Ky) * toy + 8.f * EPS24 * (float)span + kIdx;
+            dl = 104.f * EPS24 * R * R;
+            ws.x[lane][1] = ((a0.z - ozb) - g.thr) * igz - Kx * ux - Ky * uy;
+            ws.x[lane][2] = Kx * gx;
+            ws.x[lane][3] = Ky * gy;
+            ws.x[lane][4] = w;
+          }
+          ws.rng[lane][0] = (uint32_t)(p0 | ((p1 + 1) << 8));
+          ws.rng[lane][1] = (uint32_t)q0;
+          ws.tri[lane] = t;
+          ws.jm[lane] = jm | (direct ? 256 : 0);
+        }
+      }
+    }
+    const uint32_t is = warp_incl_scan(nsolve), ir = warp_incl_scan(nrow);
+    taken = (uint32_t)__popc(__ballot_sync(FULL, is <= (uint32_t)kSol && ir <= (uint32_t)kRows));
+    if (lane < taken) nun += (uint64_t)jmv;
+    if (lane == 0) ws.row[0] = 0;
+    ws.row[lane + 1] = ir;
+    if (lane < taken && nrow) {
+      ws.pre[lane] = is - nsolve;
+      uint8_t *own = ws.own + (ir - nrow);
+#pragma unroll 1
+      for (uint32_t k = 0; k < nrow; ++k) own[k] = (uint8_t)lane;
+      if (nsolve)
+        solve_rows(ws.sol + (is - nsolve), (int)nrow, ux, vx, wx, uy, vy, wy, 0.f, 0.f, gx, gy, dl, 1.1f * tox,
+                   1.1f * toy, p0, (uint32_t)p0, (uint32_t)(n2x | ((p1 + 1) << 16)), 0, 64);
+    }
+    __syncwarp();
+    {
+      const uint32_t R1 = ws.row[taken];
+#pragma unroll 1
+      for (uint32_t rb0 = 0; rb0 < R1; rb0 += 32) {
+        const uint32_t rw = rb0 + lane;
+        int p = 0, pend = 0, pi = 0, pe = 0, q = 0, jm = 0;
+        uint32_t tri = 0;
+        float X = 0.f, Kx = 0.f, wx_ = 0.f;
+        if (rw < R1) {
+          const int tl = ws.own[rw];
+          const int dq = (int)(rw - ws.row[tl]);
+          const uint32_t rx = ws.rng[tl][0];
+          jm = ws.jm[tl];
+          tri = ws.tri[tl];
+          q = (int)ws.rng[tl][1] + dq;
+          if (jm & 256) {  // nothing certain
+            jm &= 255;
+            p = (int)(rx & 255u);
+            pend = (int)(rx >> 8);
+          } else {
+            const uint32_t sxy = ws.sol[ws.pre[tl] + dq];
+            p = (int)(sxy & 255u);
+            pi = (int)((sxy >> 8) & 255u);
+            pe = (int)((sxy >> 16) & 255u);
+            pend = (int)(sxy >> 24);
+            Kx = ws.x[tl][2];
+            X = ff((float)(p - (int)(rx & 255u)), Kx, ff((float)dq, ws.x[tl][3], ws.x[tl][1]));
+            wx_ = ws.x[tl][4];
+          }
+        }
+        float dp = 0.f;
+#pragma unroll 1
+        while (__any_sync(FULL, p < pend)) {
+          bool amb = false;
+          if (p < pend) {
+            const float x = ff(dp, Kx, X);
+            const int N = min(max(__float2int_ru(x - wx_), 0), span);
+            amb = p < pi || p >= pe || N != min(max(__float2int_ru(x + wx_), 0), span);
+            if (!amb && N > 0) {
+              const int pq = q * n2x + p;
+              const int kq = __float2int_rz(((float)N + 0.5f) * inv_n2z), rem = N - kq * n2z;
+              int below;  // voxels of the chunk under layer kz0 + kq
+              bool here;  // ... and whether that layer belongs to it
+              if (kq < 32) {
+                below = __popc(layers & ((1u << kq) - 1u));
+                here = (layers >> kq) & 1u;
+              } else if (near) {
+                below = m;
+                here = false;
+              } else {
+                below = 0;
+#pragma unroll 1
+                while (below < m && kz[below] < kz0 + kq) ++below;
+                here = below < m && kz[below] == kz0 + kq;
+              }
+              const int nf = min(below, jm);
+              if (nf > 0) atomicXor(&ft[(nf - 1) * FW + (pq >> 5)], 1u << (pq & 31));
+              if (here && rem > 0 && below < jm) xor_column(par + below * W, pq, n2z, (1u << rem) - 1u);
+            }
+          }
+          nrec = queue_push(ws, nrec, amb, tri, (uint32_t)(jm | (p << 6) | (q << 11)));
+          if (nrec >= 32) {
+            fill_exact(d, ws, par, ft, kz, m, ci, cj, 32);
+            nrec = queue_shift(ws, nrec);
+          }
+          ++p;
+          dp += 1.f;
+        }
+      }
+      __syncwarp();
+    }
   }
+  if (nrec) fill_exact(d, ws, par, ft, kz, m, ci, cj, nrec);
+  __syncwarp();
 
   }
 
   // ---------------- output, top voxel first so the full-hit toggles accumulate downwards.
   // One lane per sub-column: its n2z SAT and parity bits are read once and written as n2z
   // bytes at stride n2x*n2y (consecutive lanes write consecutive bytes of each z layer).
+#pragma unroll 1
   for (int w = lane; w < FW; w += 32) ftacc[w] = 0;
   __syncwarp();
   unsigned long long nin = 0, nbd = 0;
   const uint32_t zmask_all = n2z >= 32 ? 0xffffffffu : ((1u << n2z) - 1u);
   // 16-byte stores where the layout allows them (also the fast pattern into pinned host memory);
-  // measured faster with the queued organisation (torus262k: -6%) and slower with the per-lane
-  // one on the mixed batch (+3%), so only the former uses them
   // packed codes for the host: the voxels of this launch's slab below BatchDev::pk_end (the host
   // enables it only where the 16-byte layout below applies)
   const uint32_t pkend = d.l2codes ? bd.pk_end[slab] : 0u;
-  const bool vec = (QUEUE || pkend) && (n2z == 8 || n2z == 16) && (ncol2 & 15) == 0 &&
+  const bool vec = (n2z == 8 || n2z == 16) && (ncol2 & 15) == 0 &&
                    (reinterpret_cast<uintptr_t>(d.l2) & 15) == 0;
+#pragma unroll 1
   for (int jv = m - 1; jv >= 0; --jv) {
+#pragma unroll 1
     for (int w = lane; w < FW; w += 32) ftacc[w] ^= ft[jv * FW + w];
     __syncwarp();
     const int64_t vlin = ((int64_t)kz[jv] * ny + cj) * nx + ci;
     uint8_t *out = d.l2 + (size_t)d.prefix[vlin] * cells;
     const uint32_t vidx = (uint32_t)d.prefix[vlin];
     uint32_t *codes = vidx < pkend ? d.l2codes + (size_t)vidx * (cells >> 4) : nullptr;
-    const uint32_t *satj = sat + jv * W, *parj = par + jv * W;
+    const uint32_t *satj = satm + jv * W, *parj = par + jv * W;
     if (vec) {
       if (n2z == 8) write_block_vec<8>(out, codes, satj, parj, ftacc, ncol2, lane, nbd, nin);
       else write_block_vec<16>(out, codes, satj, parj, ftacc, ncol2, lane, nbd, nin);
       __syncwarp();
       continue;
     }
+#pragma unroll 1
     for (int pq = lane; pq < ncol2; pq += 32) {
       const int off = pq * n2z, sh = off & 31;
       uint32_t sb = satj[off >> 5] >> sh, pb = parj[off >> 5] >> sh;
@@ -1185,6 +1363,7 @@ __global__ void __launch_bounds__(kWarps * 32, QUEUE ? (FQ ? 5 : 6) : 7) k_level
       nbd += (unsigned)__popc(sb);
       nin += (unsigned)__popc(ib);
       uint8_t *o = out + pq;
+#pragma unroll 1
       for (int r = 0; r < n2z; ++r)
         __stcs(reinterpret_cast<char *>(o + (size_t)r * ncol2),
                (char)(((sb >> r) & 1u) ? 254 : (((ib >> r) & 1u) ? 127 : 0)));
@@ -1211,46 +1390,32 @@ int level2_chunk(const GridDev &g, int cap) {
   return std::max(1, std::min(std::min(32, std::max(cap, 1)), kMaskWords / W));
 }
 
-// Shared-memory words one warp needs for a mesh with this grid.
-int level2_warp_words(const GridDev &g, int cap, bool stencil) {
+// Shared-memory words one warp of the two Level2 kernels needs for a mesh with this grid.
+Level2Words level2_warp_words(const GridDev &g, int cap, bool stencil) {
   const int cells = g.n2[0] * g.n2[1] * g.n2[2];
   const int W = (cells + 31) >> 5;
   const int FW = (g.n2[0] * g.n2[1] + 31) >> 5;
   const int CH = level2_chunk(g, cap);
   const int FWS = (4 * g.n2[0] * g.n2[1] + 31) >> 5;
-  return 2 * CH * W + CH * FW + CH + FW + (int)(sizeof(WarpScratch) / 4) +
-         (stencil ? 4 * CH * W + CH * FWS + FWS : 0);
-}
-
-// Measured on one GB300: the queued records win (3-10%) where the triangles span several Level2
-// cells in x and y (xycells / pairs >= 4: torus262k at 8^3, a 16k sphere at 4^3); the per-lane
-// slab work wins (10-16%) where they span about one (the same torus at 2^3 and 4^3), and on
-// mixed batches.
-bool level2_queue_pays(const MeshStats *stats, const bool *has_l2, int n) {
-  double dense = 0.0, all = 0.0;
-  for (int m = 0; m < n; ++m) {
-    if (!has_l2[m]) continue;
-    const double p = (double)stats[m].pairs;
-    all += p;
-    if ((double)stats[m].xycells >= 64.0 * p) dense += p;  // xycells carries a factor 16
-  }
-  // mixed launches do better with the per-lane organisation (the 4096-mesh mix: +3%)
-  return dense > 0.9 * all;
+  const int base = (int)(sizeof(WarpScratch) / 4) + 32;
+  return {base + CH * W, base + CH * W + CH * FW + FW + (stencil ? 4 * CH * W + CH * FWS + FWS : 0)};
 }
 
 size_t level2_smem_bytes(int warp_words) { return (size_t)warp_words * 4 * kWarps; }
 
-int64_t level2_temp_words(int64_t B) { return 7 * B + 8 + 2 * (kSlabsMax + 4) + scan_temp_words(B); }
+int64_t level2_temp_words(int64_t B) { return 10 * B + 16 + 2 * (kSlabsMax + 4) + scan_temp_words(B); }
 
 // Builds the chunk items from the sorted pair lists and runs the persistent Level2 kernel.
 void launch_level2(const BatchDev &bd, const uint32_t *keys, const uint32_t *vals,
-                   const uint32_t *useg, int64_t B, uint32_t *tmp, int warp_words, int num_sms,
+                   const uint32_t *useg, int64_t B, uint32_t *tmp, Level2Words words, int num_sms,
                    cudaStream_t s, const std::function<void()> &before_kernel, int zslab,
                    int nslab, const std::function<void(int, cudaStream_t)> &after_slab, int slab_nz,
-                   const SlabStreams *aux, bool queue, bool fillq) {
+                   const SlabStreams *aux) {
   if (B <= 0) return;
-  uint32_t *cflag = tmp, *cord = cflag + B, *colhead = cord + B, *iflag = colhead + B + 1,
-           *iord = iflag + B, *istart = iord + B, *nitems = istart + B + 1,
+  // (tmp is 256-byte aligned: the items come first)
+  Item *items = reinterpret_cast<Item *>(tmp);
+  uint32_t *cflag = tmp + 4 * B, *cord = cflag + B, *colhead = cord + B, *iflag = colhead + B + 1,
+           *iord = iflag + B, *nitems = iord + B,
            *slabcnt = nitems + 4, *ioff = slabcnt + (kSlabsMax + 4), *ilist = ioff + (kSlabsMax + 4),
            *stmp = ilist + B;
   if (nslab <= 1) zslab = 0;
@@ -1261,48 +1426,40 @@ void launch_level2(const BatchDev &bd, const uint32_t *keys, const uint32_t *val
   k_colheads<<<nb, 256, 0, s>>>(bd, cflag, cord, B, colhead);
   k_itemflags<<<nb, 256, 0, s>>>(bd, keys, useg, cflag, cord, colhead, B, zslab, iflag);
   scan_u32(iflag, iord, B, nullptr, stmp, s);
-  k_itemstarts<<<nb, 256, 0, s>>>(bd, iflag, iord, B, istart, nitems);
+  k_itemstarts<<<nb, 256, 0, s>>>(bd, keys, useg, cflag, cord, colhead, iflag, iord, B, items, nitems);
   count_launch(4);
   if (bd.fill == GPV_FILL_STENCIL && bd.stp) {
     const unsigned nbp = (unsigned)((B + kPrefixWarps - 1) / kPrefixWarps);  // items, columns <= B
     k_stencil_segment<<<nbp, kPrefixWarps * 32, 0, s>>>(bd, keys, vals, useg, cflag, cord, colhead,
-                                                         istart, nitems, B);
+                                                         items, nitems, B);
     k_stencil_scan<<<nbp, kPrefixWarps * 32, 0, s>>>(bd, cflag, cord, colhead, iflag, B);
     count_launch(2);
   }
-  const size_t smem = level2_smem_bytes(warp_words);
   const bool st = bd.fill == GPV_FILL_STENCIL;
-  using Kern = decltype(&k_level2c<false, false, false>);
-  static bool attr_set[6] = {false, false, false, false, false, false};
-  // the kernel of one SAT organisation, and its persistent grid
-  auto pick = [&](bool q, int64_t &grid) {
-    Kern k = st ? (q ? k_level2c<true, true, false> : k_level2c<true, false, false>)
-           : fillq ? (q ? k_level2c<false, true, true> : k_level2c<false, false, true>)
-                   : (q ? k_level2c<false, true, false> : k_level2c<false, false, false>);
-    const int kv = (st ? 4 : fillq ? 2 : 0) + (q ? 1 : 0);
+  using Kern = decltype(&k_level2c_sat);
+  static bool attr_set[3] = {false, false, false};
+  // a kernel's persistent grid (one-graph calls: B is a capacity, the queue ends the work)
+  auto grid_of = [&](Kern k, int kv, size_t smem) {
     if (!attr_set[kv]) {
       cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
       attr_set[kv] = true;
     }
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kWarps * 32, smem);
-    per_sm = std::max(per_sm, 1);
-    // (one-graph calls: B is a capacity, the queue ends the work)
-    grid = bd.plan ? (int64_t)num_sms * per_sm
-                   : std::min<int64_t>((B + kWarps - 1) / kWarps, (int64_t)num_sms * per_sm);
-    return k;
+    const int64_t full = (int64_t)num_sms * std::max(per_sm, 1);
+    return (unsigned)(bd.plan ? full : std::min<int64_t>((B + kWarps - 1) / kWarps, full));
   };
-  int64_t grid = 0, grid2 = 0;
-  const Kern kern = pick(queue, grid);
-  // one-graph calls: the other organisation too; the device plan leaves one of them empty
-  const Kern kern2 = bd.plan ? pick(!queue, grid2) : nullptr;
+  const Kern fill = st ? k_level2c_fill<true> : k_level2c_fill<false>;
+  const size_t smem_sat = level2_smem_bytes(words.sat), smem_fill = level2_smem_bytes(words.fill);
+  const unsigned grid_sat = grid_of(k_level2c_sat, 0, smem_sat);
+  const unsigned grid_fill = grid_of(fill, st ? 2 : 1, smem_fill);
   const int nz = slab_nz;
   if (zslab > 0) {
     // single mesh: order the items by slab so that each launch takes only its own
     cudaMemsetAsync(slabcnt, 0, (kSlabsMax + 4) * sizeof(uint32_t), s);
-    k_item_slab_count<<<nb, 256, 0, s>>>(istart, nitems, keys, useg, nz, zslab, slabcnt);
+    k_item_slab_count<<<nb, 256, 0, s>>>(items, nitems, keys, useg, nz, zslab, slabcnt);
     k_item_slab_offsets<<<1, 32, 0, s>>>(slabcnt, nslab, ioff);
-    k_item_slab_place<<<nb, 256, 0, s>>>(istart, nitems, keys, useg, nz, zslab, slabcnt, ilist);
+    k_item_slab_place<<<nb, 256, 0, s>>>(items, nitems, keys, useg, nz, zslab, slabcnt, ilist);
     count_launch(3);
   }
   if (before_kernel) before_kernel();
@@ -1310,7 +1467,7 @@ void launch_level2(const BatchDev &bd, const uint32_t *keys, const uint32_t *val
   // streams (when given) so that one slab's tail overlaps the next slab's start
   const int launches = zslab > 0 ? nslab : 1;
   const bool two = zslab > 0 && launches > 1 && aux;
-  cudaMemsetAsync(bd.queue + 1, 0, (size_t)launches * sizeof(uint32_t), s);
+  cudaMemsetAsync(bd.queue + 1, 0, (size_t)(2 * kSlabsMax) * sizeof(uint32_t), s);
   if (two) {
     cudaEventRecord(aux->fork, s);
     cudaStreamWaitEvent(aux->st[0], aux->fork, 0);
@@ -1318,16 +1475,12 @@ void launch_level2(const BatchDev &bd, const uint32_t *keys, const uint32_t *val
   }
   for (int sl = 0; sl < launches; ++sl) {
     cudaStream_t ls = two ? aux->st[sl & 1] : s;
-    kern<<<(unsigned)grid, kWarps * 32, smem, ls>>>(bd, keys, vals, useg, cflag, cord, colhead, istart,
-                                                    nitems, warp_words, sl, zslab,
-                                                    zslab > 0 ? ilist : nullptr, ioff);
-    count_launch();
-    if (kern2) {
-      kern2<<<(unsigned)grid2, kWarps * 32, smem, ls>>>(bd, keys, vals, useg, cflag, cord, colhead,
-                                                        istart, nitems, warp_words, sl, zslab,
-                                                        zslab > 0 ? ilist : nullptr, ioff);
-      count_launch();
-    }
+    const uint32_t *list = zslab > 0 ? ilist : nullptr;
+    k_level2c_sat<<<grid_sat, kWarps * 32, smem_sat, ls>>>(bd, keys, vals, useg, items, nitems, words.sat,
+                                                          sl, list, ioff);
+    fill<<<grid_fill, kWarps * 32, smem_fill, ls>>>(bd, keys, vals, useg, items, nitems, words.fill, sl,
+                                                    list, ioff);
+    count_launch(2);
     if (after_slab) after_slab(sl, ls);
   }
   if (two) {

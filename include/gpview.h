@@ -123,10 +123,8 @@ const char *gpv_last_error(gpv_ctx *ctx);
  * of boundary voxels of one Level1 column that one Level2 work item takes (1..32, default 16). */
 int gpv_set_tile(gpv_ctx *ctx, int tris_per_tile);
 int gpv_set_level2_chunk(gpv_ctx *ctx, int max_voxels);
-/* Organisation of the Level2 kernel's SAT stage (results are identical; only speed differs):
- * GPV_LEVEL2_AUTO (default) picks per launch from the item density the prep kernel measures;
- * GPV_LEVEL2_QUEUED queues the (triangle, sub-column) items that pass the z-invariant axes and
- * finishes them 32 at a time; GPV_LEVEL2_INLINE lets each item's lane finish its own item. */
+/* Organisation of the Level2 SAT.  One organisation serves every density (rows of cells solved per
+ * triangle), so the setting has no effect; it is accepted for callers that make it. */
 #define GPV_LEVEL2_AUTO 0
 #define GPV_LEVEL2_QUEUED 1
 #define GPV_LEVEL2_INLINE 2
