@@ -188,7 +188,8 @@ __device__ __forceinline__ int batch_search(const uint32_t *pre, uint32_t it) {
   return lo;
 }
 
-constexpr int kSol = 640;    // solved rows of one batch (a triangle has at most 96)
+constexpr int kSol = 640;    // solved rows of one batch (a triangle has at most 96); the output stage
+                             // keeps 16 layers of 32 lanes there
 constexpr int kRows = kSol / 2 + 32 * kDirectCells;  // its rows of sub-columns, at most
 
 struct WarpScratch {
@@ -203,6 +204,8 @@ struct WarpScratch {
   uint32_t sol[kSol];  // solved rows
   uint32_t rtri[64];   // queued exact work: triangle id and
   uint32_t rpos[64];   // voxel (or voxel count), sub-column and cell range
+  uint32_t utri[64];   // fill: queued triangles and the voxels of the chunk that see them
+  uint8_t ujm[64];
   uint8_t own[kRows];  // triangle slot of each row of sub-columns
 };
 static_assert(sizeof(WarpScratch) % 4 == 0, "word layout");
@@ -354,53 +357,127 @@ __global__ void k_item_slab_place(const Item *__restrict__ items,
 // 4 bits -> 4 bytes holding 0 or 1 (bit j to byte j; the shifted copies land on distinct bits).
 __device__ __forceinline__ uint32_t byte_flags4(uint32_t x) { return (x * 0x00204081u) & 0x01010101u; }
 
-// Output bytes of one boundary voxel when n2z is 8 or 16 and a z layer holds a multiple of 16
-// sub-columns: each lane builds 16 consecutive bytes (16 sub-columns of one layer) from the mask
-// words, where layer r of a sub-column is bit r of its n2z-bit field, and writes them with one
-// 16-byte store (a warp covers 512 contiguous bytes per instruction).  With `codes`, the same 16
-// cells go out as one word of 2-bit codes (cell k of the 16 at bits 2k: 0 outside, 1 inside,
-// 2 boundary) for the host to expand, a quarter of the bytes over the CPU-GPU link.
-template <int NZ>
-__device__ __forceinline__ void write_block_vec(uint8_t *out, uint32_t *codes,
-                                                const uint32_t *satj, const uint32_t *parj,
-                                                const uint32_t *ftacc, int ncol2, unsigned lane,
-                                                unsigned long long &nbd, unsigned long long &nin) {
-  const int chunks = NZ * ncol2 / 16;
-#pragma unroll 1
-  for (int c = (int)lane; c < chunks; c += 32) {
-    const int byte0 = c * 16;
-    const int r = byte0 / ncol2, pq0 = byte0 - r * ncol2;
-    const uint32_t f16 = (ftacc[pq0 >> 5] >> (pq0 & 31)) & 0xffffu;
-    uint32_t o[4], code = 0;
+// 16 cells' mask bits -> their output bytes, 254 boundary, 127 inside, 0 outside.
+__device__ __forceinline__ uint4 state_bytes(uint32_t sat, uint32_t in) {
+  uint32_t o[4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {  // sub-columns pq0 + 4k .. pq0 + 4k + 3
-      uint32_t sf, pf;
-      if (NZ == 8) {  // four sub-columns per word
-        const int w = (pq0 >> 2) + k;
-        sf = (satj[w] >> r) & 0x01010101u;
-        pf = (parj[w] >> r) & 0x01010101u;
-      } else {  // two sub-columns per word: layer bits at 0 and 16 of each
-        const int w = (pq0 >> 1) + 2 * k;
-        const uint32_t a = satj[w] >> r, b = satj[w + 1] >> r;
-        sf = (a & 1u) | ((a >> 8) & 0x100u) | ((b & 1u) << 16) | ((b << 8) & 0x1000000u);
-        const uint32_t c2 = parj[w] >> r, d2 = parj[w + 1] >> r;
-        pf = (c2 & 1u) | ((c2 >> 8) & 0x100u) | ((d2 & 1u) << 16) | ((d2 << 8) & 0x1000000u);
+  for (int k = 0; k < 4; ++k)
+    o[k] = byte_flags4((sat >> (4 * k)) & 0xfu) * 254u + byte_flags4((in >> (4 * k)) & 0xfu) * 127u;
+  return make_uint4(o[0], o[1], o[2], o[3]);
+}
+// 16 bits to the even bits of a word.
+__device__ __forceinline__ uint32_t spread16(uint32_t x) {
+  x = (x | (x << 8)) & 0x00ff00ffu;
+  x = (x | (x << 4)) & 0x0f0f0f0fu;
+  x = (x | (x << 2)) & 0x33333333u;
+  return (x | (x << 1)) & 0x55555555u;
+}
+
+// Transposes 16 sub-columns of a mask (NZ layers each, NZ / 2 words) in place: afterwards half r & 1
+// of word r >> 1 holds layer r, bit c for sub-column c.  The usual block swaps: halves, quarters, ...
+template <int NZ>
+__device__ __forceinline__ void transpose16(uint32_t (&w)[NZ / 2]) {
+  if constexpr (NZ == 16) {  // 16 x 16 bits, two sub-columns per word
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t t = ((w[i] >> 8) ^ w[i + 4]) & 0x00ff00ffu;
+      w[i + 4] ^= t;
+      w[i] ^= t << 8;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int i = (k & 1) + 4 * (k >> 1);
+      const uint32_t t = ((w[i] >> 4) ^ w[i + 2]) & 0x0f0f0f0fu;
+      w[i + 2] ^= t;
+      w[i] ^= t << 4;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; i += 2) {
+      const uint32_t t = ((w[i] >> 2) ^ w[i + 1]) & 0x33333333u;
+      w[i + 1] ^= t;
+      w[i] ^= t << 2;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const uint32_t t = ((w[i] >> 1) ^ (w[i] >> 16)) & 0x5555u;
+      w[i] ^= (t << 16) | (t << 1);
+    }
+  } else {  // two 8 x 8 blocks of four sub-columns per word
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      uint32_t t = (w[i] ^ (w[i] >> 7)) & 0x00aa00aau;
+      w[i] ^= t ^ (t << 7);
+      t = (w[i] ^ (w[i] >> 14)) & 0x0000ccccu;
+      w[i] ^= t ^ (t << 14);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i += 2) {
+      const uint32_t t = ((w[i] >> 4) ^ w[i + 1]) & 0x0f0f0f0fu;
+      w[i + 1] ^= t;
+      w[i] ^= t << 4;
+    }
+    // bytes: layers 0-3 of sub-columns 0-7 | layers 4-7 | the same of 8-15 -> halves by layer
+    const uint32_t a = w[0], b = w[1], c = w[2], d = w[3];
+    w[0] = __byte_perm(a, c, 0x5140);
+    w[1] = __byte_perm(a, c, 0x7362);
+    w[2] = __byte_perm(b, d, 0x5140);
+    w[3] = __byte_perm(b, d, 0x7362);
+  }
+}
+
+// Output of a chunk whose n2z is NZ (8 or 16), with a multiple of 16 sub-columns and 16-byte aligned
+// blocks.  A lane takes 16 sub-columns of one voxel: their SAT and parity bits, transposed to layers,
+// are kept in `stage` (a word per layer, conflict-free) and written layer by layer, 16 bytes each.
+// With `codes`, the voxels whose output index is below `pkend` go out as 2-bit codes instead, a word
+// per 16 cells (cell k at bits 2k: 0 outside, 1 inside, 2 boundary), for the host to expand.
+template <int NZ>
+__device__ __forceinline__ void write_chunk(uint8_t *l2, uint32_t *codes, uint32_t pkend, uint32_t vown,
+                                            const uint32_t *satm, const uint32_t *par, const uint32_t *ft,
+                                            int m, int ncol2, uint32_t *stage, unsigned long long &nbd,
+                                            unsigned long long &nin) {
+  const int lane = (int)(threadIdx.x & 31u);
+  const int upv = ncol2 >> 4, W = (ncol2 * NZ) >> 5, FW = (ncol2 + 31) >> 5;
+  uint32_t nb = 0, ni = 0;
+#pragma unroll 1
+  for (int u0 = 0; u0 < m * upv; u0 += 32) {
+    const int u = u0 + lane;
+    const bool live = u < m * upv;
+    const int jv = live ? u / upv : 0, k = u - jv * upv;  // 16 sub-columns from 16 k
+    const uint32_t vidx = __shfl_sync(FULL, vown, jv);
+    if (live) {
+      uint32_t a[NZ / 2], b[NZ / 2];
+      const uint32_t *sw = satm + jv * W + k * (NZ / 2), *pw = par + jv * W + k * (NZ / 2);
+#pragma unroll
+      for (int i = 0; i < NZ / 2; ++i) {
+        a[i] = sw[i];
+        b[i] = pw[i];
+        nb += (uint32_t)__popc(a[i]);
       }
-      pf ^= byte_flags4((f16 >> (4 * k)) & 0xfu);
-      const uint32_t inf = pf & ~sf;
-      nbd += (unsigned)__popc(sf);
-      nin += (unsigned)__popc(inf);
-      o[k] = sf * 254u + inf * 127u;  // flags are 0/1 per byte and disjoint: no carries
-      if (codes) {
-        // bytes holding 0..2 -> four 2-bit fields
-        const uint32_t c4 = sf * 2u + inf;
-        code |= ((c4 & 3u) | ((c4 >> 6) & 0xcu) | ((c4 >> 12) & 0x30u) | ((c4 >> 18) & 0xc0u)) << (8 * k);
+      transpose16<NZ>(a);
+      transpose16<NZ>(b);
+      uint32_t f = (ft[jv * FW + (k >> 1)] >> ((k & 1) * 16)) & 0xffffu;
+      f |= f << 16;
+#pragma unroll
+      for (int i = 0; i < NZ / 2; ++i) {
+        b[i] = (b[i] ^ f) & ~a[i];
+        ni += (uint32_t)__popc(b[i]);
+        stage[(2 * i) * 32 + lane] = __byte_perm(a[i], b[i], 0x5410);
+        stage[(2 * i + 1) * 32 + lane] = __byte_perm(a[i], b[i], 0x7632);
+      }
+      const size_t c0 = (size_t)vidx * (size_t)(NZ * upv) + (size_t)k;  // 16-cell group of layer 0
+      const bool packed = vidx < pkend;
+      // streaming stores: the output is not read again, so it should not displace the working set
+#pragma unroll 1
+      for (int r = 0; r < NZ; ++r) {
+        const uint32_t w = stage[r * 32 + lane], sb = w & 0xffffu, ib = w >> 16;
+        const size_t c = c0 + (size_t)(r * upv);
+        if (packed) __stcs(codes + c, spread16(sb) * 2u | spread16(ib));
+        else __stcs(reinterpret_cast<uint4 *>(l2) + c, state_bytes(sb, ib));
       }
     }
-    // streaming stores: the output is not read again, so it should not displace the working set
-    if (codes) __stcs(codes + c, code);
-    else __stcs(reinterpret_cast<uint4 *>(out + byte0), make_uint4(o[0], o[1], o[2], o[3]));
   }
+  nbd += nb;
+  nin += ni;
 }
 
 // n2z bits of a Level2 column starting at bit `off` of a mask.
@@ -979,10 +1056,10 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_fill(
   const int W = (cells + 31) >> 5;
   const int ncol2 = n2x * n2y;
   const int FW = (ncol2 + 31) >> 5;
-  uint32_t *ft = par + CH * W, *ftacc = ft + CH * FW;
+  uint32_t *ft = par + CH * W;
   // stencil fill: per voxel, (2 n2x * 2 n2y) sample columns of n2z slice toggle bits; per voxel
   // one bit per sample toggling every slice of that voxel and of the voxels above it
-  uint32_t *stg = ftacc + FW;
+  uint32_t *stg = ft + CH * FW;
   const int SWd = 4 * W;
   const int FWS = (4 * ncol2 + 31) >> 5;
   uint32_t *sft = stg + CH * SWd, *sftacc = sft + CH * FWS;
@@ -1144,11 +1221,11 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_fill(
   const float *ozt = g.o2[2];
   const int kz0 = kz[0];
   const float ozb = __ldg(ozt + (size_t)kz0 * n2z), ozl = __ldg(ozt + (size_t)kz[m - 1] * n2z + n2z - 1);
-  const float ox0 = __ldg(ox), oy0 = __ldg(oy);
+  const float ox0 = __ldg(ox), oy0 = __ldg(oy), ox1 = __ldg(ox + n2x - 1), oy1 = __ldg(oy + n2y - 1);
   // distance of the origin tables from their affine form: within a voxel two roundings; over the
   // chunk's heights the voxels' own corners (a float product and sum) too
-  const float tox = 2.02f * EPS24 * fmaxf(fabsf(ox0), fabsf(__ldg(ox + n2x - 1)));
-  const float toy = 2.02f * EPS24 * fmaxf(fabsf(oy0), fabsf(__ldg(oy + n2y - 1)));
+  const float tox = 2.02f * EPS24 * fmaxf(fabsf(ox0), fabsf(ox1));
+  const float toy = 2.02f * EPS24 * fmaxf(fabsf(oy0), fabsf(oy1));
   const float toz = EPS24 * (6.1f * fmaxf(fabsf(ozb), fabsf(ozl)) + 4.1f * fabsf(g.bmin[2]));
   const float mx = ff(tox, g.inv_g2[0], kIdx), my = ff(toy, g.inv_g2[1], kIdx);
   const int span = (kz[m - 1] - kz0 + 1) * n2z;  // ray origins from the chunk's first voxel to its last
@@ -1156,24 +1233,51 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_fill(
   // bit i: layer kz0 + i belongs to the chunk
   const uint32_t layers = __reduce_or_sync(FULL, ((int)lane < m && kz[lane] - kz0 < 32) ? 1u << (kz[lane] - kz0) : 0u);
   const bool near = kz[m - 1] - kz0 < 32;
-  uint32_t taken;  // records of a batch: 32, fewer where their rows would not fit
+  uint32_t nuni = 0;  // queued triangles (utri, ujm)
 #pragma unroll 1
-  for (uint32_t b0 = f0; b0 < f1; b0 += taken) {
-    const uint32_t e = b0 + lane;
-    const uint32_t vv = e < f1 ? vals[e] : 0u;
+  for (uint32_t b0 = f0; b0 < f1; b0 += 32) {
+    // ---- the next entries' triangles whose rays may meet the chunk: about a third of the entries, so
+    // they are queued and taken 32 at a time
+    {
+      const uint32_t e = b0 + lane;
+      const uint32_t vv = e < f1 ? vals[e] : 0u;
+      bool keep = false;
+      int jm = 0;
+      if (vv & 0x80000000u) {
+        const int dz = (int)(keys[e] - col * (uint32_t)nz) - kz0;  // layers above the chunk's first
+        if (dz >= 0) {
+          if (dz < 31) jm = __popc(layers & ((2u << dz) - 1u));
+          else if (near) jm = m;
+          else
+#pragma unroll 1
+            while (jm < m && kz[jm] - kz0 <= dz) ++jm;
+        }
+        nun += (uint64_t)jm;
+        if (jm > 0) {
+          const float4 fb = __ldg(fbox + (vv & 0x7fffffffu));
+          keep = fb.x <= ox1 && fb.z >= ox0 - tox && fb.y <= oy1 && fb.w >= oy0 - toy && fb.x <= fb.z;
+        }
+      }
+      const uint32_t bal = __ballot_sync(FULL, keep);
+      if (keep) {
+        const uint32_t k = nuni + __popc(bal & ((1u << lane) - 1u));
+        ws.utri[k] = vv & 0x7fffffffu;
+        ws.ujm[k] = (uint8_t)jm;
+      }
+      nuni += (uint32_t)__popc(bal);
+      __syncwarp();
+    }
+#pragma unroll 1
+    while (nuni >= 32 || (nuni > 0 && b0 + 32 >= f1)) {
     uint32_t nsolve = 0, nrow = 0;
-    int jmv = 0, p0 = 0, p1 = 0;
+    int p0 = 0, p1 = 0;
     float ux = 0.f, uy = 0.f, vx = 0.f, vy = 0.f, wx = 0.f, wy = 0.f, dl = 0.f;
     bool direct = false;
-    if (vv & 0x80000000u) {
-      const uint32_t t = vv & 0x7fffffffu;
-      const int zt = (int)(keys[e] - col * (uint32_t)nz);
-      int jm = 0;
-#pragma unroll 1
-      while (jm < m && kz[jm] <= zt) ++jm;
-      jmv = jm;
+    if (lane < nuni) {
+      const uint32_t t = ws.utri[lane];
+      const int jm = ws.ujm[lane];
       const float4 fb = __ldg(fbox + t);
-      if (jm > 0 && fb.x <= fb.z) {
+      {
         // sub-columns whose origins can lie in the box
         p0 = max(__float2int_ru((fb.x - ox0) * g.inv_g2[0] - mx), 0);
         p1 = min(__float2int_rd((fb.z - ox0) * g.inv_g2[0] + mx), n2x - 1);
@@ -1228,8 +1332,9 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_fill(
       }
     }
     const uint32_t is = warp_incl_scan(nsolve), ir = warp_incl_scan(nrow);
-    taken = (uint32_t)__popc(__ballot_sync(FULL, is <= (uint32_t)kSol && ir <= (uint32_t)kRows));
-    if (lane < taken) nun += (uint64_t)jmv;
+    // triangles of this batch: 32 (or the queue's last), fewer where their rows would not fit
+    const uint32_t taken = (uint32_t)__popc(
+        __ballot_sync(FULL, lane < nuni && is <= (uint32_t)kSol && ir <= (uint32_t)kRows));
     if (lane == 0) ws.row[0] = 0;
     ws.row[lane + 1] = ir;
     if (lane < taken && nrow) {
@@ -1313,62 +1418,65 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_fill(
       }
       __syncwarp();
     }
+    // the queue's rest to its front
+    {
+      const uint32_t k = lane + taken, k2 = k + 32;
+      const uint32_t t0 = k < nuni ? ws.utri[k] : 0u, t1 = k2 < nuni ? ws.utri[k2] : 0u;
+      const uint8_t j0 = k < nuni ? ws.ujm[k] : 0, j1 = k2 < nuni ? ws.ujm[k2] : 0;
+      __syncwarp();
+      if (k < nuni) { ws.utri[lane] = t0; ws.ujm[lane] = j0; }
+      if (k2 < nuni) { ws.utri[lane + 32] = t1; ws.ujm[lane + 32] = j1; }
+      nuni -= taken;
+      __syncwarp();
+    }
+    }
   }
   if (nrec) fill_exact(d, ws, par, ft, kz, m, ci, cj, nrec);
   __syncwarp();
 
   }
 
-  // ---------------- output, top voxel first so the full-hit toggles accumulate downwards.
-  // One lane per sub-column: its n2z SAT and parity bits are read once and written as n2z
-  // bytes at stride n2x*n2y (consecutive lanes write consecutive bytes of each z layer).
+  // ---------------- output.  The full-hit toggles accumulate downwards first.
 #pragma unroll 1
-  for (int w = lane; w < FW; w += 32) ftacc[w] = 0;
+  for (int w = lane; w < FW; w += 32)
+#pragma unroll 1
+    for (int jv = m - 2; jv >= 0; --jv) ft[jv * FW + w] ^= ft[(jv + 1) * FW + w];
   __syncwarp();
   unsigned long long nin = 0, nbd = 0;
   const uint32_t zmask_all = n2z >= 32 ? 0xffffffffu : ((1u << n2z) - 1u);
-  // 16-byte stores where the layout allows them (also the fast pattern into pinned host memory);
   // packed codes for the host: the voxels of this launch's slab below BatchDev::pk_end (the host
   // enables it only where the 16-byte layout below applies)
   const uint32_t pkend = d.l2codes ? bd.pk_end[slab] : 0u;
-  const bool vec = (n2z == 8 || n2z == 16) && (ncol2 & 15) == 0 &&
-                   (reinterpret_cast<uintptr_t>(d.l2) & 15) == 0;
-#pragma unroll 1
-  for (int jv = m - 1; jv >= 0; --jv) {
-#pragma unroll 1
-    for (int w = lane; w < FW; w += 32) ftacc[w] ^= ft[jv * FW + w];
+  const uint32_t vown = (int)lane < m ? (uint32_t)d.prefix[((int64_t)kz[lane] * ny + cj) * nx + ci] : 0u;
+  if ((n2z == 8 || n2z == 16) && (ncol2 & 15) == 0 && (reinterpret_cast<uintptr_t>(d.l2) & 15) == 0) {
+    if (n2z == 8) write_chunk<8>(d.l2, d.l2codes, pkend, vown, satm, par, ft, m, ncol2, ws.sol, nbd, nin);
+    else write_chunk<16>(d.l2, d.l2codes, pkend, vown, satm, par, ft, m, ncol2, ws.sol, nbd, nin);
     __syncwarp();
-    const int64_t vlin = ((int64_t)kz[jv] * ny + cj) * nx + ci;
-    uint8_t *out = d.l2 + (size_t)d.prefix[vlin] * cells;
-    const uint32_t vidx = (uint32_t)d.prefix[vlin];
-    uint32_t *codes = vidx < pkend ? d.l2codes + (size_t)vidx * (cells >> 4) : nullptr;
-    const uint32_t *satj = satm + jv * W, *parj = par + jv * W;
-    if (vec) {
-      if (n2z == 8) write_block_vec<8>(out, codes, satj, parj, ftacc, ncol2, lane, nbd, nin);
-      else write_block_vec<16>(out, codes, satj, parj, ftacc, ncol2, lane, nbd, nin);
-      __syncwarp();
-      continue;
-    }
+  } else {
+    // One lane per sub-column of the chunk: its n2z SAT and parity bits are read once and written
+    // as n2z bytes at stride n2x*n2y (consecutive lanes write consecutive bytes of each z layer).
+    uint32_t nb = 0, ni = 0;
 #pragma unroll 1
-    for (int pq = lane; pq < ncol2; pq += 32) {
-      const int off = pq * n2z, sh = off & 31;
-      uint32_t sb = satj[off >> 5] >> sh, pb = parj[off >> 5] >> sh;
-      if (sh + n2z > 32) {
-        sb |= satj[(off >> 5) + 1] << (32 - sh);
-        pb |= parj[(off >> 5) + 1] << (32 - sh);
+    for (int i0 = 0; i0 < m * ncol2; i0 += 32) {
+      const int i = i0 + (int)lane;
+      const bool live = i < m * ncol2;
+      const int jv = live ? i / ncol2 : 0, pq = i - jv * ncol2;
+      const uint32_t vidx = __shfl_sync(FULL, vown, jv);
+      if (live) {
+        const uint32_t sb = column_bits(satm + jv * W, pq * n2z, n2z) & zmask_all;
+        uint32_t pb = column_bits(par + jv * W, pq * n2z, n2z);
+        if ((ft[jv * FW + (pq >> 5)] >> (pq & 31)) & 1u) pb = ~pb;
+        const uint32_t ib = pb & ~sb & zmask_all;
+        nb += (unsigned)__popc(sb);
+        ni += (unsigned)__popc(ib);
+        uint8_t *o = d.l2 + (size_t)vidx * cells + pq;
+#pragma unroll 1
+        for (int r = 0; r < n2z; ++r)
+          __stcs(reinterpret_cast<char *>(o + (size_t)r * ncol2), (char)(((sb >> r) & 1u) * 254u + ((ib >> r) & 1u) * 127u));
       }
-      sb &= zmask_all;
-      if ((ftacc[pq >> 5] >> (pq & 31)) & 1u) pb = ~pb;
-      const uint32_t ib = pb & ~sb & zmask_all;
-      nbd += (unsigned)__popc(sb);
-      nin += (unsigned)__popc(ib);
-      uint8_t *o = out + pq;
-#pragma unroll 1
-      for (int r = 0; r < n2z; ++r)
-        __stcs(reinterpret_cast<char *>(o + (size_t)r * ncol2),
-               (char)(((sb >> r) & 1u) ? 254 : (((ib >> r) & 1u) ? 127 : 0)));
     }
-    __syncwarp();
+    nbd += nb;
+    nin += ni;
   }
   nin = warp_sum(nin);
   nbd = warp_sum(nbd);
@@ -1398,7 +1506,7 @@ Level2Words level2_warp_words(const GridDev &g, int cap, bool stencil) {
   const int CH = level2_chunk(g, cap);
   const int FWS = (4 * g.n2[0] * g.n2[1] + 31) >> 5;
   const int base = (int)(sizeof(WarpScratch) / 4) + 32;
-  return {base + CH * W, base + CH * W + CH * FW + FW + (stencil ? 4 * CH * W + CH * FWS + FWS : 0)};
+  return {base + CH * W, base + CH * W + CH * FW + (stencil ? 4 * CH * W + CH * FWS + FWS : 0)};
 }
 
 size_t level2_smem_bytes(int warp_words) { return (size_t)warp_words * 4 * kWarps; }
