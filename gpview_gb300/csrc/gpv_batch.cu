@@ -222,15 +222,15 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
     if (T[m] > 0 && (reinterpret_cast<uintptr_t>(d_tris[m]) & 15u))
       return ctx_fail(ctx, GPV_ERR_INVALID, "triangle buffers must be 16-byte aligned");
   }
-  // Level1 tile: the caller's (or the autotuner's), else the largest that still gives every SM
-  // three tiles -- larger tiles amortise the per-tile staging and barriers, but a small mesh
-  // needs small ones to occupy the GPU (torus262k: 256; a 16k-triangle sphere: 32)
+  // Level1 triangles per ticket: the caller's (or the autotuner's), else one group of 32, or two
+  // where every warp gets several (Level1 kernel, 32 / 64 / 128 per ticket: 262k triangles at 128^3
+  // 39 / 44 / 48 us, 1.3M at 256^3 118 / 115 / 128, 1M at 512^3 208 / 188 / 187, 9M in 256 meshes
+  // 1.48 / 1.46 / 1.60 ms)
   int tile = ctx->tile;
   if (tile <= 0) {
     int64_t total = 0;
     for (int m = 0; m < n; ++m) total += T[m];
-    tile = 256;
-    while (tile > 32 && total < (int64_t)tile * 3 * ctx->num_sms) tile >>= 1;
+    tile = total >= 4 * 32 * 32 * (int64_t)ctx->num_sms ? 64 : 32;
   }
   const int nmode = ctx->normals;
   const bool stencil = ctx->fill == GPV_FILL_STENCIL;
@@ -307,7 +307,6 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
   CK(ws.get(&stmp, (size_t)scan_temp_words(swords)));
   // the boundary-voxel total: past the boundary plane's words in the prefix when both are scanned
   const uint32_t *btot = kmark ? wpre + words : wtot;
-  CK(ws.get(&queue, 1 + 2 * kMaxSlabs));  // [0] Level1 tickets, then those of each slab's Level2 kernels
   // z slabs of the Level2 launch when the outputs go to the host (one mesh): the boundary ranks
   // at up to kMaxSlabs fine slab starts are read with the first phase's counts; the launch then
   // groups fine slabs into as many slabs as the Level2 output size calls for
@@ -319,7 +318,16 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
     fslab = (gh[0].n[2] + fz - 1) / fz;
     CK(ws.get(&d_slab, kMaxSlabs + 1));
   }
-  CK(ws.get(&stats, (size_t)n));
+  // the statistics, then the queue tickets and the heavy list's length: cleared together
+  const size_t stats_bytes = n * sizeof(MeshStats), acc_bytes = stats_bytes + 4 * (kQueueWords + 1);
+  {
+    unsigned char *acc;
+    CK(ws.get(&acc, acc_bytes));
+    stats = reinterpret_cast<MeshStats *>(acc);
+    queue = reinterpret_cast<uint32_t *>(acc + stats_bytes);
+  }
+  uint4 *heavy;
+  CK(ws.get(&heavy, kHeavyCap));
   CK(ws.get(&d_md, (size_t)n));
   uint32_t *stg = nullptr;  // stencil fill: Level1 sample-column toggles
   if (stencil) CK(ws.get(&stg, (size_t)stgw));
@@ -379,7 +387,11 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
   bd.total_xchunks = xchunks;
   bd.total_words = words;
   bd.queue = queue;
+  bd.heavy = heavy;
+  bd.heavy_n = queue + kQueueWords;
+  bd.heavy_cap = kHeavyCap;
   bd.normals = nmode;
+  bd.emit_all = nmode != 0;
   bd.fill = ctx->fill;
   bd.stp = nullptr;
   bd.stp_words = 0;
@@ -425,7 +437,7 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
     for (uint64_t x : {(uint64_t)(uintptr_t)bd.md, (uint64_t)bd.nmesh, (uint64_t)bd.tile,
                        (uint64_t)bd.total_tris, (uint64_t)bd.total_tiles, (uint64_t)bd.total_fwarps,
                        (uint64_t)bd.total_rows, (uint64_t)bd.total_words, (uint64_t)bd.total_xchunks,
-                       (uint64_t)(uintptr_t)bd.queue, (uint64_t)bd.normals, (uint64_t)bd.fill,
+                       (uint64_t)(uintptr_t)bd.queue, (uint64_t)(uintptr_t)bd.heavy, (uint64_t)bd.normals, (uint64_t)bd.fill,
                        (uint64_t)(uintptr_t)bd.stp, (uint64_t)bd.stp_words,
                        (uint64_t)ctx->timing, (uint64_t)ctx->num_sms, (uint64_t)bd.wait_limit,
                        (uint64_t)bd.fail_wait})
@@ -453,7 +465,7 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
     StageList in(ctx->num_sms, s);
     in.copy(d_tab, ctx->h_tables, tab_off[n] * sizeof(float));
     in.copy(d_md, ctx->h_md, n * sizeof(MeshDesc));
-    in.clear(stats, n * sizeof(MeshStats));
+    in.clear(stats, acc_bytes);
     in.clear(bplane, swords * 4);
     in.clear(toggles, togg * 4);
     if (stg) in.clear(stg, stgw * 4);

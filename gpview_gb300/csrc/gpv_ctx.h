@@ -40,7 +40,7 @@ struct gpv_ctx {
   // synchronisations, 3 second launch to the last synchronisation returning, 4 result assembly
   double host_ms[5] = {};
   std::string err;
-  int tile = 0;                        // Level1 triangles per tile (autotuned; 0: by mesh size)
+  int tile = 0;                        // Level1 triangles per ticket (autotuned; 0: by the call's size)
   // Level2 boundary voxels per chunk, upper bound (autotuned by gpv_autotune; the mask space caps
   // it at 4 for 16^3 sub-grids).  torus262k at 8^3, Level2 kernel ms: 8 -> 0.626, 16 -> 0.596,
   // 32 -> 0.712 (fewer chunks per column repeat the fill's u/v work for the triangles above them)

@@ -106,14 +106,17 @@ constexpr int kFillNone = -1;
 // than 8 for the packed host transfer (star1310k host to host 6.58 against 6.43 ms): each slab
 // launch adds its ramp and tail
 constexpr int kSlabsMax = 8;
+constexpr int kQueueWords = 1 + 2 * kSlabsMax;
+constexpr uint32_t kHeavyCap = 1u << 18;  // pieces of a call's heavy list (4 MiB)
 
 struct BatchDev {
   const MeshDesc *md;
   int nmesh;
-  int tile;              // Level1 triangles per tile (32, 64, 128, 256)
+  int tile;              // Level1 triangles per ticket (32, 64, 128, 256)
   int64_t total_tris, total_tiles, total_fwarps, total_rows, total_words;
   int64_t total_xchunks;  // 128-voxel expansion chunks of all meshes
-  uint32_t *queue;       // work-queue tickets, zeroed before each persistent launch
+  uint32_t *queue;       // work-queue tickets, zeroed by the caller: [0] Level1, [1 + k] and
+                         // [1 + kSlabsMax + k] the fill and the SAT kernel of Level2 slab k
   int normals;           // GPV_NORMALS_* of this batch
   int fill;              // GPV_FILL_* of this batch
   uint32_t *stp;         // stencil fill: per boundary voxel, the sample-coverage parity of the
@@ -121,6 +124,14 @@ struct BatchDev {
   // Level1 marks the voxel of every pair it emits for a mesh with a Level2 grid here: one
   // column-major bit plane per mesh (bit = pair key) at the mesh's word_base; nullptr: no marks
   uint32_t *kmask = nullptr;
+  // Level1 emits the (voxel, triangle) records of every mesh; otherwise only of meshes with a Level2
+  // grid (the others' are only counted)
+  int emit_all = 0;
+  // Level1 pieces of triangles with many units, {mesh, triangle, piece, valid}: written by the prep
+  // kernel, heavy_n of them (zeroed before it), room for heavy_cap; nullptr: none are split
+  uint4 *heavy = nullptr;
+  uint32_t *heavy_n = nullptr;
+  uint32_t heavy_cap = 0;
   // Level1's bounded wait for its staged tile: polls before giving up (0: the built-in limit);
   // fail_wait != 0 gives up at once (GPV_DEBUG_FAIL_WAIT, failure-detection tests)
   uint32_t wait_limit = 0;

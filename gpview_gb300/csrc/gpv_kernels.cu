@@ -4,14 +4,15 @@
 //   k_prep        per triangle: pack vertices as 3 float4, Level1 SAT candidate box (the
 //                 reference's own range, src/Object.cpp:2280-2325), conservative x/y box for the
 //                 ray tests, 1/det of the ray test, work counts.
-//   k_level1      persistent: blocks pull (mesh, triangle tile) items from a device queue; the
-//                 tile is staged in shared memory by bulk async copies (TMA) on an mbarrier.
-//                 (a) SAT units = (triangle, column) running the z run top-down; passes set the
-//                     boundary bit (atomicOr) and emit (column-major voxel key, triangle|topmost).
+//   k_level1      persistent: warps pull tickets of triangles from a device queue; groups of 32 are
+//                 staged in shared memory by bulk async copies (TMA) on the warp's mbarriers.
+//                 (a) SAT units = (triangle, column) running the z run top-down, cut to the
+//                     triangle's plane; passes set the boundary bit (atomicOr) and emit
+//                     (column-major voxel key, triangle|topmost).
 //                 (b) fill units = (triangle, column) running the column part of the +z
-//                     Moller-Trumbore test; passing pairs are queued per warp and the whole warp
-//                     evaluates t over the column (one voxel per lane, __ballot_sync), XOR-ing
-//                     parity toggles d(k) = hit(k) ^ hit(k+1) into a column-major plane.
+//                     Moller-Trumbore test; a passing unit XORs the parity toggles
+//                     d(k) = hit(k) ^ hit(k+1) into a column-major plane, from the triangle's height
+//                     over the column.
 //   k_fill_finish warp-level suffix XOR of the toggles per column -> parity, transposed to
 //                 the linear (x fastest) inside plane.
 //   k_popc + scan per-word boundary counts, boundaryPrefixSum.
@@ -149,6 +150,9 @@ __device__ __forceinline__ float4 ray_box(const float *V, const GridDev &g) {
 }
 
 // ---------------------------------------------------------------------------------------------
+constexpr int kHeavyUnits = 64;   // a triangle with more (triangle, column) units is split ...
+constexpr int kHeavyChunks = 4;   // ... into pieces of this many 32-unit chunks
+
 __global__ void __launch_bounds__(256) k_prep(BatchDev bd) {
   const int64_t gi = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const bool live = gi < bd.total_tris;
@@ -213,8 +217,21 @@ __global__ void __launch_bounds__(256) k_prep(BatchDev bd) {
     d.ptri[3 * t + 0] = make_float4(V[0], V[1], V[2], __uint_as_float(pack2(fx0, fx1)));
     d.ptri[3 * t + 1] = make_float4(V[3], V[4], V[5], __uint_as_float(pack2(fy0, fy1)));
     d.ptri[3 * t + 2] = make_float4(V[6], V[7], V[8], __fdiv_rn(1.0f, det));
+    // A triangle with many units (large against the cells) goes to the heavy list, in pieces of
+    // kHeavyChunks chunks that any warp of the Level1 kernel takes, and is flagged so that its group
+    // leaves it out; where the list is full it stays with its group.
+    int listed = 0;
+    if (bd.heavy && su + fu > (unsigned long long)kHeavyUnits) {
+      const unsigned long long pieces = ((su + 31) / 32 + (fu + 31) / 32 + kHeavyChunks - 1) / kHeavyChunks;
+      if (pieces <= bd.heavy_cap) {
+        const uint32_t pos = atomicAdd(bd.heavy_n, (uint32_t)pieces);
+        listed = pos < bd.heavy_cap && bd.heavy_cap - pos >= (uint32_t)pieces;
+        for (uint32_t k = 0; k < (uint32_t)pieces && pos < bd.heavy_cap && k < bd.heavy_cap - pos; ++k)
+          bd.heavy[pos + k] = make_uint4((uint32_t)m, (uint32_t)t, k, (uint32_t)listed);
+      }
+    }
     d.rng[t] = make_int4((int)pack2(lo[0], hi[0]), (int)pack2(lo[1], hi[1]),
-                         (int)pack2(lo[2], hi[2]), 0);
+                         (int)pack2(lo[2], hi[2]), listed);
     d.fbox[t] = fb;
   }
   block_add_prep(d.stats, sat1, su, fu, r1);
@@ -354,135 +371,288 @@ __global__ void __launch_bounds__(1024) k_plan(int nmesh, MeshDesc *md, int32_t 
 }
 
 // ---------------------------------------------------------------------------------------------
-constexpr int kL1Threads = 256;
-constexpr int kL1Warps = kL1Threads / 32;
+constexpr int kPlaneRun = 4;   // z runs past this many voxels are cut to the triangle's plane first
+constexpr int kL1Warps = 4;
+constexpr int kL1Group = 32;   // triangles of one group (a lane each)
+constexpr int kL1Pairs = 128;  // records a warp collects before it takes room for them
 constexpr uint32_t kWaitLimit = 1u << 22;
 
-// last index lt in [0,nt) with off[lt] <= u (off nondecreasing, off[0] = 0)
-__device__ __forceinline__ int tile_search(const uint32_t *off, int nt, uint32_t u) {
-  int lo = 0, hi = nt - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (off[mid] <= u) lo = mid; else hi = mid - 1;
-  }
+// last index lt in [0, 31] with off[lt] <= u (off nondecreasing, off[0] = 0)
+__device__ __forceinline__ int group_search(const uint32_t *off, uint32_t u) {
+  int lo = 0;
+#pragma unroll
+  for (int st = 16; st > 0; st >>= 1)
+    if (off[lo + st] <= u) lo += st;
   return lo;
 }
 
-template <int TILE>
-__global__ void __launch_bounds__(kL1Threads) k_level1(BatchDev bd) {
-  __shared__ __align__(16) float4 s_tri[TILE * 3];
-  __shared__ __align__(16) int4 s_rng[TILE];
-  __shared__ uint32_t s_soff[TILE + 1];
-  __shared__ uint32_t s_foff[TILE + 1];
-  __shared__ uint32_t s_q[kL1Warps][32];
-  __shared__ uint32_t s_ws[kL1Warps], s_wf[kL1Warps];
-  __shared__ uint32_t s_next;  // next 32-unit chunk of the tile (SAT chunks, then fill chunks)
-  __shared__ __align__(8) uint64_t s_bar;
-  __shared__ int64_t s_item;
+// 1/x to about an ulp (range arithmetic only, never inside a predicate).
+__device__ __forceinline__ float rcp_fast(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
 
-  const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  const unsigned lt_mask = (1u << lane) - 1u;
-  if (threadIdx.x == 0) {
-    mbar_init(&s_bar, 1);
+struct L1Warp {
+  float4 tri[3 * kL1Group];  // the staged group
+  int4 rng[kL1Group];
+  uint32_t soff[kL1Group], foff[kL1Group];  // exclusive prefixes of the SAT and fill units
+  uint32_t key[kL1Pairs], val[kL1Pairs];    // collected records
+  uint64_t bar;
+  // the current mesh's grid and planes: a shared copy, since every global atomic makes the compiler
+  // read the descriptor's fields again
+  GridDev g;
+  uint32_t *bplane, *toggles;
+};
+
+// A group of consecutive triangles of one mesh and this warp's share of its chunks of units: every
+// S-th from the part-th, or (a piece of a heavy triangle) kHeavyChunks of them from there.
+struct L1Item {
+  int m;           // mesh, -1: none left
+  int64_t t0;      // first triangle
+  int64_t tend;    // end of the ticket's triangles
+  uint32_t part;
+  bool piece;
+};
+
+// z interval outside which the SAT's plane test fails for certain in the column at (cx, cy): on
+// return [z0, z1] is cut to it.  With R the largest |V - c| (edges up to 2 R), the float test's value
+// is within 264 eps R^2 (R + h) of exact and the one below within 200; E has room for twice both and
+// for the distance of the z table from its affine form, so cells past H + E are rejected by the test.
+__device__ __forceinline__ void plane_range(const float *V, const GridDev &g, float cx, float cy,
+                                            int &z0, int &z1) {
+  const float a0 = V[3] - V[0], a1 = V[4] - V[1], a2 = V[5] - V[2];
+  const float b0 = V[6] - V[3], b1 = V[7] - V[4], b2 = V[8] - V[5];
+  const float nx = a1 * b2 - a2 * b1, ny = a2 * b0 - a0 * b2;
+  float nz = a0 * b1 - a1 * b0;
+  const float ca = __ldg(g.c1[2] + z0), cb = __ldg(g.c1[2] + z1);
+  float R = 0.f;  // the largest |V - c| of the run
+#pragma unroll
+  for (int i = 0; i < 9; i += 3)
+    R = fmaxf(R, fmaxf(fmaxf(fabsf(V[i] - cx), fabsf(V[i + 1] - cy)), fmaxf(fabsf(V[i + 2] - ca), fabsf(V[i + 2] - cb))));
+  R = fmaxf(R * 1.0001f, fmaxf(g.e1[0], fmaxf(g.e1[1], g.e1[2])));
+  if (!(R > 1e-9f && R < 1e9f)) return;
+  const float h = fmaxf(g.e1[0], fmaxf(g.e1[1], g.e1[2]));
+  const float E = 1024.f * EPS24 * R * R * (R + h) + 2.4f * EPS24 * fmaxf(fabsf(ca), fabsf(cb)) * fabsf(nz);
+  const float H = fabsf(nx) * g.e1[0] + fabsf(ny) * g.e1[1] + fabsf(nz) * g.e1[2] + E;
+  const float s = nx * (V[0] - cx) + ny * (V[1] - cy);
+  nz = copysignf(fmaxf(fabsf(nz), E * rcp_fast(512.f * R)), nz);  // (moves the value by less than E/512)
+  const float rn = rcp_fast(nz), ig = rcp_fast(2.f * g.e1[2]);
+  const float zc = V[2] - ca;
+  const float x1 = (zc + (s - H) * rn) * ig, x2 = (zc + (s + H) * rn) * ig;  // layers above z0
+  const float w = 16.f * EPS24 * (float)(z1 - z0) + 1e-4f;  // index arithmetic
+  const int b = z0;
+  z0 = b + min(max(__float2int_ru(fminf(x1, x2) - w - 16.f * EPS24 * fmaxf(fabsf(x1), fabsf(x2))), 0), z1 - b + 1);
+  z1 = b + min(__float2int_rd(fmaxf(x1, x2) + w + 16.f * EPS24 * fmaxf(fabsf(x1), fabsf(x2))), z1 - b);
+}
+
+// Toggles of one (triangle, column) pair that passed u/v: d(k) = hit(k) ^ hit(k + 1).  The exact t*
+// falls by the rise of the origin, so the hits are the voxels under the triangle's plane over the
+// column; X = the plane's height over the first centre, less 1e-6, in voxels.  As in the Level2 fill
+// the float t decides as t* outside 1.35 (8.2 eps M0 / |det| + 1e-6) of the crossing (rel <= 1/8),
+// X is off by about as much and by the centre table's distance from its affine form, and only the
+// voxels within that of the crossing (all of them for an ill-conditioned projection) run the test.
+__device__ __forceinline__ void column_toggles(const RayTri &rt, const RayCol &rc, const GridDev &g,
+                                               uint32_t *tog) {
+  const int nz = g.n[2];
+  const float *oz = g.c1[2];
+  const float ad = fabsf(rt.inv_det);
+  const float sd = fabsf(rt.e1x * rt.e2y) + fabsf(rt.e1y * rt.e2x);
+  int n1 = 0, n2 = nz;  // hits below n1 and misses from n2 for certain
+  if (4.f * EPS24 * sd * ad <= 0.125f) {
+    const float o0 = __ldg(oz), ig = rcp_fast(2.f * g.e1[2]);
+    const float atx = fabsf(rc.Tx), aty = fabsf(rc.Ty);
+    const float zt2 = 2.f * fmaxf(fabsf(rt.e1z), fmaxf(fabsf(rt.e2z), fabsf(rt.e2z - rt.e1z)));
+    const float M0 = fabsf(rt.e2x) * (aty * fabsf(rt.e1z) + zt2 * fabsf(rt.e1y)) +
+                     fabsf(rt.e2y) * (zt2 * fabsf(rt.e1x) + atx * fabsf(rt.e1z)) +
+                     fabsf(rt.e2z) * (atx * fabsf(rt.e1y) + aty * fabsf(rt.e1x));
+    const float t0 = (rt.e2x * (rc.Ty * rt.e1z) - rt.e2y * (rc.Tx * rt.e1z) +
+                      rt.e2z * (rc.Tx * rt.e1y - rc.Ty * rt.e1x)) * rt.inv_det;
+    const float X = ((rt.v1z - o0) + t0 - g.thr) * ig;
+    const float w = ig * (EPS24 * (40.f * M0 * ad + 8.f * zt2 +
+                                   4.2f * fmaxf(fabsf(g.bmin[2]), fabsf(g.bmax[2]))) + 0.35f * g.thr) +
+                    16.f * EPS24 * (float)nz + 1e-4f;
+    if (w < 1e6f) {  // (false for NaN too)
+      n1 = min(max(__float2int_ru(X - w), 0), nz);
+      n2 = min(max(__float2int_ru(X + w), 0), nz);
+    }
+  }
+  bool above = false;
+  for (int k = n2 - 1; k >= n1; --k) {
+    const bool hit = ray_t(rt, rc, __ldg(oz + k), g.thr);
+    if (hit != above) atomicXor(tog + (k >> 5), 1u << (k & 31));
+    above = hit;
+  }
+  if (n1 > 0 && !above) atomicXor(tog + ((n1 - 1) >> 5), 1u << ((n1 - 1) & 31));
+}
+
+// Every warp works by itself: it takes tickets of bd.tile triangles from the queue, stages them 32 at
+// a time by bulk async copies (TMA) on its own mbarrier and runs their SAT and fill units 32 at a
+// time.  With S > 1 (few triangles), S warps share a group's units.  Bound by instruction issue and
+// table loads where the units are many and by latency where they are few.  Against blocks of eight
+// warps on tiles of up to 256 triangles, whose closing barriers were the main stall (8 of 18 cycles per
+// issue), with every column's hits evaluated over all its voxels by a whole warp and a counter update
+// per 32 units: 262k triangles at 128^3 61 -> 36 us, 1.3M at 256^3 226 -> 108, 1M at 512^3 without
+// Level2 441 -> 176, 7k large ones at 150x170x130 265 -> 40, 9M in 256 meshes 3.8 -> 1.4 ms.  Without
+// the pieces of large triangles the last were 67 us and 4.1 ms: a group of them on one warp was the
+// launch's tail.
+__global__ void __launch_bounds__(kL1Warps * 32, 8) k_level1(BatchDev bd, uint32_t S) {
+  __shared__ __align__(16) L1Warp s_warp[kL1Warps];
+  const unsigned lane = threadIdx.x & 31u;
+  L1Warp &ws = s_warp[threadIdx.x >> 5];
+  if (lane == 0) {
+    mbar_init(&ws.bar, 1);
     fence_mbar_init();
   }
-  __syncthreads();
+  __syncwarp();
 
-  for (uint32_t iter = 0;; ++iter) {
-    // ---- pull the next (mesh, tile) item from the queue
-    if (threadIdx.x == 0) s_item = (int64_t)atomicAdd(&bd.queue[0], 1u);
-    __syncthreads();
-    const int64_t item = s_item;
-    if (item >= bd.total_tiles) break;
-    const int m = find_mesh<&MeshDesc::tile_base>(bd.md, bd.nmesh, item);
-    const MeshDesc &d = bd.md[m];
-    const GridDev &g = d.g;
-    const int64_t t0 = (item - d.tile_base) * TILE;
-    uint32_t *const kmask = bd.kmask && d.has_l2 ? bd.kmask + d.word_base : nullptr;
-    const int nt = (int)min((int64_t)TILE, d.T - t0);
-
-    // ---- stage the tile with bulk async copies completing on the mbarrier
-    if (threadIdx.x == 0) {
-      const uint32_t bt = (uint32_t)nt * 48u, br = (uint32_t)nt * 16u;
-      mbar_expect_tx(&s_bar, bt + br);
-      bulk_g2s(s_tri, d.ptri + 3 * t0, bt, &s_bar);
-      bulk_g2s(s_rng, d.rng + t0, br, &s_bar);
-    }
-    // bounded wait (bd.wait_limit polls, kWaitLimit when 0); bd.fail_wait makes it give up at
-    // once (failure-detection tests).  On giving up, the status word is raised and thread 0
-    // waits, bounded again, for the copies in flight to land before the block returns.
-    const bool ok = !bd.fail_wait &&
-                    mbar_wait_bounded(&s_bar, iter & 1u, bd.wait_limit ? bd.wait_limit : kWaitLimit);
-    if (__syncthreads_or(!ok)) {
-      if (threadIdx.x == 0) {
-        atomicOr(&d.stats->status, (unsigned)ST_WAIT_TIMEOUT);
-        mbar_wait_bounded(&s_bar, iter & 1u, kWaitLimit);  // let the copy in flight land
-      }
+  const uint32_t nheavy = bd.heavy ? min(*bd.heavy_n, bd.heavy_cap) : 0u;
+  const uint32_t nitems = nheavy + (uint32_t)(bd.total_tiles * S);
+  // the group after `it`: the next of its ticket, or the first of a new ticket
+  auto advance = [&](L1Item &it) {
+    if (it.m >= 0 && it.t0 + kL1Group < it.tend) {
+      it.t0 += kL1Group;
       return;
     }
+    uint32_t tk = 0;
+    if (lane == 0) tk = atomicAdd(&bd.queue[0], 1u);
+    tk = __shfl_sync(FULL, tk, 0);
+    if (tk >= nitems) {
+      it.m = -1;
+      return;
+    }
+    it.piece = tk < nheavy;
+    if (it.piece) {  // the heavy pieces first
+      const uint4 h = __ldg(bd.heavy + tk);
+      it.m = (int)h.x;
+      it.t0 = h.y;
+      it.tend = it.t0 + (h.w ? 1 : 0);  // (an entry of a triangle that did not fit the list: nothing)
+      it.part = h.z * kHeavyChunks;
+      return;
+    }
+    tk -= nheavy;
+    const int64_t tile = tk / S;
+    it.part = tk % S;
+    it.m = find_mesh<&MeshDesc::tile_base>(bd.md, bd.nmesh, tile);
+    const MeshDesc &d = bd.md[it.m];
+    it.t0 = (tile - d.tile_base) * bd.tile;
+    it.tend = min(d.T, it.t0 + bd.tile);
+  };
+  auto stage = [&](const L1Item &it) {
+    if (it.m < 0 || lane != 0) return;
+    const MeshDesc &d = bd.md[it.m];
+    const uint32_t n = (uint32_t)max(min((int64_t)kL1Group, it.tend - it.t0), (int64_t)1);
+    mbar_expect_tx(&ws.bar, n * 64u);
+    bulk_g2s(ws.tri, d.ptri + 3 * it.t0, n * 48u, &ws.bar);
+    bulk_g2s(ws.rng, d.rng + it.t0, n * 16u, &ws.bar);
+  };
 
-    // ---- per-triangle unit counts and their block scan
+  uint32_t nbuf = 0;  // collected records of mesh `bm`
+  int bm = -1;
+  // room for n records of a mesh in its segment; positions past its capacity raise the status
+  auto take_room = [&](MeshStats *st, uint32_t n) {
+    unsigned long long pos = 0;
+    if (lane == 0) pos = atomicAdd(&st->pairs, (unsigned long long)n);
+    return __shfl_sync(FULL, pos, 0);
+  };
+  auto flush = [&]() {
+    if (!nbuf) return;
+    const MeshDesc &d = bd.md[bm];
+    __syncwarp();
+    const unsigned long long pos = take_room(d.stats, nbuf);
+    const uint64_t cap = (uint64_t)d.pair_cap;
+    for (uint32_t i = lane; i < nbuf; i += 32) {
+      if (pos + i < cap) {
+        d.keys[pos + i] = ws.key[i];
+        d.vals[pos + i] = ws.val[i];
+      } else {
+        atomicOr(&d.stats->status, (unsigned)ST_PAIR_OVERFLOW);
+      }
+    }
+    __syncwarp();
+    nbuf = 0;
+  };
+
+  L1Item it = {-1, 0, 0, 0, false};
+  advance(it);
+  stage(it);
+  for (uint32_t phase = 0; it.m >= 0; phase ^= 1u) {
+    const MeshDesc &d = bd.md[it.m];
+    const GridDev &g = ws.g;
+    if (bm != it.m) {
+      flush();
+      bm = it.m;
+      __syncwarp();
+      const uint32_t *src = reinterpret_cast<const uint32_t *>(&d.g);
+      uint32_t *dst = reinterpret_cast<uint32_t *>(&ws.g);
+      for (int i = lane; i < (int)(sizeof(GridDev) / 4); i += 32) dst[i] = src[i];
+      if (lane == 0) {
+        ws.bplane = d.bplane;
+        ws.toggles = d.toggles;
+      }
+      __syncwarp();
+    }
+    // bounded wait (bd.wait_limit polls, kWaitLimit when 0); bd.fail_wait makes it give up at once
+    // (failure-detection tests).  On giving up, the status word is raised and the warp waits, bounded
+    // again, for the copies in flight to land before it returns.
+    const bool ok = !bd.fail_wait &&
+                    mbar_wait_bounded(&ws.bar, phase, bd.wait_limit ? bd.wait_limit : kWaitLimit);
+    if (__any_sync(FULL, !ok)) {
+      if (lane == 0) atomicOr(&d.stats->status, (unsigned)ST_WAIT_TIMEOUT);
+      mbar_wait_bounded(&ws.bar, phase, kWaitLimit);
+      return;
+    }
+    const float4 *tri = ws.tri;
+    const int4 *rng = ws.rng;
+    const int64_t t0 = it.t0;
+    const int nt = (int)min((int64_t)kL1Group, it.tend - t0);
+
+    // ---- per-triangle unit counts and their scan
     uint32_t cs = 0, cf = 0;
-    if ((int)threadIdx.x < nt) {
-      const int4 r = s_rng[threadIdx.x];
+    if ((int)lane < nt && (it.piece || !rng[lane].w)) {
+      const int4 r = rng[lane];
       const int x0 = lo16(r.x), x1 = hi16(r.x), y0 = lo16(r.y), y1 = hi16(r.y);
       if (x0 <= x1 && y0 <= y1) cs = (uint32_t)((x1 - x0 + 1) * (y1 - y0 + 1));
-      const uint32_t fxr = __float_as_uint(s_tri[3 * threadIdx.x].w);
-      const uint32_t fyr = __float_as_uint(s_tri[3 * threadIdx.x + 1].w);
+      const uint32_t fxr = __float_as_uint(tri[3 * lane].w), fyr = __float_as_uint(tri[3 * lane + 1].w);
       if (lo16(fxr) <= hi16(fxr) && lo16(fyr) <= hi16(fyr))
         cf = (uint32_t)((hi16(fxr) - lo16(fxr) + 1) * (hi16(fyr) - lo16(fyr) + 1));
     }
-    {
-      const uint32_t is = warp_incl_scan(cs), iff = warp_incl_scan(cf);
-      if (lane == 31) { s_ws[warp] = is; s_wf[warp] = iff; }
-      __syncthreads();
-      uint32_t bs = 0, bf = 0;
-      for (unsigned w = 0; w < warp; ++w) { bs += s_ws[w]; bf += s_wf[w]; }
-      if ((int)threadIdx.x < TILE) {
-        s_soff[threadIdx.x] = bs + is - cs;
-        s_foff[threadIdx.x] = bf + iff - cf;
-      }
-      if (threadIdx.x == kL1Threads - 1) {
-        s_soff[TILE] = bs + is;
-        s_foff[TILE] = bf + iff;
-      }
-      if (threadIdx.x == 0) s_next = 0;
-      __syncthreads();
-    }
-    const uint32_t Us = s_soff[TILE], Uf = s_foff[TILE];
+    const uint32_t is = warp_incl_scan(cs), iff = warp_incl_scan(cf);
+    ws.soff[lane] = is - cs;
+    ws.foff[lane] = iff - cf;
+    const uint32_t Us = __shfl_sync(FULL, is, 31), Uf = __shfl_sync(FULL, iff, 31);
+    __syncwarp();
     const int nx = g.n[0], ny = g.n[1], nz = g.n[2];
-    const uint64_t cap = (uint64_t)d.pair_cap;
-
-    // Warps take 32-unit chunks from a counter, the SAT chunks first and then the fill chunks,
-    // so that a warp whose z runs or hits were short takes more chunks instead of waiting at the
-    // tile's closing barrier for the others.
+    const bool emit = d.has_l2 || bd.emit_all;  // the records are read later (else only counted)
     const uint32_t nsc = (Us + 31u) >> 5;
-    auto next_chunk = [&]() {
-      uint32_t c = 0;
-      if (lane == 0) c = atomicAdd(&s_next, 1u);
-      return __shfl_sync(FULL, c, 0);
-    };
-    uint32_t chunk = next_chunk();
-    // ---- (a) SAT units
-    for (; chunk < nsc; chunk = next_chunk()) {
-      const uint32_t base = chunk * 32u;
-      const uint32_t u = base + lane;
+    const uint32_t step = it.piece ? 1u : S;
+    const uint32_t cend = it.piece ? min(it.part + kHeavyChunks, nsc + ((Uf + 31u) >> 5)) : nsc + ((Uf + 31u) >> 5);
+    unsigned long long counted = 0;
+    uint32_t chunk = it.part;
+
+    // ---- (a) SAT units: (triangle, column), a z run each
+    for (; chunk < min(nsc, cend); chunk += step) {
+      const uint32_t u = chunk * 32u + lane;
       int lt = 0, p = 0, q = 0, z0 = 0, zc = -1;
       float V[9];
       SatCol sc;
       if (u < Us) {
-        lt = tile_search(s_soff, nt, u);
-        const int4 r = s_rng[lt];
+        lt = group_search(ws.soff, u);
+        const int4 r = rng[lt];
         const int x0 = lo16(r.x), x1 = hi16(r.x), y0 = lo16(r.y);
         z0 = lo16(r.z);
-        const uint32_t c = u - s_soff[lt];
-        const int nxr = x1 - x0 + 1;
-        p = x0 + (int)(c % (uint32_t)nxr);
-        q = y0 + (int)(c / (uint32_t)nxr);
-        const float4 a0 = s_tri[3 * lt], a1 = s_tri[3 * lt + 1], a2 = s_tri[3 * lt + 2];
+        const uint32_t c = u - ws.soff[lt];
+        const uint32_t nxr = (uint32_t)(x1 - x0 + 1), row = c / nxr;
+        p = x0 + (int)(c - row * nxr);
+        q = y0 + (int)row;
+        const float4 a0 = tri[3 * lt], a1 = tri[3 * lt + 1], a2 = tri[3 * lt + 2];
         V[0] = a0.x; V[1] = a0.y; V[2] = a0.z; V[3] = a1.x; V[4] = a1.y; V[5] = a1.z;
         V[6] = a2.x; V[7] = a2.y; V[8] = a2.z;
-        if (sat_col(V, __ldg(g.c1[0] + p), __ldg(g.c1[1] + q), g.e1, sc)) zc = hi16(r.z);
+        const float cx = __ldg(g.c1[0] + p), cy = __ldg(g.c1[1] + q);
+        if (sat_col(V, cx, cy, g.e1, sc)) {
+          zc = hi16(r.z);
+          if (zc - z0 >= kPlaneRun) plane_range(V, g, cx, cy, z0, zc);
+        }
       }
       bool first = true;
       const uint32_t tglob = (uint32_t)(t0 + lt);
@@ -496,83 +666,73 @@ __global__ void __launch_bounds__(kL1Threads) k_level1(BatchDev bd) {
           zc -= nrun;
         }
         const uint32_t cnt = __popc(mask);
-        const uint32_t inc = warp_incl_scan(cnt);
-        const uint32_t tot = __shfl_sync(FULL, inc, 31);
-        unsigned long long basep = 0;
-        if (lane == 31 && tot) basep = atomicAdd(&d.stats->pairs, (unsigned long long)tot);
-        basep = __shfl_sync(FULL, basep, 31);
-        uint64_t pos = basep + inc - cnt;
+        uint32_t pos = 0;          // in the collected records
+        unsigned long long gpos = 0;  // or in the mesh's segment
+        bool direct = false;
+        if (emit) {
+          const uint32_t inc = warp_incl_scan(cnt);
+          const uint32_t tot = __shfl_sync(FULL, inc, 31);
+          if (tot == 0) continue;
+          if (nbuf + tot > (uint32_t)kL1Pairs) flush();
+          pos = nbuf + inc - cnt;
+          direct = tot > (uint32_t)kL1Pairs;
+          if (direct) gpos = take_room(d.stats, tot) + inc - cnt;
+          else nbuf += tot;
+        } else {
+          counted += cnt;
+        }
         while (mask) {
           const int dd = __ffs(mask) - 1;
           mask &= mask - 1u;
           const int r = ztop - dd;
           const uint32_t key = (uint32_t)(((uint64_t)q * nx + p) * nz + r);
-          if (pos < cap) {
-            d.keys[pos] = key;
-            d.vals[pos] = tglob | (first ? 0x80000000u : 0u);
-          } else {
-            atomicOr(&d.stats->status, (unsigned)ST_PAIR_OVERFLOW);
+          const uint32_t val = tglob | (first ? 0x80000000u : 0u);
+          if (direct) {
+            if (gpos < (uint64_t)d.pair_cap) {
+              d.keys[gpos] = key;
+              d.vals[gpos] = val;
+            } else {
+              atomicOr(&d.stats->status, (unsigned)ST_PAIR_OVERFLOW);
+            }
+            ++gpos;
+          } else if (emit) {
+            ws.key[pos] = key;
+            ws.val[pos] = val;
+            ++pos;
           }
-          if (kmask) atomicOr(kmask + (key >> 5), 1u << (key & 31u));
           first = false;
-          ++pos;
-          atomicOr(&d.bplane[((size_t)r * ny + q) * g.nxw + (p >> 5)], 1u << (p & 31));
+          atomicOr(&ws.bplane[((size_t)r * ny + q) * g.nxw + (p >> 5)], 1u << (p & 31));
         }
+        __syncwarp();
       }
+    }
+    if (!emit) {
+      counted = warp_sum(counted);
+      if (lane == 0 && counted) atomicAdd(&d.stats->pairs, counted);
     }
 
-    // ---- (b) fill units
-    for (; (chunk - nsc) * 32u < Uf; chunk = next_chunk()) {
-      const uint32_t base = (chunk - nsc) * 32u;
-      const uint32_t u = base + lane;
-      bool pass = false;
-      if (u < Uf) {
-        const int lt = tile_search(s_foff, nt, u);
-        const float4 a0 = s_tri[3 * lt], a1 = s_tri[3 * lt + 1], a2 = s_tri[3 * lt + 2];
-        const uint32_t fxr = __float_as_uint(a0.w), fyr = __float_as_uint(a1.w);
-        const uint32_t c = u - s_foff[lt];
-        const int nxr = hi16(fxr) - lo16(fxr) + 1;
-        const int i = lo16(fxr) + (int)(c % (uint32_t)nxr);
-        const int j = lo16(fyr) + (int)(c / (uint32_t)nxr);
-        const float V[9] = {a0.x, a0.y, a0.z, a1.x, a1.y, a1.z, a2.x, a2.y, a2.z};
-        RayTri rt;
-        ray_tri_pre(V, a2.w, rt);  // fill units exist only for triangles passing the det test
-        RayCol rc;
-        pass = ray_col(rt, __ldg(g.c1[0] + i), __ldg(g.c1[1] + j), rc);
-      }
-      const unsigned qm = __ballot_sync(FULL, pass);
-      if (pass) s_q[warp][__popc(qm & lt_mask)] = u;
-      __syncwarp();
-      const int nq = __popc(qm);
-      for (int e = 0; e < nq; ++e) {
-        const uint32_t uu = s_q[warp][e];
-        const int lt = tile_search(s_foff, nt, uu);
-        const float4 a0 = s_tri[3 * lt], a1 = s_tri[3 * lt + 1], a2 = s_tri[3 * lt + 2];
-        const uint32_t fxr = __float_as_uint(a0.w), fyr = __float_as_uint(a1.w);
-        const uint32_t c = uu - s_foff[lt];
-        const int nxr = hi16(fxr) - lo16(fxr) + 1;
-        const int i = lo16(fxr) + (int)(c % (uint32_t)nxr);
-        const int j = lo16(fyr) + (int)(c / (uint32_t)nxr);
-        const float V[9] = {a0.x, a0.y, a0.z, a1.x, a1.y, a1.z, a2.x, a2.y, a2.z};
-        RayTri rt;
-        ray_tri_pre(V, a2.w, rt);
-        RayCol rc;
-        ray_col(rt, __ldg(g.c1[0] + i), __ldg(g.c1[1] + j), rc);
-        const size_t col = (size_t)j * nx + i;
-        uint32_t carry = 0;
-        for (int w = g.nzw - 1; w >= 0; --w) {
-          const int k = w * 32 + (int)lane;
-          const bool hit = k < nz && ray_t(rt, rc, __ldg(g.c1[2] + k), g.thr);
-          const uint32_t h = __ballot_sync(FULL, hit);
-          const uint32_t dd = h ^ ((h >> 1) | (carry << 31));
-          carry = h & 1u;
-          if (lane == 0 && dd) atomicXor(&d.toggles[col * g.nzw + w], dd);
-        }
-      }
-      __syncwarp();
+    // ---- (b) fill units: (triangle, column)
+    for (; chunk < cend; chunk += step) {
+      const uint32_t u = (chunk - nsc) * 32u + lane;
+      if (u >= Uf) continue;
+      const int lt = group_search(ws.foff, u);
+      const float4 a0 = tri[3 * lt], a1 = tri[3 * lt + 1], a2 = tri[3 * lt + 2];
+      const uint32_t fxr = __float_as_uint(a0.w), fyr = __float_as_uint(a1.w);
+      const uint32_t c = u - ws.foff[lt];
+      const uint32_t nxr = (uint32_t)(hi16(fxr) - lo16(fxr) + 1), row = c / nxr;
+      const int i = lo16(fxr) + (int)(c - row * nxr), j = lo16(fyr) + (int)row;
+      const float V[9] = {a0.x, a0.y, a0.z, a1.x, a1.y, a1.z, a2.x, a2.y, a2.z};
+      RayTri rt;
+      ray_tri_pre(V, a2.w, rt);  // fill units exist only for triangles passing the det test
+      RayCol rc;
+      if (ray_col(rt, __ldg(g.c1[0] + i), __ldg(g.c1[1] + j), rc))
+        column_toggles(rt, rc, g, ws.toggles + ((size_t)j * nx + i) * g.nzw);
     }
-    __syncthreads();  // the next item overwrites the tile
+    __syncwarp();  // the buffer may be staged again
+    advance(it);
+    stage(it);
   }
+  flush();
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -645,6 +805,24 @@ __global__ void __launch_bounds__(256) k_fill_finish(BatchDev bd) {
   }
   const int k = w * 32 + (int)lane;
   if (k < nz) d.iplane[((size_t)k * ny + j) * g.nxw + ig] = mine;
+  if (!bd.kmask || !d.has_l2) return;
+  // the boundary plane transposed the other way, for the pair lists: 32 layers of 32 columns to one
+  // word per column at the columns' place in key order
+  const uint32_t bw = k < nz ? d.bplane[((size_t)k * ny + j) * g.nxw + ig] : 0u;
+  if (!__any_sync(FULL, bw != 0u)) return;
+  uint32_t cw = 0;
+#pragma unroll
+  for (int bb = 0; bb < 32; ++bb) {
+    const uint32_t mm = __ballot_sync(FULL, (bw >> bb) & 1u);
+    if ((int)lane == bb) cw = mm;
+  }
+  if (cw) {
+    uint32_t *km = bd.kmask + d.word_base;
+    const uint64_t bit = (uint64_t)col * nz + (uint64_t)w * 32;
+    const unsigned sh = (unsigned)(bit & 31u);
+    atomicOr(km + (bit >> 5), cw << sh);
+    if (sh && (cw >> (32 - sh))) atomicOr(km + (bit >> 5) + 1, cw >> (32 - sh));
+  }
 }
 
 __global__ void k_popc(const uint32_t *__restrict__ plane, int64_t nw, uint32_t *__restrict__ cnt) {
@@ -899,14 +1077,13 @@ void launch_plan(const BatchDev &bd, MeshDesc *d_md, int32_t *bindex, uint8_t *l
 
 void launch_level1(const BatchDev &bd, int num_sms, cudaStream_t s) {
   if (bd.total_tiles <= 0) return;
-  const int64_t grid = std::min<int64_t>(bd.total_tiles, (int64_t)num_sms * 8);
-  cudaMemsetAsync(bd.queue, 0, sizeof(uint32_t), s);
-  switch (bd.tile) {
-    case 32: k_level1<32><<<(unsigned)grid, kL1Threads, 0, s>>>(bd); break;
-    case 64: k_level1<64><<<(unsigned)grid, kL1Threads, 0, s>>>(bd); break;
-    case 128: k_level1<128><<<(unsigned)grid, kL1Threads, 0, s>>>(bd); break;
-    default: k_level1<256><<<(unsigned)grid, kL1Threads, 0, s>>>(bd); break;
-  }
+  // Few triangles (a coarse model on a fine grid): several warps share a group's units, so that
+  // every SM has its 32 warps.
+  const int64_t warps = (int64_t)num_sms * 8 * kL1Warps;
+  const int64_t S = std::max<int64_t>(1, std::min<int64_t>(warps / bd.total_tiles, 4096));
+  const int64_t items = bd.total_tiles * S;
+  const int64_t grid = std::min<int64_t>((items + kL1Warps - 1) / kL1Warps, (int64_t)num_sms * 8);
+  k_level1<<<(unsigned)grid, kL1Warps * 32, 0, s>>>(bd, (uint32_t)S);
   count_launch();
 }
 

@@ -1575,7 +1575,6 @@ void launch_level2(const BatchDev &bd, const uint32_t *keys, const uint32_t *val
   // streams (when given) so that one slab's tail overlaps the next slab's start
   const int launches = zslab > 0 ? nslab : 1;
   const bool two = zslab > 0 && launches > 1 && aux;
-  cudaMemsetAsync(bd.queue + 1, 0, (size_t)(2 * kSlabsMax) * sizeof(uint32_t), s);
   if (two) {
     cudaEventRecord(aux->fork, s);
     cudaStreamWaitEvent(aux->st[0], aux->fork, 0);

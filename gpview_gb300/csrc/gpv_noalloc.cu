@@ -22,6 +22,7 @@
 //   * Sizes whose intermediates do not fit the array are rejected with GPV_ERR_INVALID and a
 //     message from gpv_noalloc_last_error() (kept per host thread); nothing is launched then.
 //   * No cudaMalloc, cudaFree, host heap or library allocation is made.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -43,59 +44,6 @@ thread_local char g_err[256] = "";
 
 void set_err(const char *msg) {
   std::snprintf(g_err, sizeof(g_err), "%s", msg);
-}
-
-// Variant of the Level1 kernel without the (voxel, triangle) records: one warp per triangle,
-// whose lanes share its SAT candidate columns (boundary bits) and its fill columns (parity
-// toggles).  Inputs are the packed triangles written by the prep kernel.  A triangle's work is
-// its candidate box plus its fill columns times nz, spread over 32 lanes: a triangle whose box
-// spans the whole grid (or an ill-conditioned one, whose fill box is the whole grid) costs about
-// nx*ny*nz/32 tests per lane.
-__global__ void k_level1_nopairs(const MeshDesc *__restrict__ md) {
-  const MeshDesc &b = *md;
-  const GridDev &g = b.g;
-  const int lane = threadIdx.x & 31;
-  const int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // warp-uniform
-  if (t >= b.T) return;
-  const float4 a0 = b.ptri[3 * t], a1 = b.ptri[3 * t + 1], a2 = b.ptri[3 * t + 2];
-  const float V[9] = {a0.x, a0.y, a0.z, a1.x, a1.y, a1.z, a2.x, a2.y, a2.z};
-  const int4 rg = b.rng[t];
-  const int nx = g.n[0], ny = g.n[1], nz = g.n[2];
-  const int x0 = (int)(rg.x & 0xffff), x1 = (int)((unsigned)rg.x >> 16);
-  const int y0 = (int)(rg.y & 0xffff), y1 = (int)((unsigned)rg.y >> 16);
-  const int z0 = (int)(rg.z & 0xffff), z1 = (int)((unsigned)rg.z >> 16);
-  const int sx = max(x1 - x0 + 1, 0), sy = max(y1 - y0 + 1, 0);
-  for (int c = lane; c < sx * sy; c += 32) {
-    const int p = x0 + c % sx, q = y0 + c / sx;
-    SatCol sc;
-    if (!sat_col(V, g.c1[0][p], g.c1[1][q], g.e1, sc)) continue;
-    for (int r = z0; r <= z1; ++r)
-      if (sat_z(sc, V, g.c1[2][r], g.e1))
-        atomicOr(&b.bplane[((size_t)r * ny + q) * g.nxw + (p >> 5)], 1u << (p & 31));
-  }
-  const uint32_t fxr = __float_as_uint(a0.w), fyr = __float_as_uint(a1.w);
-  const int fx0 = (int)(fxr & 0xffff), fx1 = (int)(fxr >> 16);
-  const int fy0 = (int)(fyr & 0xffff), fy1 = (int)(fyr >> 16);
-  const int fsx = max(fx1 - fx0 + 1, 0), fsy = max(fy1 - fy0 + 1, 0);
-  RayTri rt;
-  ray_tri_pre(V, a2.w, rt);
-  for (int c = lane; c < fsx * fsy; c += 32) {
-    const int i = fx0 + c % fsx, j = fy0 + c / fsx;
-    RayCol rc;
-    if (!ray_col(rt, g.c1[0][i], g.c1[1][j], rc)) continue;
-    const size_t col = (size_t)j * nx + i;
-    uint32_t carry = 0;
-    for (int w = g.nzw - 1; w >= 0; --w) {
-      uint32_t h = 0;
-      for (int bb = 0; bb < 32; ++bb) {
-        const int k = 32 * w + bb;
-        if (k < nz && ray_t(rt, rc, g.c1[2][k], g.thr)) h |= 1u << bb;
-      }
-      const uint32_t d = h ^ ((h >> 1) | (carry << 31));
-      carry = h & 1u;
-      if (d) atomicXor(&b.toggles[col * g.nzw + w], d);
-    }
-  }
 }
 
 size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
@@ -214,6 +162,11 @@ extern "C" int gpv_voxelize_level1_noalloc(const float *d_tris, int64_t num_tria
 
   // ---- the array's device address on the current device (looked up on every call)
   unsigned char *base = nullptr;
+  int num_sms = 1;
+  {
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
+  }
   {
     void *p = nullptr;
     const cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
@@ -251,7 +204,13 @@ extern "C" int gpv_voxelize_level1_noalloc(const float *d_tris, int64_t num_tria
   std::memset(&bd, 0, sizeof(bd));
   bd.md = d_md;
   bd.nmesh = 1;
-  bd.tile = 128;
+  bd.tile = 32;
+  bd.total_tiles = (T + 31) / 32;
+  bd.queue = d_tot + 1;  // (the total takes the first word)
+  // what the array has left holds the pieces of large triangles
+  bd.heavy_cap = (uint32_t)std::min<size_t>((kScratchBytes - o) / sizeof(uint4), kHeavyCap);
+  bd.heavy = bd.heavy_cap ? reinterpret_cast<uint4 *>(base + o) : nullptr;
+  bd.heavy_n = d_tot + 2;
   bd.total_tris = T;
   bd.total_fwarps = (int64_t)g.n[1] * g.nxw * g.nzw;
   bd.total_rows = (int64_t)g.n[2] * g.n[1];
@@ -264,6 +223,7 @@ extern "C" int gpv_voxelize_level1_noalloc(const float *d_tris, int64_t num_tria
   cudaError_t e = cudaMemcpyAsync(d_tab, tab, sizeof(float) * ntab, cudaMemcpyHostToDevice, stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(d_md, &md, sizeof(md), cudaMemcpyHostToDevice, stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(md.stats, 0, sizeof(MeshStats), stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(d_tot, 0, 16, stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(md.bplane, 0, 4 * (size_t)N1w, stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(md.toggles, 0, 4 * (size_t)(ncol * g.nzw), stream);
   if (e != cudaSuccess) {
@@ -271,10 +231,7 @@ extern "C" int gpv_voxelize_level1_noalloc(const float *d_tris, int64_t num_tria
     return GPV_ERR_CUDA;
   }
   launch_prep(bd, stream);
-  if (T > 0) {
-    k_level1_nopairs<<<(unsigned)((T + 3) / 4), 128, 0, stream>>>(d_md);  // a warp per triangle
-    count_launch();
-  }
+  launch_level1(bd, num_sms, stream);  // (no Level2 grid: the records are counted, not written)
   launch_fill_finish(bd, stream);
   launch_popc(md.bplane, N1w, wcnt, stream);
   scan_u32(wcnt, wpre, N1w, d_tot, stmp, stream);

@@ -436,7 +436,7 @@ int CUDAClassifyTessellation(float *trianglesCUDAData, int numTriangles, float *
                o_rng = take(16 * (size_t)T), o_fbox = take(16 * (size_t)T),
                o_bp = take(4 * (size_t)N1w), o_ip = take(4 * (size_t)N1w),
                o_tg = take(4 * (size_t)tog), o_st = take(sizeof(MeshStats)),
-               o_md = take(sizeof(MeshDesc)), o_q = take(64);
+               o_md = take(sizeof(MeshDesc)), o_q = take(4 * (kQueueWords + 1)), o_hv = take(16 * (size_t)kHeavyCap);
   const size_t fixed = off;
   const bool aligned = (reinterpret_cast<uintptr_t>(trianglesCUDAData) & 15u) == 0;
   if (!shim_reserve(fixed) || !shim_tables((size_t)ntab)) return 1;
@@ -467,8 +467,7 @@ int CUDAClassifyTessellation(float *trianglesCUDAData, int numTriangles, float *
   md.stats = reinterpret_cast<MeshStats *>(base + o_st);
   md.ch = 1;
   MeshDesc *d_md = reinterpret_cast<MeshDesc *>(base + o_md);
-  int tile = 256;
-  while (tile > 32 && T < (int64_t)tile * 3 * g_shim.num_sms) tile >>= 1;
+  const int tile = 32;
   BatchDev bd;
   std::memset(&bd, 0, sizeof(bd));
   bd.md = d_md;
@@ -479,7 +478,15 @@ int CUDAClassifyTessellation(float *trianglesCUDAData, int numTriangles, float *
   bd.total_fwarps = (int64_t)gh.n[1] * gh.nxw * gh.nzw;
   bd.total_rows = (int64_t)gh.n[2] * gh.n[1];
   bd.total_words = N1w;
-  bd.queue = reinterpret_cast<uint32_t *>(base + o_q);
+  auto set_queue = [&] {
+    bd.queue = reinterpret_cast<uint32_t *>(base + o_q);
+    bd.heavy = reinterpret_cast<uint4 *>(base + o_hv);
+    bd.heavy_n = bd.queue + kQueueWords;
+    bd.heavy_cap = kHeavyCap;
+  };
+  set_queue();
+  cudaMemsetAsync(bd.queue, 0, 4 * (kQueueWords + 1), 0);
+  bd.emit_all = 1;
   bd.fill = kFillNone;  // SAT units only: ClassifyTessellation marks boundaries, nothing fills
   cudaMemsetAsync(md.stats, 0, sizeof(MeshStats), 0);
   cudaMemsetAsync(md.bplane, 0, 4 * (size_t)N1w, 0);
@@ -513,7 +520,7 @@ int CUDAClassifyTessellation(float *trianglesCUDAData, int numTriangles, float *
     md.stats = reinterpret_cast<MeshStats *>(base + o_st);
     d_md = reinterpret_cast<MeshDesc *>(base + o_md);
     bd.md = d_md;
-    bd.queue = reinterpret_cast<uint32_t *>(base + o_q);
+    set_queue();
   }
   uint32_t *keys = reinterpret_cast<uint32_t *>(base + o_keys);
   uint32_t *vals = reinterpret_cast<uint32_t *>(base + o_vals);
