@@ -119,6 +119,9 @@ uint64_t call_key(int n, const int64_t *T, const gpv_grid_spec *specs) {
   return h;
 }
 
+// Average triangles a voxel up to which ordering each voxel's list beats the radix sort.
+constexpr int64_t kSegSortAverage = 64;
+
 // Word of the page-locked scratch (gpv_ctx::h_u32) where a one-graph call's DevPlan lands.
 constexpr int kPlanWord = 32;
 
@@ -293,10 +296,9 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
   CK(ws.get(&ptri, 3 * (size_t)std::max<int64_t>(tris, 1)));
   CK(ws.get(&rng, (size_t)std::max<int64_t>(tris, 1)));
   CK(ws.get(&fbox, (size_t)std::max<int64_t>(tris, 1)));
-  // without normals the pair lists are built by a counting sort, which ranks the voxels of the
-  // pairs through a second, column-major bit plane after the boundary plane; one popcount and one
-  // scan cover both planes
-  const bool kmark = nmode == 0 && words > 0;
+  // the pair lists are built by a counting sort, which ranks the voxels of the pairs through a
+  // second, column-major bit plane after the boundary plane; one popcount and one scan cover both
+  const bool kmark = words > 0;
   const int64_t swords = kmark ? 2 * words : words;
   CK(ws.get(&bplane, (size_t)swords));
   CK(ws.get(&iplane, (size_t)words));
@@ -586,6 +588,7 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
     CK(ctx_malloc_async(ctx, &set->l2, std::max<int64_t>(cap.l2bytes, 16), s));
     BatchDev bdp = bd;
     bdp.plan = d_plan;
+    for (int m = 0; m < n; ++m) ctx->h_md[m].ch = level2_few_chunk(md[m].ch, cap.U, ctx->num_sms);
     std::vector<uint64_t> sig2 = sig0;
     for (uint64_t x : {(uint64_t)cap.B, (uint64_t)cap.U, (uint64_t)cap.l2bytes, (uint64_t)cap.tiles,
                        (uint64_t)cap.P,
@@ -609,7 +612,7 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
         count_sort_pairs(bdp, nullptr, cap.tiles, keys, vals, wpre + words, cap.U, cap.P, cnt,
                          useg, kalt, valt, wtot + 1, sortmp, s);
         mark(7);
-        launch_level2(bdp, kalt, valt, useg, cap.U, l2tmp, l2_words, ctx->num_sms, s,
+        launch_level2(bdp, kalt, valt, useg, cap.U, l2tmp, level2_mask_words(cap.U, cap.l2bytes), l2_words, ctx->num_sms, s,
                       [&] { mark(9); });
       } else {
         mark(7);
@@ -723,6 +726,7 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
     l2off[m + 1] = l2off[m] + (gh[m].level2 ? (int64_t)st.boundary * gh[m].cells : 0);
   }
   l2bytes = l2off[n];
+  for (int m = 0; m < n; ++m) md[m].ch = level2_few_chunk(md[m].ch, ub, ctx->num_sms);
   // host outputs into pinned memory: the Level2 kernel writes its bytes there itself (over the
   // CPU-GPU link while it computes) instead of into device memory followed by copies
   const bool l2_direct = sink && sink->l2_dev && gh[0].level2 && sink->l2_cap >= l2bytes;
@@ -785,7 +789,10 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
   // ---- phase 2: allocations and staging first, then the recorded launch sequence
   const int64_t ntiles = (int64_t)st_host.size();
   const bool do_l2 = (any_l2 || nmode) && ntiles > 0;  // sort + lists (+ Level2, normals)
-  const bool csort = do_l2 && kmark;                   // lists by the counting sort
+  // Lists by the counting sort; with normals each voxel's triangles are then put in order, which pays
+  // while they are few a voxel (430k pairs of 53k voxels: 62 us against the radix sort's 202); lists of
+  // hundreds keep the radix sort, whose passes do not depend on their lengths
+  const bool csort = do_l2 && kmark && (nmode == 0 || P2 <= kSegSortAverage * ub);
   SortTile *d_tiles = nullptr;
   int64_t *d_tb = nullptr;
   uint32_t *kalt = nullptr, *valt = nullptr, *flags = nullptr, *uidx = nullptr, *useg = nullptr,
@@ -799,7 +806,7 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
     CK(ws.get(&kalt, (size_t)std::max<int64_t>(P2, 1)));
     CK(ws.get(&valt, (size_t)std::max<int64_t>(P2, 1)));
     CK(ws.get(&flags, (size_t)std::max<int64_t>(P2, ub)));  // the counting sort's counts too
-    CK(ws.get(&uidx, (size_t)P2));
+    CK(ws.get(&uidx, (size_t)std::max<int64_t>(P2, seg_sort_words(ub))));
     CK(ws.get(&useg, (size_t)ub + 1));
     CK(ws.get(&sortmp, (size_t)std::max({sort_seg_temp_words(ntiles), scan_temp_words(P2),
                                          scan_temp_words(ub)})));
@@ -851,13 +858,15 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
   // host outputs: recorded too when only page-locked Level1 copies ride along (direct Level2)
   const bool phase1_graph = !sink || (l2_direct && sink->l1_pinned && !packed);
   std::vector<uint64_t> sig1;
+  int max_cells = 0;
+  for (int m = 0; m < n; ++m) max_cells = std::max(max_cells, gh[m].level2 ? (int)gh[m].cells : 0);
   bool any_hier = false;
   for (int m = 0; m < n; ++m) any_hier = any_hier || res_hier[m + 1] > res_hier[m];
   bd_sig(sig1);
   for (uint64_t x : {(uint64_t)(uintptr_t)wpre, (uint64_t)do_l2, (uint64_t)(uintptr_t)d_tiles,
                      (uint64_t)(uintptr_t)d_tb, (uint64_t)ntiles, (uint64_t)(uintptr_t)keys,
                      (uint64_t)(uintptr_t)vals, (uint64_t)(uintptr_t)kalt, (uint64_t)(uintptr_t)valt,
-                     (uint64_t)P2, (uint64_t)max_keybits, (uint64_t)nmode, (uint64_t)val_bits,
+                     (uint64_t)P2, (uint64_t)max_keybits, (uint64_t)csort, (uint64_t)max_cells, (uint64_t)nmode, (uint64_t)val_bits,
                      (uint64_t)(uintptr_t)sortmp, (uint64_t)(uintptr_t)flags, (uint64_t)(uintptr_t)uidx,
                      (uint64_t)(uintptr_t)wtot, (uint64_t)(uintptr_t)useg, (uint64_t)any_l2,
                      (uint64_t)ub, (uint64_t)(uintptr_t)l2tmp, (uint64_t)l2_words.sat, (uint64_t)l2_words.fill,
@@ -907,6 +916,7 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
         // lists in any triangle order: counting sort by voxel rank, segment starts from its scan
         count_sort_pairs(bd, d_tiles, ntiles, keys, vals, wpre + words, ub, P2, flags, useg, kalt,
                          valt, wtot + 1, sortmp, s);
+        if (nmode) launch_seg_sort(valt, useg, ub, uidx, ctx->num_sms, s);
       } else {
         // normals sum in ascending triangle order: radix sort by (voxel, triangle)
         const bool in_alt = sort_pairs_seg(bd, d_tiles, d_tb, ntiles, keys, vals, kalt, valt, P2,
@@ -919,7 +929,7 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
       }
       mark(7);
       if (any_l2)
-        launch_level2(bd, sk, sv, useg, ub, l2tmp, l2_words, ctx->num_sms, s, [&] { mark(9); },
+        launch_level2(bd, sk, sv, useg, ub, l2tmp, level2_mask_words(ub, l2bytes), l2_words, ctx->num_sms, s, [&] { mark(9); },
                       zslab, nslab, [&](int k, cudaStream_t ls) {
                         if (packed) {  // the host expands this slab's codes once it is done
                           cudaEventRecord(ctx->cev[1 + k], ls);
@@ -938,7 +948,7 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
         mark(9);
       if (nmode) {
         launch_face_normals(bd, s);
-        launch_normals(bd, sk, sv, useg, ub, any_l2, ctx->num_sms, s);
+        launch_normals(bd, sk, sv, useg, ub, max_cells, ctx->num_sms, s);
       }
     } else {
       mark(7);

@@ -236,6 +236,10 @@ bool sort_pairs_seg(const BatchDev &bd, const SortTile *tiles, const int64_t *ti
 constexpr int kSortTileItems = 2048;
 
 int level2_chunk(const GridDev &g, int cap = 32);
+// Few boundary voxels (B of all meshes): the warps that share one item's SAT pairs, and the chunk
+// length of ch that still leaves every warp a few items.
+int level2_parts(int64_t B, int num_sms);
+int level2_few_chunk(int ch, int64_t B, int num_sms);
 struct Level2Words { int sat, fill; };  // shared-memory words per warp of the two Level2 kernels
 Level2Words level2_warp_words(const GridDev &g, int cap = 32, bool stencil = false);
 int64_t level2_temp_words(int64_t Btot);
@@ -251,16 +255,21 @@ struct SlabStreams {  // two streams and their events for overlapping slab launc
   cudaEvent_t fork, join[2];
 };
 void launch_level2(const BatchDev &bd, const uint32_t *keys, const uint32_t *vals,
-                   const uint32_t *useg, int64_t Btot, uint32_t *tmp, Level2Words words, int num_sms,
+                   const uint32_t *useg, int64_t Btot, uint32_t *tmp, int64_t smask_words, Level2Words words, int num_sms,
                    cudaStream_t s, const std::function<void()> &before_kernel = {}, int zslab = 0,
                    int nslab = 1, const std::function<void(int, cudaStream_t)> &after_slab = {},
                    int slab_nz = 0, const SlabStreams *aux = nullptr);
 
 // ---- normals (gpv_normals.cu) ----------------------------------------------------------------
 void launch_face_normals(const BatchDev &bd, cudaStream_t s);
-// Level1 normals of the U boundary voxels of the sorted meshes, then (any_l2) Level2 normals.
+// Each voxel's triangles of counting-sorted lists in ascending id; longs: seg_sort_words(U) words.
+int64_t seg_sort_words(int64_t U);
+void launch_seg_sort(uint32_t *vals, const uint32_t *useg, int64_t U, uint32_t *longs, int num_sms,
+                     cudaStream_t s);
+// Level1 normals of the U boundary voxels of the sorted meshes, then Level2 normals of the meshes with
+// a Level2 grid (max_cells cells per voxel at most, 0: none).
 void launch_normals(const BatchDev &bd, const uint32_t *keys, const uint32_t *vals,
-                    const uint32_t *useg, int64_t U, bool any_l2, int num_sms, cudaStream_t s);
+                    const uint32_t *useg, int64_t U, int max_cells, int num_sms, cudaStream_t s);
 
 // ---- voxel box hierarchy (gpv_hierarchy.cu) ----------------------------------------------------
 int hierarchy_levels(int64_t N1);  // 0 unless N1 is a power of two >= 2

@@ -19,13 +19,13 @@
 //   k_expand      .raw bytes of Level1, boundaryPrefixSum, boundaryIndex.
 //   sort / Level2 gpv_sort.cu, gpv_level2.cu.
 #include "gpv_internal.h"
+#include "gpv_rows.cuh"
 
 namespace gpv {
 
 namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
-constexpr float EPS24 = 5.9604644775390625e-08f;  // 2^-24
 
 __device__ __forceinline__ uint32_t pack2(int lo, int hi) {
   return (uint32_t)(lo & 0xffff) | ((uint32_t)(hi & 0xffff) << 16);
@@ -384,13 +384,6 @@ __device__ __forceinline__ int group_search(const uint32_t *off, uint32_t u) {
   for (int st = 16; st > 0; st >>= 1)
     if (off[lo + st] <= u) lo += st;
   return lo;
-}
-
-// 1/x to about an ulp (range arithmetic only, never inside a predicate).
-__device__ __forceinline__ float rcp_fast(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
 }
 
 struct L1Warp {
@@ -805,7 +798,7 @@ __global__ void __launch_bounds__(256) k_fill_finish(BatchDev bd) {
   }
   const int k = w * 32 + (int)lane;
   if (k < nz) d.iplane[((size_t)k * ny + j) * g.nxw + ig] = mine;
-  if (!bd.kmask || !d.has_l2) return;
+  if (!bd.kmask || !(d.has_l2 || bd.normals)) return;
   // the boundary plane transposed the other way, for the pair lists: 32 layers of 32 columns to one
   // word per column at the columns' place in key order
   const uint32_t bw = k < nz ? d.bplane[((size_t)k * ny + j) * g.nxw + ig] : 0u;

@@ -22,13 +22,13 @@
 //            voxels expands it) and one run of bits the voxel that holds the crossing.  Rays and
 //            crossings within the error bounds run the exact float tests.
 #include "gpv_internal.h"
+#include "gpv_rows.cuh"
 
 namespace gpv {
 
 namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
-constexpr float EPS24 = 5.9604644775390625e-08f;  // 2^-24
 constexpr int kWarps = 4;
 constexpr int kDirectCells = 4;  // a triangle whose box meets at most this many cells is tested exactly
 constexpr int kMaskWords = 512;  // words of one mask kind per warp (sets the chunk length)
@@ -48,95 +48,6 @@ __device__ __forceinline__ T warp_sum(T v) {
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(FULL, v, d);
   return v;
-}
-
-// 1/x to about an ulp (range arithmetic only, never inside a predicate).
-__device__ __forceinline__ float rcp_fast(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-__device__ __forceinline__ float ff(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-
-__device__ __forceinline__ uint32_t cvt_pair_ceil(float lo, float hi) {
-  short a, b;  // (the conversion saturates)
-  asm("cvt.rpi.s16.f32 %0, %1;" : "=h"(a) : "f"(lo));
-  asm("cvt.rpi.s16.f32 %0, %1;" : "=h"(b) : "f"(hi));
-  return (uint32_t)(uint16_t)a | ((uint32_t)(uint16_t)b << 16);
-}
-__device__ __forceinline__ uint32_t cvt_pair_floor(float lo, float hi) {
-  short a, b;
-  asm("cvt.rmi.s16.f32 %0, %1;" : "=h"(a) : "f"(lo));
-  asm("cvt.rmi.s16.f32 %0, %1;" : "=h"(b) : "f"(hi));
-  return (uint32_t)(uint16_t)a | ((uint32_t)(uint16_t)b << 16);
-}
-
-// ---- rows of a two-dimensional triangle / square test ----------------------------------------
-// The squares of half sizes (ha, hb) centred at ((i - base) ga, k gb); the triangle (a[], b[]).
-// An edge (ea, eb) separates where eb * a - ea * b of the edge (t, at the square) and of the opposite
-// vertex (t + S) both exceed rad = |eb| ha + |ea| hb or both lie below -rad, so it passes for
-//   t0 + k ea gb - rad + min(S, 0)  <=  (i - base) eb ga  <=  t0 + k ea gb + rad + max(S, 0),
-// t0 being t at (0, 0).  `dl` bounds the roundings of those sides and of what the float test compares
-// (see the callers), ta and tb the distance of the centre tables from their affine form; a slope below
-// 1/512 of the bound is replaced by it, which moves a side by at most 1/16 of it over 32 cells.  kIdx
-// covers the rounding of the index arithmetic (values up to 64 with a relative error of a few 2^-23).
-// Row k passes the edge's float test for every i in [lo + w2, hi - w2] and for none outside [lo, hi],
-// with lo and hi moving by s per row.
-constexpr float kIdx = 1.f / 16384.f;
-struct EdgeRows { float lo, hi, w2, s; };
-
-__device__ __forceinline__ EdgeRows edge_rows(float ea, float eb, float a, float b, float ha, float hb,
-                                              float ga, float gb, float sn, float sp, float dl,
-                                              float ta, float tb, float base) {
-  const float t = ff(eb, a, -(ea * b));
-  const float rad = ff(fabsf(eb), ha, fabsf(ea) * hb);
-  const float d = ff(fabsf(eb), ta, ff(fabsf(ea), tb, dl));
-  const float s = eb * ga;
-  const float inv = rcp_fast(copysignf(fmaxf(fabsf(s), d * (1.f / 512.f)), s));
-  const float x1 = (t - rad + sn) * inv, x2 = (t + rad + sp) * inv;
-  const float w = ff(d, fabsf(inv), kIdx);
-  return {fminf(x1, x2) - w + base, fmaxf(x1, x2) + w + base, 2.f * w, ea * gb * inv};
-}
-
-// Solves rows 0 .. n-1 into out[]: [lo_o, end_o) holds every i of the row that can pass, [lo_i, end_i)
-// only ones that do; one byte each, lo_o | lo_i << 8 | end_i << 16 | end_o << 24.  bl and be are the
-// i that can and that certainly pass the a axis' own test (lo_o | lo_i << 16 and end_i | end_o << 16),
-// and rows outside [in_lo, in_end) may fail the b axis' own: they pass nothing for certain.
-__device__ __forceinline__ void solve_rows(uint32_t *out, int n, float a0, float a1, float a2, float b0,
-                                           float b1, float b2, float ha, float hb, float ga, float gb,
-                                           float dl, float ta, float tb, int base, uint32_t bl,
-                                           uint32_t be, int in_lo, int in_end) {
-  const float e0a = a1 - a0, e0b = b1 - b0, e1a = a2 - a1, e1b = b2 - b1, e2a = a0 - a2, e2b = b0 - b2;
-  const float S = ff(e0b, e1a, -(e0a * e1b));
-  const float sn = fminf(S, 0.f), sp = fmaxf(S, 0.f), fb = (float)base;
-  const EdgeRows r0 = edge_rows(e0a, e0b, a0, b0, ha, hb, ga, gb, sn, sp, dl, ta, tb, fb);
-  const EdgeRows r1 = edge_rows(e1a, e1b, a1, b1, ha, hb, ga, gb, sn, sp, dl, ta, tb, fb);
-  const EdgeRows r2 = edge_rows(e2a, e2b, a2, b2, ha, hb, ga, gb, sn, sp, dl, ta, tb, fb);
-  float k = 0.f;
-#pragma unroll 1
-  for (int i = 0; i < n; ++i, k += 1.f) {
-    const float l0 = ff(k, r0.s, r0.lo), l1 = ff(k, r1.s, r1.lo), l2 = ff(k, r2.s, r2.lo);
-    const float h0 = ff(k, r0.s, r0.hi), h1 = ff(k, r1.s, r1.hi), h2 = ff(k, r2.s, r2.hi);
-    const float lo_o = fmaxf(l0, fmaxf(l1, l2)), hi_o = fminf(h0, fminf(h1, h2));
-    const float lo_i = fmaxf(l0 + r0.w2, fmaxf(l1 + r1.w2, l2 + r2.w2));
-    const float hi_i = fminf(h0 - r0.w2, fminf(h1 - r1.w2, h2 - r2.w2));
-    const uint32_t L = __vmins2(__vmaxs2(cvt_pair_ceil(lo_o, lo_i), bl), 0x00400040u);
-    uint32_t E = __vmaxs2(__vmins2(cvt_pair_floor(hi_i + 1.f, hi_o + 1.f), be), 0u);
-    if (i < in_lo || i >= in_end) E &= 0xffff0000u;
-    out[i] = __byte_perm(L, E, 0x6420);
-  }
-}
-
-// Cells of one axis whose boxes can meet [tmin, tmax] ([lo, hi]) and those that certainly do
-// ([in_lo, in_end)), by the SAT's own box-axis test; `md` (cells) bounds the distance of the centre
-// table from c0 + k * g2 and the roundings.
-__device__ __forceinline__ void cell_ranges(float tmin, float tmax, float c0, float inv_g2, int n2,
-                                            float md, int &lo, int &hi, int &in_lo, int &in_end) {
-  const float f0 = ff(tmin - c0, inv_g2, 0.5f), f1 = ff(tmax - c0, inv_g2, 0.5f);
-  lo = max(__float2int_rd(f0 - md), 0);
-  hi = min(__float2int_rd(f1 + md), n2 - 1);
-  in_lo = min(max(__float2int_rd(f0 + md), 0), n2);
-  in_end = max(min(__float2int_rd(f1 - md), n2 - 1), -1) + 1;
 }
 
 // Bits of one Level2 column (n2z cells along z) start at bit (q*n2x + p)*n2z of a voxel's mask.
@@ -768,13 +679,20 @@ __device__ __forceinline__ uint32_t queue_shift(WarpScratch &ws, uint32_t nrec) 
 
 // The next work item of a persistent launch (one ticket per warp): all items, or (z slabs) this
 // launch's slab of the slab-ordered item list.  False: none left.
+// With `parts` > 1 each item comes that many times, its `part` counted up.
 __device__ __forceinline__ bool next_item(uint32_t *ticket, const Item *__restrict__ items,
                                           const uint32_t *__restrict__ nitems, int slab,
                                           const uint32_t *__restrict__ ilist,
-                                          const uint32_t *__restrict__ ioff, Item &it) {
+                                          const uint32_t *__restrict__ ioff, uint32_t parts, Item &it,
+                                          uint32_t &part) {
   uint32_t tk = 0;
   if ((threadIdx.x & 31u) == 0) tk = atomicAdd(ticket, 1u);
   tk = __shfl_sync(FULL, tk, 0);
+  part = 0;
+  if (parts > 1) {
+    part = tk % parts;
+    tk /= parts;
+  }
   if (ilist) {
     const uint32_t i0 = ioff[slab];
     if (tk >= ioff[slab + 1] - i0) return false;
@@ -808,14 +726,15 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_sat(
     BatchDev bd, const uint32_t *__restrict__ keys, const uint32_t *__restrict__ vals,
     const uint32_t *__restrict__ useg, const Item *__restrict__ items,
     const uint32_t *__restrict__ nitems, int per_warp, int slab, const uint32_t *__restrict__ ilist,
-    const uint32_t *__restrict__ ioff) {
+    const uint32_t *__restrict__ ioff, int parts) {
   extern __shared__ uint32_t sm[];
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   WarpScratch &ws = *reinterpret_cast<WarpScratch *>(sm + (size_t)warp * per_warp);
   int *const kz = reinterpret_cast<int *>(&ws + 1);
   uint32_t *const sat = reinterpret_cast<uint32_t *>(kz + 32);
   Item it;
-  while (next_item(bd.queue + 1 + kSlabsMax + slab, items, nitems, slab, ilist, ioff, it)) {
+  uint32_t part;
+  while (next_item(bd.queue + 1 + kSlabsMax + slab, items, nitems, slab, ilist, ioff, (uint32_t)parts, it, part)) {
   const uint32_t ua = it.ua;
   const MeshDesc &d = bd.md[it.m_mesh >> 7];
   const GridDev &g = d.g;
@@ -846,7 +765,10 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_sat(
   uint32_t nrec = 0;
   {
     const float h0 = g.e2[0], h1 = g.e2[1], h2 = g.e2[2];
-    const uint32_t S0 = ws.seg[0], S1 = ws.seg[m];
+    // this part's share of the pairs
+    const uint32_t n0 = ws.seg[0], np_ = ws.seg[m] - n0;
+    const uint32_t S0 = n0 + (uint32_t)((uint64_t)np_ * part / (uint32_t)parts);
+    const uint32_t S1 = n0 + (uint32_t)((uint64_t)np_ * (part + 1) / (uint32_t)parts);
     uint32_t taken;  // pairs of a batch: 32, fewer where their rows would not fit
 #pragma unroll 1
     for (uint32_t b0 = S0; b0 < S1; b0 += taken) {
@@ -1025,7 +947,10 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_sat(
   // the masks out
   uint32_t *out = sat_words(bd, d, ua, W);
 #pragma unroll 1
-  for (int w = lane; w < m * W; w += 32) out[w] = sat[w];
+  for (int w = lane; w < m * W; w += 32) {
+    if (parts == 1) out[w] = sat[w];
+    else if (sat[w]) atomicOr(out + w, sat[w]);
+  }
   __syncwarp();
   }  // next item
 }
@@ -1037,14 +962,15 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_fill(
     BatchDev bd, const uint32_t *__restrict__ keys, const uint32_t *__restrict__ vals,
     const uint32_t *__restrict__ useg, const Item *__restrict__ items,
     const uint32_t *__restrict__ nitems, int per_warp, int slab, const uint32_t *__restrict__ ilist,
-    const uint32_t *__restrict__ ioff) {
+    const uint32_t *__restrict__ ioff, int) {
   extern __shared__ uint32_t sm[];
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   WarpScratch &ws = *reinterpret_cast<WarpScratch *>(sm + (size_t)warp * per_warp);
   int *const kz = reinterpret_cast<int *>(&ws + 1);
   uint32_t *const par = reinterpret_cast<uint32_t *>(kz + 32);
   Item it;
-  while (next_item(bd.queue + 1 + slab, items, nitems, slab, ilist, ioff, it)) {
+  uint32_t part;
+  while (next_item(bd.queue + 1 + slab, items, nitems, slab, ilist, ioff, 1u, it, part)) {
   const uint32_t ua = it.ua;
   const MeshDesc &d = bd.md[it.m_mesh >> 7];
   const GridDev &g = d.g;
@@ -1509,13 +1435,22 @@ Level2Words level2_warp_words(const GridDev &g, int cap, bool stencil) {
   return {base + CH * W, base + CH * W + CH * FW + (stencil ? 4 * CH * W + CH * FWS + FWS : 0)};
 }
 
+int level2_parts(int64_t B, int num_sms) {
+  const int64_t warps = (int64_t)num_sms * 24;
+  return (int)std::max<int64_t>(1, std::min<int64_t>(64, warps / std::max<int64_t>(4 * B, 1)));
+}
+int level2_few_chunk(int ch, int64_t B, int num_sms) {
+  const int64_t warps = (int64_t)num_sms * 24;
+  return (int)std::max<int64_t>(1, std::min<int64_t>(ch, ch * B / (4 * warps)));
+}
+
 size_t level2_smem_bytes(int warp_words) { return (size_t)warp_words * 4 * kWarps; }
 
 int64_t level2_temp_words(int64_t B) { return 10 * B + 16 + 2 * (kSlabsMax + 4) + scan_temp_words(B); }
 
 // Builds the chunk items from the sorted pair lists and runs the persistent Level2 kernel.
 void launch_level2(const BatchDev &bd, const uint32_t *keys, const uint32_t *vals,
-                   const uint32_t *useg, int64_t B, uint32_t *tmp, Level2Words words, int num_sms,
+                   const uint32_t *useg, int64_t B, uint32_t *tmp, int64_t smask_words, Level2Words words, int num_sms,
                    cudaStream_t s, const std::function<void()> &before_kernel, int zslab,
                    int nslab, const std::function<void(int, cudaStream_t)> &after_slab, int slab_nz,
                    const SlabStreams *aux) {
@@ -1547,7 +1482,7 @@ void launch_level2(const BatchDev &bd, const uint32_t *keys, const uint32_t *val
   using Kern = decltype(&k_level2c_sat);
   static bool attr_set[3] = {false, false, false};
   // a kernel's persistent grid (one-graph calls: B is a capacity, the queue ends the work)
-  auto grid_of = [&](Kern k, int kv, size_t smem) {
+  auto grid_of = [&](Kern k, int kv, size_t smem, int64_t jobs) {
     if (!attr_set[kv]) {
       cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
       attr_set[kv] = true;
@@ -1555,12 +1490,16 @@ void launch_level2(const BatchDev &bd, const uint32_t *keys, const uint32_t *val
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kWarps * 32, smem);
     const int64_t full = (int64_t)num_sms * std::max(per_sm, 1);
-    return (unsigned)(bd.plan ? full : std::min<int64_t>((B + kWarps - 1) / kWarps, full));
+    return (unsigned)(bd.plan ? full : std::min<int64_t>((jobs + kWarps - 1) / kWarps, full));
   };
+  // Few voxels (a coarse grid): several warps share an item's pairs, their masks OR-ed into cleared
+  // words.  42 voxels of 7k triangles: the SAT kernel 424 -> 17 us.
+  const int parts = level2_parts(B, num_sms);
+  if (parts > 1) cudaMemsetAsync(bd.smask, 0, (size_t)smask_words * sizeof(uint32_t), s);
   const Kern fill = st ? k_level2c_fill<true> : k_level2c_fill<false>;
   const size_t smem_sat = level2_smem_bytes(words.sat), smem_fill = level2_smem_bytes(words.fill);
-  const unsigned grid_sat = grid_of(k_level2c_sat, 0, smem_sat);
-  const unsigned grid_fill = grid_of(fill, st ? 2 : 1, smem_fill);
+  const unsigned grid_sat = grid_of(k_level2c_sat, 0, smem_sat, B * parts);
+  const unsigned grid_fill = grid_of(fill, st ? 2 : 1, smem_fill, B);
   const int nz = slab_nz;
   if (zslab > 0) {
     // single mesh: order the items by slab so that each launch takes only its own
@@ -1584,9 +1523,9 @@ void launch_level2(const BatchDev &bd, const uint32_t *keys, const uint32_t *val
     cudaStream_t ls = two ? aux->st[sl & 1] : s;
     const uint32_t *list = zslab > 0 ? ilist : nullptr;
     k_level2c_sat<<<grid_sat, kWarps * 32, smem_sat, ls>>>(bd, keys, vals, useg, items, nitems, words.sat,
-                                                          sl, list, ioff);
+                                                          sl, list, ioff, parts);
     fill<<<grid_fill, kWarps * 32, smem_fill, ls>>>(bd, keys, vals, useg, items, nitems, words.fill, sl,
-                                                    list, ioff);
+                                                    list, ioff, 1);
     count_launch(2);
     if (after_slab) after_slab(sl, ls);
   }

@@ -16,7 +16,10 @@
 // Outputs per mode: GPV_NORMALS_BYTES writes the .raw encoding uint8(n * float(256/3) + 127)
 // (src/Object.cpp:2940-2941, :3033-3035), three bytes per voxel / cell; GPV_NORMALS_FLOAT writes
 // the three floats.
+#include <algorithm>
+
 #include "gpv_internal.h"
+#include "gpv_rows.cuh"
 
 namespace gpv {
 
@@ -74,21 +77,62 @@ __global__ void __launch_bounds__(256) k_face_normals(BatchDev bd) {
   d.fnorm[t] = make_float4(x, y, z, 0.f);
 }
 
-// One thread per boundary voxel of the sorted meshes: sum in list order, average, normalise.
+// One thread per boundary voxel of the sorted meshes: sum in list order, average, normalise.  The
+// loads of a list of up to kThreadList triangles run kAhead at a time; longer lists are summed by the
+// whole warp, one after the other: a load per lane, the next ones under way, and the additions in
+// list order from the lanes.  A warp takes per_warp voxels, 32 or (few voxels) one.  (A dependent load per triangle was the whole cost where a voxel holds
+// hundreds: 217 us for 42 voxels of 7k triangles, now 56.)
+constexpr int kAhead = 8;
+constexpr uint32_t kThreadList = 64;
 __global__ void __launch_bounds__(256) k_level1_normals(BatchDev bd, const uint32_t *__restrict__ keys,
                                                         const uint32_t *__restrict__ vals,
-                                                        const uint32_t *__restrict__ useg, int64_t U) {
-  const int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (u >= U) return;
-  const MeshDesc &d = bd.md[mesh_by<&MeshDesc::u_base>(bd.md, bd.nmesh, u)];
-  const uint32_t e0 = useg[u], e1 = useg[u + 1];
+                                                        const uint32_t *__restrict__ useg, int64_t U,
+                                                        int per_warp) {
+  const unsigned lane = threadIdx.x & 31u;
+  const int64_t u = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per_warp + lane;
+  const bool live = (int)lane < per_warp && u < U;
+  const MeshDesc &d = bd.md[mesh_by<&MeshDesc::u_base>(bd.md, bd.nmesh, live ? u : U - 1)];
+  const float4 *__restrict__ fnorm = d.fnorm;
+  const uint32_t e0 = live ? useg[u] : 0u, e1 = live ? useg[u + 1] : 0u;
+  const bool is_long = e1 - e0 > kThreadList;
   float sx = 0.f, sy = 0.f, sz = 0.f;
-  for (uint32_t e = e0; e < e1; ++e) {
-    const float4 f = __ldg(d.fnorm + (vals[e] & 0x7fffffffu));
-    sx = fa(sx, f.x);
-    sy = fa(sy, f.y);
-    sz = fa(sz, f.z);
+  if (!is_long)
+    for (uint32_t e = e0; e < e1; e += kAhead) {
+      float4 f[kAhead];
+#pragma unroll
+      for (int k = 0; k < kAhead; ++k) f[k] = __ldg(fnorm + (vals[min(e + k, e1 - 1)] & 0x7fffffffu));
+#pragma unroll
+      for (int k = 0; k < kAhead; ++k)
+        if (e + k < e1) {
+          sx = fa(sx, f[k].x);
+          sy = fa(sy, f[k].y);
+          sz = fa(sz, f[k].z);
+        }
+    }
+  for (uint32_t todo = __ballot_sync(FULL, is_long); todo; todo &= todo - 1u) {
+    const int own = __ffs(todo) - 1;
+    const uint32_t a = __shfl_sync(FULL, e0, own), b = __shfl_sync(FULL, e1, own);
+    const float4 *fn = reinterpret_cast<const float4 *>(__shfl_sync(FULL, (unsigned long long)fnorm, own));
+    float x = 0.f, y = 0.f, z = 0.f;
+    float4 f = __ldg(fn + (vals[min(a + lane, b - 1)] & 0x7fffffffu));
+    for (uint32_t e = a; e < b; e += 32) {
+      const float4 cur = f;
+      if (e + 32 < b) f = __ldg(fn + (vals[min(e + 32 + lane, b - 1)] & 0x7fffffffu));
+      const int n = (int)min(b - e, 32u);
+#pragma unroll 4
+      for (int k = 0; k < n; ++k) {
+        x = fa(x, __shfl_sync(FULL, cur.x, k));
+        y = fa(y, __shfl_sync(FULL, cur.y, k));
+        z = fa(z, __shfl_sync(FULL, cur.z, k));
+      }
+    }
+    if ((int)lane == own) {
+      sx = x;
+      sy = y;
+      sz = z;
+    }
   }
+  if (!live) return;
   const float cnt = (float)(e1 - e0);
   float x = __fdiv_rn(sx, cnt), y = __fdiv_rn(sy, cnt), z = __fdiv_rn(sz, cnt);
   normalize3(x, y, z);
@@ -100,90 +144,420 @@ __global__ void __launch_bounds__(256) k_level1_normals(BatchDev bd, const uint3
   store_normal(d.l1n, bd.normals, vlin, x, y, z);
 }
 
-// One warp per boundary voxel of a Level2 mesh (grid-stride).  The voxel's cells are taken in
-// tiles of kNTileCells consecutive cells (cell order r, q, p); for each tile the voxel's triangles
-// run in list order, each one's candidate cells (the triangle's box, clipped to the tile's z
-// layers) tested by the exact SAT across the lanes and accumulated in shared memory (one triangle
-// at a time, so each cell's sum follows the list order).
+// ---- a voxel's triangles by id ------------------------------------------------------------------
+// The counting sort leaves each voxel's triangles in any order; their normals are summed in ascending
+// id.  One warp per voxel: up to 32 in registers, up to kSegWarp in its shared memory; longer lists
+// are noted for k_seg_sort_long.  (With a few triangles a voxel this replaces the radix sort of all
+// pairs by id and voxel: 430k pairs of 53k voxels, sort and lists 202 -> 62 us with the counting sort.)
+constexpr int kSegWarp = 512;
+constexpr int kSegBlock = 8192;
+constexpr uint32_t kIdMask = 0x7fffffffu;
+
+// Bitonic sort by id of n <= N values in shared memory (N a power of two; padded with kIdMask).
+template <typename Sync>
+__device__ __forceinline__ void bitonic_ids(uint32_t *v, int N, int t, int nt, Sync sync) {
+  for (int k = 2; k <= N; k <<= 1)
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      for (int i = t; i < N / 2; i += nt) {
+        const int lo = 2 * i - (i & (j - 1)), hi = lo + j;
+        const uint32_t a = v[lo], b = v[hi];
+        if (((a & kIdMask) > (b & kIdMask)) == ((lo & k) == 0)) {
+          v[lo] = b;
+          v[hi] = a;
+        }
+      }
+      sync();
+    }
+}
+
+__global__ void __launch_bounds__(kNWarps * 32) k_seg_sort(uint32_t *__restrict__ vals,
+                                                           const uint32_t *__restrict__ useg, int64_t U,
+                                                           uint32_t *__restrict__ longs) {
+  __shared__ uint32_t s_v[kNWarps][kSegWarp];
+  const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const int64_t u = (int64_t)blockIdx.x * kNWarps + warp;
+  if (u >= U) return;
+  const uint32_t e0 = useg[u], n = useg[u + 1] - e0;
+  if (n <= 1) return;
+  if (n <= 32) {
+    uint32_t v = lane < n ? vals[e0 + lane] : kIdMask;
+#pragma unroll
+    for (int k = 2; k <= 32; k <<= 1)
+#pragma unroll
+      for (int j = k >> 1; j > 0; j >>= 1) {
+        const uint32_t o = __shfl_xor_sync(FULL, v, j);
+        const bool up = (lane & k) == 0, low = (lane & j) == 0;
+        if (((v & kIdMask) > (o & kIdMask)) == (up == low) && (v & kIdMask) != (o & kIdMask)) v = o;
+      }
+    if (lane < n) vals[e0 + lane] = v;
+    return;
+  }
+  if (n > (uint32_t)kSegWarp) {
+    if (lane == 0) longs[1 + atomicAdd(longs, 1u)] = (uint32_t)u;
+    return;
+  }
+  int N = 64;
+  while ((uint32_t)N < n) N <<= 1;
+  uint32_t *v = s_v[warp];
+  for (int i = lane; i < N; i += 32) v[i] = (uint32_t)i < n ? vals[e0 + i] : kIdMask;
+  __syncwarp();
+  bitonic_ids(v, N, (int)lane, 32, [] { __syncwarp(); });
+  for (uint32_t i = lane; i < n; i += 32) vals[e0 + i] = v[i];
+}
+
+// The noted lists, a block each: in shared memory up to kSegBlock, longer ones in place with the
+// same network over the next power of two (indices past the end hold the largest id: a swap that
+// would move one down cannot happen, since the partner is never larger).
+__global__ void __launch_bounds__(1024) k_seg_sort_long(uint32_t *__restrict__ vals,
+                                                        const uint32_t *__restrict__ useg,
+                                                        const uint32_t *__restrict__ longs) {
+  extern __shared__ uint32_t s_long[];
+  const uint32_t nl = longs[0];
+  for (uint32_t l = blockIdx.x; l < nl; l += gridDim.x) {
+    const uint32_t u = longs[1 + l], e0 = useg[u], n = useg[u + 1] - e0;
+    int N = 1024;
+    while ((uint32_t)N < n) N <<= 1;
+    if (n <= (uint32_t)kSegBlock) {
+      for (int i = threadIdx.x; i < N; i += 1024) s_long[i] = (uint32_t)i < n ? vals[e0 + i] : kIdMask;
+      __syncthreads();
+      bitonic_ids(s_long, N, (int)threadIdx.x, 1024, [] { __syncthreads(); });
+      for (uint32_t i = threadIdx.x; i < n; i += 1024) vals[e0 + i] = s_long[i];
+    } else {
+      // all comparisons ascending (each merge starts with a mirrored step), so that the missing
+      // largest ids stay at the end
+      uint32_t *v = vals + e0;
+      for (int64_t k = 2; k <= N; k <<= 1)
+        for (int64_t j = k >> 1; j > 0; j >>= 1) {
+          for (int64_t i = threadIdx.x; i < N / 2; i += 1024) {
+            const int64_t lo = 2 * i - (i & (j - 1));
+            const int64_t hi = j == (k >> 1) ? (lo | (k - 1)) - (lo & (k - 1)) : lo + j;
+            if (hi < n) {
+              const uint32_t a = v[lo], b = v[hi];
+              if ((a & kIdMask) > (b & kIdMask)) {
+                v[lo] = b;
+                v[hi] = a;
+              }
+            }
+          }
+          __syncthreads();
+        }
+    }
+    __syncthreads();
+  }
+}
+
+// One warp per (boundary voxel, tile of at most `tile` consecutive cells in output order).  The voxel's
+// triangles run in list order, 32 at a time: a lane each solves its rows of cells (gpv_rows.cuh), then,
+// one triangle at a time, the lanes take its sub-columns, whose cells are the run between the rows' and
+// the plane's bounds, with the exact SAT where those leave a cell open.  Each cell's sum is kept in
+// shared memory and takes its triangles in list order.  (Testing every candidate cell of every
+// triangle exactly, one triangle after the other, took 561 us on 430k pairs of 53k voxels at 8^3 and
+// 1271 us on 7k triangles in 42 voxels at 4^3; this 360 and 317.)  Bound by instruction issue on the
+// former, by the latency of the ordered sums on the latter.
+constexpr int kFewCells = 4;  // a triangle whose box meets at most this many cells is tested exactly
+constexpr int kNSol = 384;  // solved rows of one batch (a triangle has at most 96)
+
+struct NWarp {
+  float4 acc[kNTileCells];
+  float x[32][9];
+  uint32_t px[32], qy[32], rz[32];  // first, count of the triangle's sub-columns, rows; cell range
+  uint32_t so[32];                  // its solved rows; ~0: exact tests only; bit 30: its few cells'
+                                    // exact results (bit i: cell i of its box, x fastest)
+  uint32_t tri[32];
+  uint32_t que[64];                 // queued triangles that meet the tile, in list order
+  uint32_t sol[kNSol];
+};
+
 __global__ void __launch_bounds__(kNWarps * 32) k_level2_normals(BatchDev bd,
                                                                  const uint32_t *__restrict__ keys,
                                                                  const uint32_t *__restrict__ vals,
                                                                  const uint32_t *__restrict__ useg,
-                                                                 int64_t U) {
-  __shared__ float4 s_acc[kNWarps][kNTileCells];
-  const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  float4 *acc = s_acc[warp];
+                                                                 int64_t U, int tile, int max_tiles) {
+  extern __shared__ __align__(16) unsigned char s_raw[];
+  const int lane = (int)(threadIdx.x & 31u);
+  NWarp &ws = reinterpret_cast<NWarp *>(s_raw)[threadIdx.x >> 5];
+  float4 *acc = ws.acc;
   const int64_t nwarps = (int64_t)gridDim.x * kNWarps;
-  for (int64_t u = (int64_t)blockIdx.x * kNWarps + warp; u < U; u += nwarps) {
+  for (int64_t job = (int64_t)blockIdx.x * kNWarps + (threadIdx.x >> 5); job < U * max_tiles; job += nwarps) {
+    const int64_t u = job / max_tiles;
     const MeshDesc &d = bd.md[mesh_by<&MeshDesc::u_base>(bd.md, bd.nmesh, u)];
     if (!d.has_l2) continue;  // warp-uniform
     const GridDev &g = d.g;
     const int nx = g.n[0], nz = g.n[2];
     const int n2x = g.n2[0], n2y = g.n2[1], n2z = g.n2[2];
     const int ncol2 = n2x * n2y, cells = ncol2 * n2z;
+    const int c0 = (int)(job - u * max_tiles) * tile;
+    if (c0 >= cells) continue;
+    const int c1 = min(cells, c0 + tile), tc = c1 - c0;
+    const int rz0 = c0 / ncol2, rz1 = (c1 - 1) / ncol2;
+    // rows of the tile (all of them unless it lies in one layer)
+    const int ty0 = rz0 == rz1 ? (c0 - rz0 * ncol2) / n2x : 0;
+    const int ty1 = rz0 == rz1 ? (c1 - 1 - rz0 * ncol2) / n2x : n2y - 1;
     const uint32_t e0 = useg[u], e1 = useg[u + 1];
     const uint32_t key = keys[e0];
     const uint32_t col = key / (uint32_t)nz;
     const int k = (int)(key - col * (uint32_t)nz);
     const int ci = (int)(col % (uint32_t)nx), cj = (int)(col / (uint32_t)nx);
     const int64_t vlin = ((int64_t)k * g.n[1] + cj) * nx + ci;
-    const int64_t obase = (int64_t)d.prefix[vlin] * cells;
+    const int64_t obase = (int64_t)d.prefix[vlin] * cells + c0;
     const float *sx = g.c2s[0] + (size_t)ci * n2x, *sy = g.c2s[1] + (size_t)cj * n2y,
                 *szt = g.c2s[2] + (size_t)k * n2z;
     const float sx0 = __ldg(sx), sy0 = __ldg(sy), sz0 = __ldg(szt);
-    for (int c0 = 0; c0 < cells; c0 += kNTileCells) {
-      const int c1 = min(cells, c0 + kNTileCells), tc = c1 - c0;
-      const int rz0 = c0 / ncol2, rz1 = (c1 - 1) / ncol2;
-      for (int c = lane; c < tc; c += 32) acc[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float h0 = g.e2[0], h1 = g.e2[1], h2 = g.e2[2], gx = g.g2[0], gy = g.g2[1], gz = g.g2[2];
+    // (the bounds' constants as in the Level2 SAT, gpv_level2.cu)
+    const float tx = 2.02f * EPS24 * fmaxf(fabsf(sx0), fabsf(__ldg(sx + n2x - 1)));
+    const float ty = 2.02f * EPS24 * fmaxf(fabsf(sy0), fabsf(__ldg(sy + n2y - 1)));
+    const float tz = 2.02f * EPS24 * fmaxf(fabsf(sz0), fabsf(__ldg(szt + n2z - 1)));
+    for (int c = lane; c < tc; c += 32) acc[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+    __syncwarp();
+    // Where the tile is the voxel every triangle is taken; otherwise those that meet its layers and
+    // rows are queued first, so that the lanes are full.
+    const bool all = tc == cells;
+    uint32_t nq_ = 0, scan = e0;  // queued triangles, the next list entry to look at
+    uint32_t taken;
+    for (;;) {
+      if (all) nq_ = min(e1 - scan, 32u);
+      while (!all && nq_ < 32 && scan < e1) {
+        const uint32_t e = scan + (uint32_t)lane;
+        bool keep = e < e1;
+        uint32_t id = 0;
+        if (keep) {
+          id = vals[e] & 0x7fffffffu;
+          {
+            const float4 v0 = __ldg(d.ptri + 3 * (size_t)id), v1 = __ldg(d.ptri + 3 * (size_t)id + 1),
+                         v2 = __ldg(d.ptri + 3 * (size_t)id + 2);
+            int a, b, x, y;
+            cell_ranges(fminf(v0.z, fminf(v1.z, v2.z)), fmaxf(v0.z, fmaxf(v1.z, v2.z)), sz0, g.inv_g2[2], n2z,
+                        ff(tz, g.inv_g2[2], kIdx), a, b, x, y);
+            keep = max(a, rz0) <= min(b, rz1);
+            cell_ranges(fminf(v0.y, fminf(v1.y, v2.y)), fmaxf(v0.y, fmaxf(v1.y, v2.y)), sy0, g.inv_g2[1], n2y,
+                        ff(ty, g.inv_g2[1], kIdx), a, b, x, y);
+            keep = keep && max(a, ty0) <= min(b, ty1);
+          }
+        }
+        const uint32_t bal = __ballot_sync(FULL, keep);
+        if (keep) ws.que[nq_ + __popc(bal & ((1u << lane) - 1u))] = id;
+        nq_ += (uint32_t)__popc(bal);
+        scan += 32;
+        __syncwarp();
+      }
+      if (!nq_) break;
+      int p0 = 0, p1 = -1, pi = 0, pe = 0, q0 = 0, q1 = -1, qi = 0, qe = 0, r0 = 0, r1 = -1, ri = 0, re = 0;
+      uint32_t t = 0, nsolve = 0;
+      float4 a0, a1, a2;
+      float R = 0.f;
+      bool on = false, direct = false, few = false;
+      if (lane < (int)min(nq_, 32u)) {
+        t = all ? vals[scan + lane] & 0x7fffffffu : ws.que[lane];
+        a0 = __ldg(d.ptri + 3 * (size_t)t), a1 = __ldg(d.ptri + 3 * (size_t)t + 1),
+        a2 = __ldg(d.ptri + 3 * (size_t)t + 2);
+        const float xn = fminf(a0.x, fminf(a1.x, a2.x)), xx = fmaxf(a0.x, fmaxf(a1.x, a2.x));
+        const float yn = fminf(a0.y, fminf(a1.y, a2.y)), yx = fmaxf(a0.y, fmaxf(a1.y, a2.y));
+        const float zn = fminf(a0.z, fminf(a1.z, a2.z)), zx = fmaxf(a0.z, fmaxf(a1.z, a2.z));
+        cell_ranges(xn, xx, sx0, g.inv_g2[0], n2x, ff(tx, g.inv_g2[0], kIdx), p0, p1, pi, pe);
+        cell_ranges(yn, yx, sy0, g.inv_g2[1], n2y, ff(ty, g.inv_g2[1], kIdx), q0, q1, qi, qe);
+        cell_ranges(zn, zx, sz0, g.inv_g2[2], n2z, ff(tz, g.inv_g2[2], kIdx), r0, r1, ri, re);
+        on = p0 <= p1 && max(q0, ty0) <= min(q1, ty1) && max(r0, rz0) <= min(r1, rz1);
+        if (on) {
+          const int np = p1 - p0 + 1, nq = q1 - q0 + 1;
+          R = 1.0001f * fmaxf(xx - xn + 1.25f * gx + 2.f * tx,
+                              fmaxf(yx - yn + 1.25f * gy + 2.f * ty, zx - zn + 1.25f * gz + 2.f * tz));
+          few = np * nq * (r1 - r0 + 1) <= kFewCells;
+          direct = few || !(R > 1e-9f && R < 1e9f);
+          nsolve = direct ? 0u : (uint32_t)(2 * nq + np);
+        }
+      }
+      uint32_t is = nsolve;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(FULL, is, o);
+        if (lane >= o) is += v;
+      }
+      taken = (uint32_t)__popc(__ballot_sync(FULL, lane < (int)min(nq_, 32u) && is <= (uint32_t)kNSol));
+      if (lane < (int)taken && on) {
+        const int np = p1 - p0 + 1, nq = q1 - q0 + 1;
+        ws.px[lane] = (uint32_t)(p0 | (np << 8));
+        ws.qy[lane] = (uint32_t)(q0 | (nq << 8));
+        ws.rz[lane] = (uint32_t)(r0 | ((r1 + 1) << 8));
+        ws.tri[lane] = t;
+        ws.so[lane] = direct ? ~0u : is - nsolve;
+        if (few) {
+          // a lane per triangle here: one after the other, a triangle's test would wait for itself
+          const float V[9] = {a0.x, a0.y, a0.z, a1.x, a1.y, a1.z, a2.x, a2.y, a2.z};
+          const float h[3] = {h0, h1, h2};
+          uint32_t bits = 0;
+          int i = 0;
+          for (int r = r0; r <= r1; ++r)
+            for (int q = q0; q <= q1; ++q)
+              for (int p = p0; p <= p1; ++p, ++i) {
+                const float c3[3] = {__ldg(sx + p), __ldg(sy + q), __ldg(szt + r)};
+                if (tri_box(V, c3, h)) bits |= 1u << i;
+              }
+          ws.so[lane] = 0x40000000u | bits;
+        }
+        if (!direct) {
+          const float c0x = __ldg(sx + p0), c0y = __ldg(sy + q0), c0z = __ldg(szt + r0);
+          const float ux = a0.x - c0x, uy = a0.y - c0y, uz = a0.z - c0z;
+          const float vx = a1.x - c0x, vy = a1.y - c0y, vz = a1.z - c0z;
+          const float wx = a2.x - c0x, wy = a2.y - c0y, wz = a2.z - c0z;
+          float nnx = (vy - uy) * (wz - vz) - (vz - uz) * (wy - vy);
+          float nny = (vz - uz) * (wx - vx) - (vx - ux) * (wz - vz);
+          float nnz = (vx - ux) * (wy - vy) - (vy - uy) * (wx - vx);
+          if (nnz < 0.f) { nnx = -nnx; nny = -nny; nnz = -nnz; }
+          const float E = 192.f * EPS24 * R * R * (R + fmaxf(h0, fmaxf(h1, h2))) +
+                          1.1f * (fabsf(nnx) * tx + fabsf(nny) * ty + nnz * tz);
+          const float inv = rcp_fast(fmaxf(nnz * gz, E * (1.f / 512.f)));
+          const float w = ff(E, inv, kIdx);
+          ws.x[lane][0] = nnx * ux + nny * uy + nnz * uz;
+          ws.x[lane][1] = nnx * gx;
+          ws.x[lane][2] = nny * gy;
+          ws.x[lane][3] = fabsf(nnx) * h0 + fabsf(nny) * h1 + nnz * h2;
+          ws.x[lane][4] = inv;
+          ws.x[lane][5] = (float)r0 - w;
+          ws.x[lane][6] = (float)r0 + w;
+          const float dl = 72.f * EPS24 * R * R, bx = 1.1f * tx, by = 1.1f * ty, bz = 1.1f * tz;
+          uint32_t *so = ws.sol + (is - nsolve);
+          const uint32_t xl = (uint32_t)(p0 | (pi << 16)), xe = (uint32_t)(pe | ((p1 + 1) << 16));
+          const uint32_t zl = (uint32_t)(r0 | (ri << 16)), ze = (uint32_t)(re | ((r1 + 1) << 16));
+          solve_rows(so, nq, ux, vx, wx, uy, vy, wy, h0, h1, gx, gy, dl, bx, by, p0, xl, xe, qi - q0, qe - q0);
+          solve_rows(so + nq, nq, uz, vz, wz, uy, vy, wy, h2, h1, gz, gy, dl, bz, by, r0, zl, ze, qi - q0, qe - q0);
+          solve_rows(so + 2 * nq, np, uz, vz, wz, ux, vx, wx, h2, h0, gz, gx, dl, bz, bx, r0, zl, ze, pi - p0, pe - p0);
+        }
+      }
+      uint32_t left = __ballot_sync(FULL, lane < (int)taken && on);
       __syncwarp();
-      for (uint32_t e = e0; e < e1; ++e) {
-        const uint32_t t = vals[e] & 0x7fffffffu;
-        const float4 a0 = __ldg(d.ptri + 3 * (size_t)t), a1 = __ldg(d.ptri + 3 * (size_t)t + 1),
-                     a2 = __ldg(d.ptri + 3 * (size_t)t + 2);
-        const float V[9] = {a0.x, a0.y, a0.z, a1.x, a1.y, a1.z, a2.x, a2.y, a2.z};
-        const float4 fnv = __ldg(d.fnorm + t);
-        int p0, p1, q0, q1, r0, r1;
-        l2_cell_range(fminf(V[0], fminf(V[3], V[6])), fmaxf(V[0], fmaxf(V[3], V[6])), sx0,
-                      g.e2[0], g.inv_g2[0], n2x, p0, p1);
-        l2_cell_range(fminf(V[1], fminf(V[4], V[7])), fmaxf(V[1], fmaxf(V[4], V[7])), sy0,
-                      g.e2[1], g.inv_g2[1], n2y, q0, q1);
-        l2_cell_range(fminf(V[2], fminf(V[5], V[8])), fmaxf(V[2], fmaxf(V[5], V[8])), sz0,
-                      g.e2[2], g.inv_g2[2], n2z, r0, r1);
-        r0 = max(r0, rz0);
-        r1 = min(r1, rz1);
-        const int np = p1 - p0 + 1, nq = q1 - q0 + 1, nr = r1 - r0 + 1;
-        if (np > 0 && nq > 0 && nr > 0) {
-          const int tot = np * nq * nr;
-          for (int w = lane; w < tot; w += 32) {
-            const int pr = w / np, p = p0 + (w - pr * np);
-            const int qq = pr / nr, r = r0 + (pr - qq * nr), q = q0 + qq;
+      // ---- the triangles in list order
+      while (left) {
+        const int tl = __ffs(left) - 1;
+        left &= left - 1u;
+        const uint32_t px = ws.px[tl], qy = ws.qy[tl], rz = ws.rz[tl], so = ws.so[tl];
+        const int tp0 = (int)(px & 255u), np = (int)(px >> 8), tq0 = (int)(qy & 255u), nq = (int)(qy >> 8);
+        const float4 fnv = __ldg(d.fnorm + ws.tri[tl]);
+        if ((so >> 30) == 1u) {
+          const int box = np * nq, r = lane / box, pq = lane - r * box, q = pq / np;
+          const int c = ((int)(rz & 255u) + r) * ncol2 + (tq0 + q) * n2x + tp0 + (pq - q * np);
+          if (lane < kFewCells && ((so >> lane) & 1u) && c >= c0 && c < c1) {
+            float4 &a = acc[c - c0];
+            a.x = fa(a.x, fnv.x);
+            a.y = fa(a.y, fnv.y);
+            a.z = fa(a.z, fnv.z);
+            a.w = fa(a.w, 1.f);
+          }
+          __syncwarp();
+          continue;
+        }
+        const float rnp = rcp_fast((float)np);
+        for (int w = lane; w < np * nq; w += 32) {
+          // (w + 1/2) / np stays at least 1/64 away from an integer, far above the rounding
+          const int dq = __float2int_rz(((float)w + 0.5f) * rnp), dp = w - dq * np;
+          const int p = tp0 + dp, q = tq0 + dq;
+          int lo = (int)(rz & 255u), end = (int)(rz >> 8);
+          bool exact = true;
+          if (so != ~0u) {
+            const uint32_t sxy = ws.sol[so + dq];
+            if (p < (int)(sxy & 255u) || p >= (int)(sxy >> 24)) continue;
+            const uint32_t syz = ws.sol[so + nq + dq], sxz = ws.sol[so + 2 * nq + dp];
+            const float nv = ff(-(float)dp, ws.x[tl][1], ff(-(float)dq, ws.x[tl][2], ws.x[tl][0]));
+            const float va = nv - ws.x[tl][3], vb = nv + ws.x[tl][3], inv = ws.x[tl][4], k1 = ws.x[tl][5], k2 = ws.x[tl][6];
+            const uint32_t L = __vimax3_s16x2(cvt_pair_ceil(ff(va, inv, k1), ff(va, inv, k2)),
+                                              __byte_perm(syz, 0, 0x4140), __byte_perm(sxz, 0, 0x4140));
+            const uint32_t E = __vimin3_s16x2(cvt_pair_floor(ff(vb, inv, k1 + 1.f), ff(vb, inv, k2 + 1.f)),
+                                              __byte_perm(syz, 0, 0x4342), __byte_perm(sxz, 0, 0x4342));
+            lo = (int)(short)(L & 0xffffu);
+            end = (int)E >> 16;
+            exact = !(p >= (int)((sxy >> 8) & 255u) && p < (int)((sxy >> 16) & 255u) && lo == (int)L >> 16 &&
+                      end == (int)(short)(E & 0xffffu));
+          }
+          lo = max(lo, rz0);
+          end = min(end, rz1 + 1);
+          if (lo >= end) continue;
+          float V[9];
+          SatCol sc;
+          if (exact) {
+            const uint32_t tt = ws.tri[tl];
+            const float4 v0 = __ldg(d.ptri + 3 * (size_t)tt), v1 = __ldg(d.ptri + 3 * (size_t)tt + 1),
+                         v2 = __ldg(d.ptri + 3 * (size_t)tt + 2);
+            V[0] = v0.x; V[1] = v0.y; V[2] = v0.z; V[3] = v1.x; V[4] = v1.y; V[5] = v1.z;
+            V[6] = v2.x; V[7] = v2.y; V[8] = v2.z;
+            const float h[3] = {h0, h1, h2};
+            if (!sat_col(V, __ldg(sx + p), __ldg(sy + q), h, sc)) continue;
+          }
+          for (int r = lo; r < end; ++r) {
             const int c = r * ncol2 + q * n2x + p;
             if (c < c0 || c >= c1) continue;
-            const float c3[3] = {__ldg(sx + p), __ldg(sy + q), __ldg(szt + r)};
-            if (tri_box(V, c3, g.e2)) {
-              float4 &a = acc[c - c0];
-              a.x = fa(a.x, fnv.x);
-              a.y = fa(a.y, fnv.y);
-              a.z = fa(a.z, fnv.z);
-              a.w = fa(a.w, 1.f);
+            if (exact) {
+              const float h[3] = {h0, h1, h2};
+              if (!sat_z(sc, V, __ldg(szt + r), h)) continue;
             }
+            float4 &a = acc[c - c0];
+            a.x = fa(a.x, fnv.x);
+            a.y = fa(a.y, fnv.y);
+            a.z = fa(a.z, fnv.z);
+            a.w = fa(a.w, 1.f);
           }
         }
         __syncwarp();
       }
-      for (int c = lane; c < tc; c += 32) {
-        const float4 a = acc[c];
-        float x = 0.f, y = 0.f, z = 0.f;
-        if (a.w > 0.f) {
-          x = __fdiv_rn(a.x, a.w);
-          y = __fdiv_rn(a.y, a.w);
-          z = __fdiv_rn(a.z, a.w);
-          normalize3(x, y, z);
-        }
-        store_normal(d.l2n, bd.normals, obase + c0 + c, x, y, z);
+      if (all) {
+        scan += taken;
+        continue;
       }
+      // the queue's rest to its front
+      const uint32_t i0 = (uint32_t)lane + taken, i1 = i0 + 32;
+      const uint32_t k0 = i0 < nq_ ? ws.que[i0] : 0u, k1 = i1 < nq_ ? ws.que[i1] : 0u;
+      __syncwarp();
+      if (i0 < nq_) ws.que[lane] = k0;
+      if (i1 < nq_) ws.que[lane + 32] = k1;
+      nq_ -= taken;
       __syncwarp();
     }
+    // ---- averages of the cells with a triangle (about one in seven), 32 at a time
+    uint32_t nhit = 0;  // queued cells, in `sol`
+    auto finish = [&](uint32_t n) {
+      if (lane < (int)n) {
+        float4 &a = acc[ws.sol[lane]];
+        float x = __fdiv_rn(a.x, a.w), y = __fdiv_rn(a.y, a.w), z = __fdiv_rn(a.z, a.w);
+        normalize3(x, y, z);
+        a.x = x;
+        a.y = y;
+        a.z = z;
+      }
+      __syncwarp();
+    };
+    for (int cb = 0; cb < tc; cb += 32) {
+      const int c = cb + lane;
+      const bool hit = c < tc && acc[c].w > 0.f;
+      const uint32_t bal = __ballot_sync(FULL, hit);
+      if (hit) ws.sol[nhit + __popc(bal & ((1u << lane) - 1u))] = (uint32_t)c;
+      nhit += (uint32_t)__popc(bal);
+      __syncwarp();
+      const bool last = cb + 32 >= tc;
+      while (nhit >= 32 || (last && nhit)) {
+        const uint32_t n = min(nhit, 32u);
+        finish(n);
+        const uint32_t rest = (uint32_t)lane + n < nhit ? ws.sol[lane + n] : 0u;
+        __syncwarp();
+        if ((uint32_t)lane + n < nhit) ws.sol[lane] = rest;
+        nhit -= n;
+        __syncwarp();
+      }
+    }
+    // ---- out, consecutive values by consecutive lanes
+    if (bd.normals == GPV_NORMALS_FLOAT) {
+      float *o = static_cast<float *>(d.l2n) + 3 * obase;
+      for (int i = lane; i < 3 * tc; i += 32) {
+        const int c = i / 3;
+        __stcs(o + i, reinterpret_cast<const float *>(acc + c)[i - 3 * c]);
+      }
+    } else {
+      const float sc = (float)(256.0 / 3.0);
+      uint8_t *o = static_cast<uint8_t *>(d.l2n) + 3 * obase;
+      for (int i = lane; i < 3 * tc; i += 32) {
+        const int c = i / 3;
+        o[i] = (uint8_t)__float2int_rz(fa(fm(reinterpret_cast<const float *>(acc + c)[i - 3 * c], sc), 127.f));
+      }
+    }
+    __syncwarp();
   }
 }
 
@@ -195,14 +569,43 @@ void launch_face_normals(const BatchDev &bd, cudaStream_t s) {
   count_launch();
 }
 
-void launch_normals(const BatchDev &bd, const uint32_t *keys, const uint32_t *vals,
-                    const uint32_t *useg, int64_t U, bool any_l2, int num_sms, cudaStream_t s) {
+int64_t seg_sort_words(int64_t U) { return U + 1; }
+
+void launch_seg_sort(uint32_t *vals, const uint32_t *useg, int64_t U, uint32_t *longs, int num_sms,
+                     cudaStream_t s) {
   if (U <= 0) return;
-  k_level1_normals<<<(unsigned)((U + 255) / 256), 256, 0, s>>>(bd, keys, vals, useg, U);
+  cudaMemsetAsync(longs, 0, sizeof(uint32_t), s);
+  k_seg_sort<<<(unsigned)((U + kNWarps - 1) / kNWarps), kNWarps * 32, 0, s>>>(vals, useg, U, longs);
+  k_seg_sort_long<<<(unsigned)std::min<int64_t>(U, num_sms), 1024, kSegBlock * sizeof(uint32_t), s>>>(vals, useg,
+                                                                                                   longs);
+  count_launch(2);
+}
+
+void launch_normals(const BatchDev &bd, const uint32_t *keys, const uint32_t *vals,
+                    const uint32_t *useg, int64_t U, int max_cells, int num_sms, cudaStream_t s) {
+  if (U <= 0) return;
+  const int per_warp = U < (int64_t)num_sms * 32 ? 1 : 32;
+  k_level1_normals<<<(unsigned)((U + 4 * per_warp - 1) / (4 * per_warp)), 128, 0, s>>>(bd, keys, vals, useg, U,
+                                                                                     per_warp);
   count_launch();
-  if (!any_l2) return;
-  const int64_t grid = std::min<int64_t>((U + kNWarps - 1) / kNWarps, (int64_t)num_sms * 8);
-  k_level2_normals<<<(unsigned)grid, kNWarps * 32, 0, s>>>(bd, keys, vals, useg, U);
+  if (max_cells <= 0) return;
+  const size_t smem = kNWarps * sizeof(NWarp);
+  static bool attr_set = false;
+  if (!attr_set) {
+    cudaFuncSetAttribute(k_level2_normals, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    attr_set = true;
+  }
+  int per_sm = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_level2_normals, kNWarps * 32, smem);
+  const int64_t warps = (int64_t)num_sms * std::max(per_sm, 1) * kNWarps;
+  // Few voxels (a coarse grid with long lists): smaller tiles, so that every SM has warps.  A warp
+  // walks its voxel's whole list, but only the triangles that meet its tile's layers and rows cost more
+  // than their ranges.
+  int tile = std::min(kNTileCells, std::max(max_cells, 1));
+  while (tile > 4 && U * ((max_cells + tile - 1) / tile) < warps) tile = (tile + 1) / 2;
+  const int tiles = (max_cells + tile - 1) / tile;
+  const int64_t grid = std::min<int64_t>((U * tiles + kNWarps - 1) / kNWarps, (int64_t)num_sms * std::max(per_sm, 1));
+  k_level2_normals<<<(unsigned)grid, kNWarps * 32, smem, s>>>(bd, keys, vals, useg, U, tile, tiles);
   count_launch();
 }
 
