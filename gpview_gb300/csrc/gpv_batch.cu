@@ -243,7 +243,7 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
   std::vector<int64_t> tab_off(n + 1, 0), res_l1(n + 1, 0), res_pre(n + 1, 0), res_l1n(n + 1, 0),
       res_hier(n + 1, 0);
   std::vector<MeshDesc> md(n);
-  int64_t tris = 0, tiles = 0, fwarps = 0, rows = 0, xchunks = 0, words = 0, togg = 0, stgw = 0;
+  int64_t tris = 0, tiles = 0, fblks = 0, rows = 0, xchunks = 0, words = 0, togg = 0, stgw = 0;
   int max_keybits = 1;
   Level2Words l2_words = {0, 0};
   int64_t max_T = 1;
@@ -255,13 +255,13 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
     d.T = T[m];
     d.tri_base = tris;
     d.tile_base = tiles;
-    d.fwarp_base = fwarps;
+    d.fblk_base = fblks;
     d.row_base = rows;
     d.xc_base = xchunks;
     d.word_base = words;
     tris += T[m];
     tiles += (T[m] + tile - 1) / tile;
-    fwarps += (int64_t)g.n[1] * g.nxw * g.nzw;
+    fblks += finish_blocks((int64_t)g.n[1] * g.nxw);
     rows += (int64_t)g.n[2] * g.n[1];
     xchunks += ((int64_t)g.n[0] * g.n[1] * g.n[2] + 127) / 128;
     words += (int64_t)g.n[2] * g.n[1] * g.nxw;
@@ -290,20 +290,19 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
 
   float4 *ptri, *fbox;
   int4 *rng;
-  uint32_t *bplane, *iplane, *toggles, *wcnt, *wpre, *wtot, *stmp, *queue;
+  uint32_t *bplane, *iplane, *toggles, *wpre, *wtot, *stmp, *queue;
   MeshStats *stats;
   MeshDesc *d_md;
   CK(ws.get(&ptri, 3 * (size_t)std::max<int64_t>(tris, 1)));
   CK(ws.get(&rng, (size_t)std::max<int64_t>(tris, 1)));
   CK(ws.get(&fbox, (size_t)std::max<int64_t>(tris, 1)));
   // the pair lists are built by a counting sort, which ranks the voxels of the pairs through a
-  // second, column-major bit plane after the boundary plane; one popcount and one scan cover both
-  const bool kmark = words > 0;
+  // second, column-major bit plane after the boundary plane; one scan covers both
+  const bool kmark = words > 0 && (any_l2 || nmode);
   const int64_t swords = kmark ? 2 * words : words;
   CK(ws.get(&bplane, (size_t)swords));
   CK(ws.get(&iplane, (size_t)words));
   CK(ws.get(&toggles, (size_t)togg));
-  CK(ws.get(&wcnt, (size_t)swords));
   CK(ws.get(&wpre, (size_t)swords));
   CK(ws.get(&wtot, 4));
   CK(ws.get(&stmp, (size_t)scan_temp_words(swords)));
@@ -384,7 +383,7 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
   bd.tile = tile;
   bd.total_tris = tris;
   bd.total_tiles = tiles;
-  bd.total_fwarps = fwarps;
+  bd.total_fblks = fblks;
   bd.total_rows = rows;
   bd.total_xchunks = xchunks;
   bd.total_words = words;
@@ -437,7 +436,7 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
   // every value the phase's launches take (the per-mesh data reaches the kernels through d_md)
   auto bd_sig = [&](std::vector<uint64_t> &v) {
     for (uint64_t x : {(uint64_t)(uintptr_t)bd.md, (uint64_t)bd.nmesh, (uint64_t)bd.tile,
-                       (uint64_t)bd.total_tris, (uint64_t)bd.total_tiles, (uint64_t)bd.total_fwarps,
+                       (uint64_t)bd.total_tris, (uint64_t)bd.total_tiles, (uint64_t)bd.total_fblks,
                        (uint64_t)bd.total_rows, (uint64_t)bd.total_words, (uint64_t)bd.total_xchunks,
                        (uint64_t)(uintptr_t)bd.queue, (uint64_t)(uintptr_t)bd.heavy, (uint64_t)bd.normals, (uint64_t)bd.fill,
                        (uint64_t)(uintptr_t)bd.stp, (uint64_t)bd.stp_words,
@@ -449,7 +448,7 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
   bd_sig(sig0);
   for (uint64_t x : {(uint64_t)(uintptr_t)d_md, (uint64_t)(uintptr_t)keys, (uint64_t)(uintptr_t)vals,
                      (uint64_t)pair_cap, (uint64_t)(uintptr_t)bplane, (uint64_t)words,
-                     (uint64_t)(uintptr_t)wcnt, (uint64_t)(uintptr_t)wpre, (uint64_t)(uintptr_t)wtot,
+                     (uint64_t)(uintptr_t)wpre, (uint64_t)(uintptr_t)wtot,
                      (uint64_t)(uintptr_t)stmp, (uint64_t)(uintptr_t)d_slab,
                      (uint64_t)(d_slab ? (int64_t)gh[0].n[1] * gh[0].nxw : 0),
                      (uint64_t)(d_slab ? gh[0].n[2] : 0), (uint64_t)fz, (uint64_t)fslab,
@@ -485,8 +484,7 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
     if (stencil) launch_stencil1(bd, s);
     mark(3);
     launch_fill_finish(bd, s);
-    launch_popc(bplane, swords, wcnt, s);
-    scan_u32(wcnt, wpre, swords, wtot, stmp, s);
+    scan_u32(bplane, wpre, swords, wtot, stmp, s, true);
     launch_boundary_counts(bd, wpre, btot, s);
     if (d_slab)
       launch_slab_offsets(wpre, btot, (int64_t)gh[0].n[1] * gh[0].nxw, gh[0].n[2], fz, fslab,

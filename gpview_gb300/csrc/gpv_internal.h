@@ -17,8 +17,9 @@ void count_launch(uint64_t n = 1);
 
 // ---- scan / sort (gpv_sort.cu) ---------------------------------------------------------------
 int64_t scan_temp_words(int64_t n);
+// Exclusive scan of in[0..n), of the values or (bits) of their bit counts.
 void scan_u32(const uint32_t *in, uint32_t *out, int64_t n, uint32_t *d_total, uint32_t *temp,
-              cudaStream_t s);
+              cudaStream_t s, bool bits = false);
 int64_t sort_temp_words(int64_t n);
 bool sort_pairs(uint32_t *keys, uint32_t *vals, uint32_t *kalt, uint32_t *valt, int64_t n,
                 int key_bits, uint32_t *temp, cudaStream_t s);
@@ -53,7 +54,7 @@ struct MeshDesc {
   float4 *fbox;          // conservative x/y box for the ray tests per triangle
   uint32_t *bplane;      // boundary bit plane (padded rows), slice of the batch plane
   uint32_t *iplane;      // inside (parity) bit plane, slice
-  uint32_t *toggles;     // column-major parity toggles
+  uint32_t *toggles;     // parity toggles, 32 layers a word: word w of column c at w * nx * ny + c
   uint32_t *keys, *vals; // pair emission segment (capacity pair_cap)
   MeshStats *stats;
   uint8_t *l1;           // outputs
@@ -63,7 +64,7 @@ struct MeshDesc {
   int64_t T, pair_cap;
   int64_t tri_base;      // prefix over meshes of triangles
   int64_t tile_base;     // ... of Level1 tiles
-  int64_t fwarp_base;    // ... of fill-finish warps (ny * nxw * nzw)
+  int64_t fblk_base;     // ... of fill-finish blocks (ny * nxw words of a layer, kFinishGroups each)
   int64_t row_base;      // ... of Level1 rows (nz * ny)
   int64_t xc_base;       // ... of 128-voxel expansion chunks (ceil(N1 / 128))
   int64_t word_base;     // ... of bit-plane words (nz * ny * nxw)
@@ -109,11 +110,14 @@ constexpr int kSlabsMax = 8;
 constexpr int kQueueWords = 1 + 2 * kSlabsMax;
 constexpr uint32_t kHeavyCap = 1u << 18;  // pieces of a call's heavy list (4 MiB)
 
+constexpr int kFinishGroups = 8;  // plane words of a layer that one fill-finish block takes
+inline int64_t finish_blocks(int64_t layer_words) { return (layer_words + kFinishGroups - 1) / kFinishGroups; }
+
 struct BatchDev {
   const MeshDesc *md;
   int nmesh;
   int tile;              // Level1 triangles per ticket (32, 64, 128, 256)
-  int64_t total_tris, total_tiles, total_fwarps, total_rows, total_words;
+  int64_t total_tris, total_tiles, total_fblks, total_rows, total_words;
   int64_t total_xchunks;  // 128-voxel expansion chunks of all meshes
   uint32_t *queue;       // work-queue tickets, zeroed by the caller: [0] Level1, [1 + k] and
                          // [1 + kSlabsMax + k] the fill and the SAT kernel of Level2 slab k
@@ -204,7 +208,6 @@ void launch_fill_finish(const BatchDev &bd, cudaStream_t s);
 // Stencil fill, Level1 (gpv_stencil.cu): per-sample-column slice toggles of every triangle into
 // MeshDesc::stg (zeroed by the caller); launch_fill_finish then reduces them.
 void launch_stencil1(const BatchDev &bd, cudaStream_t s);
-void launch_popc(const uint32_t *plane, int64_t nwords, uint32_t *cnt, cudaStream_t s);
 void launch_boundary_counts(const BatchDev &bd, const uint32_t *wpre, const uint32_t *wtotal,
                             cudaStream_t s);
 void launch_expand(const BatchDev &bd, const uint32_t *wpre, cudaStream_t s);

@@ -13,9 +13,9 @@
 //                     Moller-Trumbore test; a passing unit XORs the parity toggles
 //                     d(k) = hit(k) ^ hit(k+1) into a column-major plane, from the triangle's height
 //                     over the column.
-//   k_fill_finish warp-level suffix XOR of the toggles per column -> parity, transposed to
-//                 the linear (x fastest) inside plane.
-//   k_popc + scan per-word boundary counts, boundaryPrefixSum.
+//   k_fill_finish suffix XOR of the toggles per column -> parity, transposed to the linear (x fastest)
+//                 inside plane; the boundary plane transposed to the pair keys' order.
+//   scan          per-word boundary counts, boundaryPrefixSum.
 //   k_expand      .raw bytes of Level1, boundaryPrefixSum, boundaryIndex.
 //   sort / Level2 gpv_sort.cu, gpv_level2.cu.
 #include "gpv_internal.h"
@@ -446,7 +446,7 @@ __device__ __forceinline__ void plane_range(const float *V, const GridDev &g, fl
 // X is off by about as much and by the centre table's distance from its affine form, and only the
 // voxels within that of the crossing (all of them for an ill-conditioned projection) run the test.
 __device__ __forceinline__ void column_toggles(const RayTri &rt, const RayCol &rc, const GridDev &g,
-                                               uint32_t *tog) {
+                                               uint32_t *tog, size_t stride) {
   const int nz = g.n[2];
   const float *oz = g.c1[2];
   const float ad = fabsf(rt.inv_det);
@@ -473,10 +473,10 @@ __device__ __forceinline__ void column_toggles(const RayTri &rt, const RayCol &r
   bool above = false;
   for (int k = n2 - 1; k >= n1; --k) {
     const bool hit = ray_t(rt, rc, __ldg(oz + k), g.thr);
-    if (hit != above) atomicXor(tog + (k >> 5), 1u << (k & 31));
+    if (hit != above) atomicXor(tog + (size_t)(k >> 5) * stride, 1u << (k & 31));
     above = hit;
   }
-  if (n1 > 0 && !above) atomicXor(tog + ((n1 - 1) >> 5), 1u << ((n1 - 1) & 31));
+  if (n1 > 0 && !above) atomicXor(tog + (size_t)((n1 - 1) >> 5) * stride, 1u << ((n1 - 1) & 31));
 }
 
 // Every warp works by itself: it takes tickets of bd.tile triangles from the queue, stages them 32 at
@@ -719,7 +719,7 @@ __global__ void __launch_bounds__(kL1Warps * 32, 8) k_level1(BatchDev bd, uint32
       ray_tri_pre(V, a2.w, rt);  // fill units exist only for triangles passing the det test
       RayCol rc;
       if (ray_col(rt, __ldg(g.c1[0] + i), __ldg(g.c1[1] + j), rc))
-        column_toggles(rt, rc, g, ws.toggles + ((size_t)j * nx + i) * g.nzw);
+        column_toggles(rt, rc, g, ws.toggles + (size_t)j * nx + i, (size_t)nx * ny);
     }
     __syncwarp();  // the buffer may be staged again
     advance(it);
@@ -729,98 +729,108 @@ __global__ void __launch_bounds__(kL1Warps * 32, 8) k_level1(BatchDev bd, uint32
 }
 
 // ---------------------------------------------------------------------------------------------
-// One warp per (mesh, row j, 32-column group, 32-layer word w): suffix XOR of each column's
-// toggles gives the parity of every voxel (the toggles of the words above w give the carry); 32
-// ballots transpose the word into the linear inside plane.
-// Stencil fill: the parity of each of the voxel column's four sample columns is the prefix XOR
-// of its slice toggles (lowest slice first), and a voxel is inside where at least three of the
-// four are odd.
-__global__ void __launch_bounds__(256) k_fill_finish(BatchDev bd) {
-  const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+// 32 x 32 bits across a warp: bit c of lane r becomes bit r of lane c.
+__device__ __forceinline__ uint32_t warp_transpose(uint32_t x) {
   const unsigned lane = threadIdx.x & 31u;
-  if (gw >= bd.total_fwarps) return;
-  const int m = find_mesh<&MeshDesc::fwarp_base>(bd.md, bd.nmesh, gw);
-  const MeshDesc &d = bd.md[m];
-  const GridDev &g = d.g;
-  const int64_t lw = gw - d.fwarp_base;
-  const int nx = g.n[0], ny = g.n[1], nz = g.n[2];
-  const int w = (int)(lw % g.nzw);
-  const int64_t cgrp = lw / g.nzw;
-  const int j = (int)(cgrp / g.nxw), ig = (int)(cgrp % g.nxw);
-  const int i = ig * 32 + (int)lane;
-  const bool valid = i < nx;
-  const size_t col = (size_t)j * nx + i;
-  const bool stencil = bd.fill == GPV_FILL_STENCIL;
-  const uint32_t *sc[4] = {nullptr, nullptr, nullptr, nullptr};
-  uint32_t s;
-  if (stencil) {
-    // bit a: toggle parity of sample column a in all words / in the words above w
-    uint32_t tot = 0, above = 0;
-    if (valid) {
-      const size_t SW = 2 * (size_t)nx;
-      sc[0] = d.stg + ((size_t)(2 * j) * SW + 2 * (size_t)i) * g.nzw;
-      sc[1] = sc[0] + g.nzw;
-      sc[2] = sc[0] + SW * g.nzw;
-      sc[3] = sc[2] + g.nzw;
-      for (int v = 0; v < g.nzw; ++v)
+  uint32_t m = 0x0000ffffu;
 #pragma unroll
-        for (int a = 0; a < 4; ++a) {
-          const uint32_t pv = (uint32_t)(__popc(sc[a][v]) & 1) << a;
-          tot ^= pv;
-          if (v > w) above ^= pv;
-        }
-    }
-    uint32_t x[4];
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      const uint32_t D = valid ? sc[a][w] : 0u;
-      const uint32_t pd = (uint32_t)(__popc(D) & 1);
-      uint32_t y = D;  // prefix XOR from the lowest slice of the word
-      y ^= y << 1; y ^= y << 2; y ^= y << 4; y ^= y << 8; y ^= y << 16;
-      if ((((tot ^ above) >> a) & 1u) ^ pd) y = ~y;  // odd toggles in the words below
-      x[a] = y;
-    }
-    s = (x[0] & x[1] & (x[2] | x[3])) | (x[2] & x[3] & (x[0] | x[1]));
-  } else {
-    uint32_t carry = 0;  // toggle parity of the column in the words above w
-    if (valid)
-      for (int v = w + 1; v < g.nzw; ++v) carry ^= (uint32_t)(__popc(d.toggles[col * g.nzw + v]) & 1);
-    const uint32_t D = valid ? d.toggles[col * g.nzw + w] : 0u;
-    s = D;
-    s ^= s >> 1; s ^= s >> 2; s ^= s >> 4; s ^= s >> 8; s ^= s >> 16;
-    if (carry) s = ~s;
+  for (int j = 16; j > 0; j >>= 1, m ^= m << j) {
+    const uint32_t y = __shfl_xor_sync(FULL, x, j);
+    x = (lane & j) ? ((x & ~m) | ((y >> j) & m)) : ((x & m) | ((y & m) << j));
   }
-  uint32_t mine = 0;
-#pragma unroll
-  for (int bb = 0; bb < 32; ++bb) {
-    const uint32_t mm = __ballot_sync(FULL, (s >> bb) & 1u);
-    if ((int)lane == bb) mine = mm;
-  }
-  const int k = w * 32 + (int)lane;
-  if (k < nz) d.iplane[((size_t)k * ny + j) * g.nxw + ig] = mine;
-  if (!bd.kmask || !(d.has_l2 || bd.normals)) return;
-  // the boundary plane transposed the other way, for the pair lists: 32 layers of 32 columns to one
-  // word per column at the columns' place in key order
-  const uint32_t bw = k < nz ? d.bplane[((size_t)k * ny + j) * g.nxw + ig] : 0u;
-  if (!__any_sync(FULL, bw != 0u)) return;
-  uint32_t cw = 0;
-#pragma unroll
-  for (int bb = 0; bb < 32; ++bb) {
-    const uint32_t mm = __ballot_sync(FULL, (bw >> bb) & 1u);
-    if ((int)lane == bb) cw = mm;
-  }
-  if (cw) {
-    uint32_t *km = bd.kmask + d.word_base;
-    const uint64_t bit = (uint64_t)col * nz + (uint64_t)w * 32;
-    const unsigned sh = (unsigned)(bit & 31u);
-    atomicOr(km + (bit >> 5), cw << sh);
-    if (sh && (cw >> (32 - sh))) atomicOr(km + (bit >> 5) + 1, cw >> (32 - sh));
-  }
+  return x;
 }
 
-__global__ void k_popc(const uint32_t *__restrict__ plane, int64_t nw, uint32_t *__restrict__ cnt) {
-  const int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (w < nw) cnt[w] = __popc(plane[w]);
+// A block takes kFinishGroups consecutive groups of 32 columns (a warp each; consecutive words of a
+// layer's plane) and walks their layers 32 at a time: the parity of each column's voxels from its
+// toggles, transposed to the linear inside plane, and, for meshes with pair lists, the boundary plane
+// transposed the other way, to one word per column at the columns' place in key order.  Both planes
+// move through shared memory, 32 bytes of a layer together.  Ray fill: the suffix XOR of the toggles, from
+// the top layers down.  Stencil fill: the parity of each of the voxel column's four sample columns is
+// the prefix XOR of its slice toggles, lowest slice first, and a voxel is inside where at least three
+// of the four are odd.  Bound by latency on small grids and by the planes' traffic on large ones (a
+// warp per 32 columns and 32 layers, which read all words above its own for the carry and wrote four
+// bytes of a sector, took 102 us at 512^3 and 17 at 256^3; this 25 and 10).
+__global__ void __launch_bounds__(kFinishGroups * 32) k_fill_finish(BatchDev bd) {
+  __shared__ uint32_t s_in[2][32][kFinishGroups + 1], s_bd[2][32][kFinishGroups + 1];
+  const int lane = (int)(threadIdx.x & 31u), warp = (int)(threadIdx.x >> 5);
+  const int m = find_mesh<&MeshDesc::fblk_base>(bd.md, bd.nmesh, blockIdx.x);
+  const MeshDesc &d = bd.md[m];
+  const GridDev &g = d.g;
+  const int nx = g.n[0], ny = g.n[1], nz = g.n[2], nzw = g.nzw;
+  const int64_t ngrp = (int64_t)ny * g.nxw;  // words of a plane's layer
+  const int64_t grp0 = ((int64_t)blockIdx.x - d.fblk_base) * kFinishGroups, grp = grp0 + warp;
+  const int j = (int)(grp / g.nxw), ig = (int)(grp - (int64_t)j * g.nxw);
+  const int i = ig * 32 + lane;
+  const bool valid = grp < ngrp && i < nx;
+  const size_t ncol = (size_t)nx * ny, col = (size_t)j * nx + i;
+  const bool stencil = bd.fill == GPV_FILL_STENCIL;
+  uint32_t *const km = bd.kmask && (d.has_l2 || bd.normals) ? bd.kmask + d.word_base : nullptr;
+  // this thread's place in a plane tile: layer tl, group tg
+  const int tl = (int)threadIdx.x / kFinishGroups, tg = (int)threadIdx.x % kFinishGroups;
+  const bool tok = grp0 + tg < ngrp;
+  const uint32_t *sc[4] = {nullptr, nullptr, nullptr, nullptr};
+  if (stencil && valid) {
+    const size_t SW = 2 * (size_t)nx;
+    sc[0] = d.stg + ((size_t)(2 * j) * SW + 2 * (size_t)i) * nzw;
+    sc[1] = sc[0] + nzw;
+    sc[2] = sc[0] + SW * nzw;
+    sc[3] = sc[2] + nzw;
+  }
+  uint32_t carry = 0;  // ray: the toggles above are odd; stencil, bit a: those below of sample a
+  constexpr int kAhead = 4;
+  for (int t0 = 0; t0 < nzw; t0 += kAhead) {
+    // the next words' loads together
+    uint32_t dv[kAhead], bv[kAhead];
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+      const int t = t0 + k, w = stencil ? t : nzw - 1 - t, z = w * 32 + tl;
+      dv[k] = t < nzw && valid && !stencil ? __ldg(d.toggles + (size_t)w * ncol + col) : 0u;
+      bv[k] = t < nzw && km && tok && z < nz ? __ldg(d.bplane + (size_t)z * ngrp + grp0 + tg) : 0u;
+    }
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+      const int t = t0 + k;
+      if (t >= nzw) break;
+      const int w = stencil ? t : nzw - 1 - t, buf = t & 1;
+      uint32_t s;
+      if (stencil) {
+        uint32_t x[4];
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+          const uint32_t D = valid ? sc[a][w] : 0u;
+          uint32_t y = D;
+          y ^= y << 1; y ^= y << 2; y ^= y << 4; y ^= y << 8; y ^= y << 16;
+          if ((carry >> a) & 1u) y = ~y;
+          carry ^= (uint32_t)(__popc(D) & 1) << a;
+          x[a] = y;
+        }
+        s = (x[0] & x[1] & (x[2] | x[3])) | (x[2] & x[3] & (x[0] | x[1]));
+      } else {
+        s = dv[k];
+        s ^= s >> 1; s ^= s >> 2; s ^= s >> 4; s ^= s >> 8; s ^= s >> 16;
+        if (carry) s = ~s;
+        carry ^= (uint32_t)(__popc(dv[k]) & 1);
+      }
+      s_in[buf][lane][warp] = warp_transpose(s);
+      if (km) s_bd[buf][tl][tg] = bv[k];
+      __syncthreads();
+      const int z = w * 32 + tl;
+      if (tok && z < nz) d.iplane[(size_t)z * ngrp + grp0 + tg] = s_in[buf][tl][tg];
+      if (km) {
+        const uint32_t bw = s_bd[buf][lane][warp];
+        if (__any_sync(FULL, bw != 0u)) {
+          const uint32_t cw = warp_transpose(bw);
+          if (cw) {
+            const uint64_t bit = (uint64_t)col * nz + (uint64_t)w * 32;
+            const unsigned sh = (unsigned)(bit & 31u);
+            atomicOr(km + (bit >> 5), cw << sh);
+            if (sh && (cw >> (32 - sh))) atomicOr(km + (bit >> 5) + 1, cw >> (32 - sh));
+          }
+        }
+      }
+    }
+  }
 }
 
 // B_m = boundary voxels of mesh m, from the exclusive scan over the batch's plane words.
@@ -833,71 +843,71 @@ __global__ void k_boundary_counts(BatchDev bd, const uint32_t *__restrict__ wpre
   bd.md[m].stats->boundary = e - s;
 }
 
-// One warp per chunk of 128 consecutive voxels of one mesh's linear index (x fastest),
-// kExpandWarps chunks per block: state bytes, boundaryPrefixSum, boundaryIndex.  Every lane of a
-// chunk works whatever the row length (a warp per row left three quarters of the lanes idle on a
-// 32-voxel row), and a block whose chunks lie in one mesh looks the mesh up once.
+// One warp per chunk of 128 consecutive voxels of one mesh's linear index (x fastest), four per lane:
+// state bytes, boundaryPrefixSum, boundaryIndex.  Every lane of a chunk works whatever the row length (a
+// warp per row left three quarters of the lanes idle on a 32-voxel row).  The mesh's fields are kept in
+// registers and the planes read through the read-only path, so that several chunks' loads are in
+// flight; with them read again after every store and 64-bit index arithmetic the kernel was bound by
+// its instructions (512^3: 302 us, now 215, 3.2 TB/s).
 constexpr int kExpandWarps = 8;
 constexpr int kExpandVox = 128;
-// One chunk by one warp; returns the lane's inside-voxel count and the chunk's mesh statistics.
-__device__ __forceinline__ unsigned long long expand_chunk(const BatchDev &bd,
-                                                           const uint32_t *__restrict__ wpre, int m,
-                                                           int64_t gc, unsigned lane,
-                                                           MeshStats *&st) {
-  const MeshDesc &d = bd.md[m];
-  const GridDev &g = d.g;
-  st = d.stats;
-  const int nx = g.n[0];
-  const int64_t N1 = (int64_t)nx * g.n[1] * g.n[2];
-  const int64_t v0 = (gc - d.xc_base) * kExpandVox + (int64_t)lane * 4;
-  if (v0 >= N1) return 0;
-  const uint32_t pbase = wpre[d.word_base];
-  const uint32_t *bplane = d.bplane, *iplane = d.iplane;
-  const uint32_t *wp = wpre + d.word_base;
-  unsigned long long nin = 0;
-  // (the 4- and 16-byte stores need aligned outputs: the batch's arenas are, a no-alloc caller's
-  // buffers may not be)
-  if ((nx & 3) == 0 && (reinterpret_cast<uintptr_t>(d.l1) & 3u) == 0 &&
-      (reinterpret_cast<uintptr_t>(d.prefix) & 15u) == 0) {
-    // the lane's four voxels share a row and a plane word (nx and v0 are multiples of 4), and
-    // N1 is a multiple of 4 too
-    const int64_t row = v0 / nx;
-    const int x0 = (int)(v0 - row * nx);
-    const size_t w = (size_t)row * g.nxw + (x0 >> 5);
-    const int b0 = x0 & 31;
-    const uint32_t bw = bplane[w], iw = iplane[w];
-    uint32_t p = wp[w] - pbase + __popc(bw & ((1u << b0) - 1u));
-    uint32_t bytes = 0;
-    int32_t pre[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const bool isb = (bw >> (b0 + e)) & 1u, isi = (iw >> (b0 + e)) & 1u;
-      pre[e] = (int32_t)p;
-      if (isb) {
-        d.bindex[p] = (int32_t)(v0 + e);
-        ++p;
-      }
-      nin += (!isb && isi);
-      bytes |= (isb ? 254u : (isi ? 127u : 0u)) << (8 * e);
-    }
-    *reinterpret_cast<uint32_t *>(d.l1 + v0) = bytes;
-    *reinterpret_cast<int4 *>(d.prefix + v0) = make_int4(pre[0], pre[1], pre[2], pre[3]);
-  } else {
-    for (int e = 0; e < 4; ++e) {
-      const int64_t v = v0 + e;
-      if (v >= N1) break;
-      const int64_t row = v / nx;
-      const int x = (int)(v - row * nx);
-      const size_t w = (size_t)row * g.nxw + (x >> 5);
-      const int bit = x & 31;
-      const uint32_t bw = bplane[w], iw = iplane[w];
-      const uint32_t p = wp[w] - pbase + __popc(bw & ((1u << bit) - 1u));
-      const bool isb = (bw >> bit) & 1u, isi = (iw >> bit) & 1u;
-      nin += (!isb && isi);
-      if (isb) d.bindex[p] = (int32_t)v;
-      d.l1[v] = (uint8_t)(isb ? 254u : (isi ? 127u : 0u));
-      d.prefix[v] = (int32_t)p;
-    }
+struct ExpandMesh {
+  const uint32_t *bplane, *iplane, *wp;
+  uint8_t *l1;
+  int32_t *prefix, *bindex;
+  int64_t first;  // its first chunk
+  uint32_t N1, nx, nxw, pbase;
+  bool vec;       // rows of a multiple of four voxels and aligned outputs (the batch's arenas are, a
+                  // no-alloc caller's buffers may not be)
+};
+__device__ __forceinline__ ExpandMesh expand_mesh(const MeshDesc &d, const uint32_t *__restrict__ wpre) {
+  ExpandMesh e;
+  e.bplane = d.bplane;
+  e.iplane = d.iplane;
+  e.wp = wpre + d.word_base;
+  e.l1 = d.l1;
+  e.prefix = d.prefix;
+  e.bindex = d.bindex;
+  e.first = d.xc_base;
+  e.nx = (uint32_t)d.g.n[0];
+  e.N1 = e.nx * (uint32_t)d.g.n[1] * (uint32_t)d.g.n[2];
+  e.nxw = (uint32_t)d.g.nxw;
+  e.pbase = wpre[d.word_base];
+  e.vec = (e.nx & 3u) == 0 && (reinterpret_cast<uintptr_t>(d.l1) & 3u) == 0 &&
+          (reinterpret_cast<uintptr_t>(d.prefix) & 15u) == 0;
+  return e;
+}
+// One chunk by one warp; returns the lane's inside-voxel count.
+__device__ __forceinline__ uint32_t expand_chunk(const ExpandMesh &e, int64_t gc, uint32_t lane) {
+  const uint32_t v0 = (uint32_t)(gc - e.first) * kExpandVox + lane * 4u;
+  if (v0 >= e.N1) return 0;
+  if (e.vec) {
+    // the lane's four voxels share a row and a plane word (nx, v0 and N1 are multiples of 4)
+    const uint32_t row = v0 / e.nx, x0 = v0 - row * e.nx;
+    const uint32_t w = row * e.nxw + (x0 >> 5), b0 = x0 & 31u;
+    const uint32_t bw = __ldg(e.bplane + w), iw = __ldg(e.iplane + w);
+    const uint32_t p = __ldg(e.wp + w) - e.pbase + __popc(bw & ((1u << b0) - 1u));
+    const uint32_t bb = (bw >> b0) & 0xfu, ib = (iw >> b0) & 0xfu & ~bb;
+    // (4 bits to 4 bytes: bit j to byte j)
+    const uint32_t bytes = ((bb * 0x00204081u) & 0x01010101u) * 254u + ((ib * 0x00204081u) & 0x01010101u) * 127u;
+    const uint32_t p1 = p + (bb & 1u), p2 = p1 + ((bb >> 1) & 1u), p3 = p2 + ((bb >> 2) & 1u);
+    *reinterpret_cast<uint32_t *>(e.l1 + v0) = bytes;
+    *reinterpret_cast<int4 *>(e.prefix + v0) = make_int4((int)p, (int)p1, (int)p2, (int)p3);
+    uint32_t q = p;
+    for (uint32_t k = bb; k; k &= k - 1u) e.bindex[q++] = (int32_t)(v0 + (uint32_t)__ffs(k) - 1u);
+    return (uint32_t)__popc(ib);
+  }
+  uint32_t nin = 0;
+  for (uint32_t k = 0; k < 4u && v0 + k < e.N1; ++k) {
+    const uint32_t v = v0 + k, row = v / e.nx, x = v - row * e.nx;
+    const uint32_t w = row * e.nxw + (x >> 5), bit = x & 31u;
+    const uint32_t bw = __ldg(e.bplane + w), iw = __ldg(e.iplane + w);
+    const uint32_t p = __ldg(e.wp + w) - e.pbase + __popc(bw & ((1u << bit) - 1u));
+    const bool isb = (bw >> bit) & 1u, isi = (iw >> bit) & 1u;
+    nin += (!isb && isi);
+    if (isb) e.bindex[p] = (int32_t)v;
+    e.l1[v] = (uint8_t)(isb ? 254u : (isi ? 127u : 0u));
+    e.prefix[v] = (int32_t)p;
   }
   return nin;
 }
@@ -920,20 +930,22 @@ __global__ void __launch_bounds__(kExpandWarps * 32) k_expand(BatchDev bd,
   if (threadIdx.x == 0) s_mesh = find_mesh<&MeshDesc::xc_base>(bd.md, bd.nmesh, c0);
   __syncthreads();
   int m = s_mesh;
+  ExpandMesh em = expand_mesh(bd.md[m], wpre);
+  int64_t next = m + 1 < bd.nmesh ? bd.md[m + 1].xc_base : bd.total_xchunks;
   unsigned long long nin = 0;
+#pragma unroll 4
   for (int k = 0; k < iters; ++k) {
     const int64_t gc = c0 + (int64_t)k * kExpandWarps + warp;
     if (gc >= bd.total_xchunks) break;  // warp-uniform
-    int mn = m;
-    while (mn + 1 < bd.nmesh && bd.md[mn + 1].xc_base <= gc) ++mn;
-    if (mn != m) {
+    if (gc >= next) {
       const unsigned long long t = warp_sum(nin);
       if (lane == 0 && t) atomicAdd(&bd.md[m].stats->l1_inside, t);
       nin = 0;
-      m = mn;
+      while (m + 1 < bd.nmesh && bd.md[m + 1].xc_base <= gc) ++m;
+      em = expand_mesh(bd.md[m], wpre);
+      next = m + 1 < bd.nmesh ? bd.md[m + 1].xc_base : bd.total_xchunks;
     }
-    MeshStats *st = nullptr;
-    nin += expand_chunk(bd, wpre, m, gc, lane, st);
+    nin += expand_chunk(em, gc, lane);
   }
   // the warps' last mesh runs: one atomic per mesh of the block
   const unsigned long long t = warp_sum(nin);
@@ -1081,14 +1093,8 @@ void launch_level1(const BatchDev &bd, int num_sms, cudaStream_t s) {
 }
 
 void launch_fill_finish(const BatchDev &bd, cudaStream_t s) {
-  if (bd.total_fwarps <= 0) return;
-  k_fill_finish<<<(unsigned)((bd.total_fwarps * 32 + 255) / 256), 256, 0, s>>>(bd);
-  count_launch();
-}
-
-void launch_popc(const uint32_t *plane, int64_t nwords, uint32_t *cnt, cudaStream_t s) {
-  if (nwords <= 0) return;
-  k_popc<<<(unsigned)((nwords + 255) / 256), 256, 0, s>>>(plane, nwords, cnt);
+  if (bd.total_fblks <= 0) return;
+  k_fill_finish<<<(unsigned)bd.total_fblks, kFinishGroups * 32, 0, s>>>(bd);
   count_launch();
 }
 

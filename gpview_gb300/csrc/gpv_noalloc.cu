@@ -145,7 +145,7 @@ extern "C" int gpv_voxelize_level1_noalloc(const float *d_tris, int64_t num_tria
   const size_t o_bp = take(4 * (size_t)N1w);
   const size_t o_ip = take(4 * (size_t)N1w);
   const size_t o_tg = take(4 * (size_t)(ncol * g.nzw));
-  const size_t o_wc = take(4 * (size_t)N1w);
+  const size_t o_hv = take(4 * (size_t)N1w);  // pieces of large triangles
   const size_t o_wp = take(4 * (size_t)N1w);
   const size_t o_sc = take(4 * (size_t)scan_temp_words(N1w));
   const size_t o_st = take(sizeof(MeshStats));
@@ -196,7 +196,6 @@ extern "C" int gpv_voxelize_level1_noalloc(const float *d_tris, int64_t num_tria
   md.prefix = d_level1_prefix;
   md.bindex = d_boundary_index;
   MeshDesc *d_md = reinterpret_cast<MeshDesc *>(base + o_md);
-  uint32_t *wcnt = reinterpret_cast<uint32_t *>(base + o_wc);
   uint32_t *wpre = reinterpret_cast<uint32_t *>(base + o_wp);
   uint32_t *stmp = reinterpret_cast<uint32_t *>(base + o_sc);
   uint32_t *d_tot = reinterpret_cast<uint32_t *>(base + o_tot);
@@ -207,12 +206,13 @@ extern "C" int gpv_voxelize_level1_noalloc(const float *d_tris, int64_t num_tria
   bd.tile = 32;
   bd.total_tiles = (T + 31) / 32;
   bd.queue = d_tot + 1;  // (the total takes the first word)
-  // what the array has left holds the pieces of large triangles
-  bd.heavy_cap = (uint32_t)std::min<size_t>((kScratchBytes - o) / sizeof(uint4), kHeavyCap);
-  bd.heavy = bd.heavy_cap ? reinterpret_cast<uint4 *>(base + o) : nullptr;
+  // the pieces of large triangles: their own region, or what the array has left where that is more
+  const size_t own_cap = (size_t)N1w / 4, rest_cap = (kScratchBytes - o) / sizeof(uint4);
+  bd.heavy_cap = (uint32_t)std::min<size_t>(std::max(own_cap, rest_cap), kHeavyCap);
+  bd.heavy = bd.heavy_cap ? reinterpret_cast<uint4 *>(base + (rest_cap > own_cap ? o : o_hv)) : nullptr;
   bd.heavy_n = d_tot + 2;
   bd.total_tris = T;
-  bd.total_fwarps = (int64_t)g.n[1] * g.nxw * g.nzw;
+  bd.total_fblks = finish_blocks((int64_t)g.n[1] * g.nxw);
   bd.total_rows = (int64_t)g.n[2] * g.n[1];
   bd.total_xchunks = (N1 + 127) / 128;
   bd.total_words = N1w;
@@ -233,8 +233,7 @@ extern "C" int gpv_voxelize_level1_noalloc(const float *d_tris, int64_t num_tria
   launch_prep(bd, stream);
   launch_level1(bd, num_sms, stream);  // (no Level2 grid: the records are counted, not written)
   launch_fill_finish(bd, stream);
-  launch_popc(md.bplane, N1w, wcnt, stream);
-  scan_u32(wcnt, wpre, N1w, d_tot, stmp, stream);
+  scan_u32(md.bplane, wpre, N1w, d_tot, stmp, stream, true);
   launch_expand(bd, wpre, stream);
   uint32_t nb = 0;
   MeshStats hs;

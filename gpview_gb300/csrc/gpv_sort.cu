@@ -2,7 +2,7 @@
 // triangle lists (the reference builds them on the host, src/Object.cpp:2146-2180, and
 // compacts boundary voxels there too, :3271-3279).
 //
-// scan_u32:  reduce-then-scan, no inter-block waiting: tile sums, then a down-sweep in which every
+// scan_u32:  (of values or bit counts) reduce-then-scan, no inter-block waiting: tile sums, then a down-sweep in which every
 //            block adds up the sums of the tiles before it (up to 1024 tiles; beyond that a
 //            separate single-block scan of the tile sums runs in between).
 // sort_pairs: stable LSD radix sort of (u32 key, u32 value), 8-bit digits; per pass a tile
@@ -53,15 +53,54 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t &total)
   return r;
 }
 
-__global__ void k_scan_reduce(const uint32_t *__restrict__ in, int64_t n,
-                              uint32_t *__restrict__ part) {
-  const int64_t base = (int64_t)blockIdx.x * kScanTile;
-  uint32_t s = 0;
+// A thread's kScanItems consecutive values (or bit counts), zero past the end: two 16-byte loads
+// inside the array (bases are 16-byte aligned where `vec`).
+template <bool BITS>
+__device__ __forceinline__ void scan_load(const uint32_t *__restrict__ in, int64_t n, int64_t tb, bool vec,
+                                          uint32_t (&v)[kScanItems]) {
+  if (vec && tb + kScanItems <= n) {
 #pragma unroll
-  for (int k = 0; k < kScanItems; ++k) {
-    int64_t i = base + (int64_t)k * kScanThreads + threadIdx.x;
-    if (i < n) s += in[i];
+    for (int k = 0; k < kScanItems; k += 4) {
+      const uint4 x = __ldg(reinterpret_cast<const uint4 *>(in + tb + k));
+      v[k] = x.x; v[k + 1] = x.y; v[k + 2] = x.z; v[k + 3] = x.w;
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) v[k] = tb + k < n ? in[tb + k] : 0u;
   }
+  if (BITS) {
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) v[k] = (uint32_t)__popc(v[k]);
+  }
+}
+__device__ __forceinline__ void scan_store(uint32_t *__restrict__ out, int64_t n, int64_t tb, bool vec,
+                                           uint32_t ex, const uint32_t (&v)[kScanItems]) {
+  if (vec && tb + kScanItems <= n) {
+#pragma unroll
+    for (int k = 0; k < kScanItems; k += 4) {
+      uint4 x;
+      x.x = ex; ex += v[k];
+      x.y = ex; ex += v[k + 1];
+      x.z = ex; ex += v[k + 2];
+      x.w = ex; ex += v[k + 3];
+      *reinterpret_cast<uint4 *>(out + tb + k) = x;
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) {
+      if (tb + k < n) out[tb + k] = ex;
+      ex += v[k];
+    }
+  }
+}
+
+template <bool BITS>
+__global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const uint32_t *__restrict__ in, int64_t n,
+                                                             bool vec, uint32_t *__restrict__ part) {
+  uint32_t v[kScanItems], s = 0;
+  scan_load<BITS>(in, n, (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems, vec, v);
+#pragma unroll
+  for (int k = 0; k < kScanItems; ++k) s += v[k];
   uint32_t tot;
   block_excl_scan<kScanThreads>(s, tot);
   if (threadIdx.x == 0) part[blockIdx.x] = tot;
@@ -82,62 +121,38 @@ __global__ void k_scan_partials(uint32_t *__restrict__ part, int64_t nb,
   if (threadIdx.x == 0 && total) *total = carry;
 }
 
-__global__ void k_scan_down(const uint32_t *__restrict__ in, int64_t n,
-                            const uint32_t *__restrict__ part, uint32_t *__restrict__ out) {
-  const int64_t base = (int64_t)blockIdx.x * kScanTile;
-  // blocked arrangement: thread owns kScanItems consecutive items
-  uint32_t v[kScanItems];
-  uint32_t s = 0;
-  const int64_t tb = base + (int64_t)threadIdx.x * kScanItems;
-#pragma unroll
-  for (int k = 0; k < kScanItems; ++k) {
-    int64_t i = tb + k;
-    v[k] = i < n ? in[i] : 0u;
-    s += v[k];
-  }
-  uint32_t tot;
-  uint32_t ex = block_excl_scan<kScanThreads>(s, tot) + part[blockIdx.x];
-#pragma unroll
-  for (int k = 0; k < kScanItems; ++k) {
-    int64_t i = tb + k;
-    if (i < n) out[i] = ex;
-    ex += v[k];
-  }
-}
-
-// Down-sweep that also finds its own tile offset: the sum of the partials of the tiles before it
+// Down-sweep.  SELF: it also finds its own tile offset, the sum of the partials of the tiles before it
 // (for up to kFusedTiles tiles, where that sum is cheap), so the partials need no separate scan.
 constexpr int64_t kFusedTiles = 1024;
 
-__global__ void k_scan_down_fused(const uint32_t *__restrict__ in, int64_t n,
-                                  const uint32_t *__restrict__ part, uint32_t *__restrict__ out,
-                                  uint32_t *__restrict__ total) {
+template <bool BITS, bool SELF>
+__global__ void __launch_bounds__(kScanThreads) k_scan_down(const uint32_t *__restrict__ in, int64_t n,
+                                                           bool vec, const uint32_t *__restrict__ part,
+                                                           uint32_t *__restrict__ out,
+                                                           uint32_t *__restrict__ total) {
   __shared__ uint32_t s_base;
-  uint32_t acc = 0;
-  for (int64_t k = threadIdx.x; k < blockIdx.x; k += kScanThreads) acc += part[k];
-  uint32_t sum;
-  block_excl_scan<kScanThreads>(acc, sum);
-  if (threadIdx.x == 0) s_base = sum;
-  __syncthreads();
-  const int64_t base = (int64_t)blockIdx.x * kScanTile;
-  uint32_t v[kScanItems];
-  uint32_t s = 0;
-  const int64_t tb = base + (int64_t)threadIdx.x * kScanItems;
-#pragma unroll
-  for (int k = 0; k < kScanItems; ++k) {
-    int64_t i = tb + k;
-    v[k] = i < n ? in[i] : 0u;
-    s += v[k];
+  // blocked arrangement: thread owns kScanItems consecutive items
+  const int64_t tb = (int64_t)blockIdx.x * kScanTile + (int64_t)threadIdx.x * kScanItems;
+  uint32_t v[kScanItems], s = 0;
+  scan_load<BITS>(in, n, tb, vec, v);
+  uint32_t base;
+  if (SELF) {
+    uint32_t acc = 0;
+    for (int64_t k = threadIdx.x; k < blockIdx.x; k += kScanThreads) acc += part[k];
+    uint32_t sum;
+    block_excl_scan<kScanThreads>(acc, sum);
+    if (threadIdx.x == 0) s_base = sum;
+    __syncthreads();
+    base = s_base;
+  } else {
+    base = part[blockIdx.x];
   }
+#pragma unroll
+  for (int k = 0; k < kScanItems; ++k) s += v[k];
   uint32_t tot;
-  uint32_t ex = block_excl_scan<kScanThreads>(s, tot) + s_base;
-#pragma unroll
-  for (int k = 0; k < kScanItems; ++k) {
-    int64_t i = tb + k;
-    if (i < n) out[i] = ex;
-    ex += v[k];
-  }
-  if (total && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *total = s_base + tot;
+  const uint32_t ex = block_excl_scan<kScanThreads>(s, tot) + base;
+  scan_store(out, n, tb, vec, ex, v);
+  if (SELF && total && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *total = base + tot;
 }
 
 // ---- radix sort ---------------------------------------------------------------------------
@@ -308,22 +323,33 @@ void count_launch(uint64_t n) { g_launches.fetch_add(n); }
 
 int64_t scan_temp_words(int64_t n) { return (n + kScanTile - 1) / kScanTile + 1; }
 
-void scan_u32(const uint32_t *in, uint32_t *out, int64_t n, uint32_t *d_total, uint32_t *temp,
+namespace {
+template <bool BITS>
+void scan_any(const uint32_t *in, uint32_t *out, int64_t n, uint32_t *d_total, uint32_t *temp,
               cudaStream_t s) {
-  if (n <= 0) {
-    if (d_total) cudaMemsetAsync(d_total, 0, sizeof(uint32_t), s);
-    return;
-  }
   const int64_t nb = (n + kScanTile - 1) / kScanTile;
-  k_scan_reduce<<<(unsigned)nb, kScanThreads, 0, s>>>(in, n, temp);
+  const bool vin = (reinterpret_cast<uintptr_t>(in) & 15u) == 0;
+  const bool vec = vin && (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
+  k_scan_reduce<BITS><<<(unsigned)nb, kScanThreads, 0, s>>>(in, n, vin, temp);
   if (nb <= kFusedTiles) {
-    k_scan_down_fused<<<(unsigned)nb, kScanThreads, 0, s>>>(in, n, temp, out, d_total);
+    k_scan_down<BITS, true><<<(unsigned)nb, kScanThreads, 0, s>>>(in, n, vec, temp, out, d_total);
     count_launch(2);
     return;
   }
   k_scan_partials<<<1, 1024, 0, s>>>(temp, nb, d_total);
-  k_scan_down<<<(unsigned)nb, kScanThreads, 0, s>>>(in, n, temp, out);
+  k_scan_down<BITS, false><<<(unsigned)nb, kScanThreads, 0, s>>>(in, n, vec, temp, out, nullptr);
   count_launch(3);
+}
+}  // namespace
+
+void scan_u32(const uint32_t *in, uint32_t *out, int64_t n, uint32_t *d_total, uint32_t *temp,
+              cudaStream_t s, bool bits) {
+  if (n <= 0) {
+    if (d_total) cudaMemsetAsync(d_total, 0, sizeof(uint32_t), s);
+    return;
+  }
+  if (bits) scan_any<true>(in, out, n, d_total, temp, s);
+  else scan_any<false>(in, out, n, d_total, temp, s);
 }
 
 int64_t sort_temp_words(int64_t n) {
@@ -370,9 +396,9 @@ __device__ __forceinline__ uint32_t cs_rank(const BatchDev &bd, const MeshDesc &
                                             const uint32_t *__restrict__ kpre, uint32_t key,
                                             int64_t nseg) {
   const int64_t w = d.word_base + (key >> 5);
-  const uint32_t word = bd.kmask[w], bit = 1u << (key & 31u);
-  if (!(word & bit)) return (uint32_t)nseg;
-  return kpre[w] - kpre[0] + __popc(word & (bit - 1u));
+  const uint32_t word = __ldg(bd.kmask + w), bit = 1u << (key & 31u);
+  const uint32_t rank = __ldg(kpre + w) - __ldg(kpre) + __popc(word & (bit - 1u));
+  return (word & bit) ? rank : (uint32_t)nseg;
 }
 
 // The block's pair tile: from the host's list, or (one-graph calls, tiles == nullptr) from the
@@ -402,10 +428,21 @@ __global__ void __launch_bounds__(kSortThreads) k_cs_count(BatchDev bd,
   if (bd.plan) nseg = bd.plan->ub;
   const MeshDesc &d = bd.md[st.mesh];
   const int64_t in0 = d.emit_base + (int64_t)st.j * kSortTile;
-  for (int i = threadIdx.x; i < st.count; i += kSortThreads) {
-    const uint32_t g = cs_rank(bd, d, kpre, keys[in0 + i], nseg);
-    if (g < nseg) atomicAdd(cnt + g, 1u);
+  // a tile's pairs at once, so that a thread's loads are in flight together (one pair after the other,
+  // the count and the scatter took 11 and 20 us from 90k to 850k pairs; now 8 and 10 to 9 and 14)
+  uint32_t key[kSortRounds];
+#pragma unroll
+  for (int r = 0; r < kSortRounds; ++r) {
+    const int i = r * kSortThreads + (int)threadIdx.x;
+    key[r] = i < st.count ? __ldg(keys + in0 + i) : 0u;
   }
+  uint32_t g[kSortRounds];
+#pragma unroll
+  for (int r = 0; r < kSortRounds; ++r)
+    g[r] = r * kSortThreads + (int)threadIdx.x < st.count ? cs_rank(bd, d, kpre, key[r], nseg) : (uint32_t)nseg;
+#pragma unroll
+  for (int r = 0; r < kSortRounds; ++r)
+    if (g[r] < nseg) atomicAdd(cnt + g[r], 1u);
 }
 
 // Places each pair at its voxel's segment start + (pairs of the voxel still unplaced - 1), so the
@@ -427,16 +464,29 @@ __global__ void __launch_bounds__(kSortThreads) k_cs_scatter(
   const MeshDesc &d = bd.md[st.mesh];
   const int64_t in0 = d.emit_base + (int64_t)st.j * kSortTile;
   uint32_t fin = 0;
-  for (int i = threadIdx.x; i < st.count; i += kSortThreads) {
-    const uint32_t key = keys[in0 + i];
-    const uint32_t g = cs_rank(bd, d, kpre, key, nseg);
-    if (g >= nseg) continue;
-    const uint32_t left = atomicSub(cnt + g, 1u);
-    const int64_t pos = (int64_t)useg[g] + left - 1;
-    if (left == 0 || pos >= P) continue;
-    kout[pos] = key;
-    vout[pos] = vals[in0 + i];
-    fin += left == 1u;
+  uint32_t key[kSortRounds], val[kSortRounds], g[kSortRounds];
+#pragma unroll
+  for (int r = 0; r < kSortRounds; ++r) {
+    const int i = r * kSortThreads + (int)threadIdx.x;
+    key[r] = i < st.count ? __ldg(keys + in0 + i) : 0u;
+    val[r] = i < st.count ? __ldg(vals + in0 + i) : 0u;
+  }
+#pragma unroll
+  for (int r = 0; r < kSortRounds; ++r)
+    g[r] = r * kSortThreads + (int)threadIdx.x < st.count ? cs_rank(bd, d, kpre, key[r], nseg) : (uint32_t)nseg;
+  uint32_t at[kSortRounds], left[kSortRounds];
+#pragma unroll
+  for (int r = 0; r < kSortRounds; ++r) {
+    at[r] = g[r] < nseg ? __ldg(useg + g[r]) : 0u;
+    left[r] = g[r] < nseg ? atomicSub(cnt + g[r], 1u) : 0u;
+  }
+#pragma unroll
+  for (int r = 0; r < kSortRounds; ++r) {
+    const int64_t pos = (int64_t)at[r] + left[r] - 1;
+    if (left[r] == 0 || pos >= P) continue;
+    kout[pos] = key[r];
+    vout[pos] = val[r];
+    fin += left[r] == 1u;
   }
   fin = __reduce_add_sync(0xffffffffu, fin);
   if ((threadIdx.x & 31u) == 0 && fin) atomicAdd(&s_done, fin);
