@@ -9,7 +9,7 @@
 //   SAT   -- each axis test of the SAT that crosses an edge with a box axis depends on two of the
 //            three coordinates, so the cells that pass the nine of them are the ones whose x/y, y/z
 //            and x/z squares pass three two-dimensional tests.  Those are solved a row at a time
-//            (row_span): the interval of cells that certainly pass and the one outside which every
+//            (solve_rows): the interval of cells that certainly pass and the one outside which every
 //            cell certainly fails, with the float tests' error bounds.  A sub-column's cells are the
 //            intersection of two such intervals with the plane test's, written with one atomic.
 //            Only sub-columns with a cell between the two intervals (about one in a hundred) run
@@ -99,27 +99,39 @@ __device__ __forceinline__ int batch_search(const uint32_t *pre, uint32_t it) {
   return lo;
 }
 
-constexpr int kSol = 640;    // solved rows of one batch (a triangle has at most 96); the output stage
+constexpr int kSol = 512;    // solved rows of one batch (a triangle has at most 96); the output stage
                              // keeps 16 layers of 32 lanes there
-constexpr int kRows = kSol / 2 + 32 * kDirectCells;  // its rows of sub-columns, at most
+constexpr int kCols = 1024;  // its sub-columns (a triangle has at most that many)
 
-struct WarpScratch {
-  float x[32][9];      // per-triangle constants (odd stride: no bank conflicts)
-  uint32_t rng[32][3]; // first sub-column, first row, cell range of exact-only triangles
-  uint32_t tri[32];    // triangle id
-  int jm[32];          // SAT: the triangle's voxel in the chunk; fill: voxels of the chunk up to the
-                       // triangle's topmost voxel; bit 8: exact tests only
-  uint32_t pre[33];    // exclusive prefix of the solved rows
-  uint32_t row[33];    // exclusive prefix of the rows of sub-columns
-  uint32_t seg[33];    // SAT: first pair of each voxel of the chunk, and the end
+struct __align__(16) WarpScratch {
+  float4 xa[32], xb[32];  // per-triangle constants
+  uint4 me[32];        // triangle id; voxel in the chunk (fill: voxels of the chunk up to its topmost) |
+                       // exact tests only << 8 | first sub-column << 16 | first row << 24; its solved
+                       // rows of y/z | of x/z << 16; first layer | end << 8 where tests are exact
+  uint32_t seg[36];    // SAT: first pair of each voxel of the chunk, and the end
   uint32_t sol[kSol];  // solved rows
   uint32_t rtri[64];   // queued exact work: triangle id and
   uint32_t rpos[64];   // voxel (or voxel count), sub-column and cell range
   uint32_t utri[64];   // fill: queued triangles and the voxels of the chunk that see them
   uint8_t ujm[64];
-  uint8_t own[kRows];  // triangle slot of each row of sub-columns
+  uint16_t cols[kCols];  // the batch's sub-columns: triangle slot | row << 5 | column << 10 (both from
+                         // the triangle's first) | certain to pass the x/y tests << 15
 };
-static_assert(sizeof(WarpScratch) % 4 == 0, "word layout");
+static_assert(sizeof(WarpScratch) % 16 == 0, "layout");
+
+// Lists a triangle's sub-columns from its solved x/y rows (nullptr: all np x nq, none certain).
+__device__ __forceinline__ void list_columns(uint16_t *out, const uint32_t *xy, int slot, int p0, int np,
+                                             int nq) {
+#pragma unroll 1
+  for (int dq = 0; dq < nq; ++dq) {
+    const uint32_t w = xy ? xy[dq] : (uint32_t)(p0 | ((p0 + np) << 24));
+    const int lo_i = (int)((w >> 8) & 255u), end_i = (int)((w >> 16) & 255u), end = (int)(w >> 24);
+    const uint32_t e = (uint32_t)(slot | (dq << 5));
+#pragma unroll 1
+    for (int p = (int)(w & 255u); p < end; ++p)
+      *out++ = (uint16_t)(e | (uint32_t)((p - p0) << 10) | (p >= lo_i && p < end_i ? 0x8000u : 0u));
+  }
+}
 
 struct StScratch {    // stencil fill: the batch's triangles
   float v[32][9];     // snapped vertices and heights
@@ -716,10 +728,13 @@ __device__ __forceinline__ uint32_t *sat_words(const BatchDev &bd, const MeshDes
 // 262k-triangle torus, 128^3 / 8^3; 0.2 with two kernels).  The SAT masks go through device memory
 // (one bit per cell).  Both kernels are bound by instruction issue.  Measured against one kernel
 // testing every (triangle, sub-column) and listed cell exactly, both kernels together: the torus
-// 487 -> 275 us, a 1.3M-triangle star at 256^3 / 16^3 3.51 -> 1.76 ms, 256 mixed meshes in one call
-// 19.9 -> 11.7 ms, 7k large triangles at 150x170x130 / 6^3 279 -> 154 us.  A twentieth of the
-// instructions are exact tests (0.4-2.7% of the sub-columns); a lane per solved row instead of a lane
-// per triangle looping over its rows took 190 us for the torus' SAT against 134.
+// 487 -> 197 us, a 1.3M-triangle star at 256^3 / 16^3 3.51 -> 1.27 ms, 256 mixed meshes in one call
+// 19.9 -> 9.9 ms.  A twentieth of the instructions are exact tests (0.4-2.7% of the sub-columns).
+// Rows are solved by a lane per triangle looping over them (a lane per row took 190 us for the torus'
+// SAT against 134); the sub-columns they leave are listed and taken a lane each, because lanes that
+// walked their own row had 43-52% of them at work in the SAT and 34% in the fill (the star: SAT
+// 787 -> 690 us, fill 712 -> 577; the torus 135 -> 113 and 101 -> 84; the batch 5.7 -> 5.4 ms and
+// 5.1 -> 4.5).
 //
 // k_level2c_sat: bd.smask gets every boundary voxel's mask of Level2 boundary cells.
 __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_sat(
@@ -727,7 +742,7 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_sat(
     const uint32_t *__restrict__ useg, const Item *__restrict__ items,
     const uint32_t *__restrict__ nitems, int per_warp, int slab, const uint32_t *__restrict__ ilist,
     const uint32_t *__restrict__ ioff, int parts) {
-  extern __shared__ uint32_t sm[];
+  extern __shared__ __align__(16) uint32_t sm[];
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   WarpScratch &ws = *reinterpret_cast<WarpScratch *>(sm + (size_t)warp * per_warp);
   int *const kz = reinterpret_cast<int *>(&ws + 1);
@@ -769,14 +784,14 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_sat(
     const uint32_t n0 = ws.seg[0], np_ = ws.seg[m] - n0;
     const uint32_t S0 = n0 + (uint32_t)((uint64_t)np_ * part / (uint32_t)parts);
     const uint32_t S1 = n0 + (uint32_t)((uint64_t)np_ * (part + 1) / (uint32_t)parts);
-    uint32_t taken;  // pairs of a batch: 32, fewer where their rows would not fit
+    uint32_t taken;  // pairs of a batch: 32, fewer where their rows or sub-columns would not fit
 #pragma unroll 1
     for (uint32_t b0 = S0; b0 < S1; b0 += taken) {
       // ---- one triangle per lane: its cell ranges, its plane and its rows
       const uint32_t e = b0 + lane;
       int p0 = 0, p1 = -1, pi = 0, pe = 0, q0 = 0, q1 = -1, qi = 0, qe = 0, r0 = 0, r1 = -1, ri = 0, re = 0;
-      bool direct = false;
-      uint32_t nsolve = 0, nrow = 0, t = 0;
+      bool direct = false, on = false;
+      uint32_t nsolve = 0, ncol = 0, t = 0;
       int jv = 0;  // last voxel whose segment starts at or before e
       float4 a0, a1, a2;
       float R = 0.f, tz = 0.f;
@@ -810,25 +825,20 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_sat(
           // A few cells are tested as fast as they are solved; outside these magnitudes the
           // bounds' own arithmetic could leave the normal range.
           direct = np * nq * (r1 - r0 + 1) <= kDirectCells || !(R > 1e-9f && R < 1e9f);
-          nrow = (uint32_t)nq;
+          on = true;
           nsolve = direct ? 0u : (uint32_t)(2 * nq + np);
-          // (exact-only triangles outside the magnitudes have rows too, without solved ones)
         }
       }
-      const uint32_t is = warp_incl_scan(nsolve), ir = warp_incl_scan(nrow);
-      taken = (uint32_t)__popc(__ballot_sync(FULL, is <= (uint32_t)kSol && ir <= (uint32_t)kRows));
-      if (lane == 0) ws.row[0] = 0;
-      ws.row[lane + 1] = ir;
-      if (lane < taken && nrow) {
-        ws.rng[lane][0] = (uint32_t)(p0 | ((p1 + 1) << 8));
-        ws.rng[lane][1] = (uint32_t)q0;
-        ws.rng[lane][2] = (uint32_t)(r0 | ((r1 + 1) << 8));
-        ws.tri[lane] = t;
-        ws.jm[lane] = jv | (direct ? 256 : 0);
-        ws.pre[lane] = is - nsolve;
-        uint8_t *own = ws.own + (ir - nrow);
-#pragma unroll 1
-        for (uint32_t k = 0; k < nrow; ++k) own[k] = (uint8_t)lane;
+      const uint32_t is = warp_incl_scan(nsolve);
+      taken = (uint32_t)__popc(__ballot_sync(FULL, is <= (uint32_t)kSol));
+      on = on && lane < taken;
+      const uint32_t so0 = is - nsolve;
+      if (on) {
+        const int np_ = p1 - p0 + 1, nq_ = q1 - q0 + 1;
+        ws.me[lane] = make_uint4(t, (uint32_t)(jv | (direct ? 256 : 0) | (p0 << 16) | (q0 << 24)),
+                                 (so0 + (uint32_t)nq_) | ((so0 + 2u * (uint32_t)nq_) << 16),
+                                 (uint32_t)(r0 | ((r1 + 1) << 8)));
+        ncol = (uint32_t)(np_ * nq_);
         if (!direct) {
           const int np = p1 - p0 + 1, nq = q1 - q0 + 1;
           const float c0x = __ldg(sx + p0), c0y = __ldg(sy + q0), c0z = __ldg(sz + r0);
@@ -844,99 +854,67 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_sat(
                           1.1f * (fabsf(nx) * tx + fabsf(ny) * ty + nz_ * tz);
           const float inv = rcp_fast(fmaxf(nz_ * gz, E * (1.f / 512.f)));
           const float w = ff(E, inv, kIdx);
-          ws.x[lane][0] = nx * ux + ny * uy + nz_ * uz;
-          ws.x[lane][1] = nx * gx;
-          ws.x[lane][2] = ny * gy;
-          ws.x[lane][3] = fabsf(nx) * h0 + fabsf(ny) * h1 + nz_ * h2;
-          ws.x[lane][4] = inv;
-          ws.x[lane][5] = (float)r0 - w;
-          ws.x[lane][6] = (float)r0 + w;
+          ws.xa[lane] = make_float4(nx * ux + ny * uy + nz_ * uz, nx * gx, ny * gy,
+                                    fabsf(nx) * h0 + fabsf(ny) * h1 + nz_ * h2);
+          ws.xb[lane] = make_float4(inv, (float)r0 - w, (float)r0 + w, 0.f);
           const float dl = 72.f * EPS24 * R * R, bx = 1.1f * tx, by = 1.1f * ty, bz = 1.1f * tz;
-          uint32_t *so = ws.sol + (is - nsolve);
+          uint32_t *so = ws.sol + so0;
           const uint32_t xl = (uint32_t)(p0 | (pi << 16)), xe = (uint32_t)(pe | ((p1 + 1) << 16));
           const uint32_t zl = (uint32_t)(r0 | (ri << 16)), ze = (uint32_t)(re | ((r1 + 1) << 16));
-          solve_rows(so, nq, ux, vx, wx, uy, vy, wy, h0, h1, gx, gy, dl, bx, by, p0, xl, xe, qi - q0, qe - q0);
+          ncol = solve_rows(so, nq, ux, vx, wx, uy, vy, wy, h0, h1, gx, gy, dl, bx, by, p0, xl, xe, qi - q0, qe - q0);
           solve_rows(so + nq, nq, uz, vz, wz, uy, vy, wy, h2, h1, gz, gy, dl, bz, by, r0, zl, ze, qi - q0, qe - q0);
           solve_rows(so + 2 * nq, np, uz, vz, wz, ux, vx, wx, h2, h0, gz, gx, dl, bz, bx, r0, zl, ze, pi - p0, pe - p0);
         }
       }
+      // ---- the sub-columns that can pass x/y, listed so that every lane takes one
+      if (!on) ncol = 0;
+      const uint32_t ic = warp_incl_scan(ncol);
+      taken = (uint32_t)__popc(__ballot_sync(FULL, lane < taken && ic <= (uint32_t)kCols));
+      if (on && lane < taken)
+        list_columns(ws.cols + (ic - ncol), direct ? nullptr : ws.sol + so0, (int)lane, p0, p1 - p0 + 1, q1 - q0 + 1);
+      const uint32_t C = __shfl_sync(FULL, ic, (int)taken - 1);
       __syncwarp();
-      // ---- one lane per row of sub-columns, a sub-column at a time
-      const uint32_t R1 = ws.row[taken];
 #pragma unroll 1
-      for (uint32_t rb0 = 0; rb0 < R1; rb0 += 32) {
-        const uint32_t rw = rb0 + lane;
-        int p = 0, pend = 0, pi_ = 0, pe_ = 0, q = 0, jv_ = 0, solz = 0, rlo = 0, rend = 0;
-        uint32_t YL = 0, YE = 0, tri = 0;
-        float num = 0.f, nxg = 0.f, Hs = 0.f, inv = 0.f, k1 = 0.f, k2 = 0.f;
-        bool dir = false;
-        if (rw < R1) {
-          const int tl = ws.own[rw];
-          const int dq = (int)(rw - ws.row[tl]), nq = (int)(ws.row[tl + 1] - ws.row[tl]);
-          const int jm = ws.jm[tl];
-          jv_ = jm & 255;
-          dir = (jm & 256) != 0;
-          tri = ws.tri[tl];
-          q = (int)ws.rng[tl][1] + dq;
-          const uint32_t rx = ws.rng[tl][0];
-          p = (int)(rx & 255u);
-          if (dir) {
-            const uint32_t rz = ws.rng[tl][2];
-            pend = (int)(rx >> 8);
-            rlo = (int)(rz & 255u);
-            rend = (int)(rz >> 8);
+      for (uint32_t c0 = 0; c0 < C; c0 += 32) {
+        const uint32_t c = c0 + lane;
+        bool amb = false;
+        uint32_t tri = 0, pos = 0;
+        if (c < C) {
+          const uint32_t en = ws.cols[c];
+          const int tl = (int)(en & 31u), dq = (int)((en >> 5) & 31u), dp = (int)((en >> 10) & 31u);
+          const uint4 me = ws.me[tl];
+          const int p = (int)((me.y >> 16) & 255u) + dp, q = (int)(me.y >> 24) + dq;
+          const int j = (int)(me.y & 255u);
+          int lo, end;
+          if (me.y & 256u) {
+            lo = (int)(me.w & 255u);
+            end = (int)(me.w >> 8);
+            amb = true;
           } else {
-            const uint32_t *so = ws.sol + ws.pre[tl];
-            const uint32_t sxy = so[dq], syz = so[nq + dq];
-            solz = (int)ws.pre[tl] + 2 * nq - p;
-            p = (int)(sxy & 255u);
-            pi_ = (int)((sxy >> 8) & 255u);
-            pe_ = (int)((sxy >> 16) & 255u);
-            pend = (int)(sxy >> 24);
-            YL = __byte_perm(syz, 0, 0x4140);
-            YE = __byte_perm(syz, 0, 0x4342);
-            nxg = ws.x[tl][1];
-            num = ff(-(float)(p - (int)(rx & 255u)), nxg, ff(-(float)dq, ws.x[tl][2], ws.x[tl][0]));
-            Hs = ws.x[tl][3];
-            inv = ws.x[tl][4];
-            k1 = ws.x[tl][5];
-            k2 = ws.x[tl][6];
+            const float4 xa = ws.xa[tl], xb = ws.xb[tl];
+            const uint32_t syz = ws.sol[(me.z & 0xffffu) + (uint32_t)dq], sxz = ws.sol[(me.z >> 16) + (uint32_t)dp];
+            const float nv = ff(-(float)dp, xa.y, ff(-(float)dq, xa.z, xa.x));
+            const float va = nv - xa.w, vb = nv + xa.w;
+            const uint32_t L = __vimax3_s16x2(cvt_pair_ceil(ff(va, xb.x, xb.y), ff(va, xb.x, xb.z)),
+                                              __byte_perm(syz, 0, 0x4140), __byte_perm(sxz, 0, 0x4140));
+            const uint32_t E = __vimin3_s16x2(
+                cvt_pair_floor(ff(vb, xb.x, xb.y + 1.f), ff(vb, xb.x, xb.z + 1.f)),
+                __byte_perm(syz, 0, 0x4342), __byte_perm(sxz, 0, 0x4342));
+            const int lo_i = (int)L >> 16, end_i = (int)(short)(E & 0xffffu);
+            lo = (int)(short)(L & 0xffffu);
+            end = (int)E >> 16;
+            const bool sure = (en & 0x8000u) != 0;
+            if (sure && lo_i < end_i)
+              or_column(sat + j * W, q * n2x + p, n2z, (0xffffffffu >> (32 - (end_i - lo_i))) << lo_i);
+            amb = lo < end && !(sure && lo == lo_i && end == end_i);
           }
+          tri = me.x;
+          pos = (uint32_t)(j | (p << 5) | (q << 10) | (lo << 15) | (end << 21));
         }
-        uint32_t *satj = sat + jv_ * W;
-        float dp = 0.f;
-        const float k1e = k1 + 1.f, k2e = k2 + 1.f;
-#pragma unroll 1
-        while (__any_sync(FULL, p < pend)) {
-          bool amb = false;
-          int lo = rlo, end = rend;
-          if (p < pend) {
-            amb = dir;
-            if (!dir) {
-              const float nv = ff(-dp, nxg, num);
-              const float va = nv - Hs, vb = nv + Hs;
-              const uint32_t sxz = ws.sol[solz + p];
-              const uint32_t L = __vimax3_s16x2(cvt_pair_ceil(ff(va, inv, k1), ff(va, inv, k2)), YL,
-                                                __byte_perm(sxz, 0, 0x4140));
-              const uint32_t E = __vimin3_s16x2(cvt_pair_floor(ff(vb, inv, k1e), ff(vb, inv, k2e)), YE,
-                                                __byte_perm(sxz, 0, 0x4342));
-              const int lo_i = (int)L >> 16, end_i = (int)(short)(E & 0xffffu);
-              lo = (int)(short)(L & 0xffffu);
-              end = (int)E >> 16;
-              const bool sure = p >= pi_ && p < pe_;
-              if (sure && lo_i < end_i)
-                or_column(satj, q * n2x + p, n2z, (0xffffffffu >> (32 - (end_i - lo_i))) << lo_i);
-              amb = lo < end && !(sure && lo == lo_i && end == end_i);
-            }
-          }
-          nrec = queue_push(ws, nrec, amb, tri,
-                            (uint32_t)(jv_ | (p << 5) | (q << 10) | (lo << 15) | (end << 21)));
-          if (nrec >= 32) {
-            sat_exact(d, ws, sat, kz, ci, cj, 32);
-            nrec = queue_shift(ws, nrec);
-          }
-          ++p;
-          dp += 1.f;
+        nrec = queue_push(ws, nrec, amb, tri, pos);
+        if (nrec >= 32) {
+          sat_exact(d, ws, sat, kz, ci, cj, 32);
+          nrec = queue_shift(ws, nrec);
         }
       }
       __syncwarp();
@@ -963,7 +941,7 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_fill(
     const uint32_t *__restrict__ useg, const Item *__restrict__ items,
     const uint32_t *__restrict__ nitems, int per_warp, int slab, const uint32_t *__restrict__ ilist,
     const uint32_t *__restrict__ ioff, int) {
-  extern __shared__ uint32_t sm[];
+  extern __shared__ __align__(16) uint32_t sm[];
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   WarpScratch &ws = *reinterpret_cast<WarpScratch *>(sm + (size_t)warp * per_warp);
   int *const kz = reinterpret_cast<int *>(&ws + 1);
@@ -1195,8 +1173,8 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_fill(
     }
 #pragma unroll 1
     while (nuni >= 32 || (nuni > 0 && b0 + 32 >= f1)) {
-    uint32_t nsolve = 0, nrow = 0;
-    int p0 = 0, p1 = 0;
+    uint32_t nsolve = 0, ncol = 0;
+    int p0 = 0, p1 = 0, nq = 0;
     float ux = 0.f, uy = 0.f, vx = 0.f, vy = 0.f, wx = 0.f, wy = 0.f, dl = 0.f;
     bool direct = false;
     if (lane < nuni) {
@@ -1210,7 +1188,8 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_fill(
         const int q0 = max(__float2int_ru((fb.y - oy0) * g.inv_g2[1] - my), 0);
         const int q1 = min(__float2int_rd((fb.w - oy0) * g.inv_g2[1] + my), n2y - 1);
         if (p0 <= p1 && q0 <= q1) {
-          const int np = p1 - p0 + 1, nq = q1 - q0 + 1;
+          const int np = p1 - p0 + 1;
+          nq = q1 - q0 + 1;
           const float4 a0 = __ldg(ptri + 3 * (size_t)t), a1 = __ldg(ptri + 3 * (size_t)t + 1),
                        a2 = __ldg(ptri + 3 * (size_t)t + 2);
           const float o0 = __ldg(ox + p0), o1 = __ldg(oy + q0);
@@ -1224,7 +1203,7 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_fill(
           // solve_rows' sides by less than 42: 90, 96 with the slope's.  An unbounded box marks an
           // ill-conditioned x/y projection, which has no bound on t: exact tests only.
           direct = !g.oz_monotone || isinf(fb.x) || isinf(fb.z) || !(R > 1e-9f && R < 1e9f);
-          nrow = (uint32_t)nq;
+          ncol = (uint32_t)(np * nq);
           if (!direct) {
             nsolve = (uint32_t)nq;
             // The plane's height over an origin is affine in (p, q): X = its height above the
@@ -1245,72 +1224,44 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_fill(
             const float w = igz * (EPS24 * (40.f * M0 * fabsf(rn) + 8.f * zt2) + toz + 0.35f * g.thr) +
                             fabsf(Kx) * tox + fabsf(Ky) * toy + 8.f * EPS24 * (float)span + kIdx;
             dl = 104.f * EPS24 * R * R;
-            ws.x[lane][1] = ((a0.z - ozb) - g.thr) * igz - Kx * ux - Ky * uy;
-            ws.x[lane][2] = Kx * gx;
-            ws.x[lane][3] = Ky * gy;
-            ws.x[lane][4] = w;
+            ws.xa[lane] = make_float4(((a0.z - ozb) - g.thr) * igz - Kx * ux - Ky * uy, Kx * gx, Ky * gy, w);
           }
-          ws.rng[lane][0] = (uint32_t)(p0 | ((p1 + 1) << 8));
-          ws.rng[lane][1] = (uint32_t)q0;
-          ws.tri[lane] = t;
-          ws.jm[lane] = jm | (direct ? 256 : 0);
+          ws.me[lane] = make_uint4(t, (uint32_t)(jm | (direct ? 256 : 0) | (p0 << 16) | (q0 << 24)), 0u, 0u);
         }
       }
     }
-    const uint32_t is = warp_incl_scan(nsolve), ir = warp_incl_scan(nrow);
-    // triangles of this batch: 32 (or the queue's last), fewer where their rows would not fit
-    const uint32_t taken = (uint32_t)__popc(
-        __ballot_sync(FULL, lane < nuni && is <= (uint32_t)kSol && ir <= (uint32_t)kRows));
-    if (lane == 0) ws.row[0] = 0;
-    ws.row[lane + 1] = ir;
-    if (lane < taken && nrow) {
-      ws.pre[lane] = is - nsolve;
-      uint8_t *own = ws.own + (ir - nrow);
-#pragma unroll 1
-      for (uint32_t k = 0; k < nrow; ++k) own[k] = (uint8_t)lane;
-      if (nsolve)
-        solve_rows(ws.sol + (is - nsolve), (int)nrow, ux, vx, wx, uy, vy, wy, 0.f, 0.f, gx, gy, dl, 1.1f * tox,
-                   1.1f * toy, p0, (uint32_t)p0, (uint32_t)(n2x | ((p1 + 1) << 16)), 0, 64);
-    }
+    const uint32_t is = warp_incl_scan(nsolve);
+    // triangles of this batch: 32 (or the queue's last), fewer where their rows or sub-columns would
+    // not fit
+    uint32_t taken = (uint32_t)__popc(__ballot_sync(FULL, lane < nuni && is <= (uint32_t)kSol));
+    if (lane >= taken) ncol = 0;
+    if (ncol && nsolve)
+      ncol = solve_rows(ws.sol + (is - nsolve), nq, ux, vx, wx, uy, vy, wy, 0.f, 0.f, gx, gy, dl, 1.1f * tox,
+                        1.1f * toy, p0, (uint32_t)p0, (uint32_t)(n2x | ((p1 + 1) << 16)), 0, 64);
+    const uint32_t ic = warp_incl_scan(ncol);
+    taken = (uint32_t)__popc(__ballot_sync(FULL, lane < taken && ic <= (uint32_t)kCols));
+    if (ncol && lane < taken)
+      list_columns(ws.cols + (ic - ncol), nsolve ? ws.sol + (is - nsolve) : nullptr, (int)lane, p0, p1 - p0 + 1, nq);
+    const uint32_t C = __shfl_sync(FULL, ic, (int)taken - 1);
     __syncwarp();
     {
-      const uint32_t R1 = ws.row[taken];
 #pragma unroll 1
-      for (uint32_t rb0 = 0; rb0 < R1; rb0 += 32) {
-        const uint32_t rw = rb0 + lane;
-        int p = 0, pend = 0, pi = 0, pe = 0, q = 0, jm = 0;
-        uint32_t tri = 0;
-        float X = 0.f, Kx = 0.f, wx_ = 0.f;
-        if (rw < R1) {
-          const int tl = ws.own[rw];
-          const int dq = (int)(rw - ws.row[tl]);
-          const uint32_t rx = ws.rng[tl][0];
-          jm = ws.jm[tl];
-          tri = ws.tri[tl];
-          q = (int)ws.rng[tl][1] + dq;
-          if (jm & 256) {  // nothing certain
-            jm &= 255;
-            p = (int)(rx & 255u);
-            pend = (int)(rx >> 8);
-          } else {
-            const uint32_t sxy = ws.sol[ws.pre[tl] + dq];
-            p = (int)(sxy & 255u);
-            pi = (int)((sxy >> 8) & 255u);
-            pe = (int)((sxy >> 16) & 255u);
-            pend = (int)(sxy >> 24);
-            Kx = ws.x[tl][2];
-            X = ff((float)(p - (int)(rx & 255u)), Kx, ff((float)dq, ws.x[tl][3], ws.x[tl][1]));
-            wx_ = ws.x[tl][4];
-          }
-        }
-        float dp = 0.f;
-#pragma unroll 1
-        while (__any_sync(FULL, p < pend)) {
-          bool amb = false;
-          if (p < pend) {
-            const float x = ff(dp, Kx, X);
-            const int N = min(max(__float2int_ru(x - wx_), 0), span);
-            amb = p < pi || p >= pe || N != min(max(__float2int_ru(x + wx_), 0), span);
+      for (uint32_t c0 = 0; c0 < C; c0 += 32) {
+        const uint32_t c = c0 + lane;
+        bool amb = false;
+        uint32_t tri = 0, pos = 0;
+        if (c < C) {
+          const uint32_t en = ws.cols[c];
+          const int tl = (int)(en & 31u), dq = (int)((en >> 5) & 31u), dp = (int)((en >> 10) & 31u);
+          const uint4 me = ws.me[tl];
+          const int p = (int)((me.y >> 16) & 255u) + dp, q = (int)(me.y >> 24) + dq;
+          const int jm = (int)(me.y & 255u);
+          amb = !(en & 0x8000u);
+          if (!amb) {
+            const float4 xa = ws.xa[tl];
+            const float x = ff((float)dp, xa.y, ff((float)dq, xa.z, xa.x));
+            const int N = min(max(__float2int_ru(x - xa.w), 0), span);
+            amb = N != min(max(__float2int_ru(x + xa.w), 0), span);
             if (!amb && N > 0) {
               const int pq = q * n2x + p;
               const int kq = __float2int_rz(((float)N + 0.5f) * inv_n2z), rem = N - kq * n2z;
@@ -1333,13 +1284,13 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_fill(
               if (here && rem > 0 && below < jm) xor_column(par + below * W, pq, n2z, (1u << rem) - 1u);
             }
           }
-          nrec = queue_push(ws, nrec, amb, tri, (uint32_t)(jm | (p << 6) | (q << 11)));
-          if (nrec >= 32) {
-            fill_exact(d, ws, par, ft, kz, m, ci, cj, 32);
-            nrec = queue_shift(ws, nrec);
-          }
-          ++p;
-          dp += 1.f;
+          tri = me.x;
+          pos = (uint32_t)(jm | (p << 6) | (q << 11));
+        }
+        nrec = queue_push(ws, nrec, amb, tri, pos);
+        if (nrec >= 32) {
+          fill_exact(d, ws, par, ft, kz, m, ci, cj, 32);
+          nrec = queue_shift(ws, nrec);
         }
       }
       __syncwarp();
@@ -1432,7 +1383,8 @@ Level2Words level2_warp_words(const GridDev &g, int cap, bool stencil) {
   const int CH = level2_chunk(g, cap);
   const int FWS = (4 * g.n2[0] * g.n2[1] + 31) >> 5;
   const int base = (int)(sizeof(WarpScratch) / 4) + 32;
-  return {base + CH * W, base + CH * W + CH * FW + (stencil ? 4 * CH * W + CH * FWS + FWS : 0)};
+  auto al = [](int words) { return (words + 3) & ~3; };  // a warp's region starts 16-byte aligned
+  return {al(base + CH * W), al(base + CH * W + CH * FW + (stencil ? 4 * CH * W + CH * FWS + FWS : 0))};
 }
 
 int level2_parts(int64_t B, int num_sms) {

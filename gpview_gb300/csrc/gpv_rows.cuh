@@ -57,11 +57,11 @@ __device__ __forceinline__ EdgeRows edge_rows(float ea, float eb, float a, float
   return {fminf(x1, x2) - w + base, fmaxf(x1, x2) + w + base, 2.f * w, ea * gb * inv};
 }
 
-// Solves rows 0 .. n-1 into out[]: [lo_o, end_o) holds every i of the row that can pass, [lo_i, end_i)
-// only ones that do; one byte each, lo_o | lo_i << 8 | end_i << 16 | end_o << 24.  bl and be are the
+// Solves rows 0 .. n-1 into out[] and returns the number of cells that can pass.  A row's [lo_o, end_o)
+// holds every i that can pass, [lo_i, end_i) only ones that do; one byte each, lo_o | lo_i << 8 | end_i << 16 | end_o << 24.  bl and be are the
 // i that can and that certainly pass the a axis' own test (lo_o | lo_i << 16 and end_i | end_o << 16),
 // and rows outside [in_lo, in_end) may fail the b axis' own: they pass nothing for certain.
-__device__ __forceinline__ void solve_rows(uint32_t *out, int n, float a0, float a1, float a2, float b0,
+__device__ __forceinline__ uint32_t solve_rows(uint32_t *out, int n, float a0, float a1, float a2, float b0,
                                            float b1, float b2, float ha, float hb, float ga, float gb,
                                            float dl, float ta, float tb, int base, uint32_t bl,
                                            uint32_t be, int in_lo, int in_end) {
@@ -72,6 +72,7 @@ __device__ __forceinline__ void solve_rows(uint32_t *out, int n, float a0, float
   const EdgeRows r1 = edge_rows(e1a, e1b, a1, b1, ha, hb, ga, gb, sn, sp, dl, ta, tb, fb);
   const EdgeRows r2 = edge_rows(e2a, e2b, a2, b2, ha, hb, ga, gb, sn, sp, dl, ta, tb, fb);
   float k = 0.f;
+  uint32_t cells = 0;
 #pragma unroll 1
   for (int i = 0; i < n; ++i, k += 1.f) {
     const float l0 = ff(k, r0.s, r0.lo), l1 = ff(k, r1.s, r1.lo), l2 = ff(k, r2.s, r2.lo);
@@ -83,7 +84,9 @@ __device__ __forceinline__ void solve_rows(uint32_t *out, int n, float a0, float
     uint32_t E = __vmaxs2(__vmins2(cvt_pair_floor(hi_i + 1.f, hi_o + 1.f), be), 0u);
     if (i < in_lo || i >= in_end) E &= 0xffff0000u;
     out[i] = __byte_perm(L, E, 0x6420);
+    cells += (uint32_t)max((int)E >> 16, (int)(L & 0xffffu)) - (L & 0xffffu);
   }
+  return cells;
 }
 
 // Cells of one axis whose boxes can meet [tmin, tmax] ([lo, hi]) and those that certainly do

@@ -68,3 +68,16 @@ def test_large_triangles(ctx, built, n1, n2):
     tris = np.ascontiguousarray(np.concatenate([box, sliver]), np.float32).reshape(-1)
     mn, mx = gpv.mesh_bounds(tris)
     _check(ctx, gpv, tris, gpv.grid_padded(mn, mx, n1, n2))
+
+
+@pytest.mark.parametrize("n2", [(32, 32, 1), (32, 32, 32), (31, 32, 5), (16, 32, 8)])
+def test_full_column_lists(ctx, built, n2):
+    # near-horizontal sheets wider than the grid: each triangle leaves (nearly) all sub-columns of its
+    # voxels, so one triangle fills the list of a batch and the others wait for the next
+    gpv = built
+    z = np.array([0.11, 0.12, 0.48, 0.48, 0.83])
+    quad = np.array([[[-9, -9, 0], [9, -9, 0], [9, 9, 0]], [[-9, -9, 0], [9, 9, 0], [-9, 9, 0]]], np.float64)
+    t = np.concatenate([quad + [0, 0, v] for v in z])
+    t[4:] += t[4:, :, :1] * [0, 0, 0.013] + t[4:, :, 1:2] * [0, 0, 0.007]
+    tris = np.ascontiguousarray(t, np.float32).reshape(-1)
+    _check(ctx, gpv, tris, _spec(gpv, (0, 0, 0), (1, 1, 1), [2, 3, 4], list(n2)))
