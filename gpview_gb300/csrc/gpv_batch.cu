@@ -610,7 +610,7 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
         count_sort_pairs(bdp, nullptr, cap.tiles, keys, vals, wpre + words, cap.U, cap.P, cnt,
                          useg, kalt, valt, wtot + 1, sortmp, s);
         mark(7);
-        launch_level2(bdp, kalt, valt, useg, cap.U, l2tmp, level2_mask_words(cap.U, cap.l2bytes), l2_words, ctx->num_sms, s,
+        launch_level2(bdp, kalt, valt, useg, wpre + words, cap.U, l2tmp, level2_mask_words(cap.U, cap.l2bytes), l2_words, ctx->num_sms, s,
                       [&] { mark(9); });
       } else {
         mark(7);
@@ -927,7 +927,7 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
       }
       mark(7);
       if (any_l2)
-        launch_level2(bd, sk, sv, useg, ub, l2tmp, level2_mask_words(ub, l2bytes), l2_words, ctx->num_sms, s, [&] { mark(9); },
+        launch_level2(bd, sk, sv, useg, wpre + words, ub, l2tmp, level2_mask_words(ub, l2bytes), l2_words, ctx->num_sms, s, [&] { mark(9); },
                       zslab, nslab, [&](int k, cudaStream_t ls) {
                         if (packed) {  // the host expands this slab's codes once it is done
                           cudaEventRecord(ctx->cev[1 + k], ls);

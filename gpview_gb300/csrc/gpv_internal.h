@@ -107,7 +107,8 @@ constexpr int kFillNone = -1;
 // than 8 for the packed host transfer (star1310k host to host 6.58 against 6.43 ms): each slab
 // launch adds its ramp and tail
 constexpr int kSlabsMax = 8;
-constexpr int kQueueWords = 1 + 2 * kSlabsMax;
+constexpr int kQueueItems = 1 + 2 * kSlabsMax;
+constexpr int kQueueWords = kQueueItems + 1;
 constexpr uint32_t kHeavyCap = 1u << 18;  // pieces of a call's heavy list (4 MiB)
 
 constexpr int kFinishGroups = 8;  // plane words of a layer that one fill-finish block takes
@@ -120,7 +121,8 @@ struct BatchDev {
   int64_t total_tris, total_tiles, total_fblks, total_rows, total_words;
   int64_t total_xchunks;  // 128-voxel expansion chunks of all meshes
   uint32_t *queue;       // work-queue tickets, zeroed by the caller: [0] Level1, [1 + k] and
-                         // [1 + kSlabsMax + k] the fill and the SAT kernel of Level2 slab k
+                         // [1 + kSlabsMax + k] the fill and the SAT kernel of Level2 slab k,
+                         // [kQueueItems] the number of Level2 work items
   int normals;           // GPV_NORMALS_* of this batch
   int fill;              // GPV_FILL_* of this batch
   uint32_t *stp;         // stencil fill: per boundary voxel, the sample-coverage parity of the
@@ -258,7 +260,7 @@ struct SlabStreams {  // two streams and their events for overlapping slab launc
   cudaEvent_t fork, join[2];
 };
 void launch_level2(const BatchDev &bd, const uint32_t *keys, const uint32_t *vals,
-                   const uint32_t *useg, int64_t Btot, uint32_t *tmp, int64_t smask_words, Level2Words words, int num_sms,
+                   const uint32_t *useg, const uint32_t *kpre, int64_t Btot, uint32_t *tmp, int64_t smask_words, Level2Words words, int num_sms,
                    cudaStream_t s, const std::function<void()> &before_kernel = {}, int zslab = 0,
                    int nslab = 1, const std::function<void(int, cudaStream_t)> &after_slab = {},
                    int slab_nz = 0, const SlabStreams *aux = nullptr);

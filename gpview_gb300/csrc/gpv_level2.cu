@@ -159,59 +159,6 @@ __device__ __forceinline__ int64_t sorted_voxels(const BatchDev &bd, int64_t B) 
   return bd.plan->ok ? min(B, (int64_t)bd.plan->ub) : 0;
 }
 
-// cflag[u] = 1 where a new Level1 column starts (a mesh's first boundary voxel, or a column
-// change within the mesh).  One-graph calls: zero past the device count (the scans run over the
-// capacity), and no work items until k_itemstarts counts them.
-__global__ void k_colflags(BatchDev bd, const uint32_t *__restrict__ keys,
-                           const uint32_t *__restrict__ useg, int64_t Bcap,
-                           uint32_t *__restrict__ cflag, uint32_t *__restrict__ nitems) {
-  const int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (u >= Bcap) return;
-  if (bd.plan && u == 0) *nitems = 0;
-  const int64_t B = sorted_voxels(bd, Bcap);
-  if (u >= B) {
-    cflag[u] = 0;
-    return;
-  }
-  const int m = mesh_of_u(bd.md, bd.nmesh, u);
-  const uint32_t nz = (uint32_t)bd.md[m].g.n[2];
-  const uint32_t col = keys[useg[u]] / nz;
-  cflag[u] = (u == bd.md[m].u_base || keys[useg[u - 1]] / nz != col) ? 1u : 0u;
-}
-
-__global__ void k_colheads(BatchDev bd, const uint32_t *__restrict__ cflag,
-                           const uint32_t *__restrict__ cord, int64_t Bcap,
-                           uint32_t *__restrict__ colhead) {
-  const int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t B = sorted_voxels(bd, Bcap);
-  if (u >= B) return;
-  if (cflag[u]) colhead[cord[u]] = (uint32_t)u;
-  if (u == B - 1) colhead[cord[u] + cflag[u]] = (uint32_t)B;
-}
-
-// An item starts every CH voxels from its column's first boundary voxel and, with z slabs
-// (zslab > 0), also where the column enters a new slab of zslab Level1 layers.
-__global__ void k_itemflags(BatchDev bd, const uint32_t *__restrict__ keys,
-                            const uint32_t *__restrict__ useg, const uint32_t *__restrict__ cflag,
-                            const uint32_t *__restrict__ cord, const uint32_t *__restrict__ colhead,
-                            int64_t Bcap, int zslab, uint32_t *__restrict__ iflag) {
-  const int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (u >= Bcap) return;
-  if (u >= sorted_voxels(bd, Bcap)) {
-    iflag[u] = 0;
-    return;
-  }
-  const MeshDesc &d = bd.md[mesh_of_u(bd.md, bd.nmesh, u)];
-  const uint32_t c = cord[u] + cflag[u] - 1u;
-  bool start = (u - colhead[c]) % d.ch == 0;
-  if (zslab > 0 && !start) {
-    const uint32_t nz = (uint32_t)d.g.n[2];
-    start = (keys[useg[u]] % nz) / (uint32_t)zslab != (keys[useg[u - 1]] % nz) / (uint32_t)zslab;
-  }
-  // meshes without a Level2 grid (sorted for their normals only) get no Level2 work items
-  iflag[u] = (d.has_l2 && start) ? 1u : 0u;
-}
-
 // Work item of the Level2 kernels: a run of boundary voxels of one Level1 column.
 struct __align__(16) Item {
   uint32_t ua;       // first boundary voxel
@@ -220,29 +167,72 @@ struct __align__(16) Item {
   uint32_t col_end;  // first boundary voxel of the next column
 };
 
-__global__ void k_itemstarts(BatchDev bd, const uint32_t *__restrict__ keys,
-                             const uint32_t *__restrict__ useg, const uint32_t *__restrict__ cflag,
-                             const uint32_t *__restrict__ cord, const uint32_t *__restrict__ colhead,
-                             const uint32_t *__restrict__ iflag, const uint32_t *__restrict__ iord,
-                             int64_t Bcap, Item *__restrict__ items, uint32_t *__restrict__ nitems) {
-  const int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// Marked voxels of all meshes up to and with `key` of mesh d (kpre: the exclusive prefix of kmask's
+// bits by word, kpre[0] the bits before the plane).
+__device__ __forceinline__ uint32_t marked_through(const BatchDev &bd, const MeshDesc &d,
+                                                   const uint32_t *__restrict__ kpre, uint32_t key) {
+  const int64_t w = d.word_base + (key >> 5);
+  return __ldg(kpre + w) - __ldg(kpre) + __popc(__ldg(bd.kmask + w) & (0xffffffffu >> (31u - (key & 31u))));
+}
+
+// The items: one starts every MeshDesc::ch voxels from its column's first boundary voxel and, with z
+// slabs (zslab > 0), also where the column enters a new slab of zslab Level1 layers.  The ends of a
+// voxel's column and slab are ranks among the marked voxels, so each voxel knows by itself whether an
+// item starts there and how long it is; blocks append theirs in any order.  iflag (stencil fill, else
+// nullptr): 1 where an item starts.  Bound by latency; two scans over the voxels and four kernels
+// instead (column flags, heads, item flags, starts) made a 16k-triangle call 25 us longer, the 262k-
+// triangle torus (98k boundary voxels) 21 us.
+constexpr int kItemThreads = 256;
+__global__ void __launch_bounds__(kItemThreads) k_items(
+    BatchDev bd, const uint32_t *__restrict__ kpre, const uint32_t *__restrict__ keys,
+    const uint32_t *__restrict__ useg, int64_t Bcap, int zslab, uint32_t *__restrict__ iflag,
+    Item *__restrict__ items, uint32_t *__restrict__ nitems) {
+  __shared__ int s_mesh[2];
+  __shared__ uint32_t s_cnt[kItemThreads / 32 + 1];
   const int64_t B = sorted_voxels(bd, Bcap);
-  if (u >= B) return;
-  if (iflag[u]) {
-    const int mesh = mesh_of_u(bd.md, bd.nmesh, u);
+  const int64_t u0 = (int64_t)blockIdx.x * kItemThreads, u = u0 + threadIdx.x;
+  if (u0 >= B) return;
+  if ((threadIdx.x & 31u) == 0 && threadIdx.x < 64)
+    s_mesh[threadIdx.x >> 5] = mesh_of_u(bd.md, bd.nmesh, threadIdx.x ? min(u0 + kItemThreads, B) - 1 : u0);
+  __syncthreads();
+  Item it = {};
+  bool start = false;
+  if (u < B) {
+    const int m0 = s_mesh[0], mesh = m0 + mesh_of_u(bd.md + m0, s_mesh[1] - m0 + 1, u);
     const MeshDesc &d = bd.md[mesh];
-    Item it;
-    it.ua = (uint32_t)u;
-    it.col = keys[useg[u]] / (uint32_t)d.g.n[2];
-    it.col_end = colhead[cord[u] + cflag[u]];
-    // (an item ends where the next one of its column starts)
-    const uint32_t end = min(it.col_end, (uint32_t)u + (uint32_t)d.ch);
-    uint32_t e = (uint32_t)u + 1;
-    while (e < end && !iflag[e]) ++e;
-    it.m_mesh = (e - (uint32_t)u) | (cflag[u] << 6) | ((uint32_t)mesh << 7);
-    items[iord[u]] = it;
+    if (d.has_l2) {  // meshes sorted for their normals only get no items
+      const uint32_t nz = (uint32_t)d.g.n[2], key = __ldg(keys + __ldg(useg + u)), col = key / nz;
+      const uint32_t k0 = col * nz, uu = (uint32_t)u;
+      const uint32_t head = k0 ? marked_through(bd, d, kpre, k0 - 1u) : (uint32_t)d.u_base;
+      it.ua = uu;
+      it.col = col;
+      it.col_end = marked_through(bd, d, kpre, k0 + nz - 1u);
+      const uint32_t ch = (uint32_t)d.ch, r = (uu - head) % ch;
+      uint32_t end = min(it.col_end, uu + ch - r);
+      start = r == 0;
+      if (zslab > 0) {
+        const uint32_t z0 = (key - k0) / (uint32_t)zslab * (uint32_t)zslab;
+        const uint32_t z1 = min(nz, z0 + (uint32_t)zslab);
+        start = start || (z0 && uu == marked_through(bd, d, kpre, k0 + z0 - 1u));
+        end = min(end, marked_through(bd, d, kpre, k0 + z1 - 1u));
+      }
+      it.m_mesh = (end - uu) | (uu == head ? 64u : 0u) | ((uint32_t)mesh << 7);
+    }
+    if (iflag) iflag[u] = start ? 1u : 0u;
   }
-  if (u == B - 1) *nitems = iord[u] + iflag[u];
+  const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint32_t bal = __ballot_sync(FULL, start);
+  if (lane == 0) s_cnt[warp] = (uint32_t)__popc(bal);
+  __syncthreads();
+  if (warp == 0) {
+    const uint32_t c = lane < kItemThreads / 32 ? s_cnt[lane] : 0u, inc = warp_incl_scan(c);
+    uint32_t base = 0;
+    if (lane == 31 && inc) base = atomicAdd(nitems, inc);
+    base = __shfl_sync(FULL, base, 31);
+    if (lane < kItemThreads / 32) s_cnt[lane] = base + inc - c;
+  }
+  __syncthreads();
+  if (start) items[s_cnt[warp] + (uint32_t)__popc(bal & ((1u << lane) - 1u))] = it;
 }
 
 // Items of one mesh ordered by z slab (order within a slab is free): per-slab counts, their
@@ -430,27 +420,23 @@ constexpr int kPrefixWarps = 4;
 constexpr int kPrefixMaskWords = 128;  // 4 * 32 * 32 samples / 32
 
 __global__ void __launch_bounds__(kPrefixWarps * 32) k_stencil_segment(
-    BatchDev bd, const uint32_t *__restrict__ keys, const uint32_t *__restrict__ vals,
-    const uint32_t *__restrict__ useg, const uint32_t *__restrict__ cflag,
-    const uint32_t *__restrict__ cord, const uint32_t *__restrict__ colhead,
-    const Item *__restrict__ items, const uint32_t *__restrict__ nitems, int64_t B) {
+    BatchDev bd, const uint32_t *__restrict__ vals, const uint32_t *__restrict__ useg,
+    const Item *__restrict__ items, const uint32_t *__restrict__ nitems) {
   __shared__ uint32_t s_mask[kPrefixWarps][kPrefixMaskWords];
   __shared__ StTri s_t[kPrefixWarps][32];
   __shared__ uint32_t s_pre[kPrefixWarps][32];
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const int64_t it = (int64_t)blockIdx.x * kPrefixWarps + warp;
-  const int64_t NI = (int64_t)*nitems;
-  if (it >= NI) return;
-  const uint32_t ua = items[it].ua;
-  const uint32_t ue = it + 1 < NI ? items[it + 1].ua : (uint32_t)B;  // the item's voxels [ua, ue)
-  if (ue >= colhead[cord[ua] + cflag[ua]]) return;  // the column's last item: no item reads it
-  const MeshDesc &d = bd.md[mesh_of_u(bd.md, bd.nmesh, ua)];
-  if (!d.has_l2) return;
+  if (it >= (int64_t)*nitems) return;
+  const Item w = items[it];
+  const uint32_t ua = w.ua, ue = ua + (w.m_mesh & 63u);  // the item's voxels [ua, ue)
+  if (ue >= w.col_end) return;  // the column's last item: no item reads it
+  const MeshDesc &d = bd.md[w.m_mesh >> 7];
   const GridDev &g = d.g;
-  const int n2x = g.n2[0], n2y = g.n2[1], nz = g.n[2], nx = g.n[0];
+  const int n2x = g.n2[0], n2y = g.n2[1], nx = g.n[0];
   const int SW = 2 * n2x, SH = 2 * n2y;
   const int FWS = (4 * n2x * n2y + 31) >> 5;
-  const uint32_t col = keys[useg[ua]] / (uint32_t)nz;
+  const uint32_t col = w.col;
   const int ci = (int)(col % (uint32_t)nx), cj = (int)(col / (uint32_t)nx);
   const float lx = fa(fm((float)ci, g.g[0]), g.bmin[0]), hx = fa(lx, g.g[0]);
   const float ly = fa(fm((float)cj, g.g[1]), g.bmin[1]), hy = fa(ly, g.g[1]);
@@ -503,19 +489,16 @@ __global__ void __launch_bounds__(kPrefixWarps * 32) k_stencil_segment(
 }
 
 __global__ void __launch_bounds__(kPrefixWarps * 32) k_stencil_scan(
-    BatchDev bd, const uint32_t *__restrict__ cflag, const uint32_t *__restrict__ cord,
-    const uint32_t *__restrict__ colhead, const uint32_t *__restrict__ iflag, int64_t B) {
+    BatchDev bd, const uint32_t *__restrict__ iflag, const Item *__restrict__ items,
+    const uint32_t *__restrict__ nitems) {
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  const int64_t c = (int64_t)blockIdx.x * kPrefixWarps + warp;
-  const int64_t ncols = (int64_t)cord[B - 1] + cflag[B - 1];
-  if (c >= ncols) return;
-  const uint32_t u0 = colhead[c], u1 = colhead[c + 1];
-  const MeshDesc &d = bd.md[mesh_of_u(bd.md, bd.nmesh, u0)];
-  if (!d.has_l2) return;
-  // a one-item column has nothing to scan
-  bool more = false;
-  for (uint32_t u = u0 + 1 + lane; u < u1 && !more; u += 32) more = iflag[u] != 0u;
-  if (!__any_sync(FULL, more)) return;
+  const int64_t it = (int64_t)blockIdx.x * kPrefixWarps + warp;
+  if (it >= (int64_t)*nitems) return;
+  const Item w0 = items[it];
+  const uint32_t u0 = w0.ua, u1 = w0.col_end;
+  // the warp of a column's first item takes the column; a one-item column has nothing to scan
+  if (!((w0.m_mesh >> 6) & 1u) || u0 + (w0.m_mesh & 63u) >= u1) return;
+  const MeshDesc &d = bd.md[w0.m_mesh >> 7];
   const int FWS = (4 * d.g.n2[0] * d.g.n2[1] + 31) >> 5;  // <= kPrefixMaskWords
   uint32_t acc[kPrefixMaskWords / 32] = {};
   // the column's item starts 32 voxels at a time (one flag load per lane), then each in order
@@ -1398,36 +1381,30 @@ int level2_few_chunk(int ch, int64_t B, int num_sms) {
 
 size_t level2_smem_bytes(int warp_words) { return (size_t)warp_words * 4 * kWarps; }
 
-int64_t level2_temp_words(int64_t B) { return 10 * B + 16 + 2 * (kSlabsMax + 4) + scan_temp_words(B); }
+int64_t level2_temp_words(int64_t B) { return 6 * B + 16 + 2 * (kSlabsMax + 4); }
 
 // Builds the chunk items from the sorted pair lists and runs the persistent Level2 kernel.
 void launch_level2(const BatchDev &bd, const uint32_t *keys, const uint32_t *vals,
-                   const uint32_t *useg, int64_t B, uint32_t *tmp, int64_t smask_words, Level2Words words, int num_sms,
+                   const uint32_t *useg, const uint32_t *kpre, int64_t B, uint32_t *tmp, int64_t smask_words, Level2Words words, int num_sms,
                    cudaStream_t s, const std::function<void()> &before_kernel, int zslab,
                    int nslab, const std::function<void(int, cudaStream_t)> &after_slab, int slab_nz,
                    const SlabStreams *aux) {
   if (B <= 0) return;
   // (tmp is 256-byte aligned: the items come first)
   Item *items = reinterpret_cast<Item *>(tmp);
-  uint32_t *cflag = tmp + 4 * B, *cord = cflag + B, *colhead = cord + B, *iflag = colhead + B + 1,
-           *iord = iflag + B, *nitems = iord + B,
-           *slabcnt = nitems + 4, *ioff = slabcnt + (kSlabsMax + 4), *ilist = ioff + (kSlabsMax + 4),
-           *stmp = ilist + B;
+  uint32_t *iflag = tmp + 4 * B, *slabcnt = iflag + B, *ioff = slabcnt + (kSlabsMax + 4),
+           *ilist = ioff + (kSlabsMax + 4), *nitems = bd.queue + kQueueItems;
   if (nslab <= 1) zslab = 0;
   const unsigned nb = (unsigned)((B + 255) / 256);
+  const bool stp = bd.fill == GPV_FILL_STENCIL && bd.stp;
   // (one-graph calls: B is the capacity, the kernels read the device count)
-  k_colflags<<<nb, 256, 0, s>>>(bd, keys, useg, B, cflag, nitems);
-  scan_u32(cflag, cord, B, nullptr, stmp, s);
-  k_colheads<<<nb, 256, 0, s>>>(bd, cflag, cord, B, colhead);
-  k_itemflags<<<nb, 256, 0, s>>>(bd, keys, useg, cflag, cord, colhead, B, zslab, iflag);
-  scan_u32(iflag, iord, B, nullptr, stmp, s);
-  k_itemstarts<<<nb, 256, 0, s>>>(bd, keys, useg, cflag, cord, colhead, iflag, iord, B, items, nitems);
-  count_launch(4);
-  if (bd.fill == GPV_FILL_STENCIL && bd.stp) {
-    const unsigned nbp = (unsigned)((B + kPrefixWarps - 1) / kPrefixWarps);  // items, columns <= B
-    k_stencil_segment<<<nbp, kPrefixWarps * 32, 0, s>>>(bd, keys, vals, useg, cflag, cord, colhead,
-                                                         items, nitems, B);
-    k_stencil_scan<<<nbp, kPrefixWarps * 32, 0, s>>>(bd, cflag, cord, colhead, iflag, B);
+  k_items<<<(unsigned)((B + kItemThreads - 1) / kItemThreads), kItemThreads, 0, s>>>(
+      bd, kpre, keys, useg, B, zslab, stp ? iflag : nullptr, items, nitems);
+  count_launch(1);
+  if (stp) {
+    const unsigned nbp = (unsigned)((B + kPrefixWarps - 1) / kPrefixWarps);  // items <= B
+    k_stencil_segment<<<nbp, kPrefixWarps * 32, 0, s>>>(bd, vals, useg, items, nitems);
+    k_stencil_scan<<<nbp, kPrefixWarps * 32, 0, s>>>(bd, iflag, items, nitems);
     count_launch(2);
   }
   const bool st = bd.fill == GPV_FILL_STENCIL;
