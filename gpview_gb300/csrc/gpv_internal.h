@@ -108,7 +108,7 @@ constexpr int kFillNone = -1;
 // launch adds its ramp and tail
 constexpr int kSlabsMax = 8;
 constexpr int kQueueItems = 1 + 2 * kSlabsMax;
-constexpr int kQueueWords = kQueueItems + 1;
+constexpr int kQueueWords = kQueueItems + 2;
 constexpr uint32_t kHeavyCap = 1u << 18;  // pieces of a call's heavy list (4 MiB)
 
 constexpr int kFinishGroups = 8;  // plane words of a layer that one fill-finish block takes
@@ -122,7 +122,7 @@ struct BatchDev {
   int64_t total_xchunks;  // 128-voxel expansion chunks of all meshes
   uint32_t *queue;       // work-queue tickets, zeroed by the caller: [0] Level1, [1 + k] and
                          // [1 + kSlabsMax + k] the fill and the SAT kernel of Level2 slab k,
-                         // [kQueueItems] the number of Level2 work items
+                         // [kQueueItems] the numbers of Level2 items and SAT runs
   int normals;           // GPV_NORMALS_* of this batch
   int fill;              // GPV_FILL_* of this batch
   uint32_t *stp;         // stencil fill: per boundary voxel, the sample-coverage parity of the

@@ -5,7 +5,8 @@
 // the +z ray from the cell's origin crosses an odd number of distinct triangles among those
 // recorded in voxels (i,j,z) with z >= k; otherwise 0.
 //
-// Work unit: a chunk of up to CH consecutive boundary voxels of one Level1 column (one warp).
+// Work unit (one warp): the SAT's is a run of consecutive boundary voxels, the fill's a chunk of up to
+// CH consecutive boundary voxels of one Level1 column.
 //   SAT   -- each axis test of the SAT that crosses an edge with a box axis depends on two of the
 //            three coordinates, so the cells that pass the nine of them are the ones whose x/y, y/z
 //            and x/z squares pass three two-dimensional tests.  Those are solved a row at a time
@@ -163,6 +164,7 @@ __device__ __forceinline__ int64_t sorted_voxels(const BatchDev &bd, int64_t B) 
 struct __align__(16) Item {
   uint32_t ua;       // first boundary voxel
   uint32_t m_mesh;   // voxels (1..32) | first of its column << 6 | mesh << 7
+                     // (a SAT run has the voxels and the mesh only)
   uint32_t col;      // column (y * nx + x)
   uint32_t col_end;  // first boundary voxel of the next column
 };
@@ -175,10 +177,42 @@ __device__ __forceinline__ uint32_t marked_through(const BatchDev &bd, const Mes
   return __ldg(kpre + w) - __ldg(kpre) + __popc(__ldg(bd.kmask + w) & (0xffffffffu >> (31u - (key & 31u))));
 }
 
+// The SAT kernel takes runs of consecutive boundary voxels, whatever their columns: its pairs are
+// tested by voxel.  A run ends where its masks fill the warp's share of shared memory and, so that
+// batches of 32 pairs are full and warps finish together, after about q pairs: nb batches less an
+// average list (a run's pairs vary by about one list around q), nb giving a warp two runs, and a
+// quarter of that for the last eighth of the pairs.  Where a full run's masks hold less than two
+// batches, pairs only bound the longest lists.  Against the fill's items, whose columns are mostly
+// short: a 16k-triangle sphere at 64^3 / 8^3 52 -> 31 us (its longest columns took that long), 7k
+// triangles at 150x170x130 / 6^3 73 -> 53, 256 mixed meshes 5.4 -> 4.0 ms, the 1.3M-triangle star at
+// 256^3 / 16^3 690 -> 677; a 262k-triangle torus, whose columns are long, 113..119 -> 119.  One run
+// a warp instead of two: torus 135 us, batch 4.1 ms; three: batch 3.9 ms, star 684 us.
+constexpr int kSatWords = 512;  // (1024, with a block less per SM, took 688 us for the star)
+__host__ __device__ __forceinline__ int sat_run_cap(const GridDev &g) {
+  const int n = kSatWords / ((g.n2[0] * g.n2[1] * g.n2[2] + 31) >> 5);
+  return n < 1 ? 1 : n > 32 ? 32 : n;
+}
+struct SatRuns {
+  uint32_t q, qt, tail, nq;
+  __device__ __forceinline__ SatRuns(uint32_t pairs, uint32_t voxels, int slots, uint32_t cap) {
+    const uint32_t avg = pairs / voxels, nb = max(pairs / (32u * (uint32_t)slots), 1u);
+    q = max(32u * nb, avg + 16u) - avg;
+    qt = max(32u * max(nb / 4u, 1u), avg + 16u) - avg;
+    if (cap * avg < 64u) {
+      q = max(q, 256u);
+      qt = q;
+    }
+    tail = pairs - pairs / 8u;
+    nq = tail / q + 1u;
+  }
+  __device__ __forceinline__ uint32_t bucket(uint32_t e) const { return e < tail ? e / q : nq + (e - tail) / qt; }
+};
+
 // The items: one starts every MeshDesc::ch voxels from its column's first boundary voxel and, with z
 // slabs (zslab > 0), also where the column enters a new slab of zslab Level1 layers.  The ends of a
 // voxel's column and slab are ranks among the marked voxels, so each voxel knows by itself whether an
-// item starts there and how long it is; blocks append theirs in any order.  iflag (stencil fill, else
+// item starts there and how long it is; blocks append theirs in any order.  runs (nullptr with z slabs,
+// where the SAT takes the items): the SAT kernel's; counts: the numbers of both.  iflag (stencil fill, else
 // nullptr): 1 where an item starts.  Bound by latency; two scans over the voxels and four kernels
 // instead (column flags, heads, item flags, starts) made a 16k-triangle call 25 us longer, the 262k-
 // triangle torus (98k boundary voxels) 21 us.
@@ -186,17 +220,17 @@ constexpr int kItemThreads = 256;
 __global__ void __launch_bounds__(kItemThreads) k_items(
     BatchDev bd, const uint32_t *__restrict__ kpre, const uint32_t *__restrict__ keys,
     const uint32_t *__restrict__ useg, int64_t Bcap, int zslab, uint32_t *__restrict__ iflag,
-    Item *__restrict__ items, uint32_t *__restrict__ nitems) {
+    Item *__restrict__ items, Item *__restrict__ runs, int slots, uint32_t *__restrict__ counts) {
   __shared__ int s_mesh[2];
-  __shared__ uint32_t s_cnt[kItemThreads / 32 + 1];
+  __shared__ uint32_t s_cnt[2][kItemThreads / 32];
   const int64_t B = sorted_voxels(bd, Bcap);
   const int64_t u0 = (int64_t)blockIdx.x * kItemThreads, u = u0 + threadIdx.x;
   if (u0 >= B) return;
   if ((threadIdx.x & 31u) == 0 && threadIdx.x < 64)
     s_mesh[threadIdx.x >> 5] = mesh_of_u(bd.md, bd.nmesh, threadIdx.x ? min(u0 + kItemThreads, B) - 1 : u0);
   __syncthreads();
-  Item it = {};
-  bool start = false;
+  Item it = {}, run = {};
+  bool start = false, rstart = false;
   if (u < B) {
     const int m0 = s_mesh[0], mesh = m0 + mesh_of_u(bd.md + m0, s_mesh[1] - m0 + 1, u);
     const MeshDesc &d = bd.md[mesh];
@@ -217,22 +251,41 @@ __global__ void __launch_bounds__(kItemThreads) k_items(
         end = min(end, marked_through(bd, d, kpre, k0 + z1 - 1u));
       }
       it.m_mesh = (end - uu) | (uu == head ? 64u : 0u) | ((uint32_t)mesh << 7);
+      if (runs) {
+        const uint32_t cap = (uint32_t)sat_run_cap(d.g);
+        const SatRuns sr(__ldg(useg + B), (uint32_t)B, slots, cap);
+        const uint32_t r0 = (uu - (uint32_t)d.u_base) % cap, b = sr.bucket(__ldg(useg + u));
+        rstart = r0 == 0 || sr.bucket(__ldg(useg + u - 1)) != b;
+        if (rstart) {
+          const uint32_t mend = mesh + 1 < bd.nmesh ? (uint32_t)bd.md[mesh + 1].u_base : (uint32_t)B;
+          const uint32_t last = min(mend, uu + cap - r0);
+          uint32_t e = uu + 1;
+          while (e < last && sr.bucket(__ldg(useg + e)) == b) ++e;
+          run.ua = uu;
+          run.m_mesh = (e - uu) | ((uint32_t)mesh << 7);
+        }
+      }
     }
     if (iflag) iflag[u] = start ? 1u : 0u;
   }
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  const uint32_t bal = __ballot_sync(FULL, start);
-  if (lane == 0) s_cnt[warp] = (uint32_t)__popc(bal);
-  __syncthreads();
-  if (warp == 0) {
-    const uint32_t c = lane < kItemThreads / 32 ? s_cnt[lane] : 0u, inc = warp_incl_scan(c);
-    uint32_t base = 0;
-    if (lane == 31 && inc) base = atomicAdd(nitems, inc);
-    base = __shfl_sync(FULL, base, 31);
-    if (lane < kItemThreads / 32) s_cnt[lane] = base + inc - c;
+  const uint32_t bal = __ballot_sync(FULL, start), rbal = __ballot_sync(FULL, rstart);
+  if (lane == 0) {
+    s_cnt[0][warp] = (uint32_t)__popc(bal);
+    s_cnt[1][warp] = (uint32_t)__popc(rbal);
   }
   __syncthreads();
-  if (start) items[s_cnt[warp] + (uint32_t)__popc(bal & ((1u << lane) - 1u))] = it;
+  if (warp < 2) {
+    const uint32_t c = lane < kItemThreads / 32 ? s_cnt[warp][lane] : 0u, inc = warp_incl_scan(c);
+    uint32_t base = 0;
+    if (lane == 31 && inc) base = atomicAdd(counts + warp, inc);
+    base = __shfl_sync(FULL, base, 31);
+    if (lane < kItemThreads / 32) s_cnt[warp][lane] = base + inc - c;
+  }
+  __syncthreads();
+  const uint32_t below = (1u << lane) - 1u;
+  if (start) items[s_cnt[0][warp] + (uint32_t)__popc(bal & below)] = it;
+  if (rstart) runs[s_cnt[1][warp] + (uint32_t)__popc(rbal & below)] = run;
 }
 
 // Items of one mesh ordered by z slab (order within a slab is free): per-slab counts, their
@@ -526,7 +579,7 @@ __global__ void __launch_bounds__(kPrefixWarps * 32) k_stencil_scan(
 // The exact SAT of queued (triangle, voxel, sub-column, cell range) records, one per lane: cells
 // that another triangle has marked already are left out (the state is an OR).
 __device__ __noinline__ void sat_exact(const MeshDesc &d, WarpScratch &ws, uint32_t *sat,
-                                       const int *kz, int ci, int cj, uint32_t nr) {
+                                       const int *kz, const uint32_t *xy, uint32_t nr) {
   const unsigned lane = threadIdx.x & 31u;
   __syncwarp();
   if (lane < nr) {
@@ -546,9 +599,10 @@ __device__ __noinline__ void sat_exact(const MeshDesc &d, WarpScratch &ws, uint3
                    a2 = __ldg(d.ptri + 3 * (size_t)t + 2);
       const float V[9] = {a0.x, a0.y, a0.z, a1.x, a1.y, a1.z, a2.x, a2.y, a2.z};
       const float h[3] = {g.e2[0], g.e2[1], g.e2[2]};
+      const uint32_t c = xy[jv];
       SatCol sc;
-      if (sat_col(V, __ldg(g.c2s[0] + (size_t)ci * n2x + p),
-                  __ldg(g.c2s[1] + (size_t)cj * g.n2[1] + q), h, sc)) {
+      if (sat_col(V, __ldg(g.c2s[0] + (size_t)(c & 0xffffu) * n2x + p),
+                  __ldg(g.c2s[1] + (size_t)(c >> 16) * g.n2[1] + q), h, sc)) {
         const float *sz = g.c2s[2] + (size_t)kz[jv] * n2z;
         uint32_t bits = 0;
 #pragma unroll 1
@@ -729,7 +783,7 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_sat(
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   WarpScratch &ws = *reinterpret_cast<WarpScratch *>(sm + (size_t)warp * per_warp);
   int *const kz = reinterpret_cast<int *>(&ws + 1);
-  uint32_t *const sat = reinterpret_cast<uint32_t *>(kz + 32);
+  uint32_t *const xy = reinterpret_cast<uint32_t *>(kz + 32), *const sat = xy + 32;
   Item it;
   uint32_t part;
   while (next_item(bd.queue + 1 + kSlabsMax + slab, items, nitems, slab, ilist, ioff, (uint32_t)parts, it, part)) {
@@ -739,27 +793,22 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_sat(
   const float4 *__restrict__ ptri = d.ptri;
   const int n2x = g.n2[0], n2y = g.n2[1], n2z = g.n2[2];
   const int W = (n2x * n2y * n2z + 31) >> 5;
-  const int nx = g.n[0], nz = g.n[2];
   const int m = (int)(it.m_mesh & 63u);
-  const int ci = (int)(it.col % (uint32_t)nx), cj = (int)(it.col / (uint32_t)nx);
 #pragma unroll 1
   for (int w = lane; w < m * W; w += 32) sat[w] = 0;
   if ((int)lane < m) {
-    const uint32_t e = useg[ua + lane];
+    const uint32_t e = useg[ua + lane], key = keys[e], col = key / (uint32_t)g.n[2];
+    const uint32_t cj = col / (uint32_t)g.n[0];
     ws.seg[lane] = e;
-    kz[lane] = (int)(keys[e] - it.col * (uint32_t)nz);
+    kz[lane] = (int)(key - col * (uint32_t)g.n[2]);
+    xy[lane] = (col - cj * (uint32_t)g.n[0]) | (cj << 16);
   }
   if (lane == 0) ws.seg[m] = useg[ua + m];
   __syncwarp();
-  const float *sx = g.c2s[0] + (size_t)ci * n2x, *sy = g.c2s[1] + (size_t)cj * n2y;
-  const float sx0 = __ldg(sx), sx1 = __ldg(sx + n2x - 1), sy0 = __ldg(sy), sy1 = __ldg(sy + n2y - 1);
 
-  // ---------------- SAT of each voxel's own triangles: the chunk's (voxel, triangle) pairs are
+  // ---------------- SAT of each voxel's own triangles: the run's (voxel, triangle) pairs are
   // contiguous in the sorted lists and are taken 32 at a time across voxel boundaries.
   const float gx = g.g2[0], gy = g.g2[1], gz = g.g2[2];
-  // Distance of the centre tables from their affine form within a voxel: two roundings (eps times
-  // the coordinate) of the formulas' doubles.
-  const float tx = 2.02f * EPS24 * fmaxf(fabsf(sx0), fabsf(sx1)), ty = 2.02f * EPS24 * fmaxf(fabsf(sy0), fabsf(sy1));
   uint32_t nrec = 0;
   {
     const float h0 = g.e2[0], h1 = g.e2[1], h2 = g.e2[2];
@@ -777,13 +826,17 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_sat(
       uint32_t nsolve = 0, ncol = 0, t = 0;
       int jv = 0;  // last voxel whose segment starts at or before e
       float4 a0, a1, a2;
-      float R = 0.f, tz = 0.f;
-      const float *sz = nullptr;
+      float R = 0.f, tx = 0.f, ty = 0.f, tz = 0.f;
+      const float *sx = nullptr, *sy = nullptr, *sz = nullptr;
       if (e < S1) {
 #pragma unroll
         for (int st = 16; st > 0; st >>= 1)
           if (jv + st <= m - 1 && ws.seg[jv + st] <= e) jv += st;
+        const uint32_t c = xy[jv];
+        sx = g.c2s[0] + (size_t)(c & 0xffffu) * n2x;
+        sy = g.c2s[1] + (size_t)(c >> 16) * n2y;
         sz = g.c2s[2] + (size_t)kz[jv] * n2z;
+        const float sx0 = __ldg(sx), sx1 = __ldg(sx + n2x - 1), sy0 = __ldg(sy), sy1 = __ldg(sy + n2y - 1);
         const float sz0 = __ldg(sz), sz1 = __ldg(sz + n2z - 1);
         t = vals[e] & 0x7fffffffu;
         a0 = __ldg(ptri + 3 * (size_t)t), a1 = __ldg(ptri + 3 * (size_t)t + 1),
@@ -791,6 +844,10 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_sat(
         const float xn = fminf(a0.x, fminf(a1.x, a2.x)), xx = fmaxf(a0.x, fmaxf(a1.x, a2.x));
         const float yn = fminf(a0.y, fminf(a1.y, a2.y)), yx = fmaxf(a0.y, fmaxf(a1.y, a2.y));
         const float zn = fminf(a0.z, fminf(a1.z, a2.z)), zx = fmaxf(a0.z, fmaxf(a1.z, a2.z));
+        // Distance of the centre tables from their affine form within a voxel: two roundings (eps
+        // times the coordinate) of the formulas' doubles.
+        tx = 2.02f * EPS24 * fmaxf(fabsf(sx0), fabsf(sx1));
+        ty = 2.02f * EPS24 * fmaxf(fabsf(sy0), fabsf(sy1));
         tz = 2.02f * EPS24 * fmaxf(fabsf(sz0), fabsf(sz1));
         cell_ranges(xn, xx, sx0, g.inv_g2[0], n2x, ff(tx, g.inv_g2[0], kIdx), p0, p1, pi, pe);
         cell_ranges(yn, yx, sy0, g.inv_g2[1], n2y, ff(ty, g.inv_g2[1], kIdx), q0, q1, qi, qe);
@@ -896,13 +953,13 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_sat(
         }
         nrec = queue_push(ws, nrec, amb, tri, pos);
         if (nrec >= 32) {
-          sat_exact(d, ws, sat, kz, ci, cj, 32);
+          sat_exact(d, ws, sat, kz, xy, 32);
           nrec = queue_shift(ws, nrec);
         }
       }
       __syncwarp();
     }
-    if (nrec) sat_exact(d, ws, sat, kz, ci, cj, nrec);
+    if (nrec) sat_exact(d, ws, sat, kz, xy, nrec);
     nrec = 0;
   }
   // the masks out
@@ -1367,7 +1424,7 @@ Level2Words level2_warp_words(const GridDev &g, int cap, bool stencil) {
   const int FWS = (4 * g.n2[0] * g.n2[1] + 31) >> 5;
   const int base = (int)(sizeof(WarpScratch) / 4) + 32;
   auto al = [](int words) { return (words + 3) & ~3; };  // a warp's region starts 16-byte aligned
-  return {al(base + CH * W), al(base + CH * W + CH * FW + (stencil ? 4 * CH * W + CH * FWS + FWS : 0))};
+  return {al(base + 32 + std::max(CH, sat_run_cap(g)) * W), al(base + CH * W + CH * FW + (stencil ? 4 * CH * W + CH * FWS + FWS : 0))};
 }
 
 int level2_parts(int64_t B, int num_sms) {
@@ -1381,7 +1438,7 @@ int level2_few_chunk(int ch, int64_t B, int num_sms) {
 
 size_t level2_smem_bytes(int warp_words) { return (size_t)warp_words * 4 * kWarps; }
 
-int64_t level2_temp_words(int64_t B) { return 6 * B + 16 + 2 * (kSlabsMax + 4); }
+int64_t level2_temp_words(int64_t B) { return 10 * B + 16 + 2 * (kSlabsMax + 4); }
 
 // Builds the chunk items from the sorted pair lists and runs the persistent Level2 kernel.
 void launch_level2(const BatchDev &bd, const uint32_t *keys, const uint32_t *vals,
@@ -1392,14 +1449,16 @@ void launch_level2(const BatchDev &bd, const uint32_t *keys, const uint32_t *val
   if (B <= 0) return;
   // (tmp is 256-byte aligned: the items come first)
   Item *items = reinterpret_cast<Item *>(tmp);
-  uint32_t *iflag = tmp + 4 * B, *slabcnt = iflag + B, *ioff = slabcnt + (kSlabsMax + 4),
+  Item *runs = items + B;
+  uint32_t *iflag = tmp + 8 * B, *slabcnt = iflag + B, *ioff = slabcnt + (kSlabsMax + 4),
            *ilist = ioff + (kSlabsMax + 4), *nitems = bd.queue + kQueueItems;
   if (nslab <= 1) zslab = 0;
+  if (zslab > 0) runs = nullptr;
   const unsigned nb = (unsigned)((B + 255) / 256);
   const bool stp = bd.fill == GPV_FILL_STENCIL && bd.stp;
   // (one-graph calls: B is the capacity, the kernels read the device count)
   k_items<<<(unsigned)((B + kItemThreads - 1) / kItemThreads), kItemThreads, 0, s>>>(
-      bd, kpre, keys, useg, B, zslab, stp ? iflag : nullptr, items, nitems);
+      bd, kpre, keys, useg, B, zslab, stp ? iflag : nullptr, items, runs, 2 * 24 * num_sms, nitems);
   count_launch(1);
   if (stp) {
     const unsigned nbp = (unsigned)((B + kPrefixWarps - 1) / kPrefixWarps);  // items <= B
@@ -1451,8 +1510,9 @@ void launch_level2(const BatchDev &bd, const uint32_t *keys, const uint32_t *val
   for (int sl = 0; sl < launches; ++sl) {
     cudaStream_t ls = two ? aux->st[sl & 1] : s;
     const uint32_t *list = zslab > 0 ? ilist : nullptr;
-    k_level2c_sat<<<grid_sat, kWarps * 32, smem_sat, ls>>>(bd, keys, vals, useg, items, nitems, words.sat,
-                                                          sl, list, ioff, parts);
+    k_level2c_sat<<<grid_sat, kWarps * 32, smem_sat, ls>>>(bd, keys, vals, useg, runs ? runs : items,
+                                                          nitems + (runs ? 1 : 0), words.sat, sl, list, ioff,
+                                                          parts);
     fill<<<grid_fill, kWarps * 32, smem_fill, ls>>>(bd, keys, vals, useg, items, nitems, words.fill, sl,
                                                     list, ioff, 1);
     count_launch(2);
