@@ -946,7 +946,7 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
         mark(9);
       if (nmode) {
         launch_face_normals(bd, s);
-        launch_normals(bd, sk, sv, useg, ub, max_cells, ctx->num_sms, s);
+        launch_normals(bd, sk, sv, useg, ub, P2, max_cells, ctx->num_sms, s);
       }
     } else {
       mark(7);

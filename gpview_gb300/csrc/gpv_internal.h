@@ -108,7 +108,8 @@ constexpr int kFillNone = -1;
 // launch adds its ramp and tail
 constexpr int kSlabsMax = 8;
 constexpr int kQueueItems = 1 + 2 * kSlabsMax;
-constexpr int kQueueWords = kQueueItems + 2;
+constexpr int kQueueNormals = kQueueItems + 2;
+constexpr int kQueueWords = kQueueNormals + 1;
 constexpr uint32_t kHeavyCap = 1u << 18;  // pieces of a call's heavy list (4 MiB)
 
 constexpr int kFinishGroups = 8;  // plane words of a layer that one fill-finish block takes
@@ -122,7 +123,8 @@ struct BatchDev {
   int64_t total_xchunks;  // 128-voxel expansion chunks of all meshes
   uint32_t *queue;       // work-queue tickets, zeroed by the caller: [0] Level1, [1 + k] and
                          // [1 + kSlabsMax + k] the fill and the SAT kernel of Level2 slab k,
-                         // [kQueueItems] the numbers of Level2 items and SAT runs
+                         // [kQueueItems] the numbers of Level2 items and SAT runs,
+                         // [kQueueNormals] the Level2 normals
   int normals;           // GPV_NORMALS_* of this batch
   int fill;              // GPV_FILL_* of this batch
   uint32_t *stp;         // stencil fill: per boundary voxel, the sample-coverage parity of the
@@ -274,7 +276,7 @@ void launch_seg_sort(uint32_t *vals, const uint32_t *useg, int64_t U, uint32_t *
 // Level1 normals of the U boundary voxels of the sorted meshes, then Level2 normals of the meshes with
 // a Level2 grid (max_cells cells per voxel at most, 0: none).
 void launch_normals(const BatchDev &bd, const uint32_t *keys, const uint32_t *vals,
-                    const uint32_t *useg, int64_t U, int max_cells, int num_sms, cudaStream_t s);
+                    const uint32_t *useg, int64_t U, int64_t P, int max_cells, int num_sms, cudaStream_t s);
 
 // ---- voxel box hierarchy (gpv_hierarchy.cu) ----------------------------------------------------
 int hierarchy_levels(int64_t N1);  // 0 unless N1 is a power of two >= 2

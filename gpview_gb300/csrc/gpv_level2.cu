@@ -120,20 +120,6 @@ struct __align__(16) WarpScratch {
 };
 static_assert(sizeof(WarpScratch) % 16 == 0, "layout");
 
-// Lists a triangle's sub-columns from its solved x/y rows (nullptr: all np x nq, none certain).
-__device__ __forceinline__ void list_columns(uint16_t *out, const uint32_t *xy, int slot, int p0, int np,
-                                             int nq) {
-#pragma unroll 1
-  for (int dq = 0; dq < nq; ++dq) {
-    const uint32_t w = xy ? xy[dq] : (uint32_t)(p0 | ((p0 + np) << 24));
-    const int lo_i = (int)((w >> 8) & 255u), end_i = (int)((w >> 16) & 255u), end = (int)(w >> 24);
-    const uint32_t e = (uint32_t)(slot | (dq << 5));
-#pragma unroll 1
-    for (int p = (int)(w & 255u); p < end; ++p)
-      *out++ = (uint16_t)(e | (uint32_t)((p - p0) << 10) | (p >= lo_i && p < end_i ? 0x8000u : 0u));
-  }
-}
-
 struct StScratch {    // stencil fill: the batch's triangles
   float v[32][9];     // snapped vertices and heights
   float rA[32];
@@ -911,7 +897,7 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_sat(
       const uint32_t ic = warp_incl_scan(ncol);
       taken = (uint32_t)__popc(__ballot_sync(FULL, lane < taken && ic <= (uint32_t)kCols));
       if (on && lane < taken)
-        list_columns(ws.cols + (ic - ncol), direct ? nullptr : ws.sol + so0, (int)lane, p0, p1 - p0 + 1, q1 - q0 + 1);
+        list_columns(ws.cols + (ic - ncol), direct ? nullptr : ws.sol + so0, (int)lane, p0, p1 - p0 + 1, 0, q1 - q0 + 1);
       const uint32_t C = __shfl_sync(FULL, ic, (int)taken - 1);
       __syncwarp();
 #pragma unroll 1
@@ -1281,7 +1267,7 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_fill(
     const uint32_t ic = warp_incl_scan(ncol);
     taken = (uint32_t)__popc(__ballot_sync(FULL, lane < taken && ic <= (uint32_t)kCols));
     if (ncol && lane < taken)
-      list_columns(ws.cols + (ic - ncol), nsolve ? ws.sol + (is - nsolve) : nullptr, (int)lane, p0, p1 - p0 + 1, nq);
+      list_columns(ws.cols + (ic - ncol), nsolve ? ws.sol + (is - nsolve) : nullptr, (int)lane, p0, p1 - p0 + 1, 0, nq);
     const uint32_t C = __shfl_sync(FULL, ic, (int)taken - 1);
     __syncwarp();
     {

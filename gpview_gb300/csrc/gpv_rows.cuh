@@ -89,6 +89,21 @@ __device__ __forceinline__ uint32_t solve_rows(uint32_t *out, int n, float a0, f
   return cells;
 }
 
+// Lists a triangle's sub-columns (slot | row << 5 | column << 10, both from the triangle's first, | certain
+// to pass the x/y tests << 15) in rows [d0, d1) from its solved x/y rows (nullptr: all np x nq, none certain).
+__device__ __forceinline__ void list_columns(uint16_t *out, const uint32_t *xy, int slot, int p0, int np,
+                                             int d0, int d1) {
+#pragma unroll 1
+  for (int dq = d0; dq < d1; ++dq) {
+    const uint32_t w = xy ? xy[dq] : (uint32_t)(p0 | ((p0 + np) << 24));
+    const int lo_i = (int)((w >> 8) & 255u), end_i = (int)((w >> 16) & 255u), end = (int)(w >> 24);
+    const uint32_t e = (uint32_t)(slot | (dq << 5));
+#pragma unroll 1
+    for (int p = (int)(w & 255u); p < end; ++p)
+      *out++ = (uint16_t)(e | (uint32_t)((p - p0) << 10) | (p >= lo_i && p < end_i ? 0x8000u : 0u));
+  }
+}
+
 // Cells of one axis whose boxes can meet [tmin, tmax] ([lo, hi]) and those that certainly do
 // ([in_lo, in_end)), by the SAT's own box-axis test; `md` (cells) bounds the distance of the centre
 // table from c0 + k * g2 and the roundings.
