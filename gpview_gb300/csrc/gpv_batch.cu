@@ -263,7 +263,7 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
     tiles += (T[m] + tile - 1) / tile;
     fblks += finish_blocks((int64_t)g.n[1] * g.nxw);
     rows += (int64_t)g.n[2] * g.n[1];
-    xchunks += ((int64_t)g.n[0] * g.n[1] * g.n[2] + 127) / 128;
+    xchunks += ((int64_t)g.n[2] * g.n[1] * g.nxw + 31) / 32;
     words += (int64_t)g.n[2] * g.n[1] * g.nxw;
     togg += (int64_t)g.n[0] * g.n[1] * g.nzw;
     if (stencil) stgw += 4 * (int64_t)g.n[0] * g.n[1] * g.nzw;

@@ -66,7 +66,7 @@ struct MeshDesc {
   int64_t tile_base;     // ... of Level1 tiles
   int64_t fblk_base;     // ... of fill-finish blocks (ny * nxw words of a layer, kFinishGroups each)
   int64_t row_base;      // ... of Level1 rows (nz * ny)
-  int64_t xc_base;       // ... of 128-voxel expansion chunks (ceil(N1 / 128))
+  int64_t xc_base;       // ... of expansion chunks (32 bit-plane words)
   int64_t word_base;     // ... of bit-plane words (nz * ny * nxw)
   int64_t emit_base;     // ... of pair capacities (emission segments)
   int64_t pair_base;     // ... of pairs (dense layout after the sort)
@@ -120,7 +120,7 @@ struct BatchDev {
   int nmesh;
   int tile;              // Level1 triangles per ticket (32, 64, 128, 256)
   int64_t total_tris, total_tiles, total_fblks, total_rows, total_words;
-  int64_t total_xchunks;  // 128-voxel expansion chunks of all meshes
+  int64_t total_xchunks;  // expansion chunks of all meshes
   uint32_t *queue;       // work-queue tickets, zeroed by the caller: [0] Level1, [1 + k] and
                          // [1 + kSlabsMax + k] the fill and the SAT kernel of Level2 slab k,
                          // [kQueueItems] the numbers of Level2 items and SAT runs,

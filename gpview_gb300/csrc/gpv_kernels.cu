@@ -843,20 +843,19 @@ __global__ void k_boundary_counts(BatchDev bd, const uint32_t *__restrict__ wpre
   bd.md[m].stats->boundary = e - s;
 }
 
-// One warp per chunk of 128 consecutive voxels of one mesh's linear index (x fastest), four per lane:
-// state bytes, boundaryPrefixSum, boundaryIndex.  Every lane of a chunk works whatever the row length (a
-// warp per row left three quarters of the lanes idle on a 32-voxel row).  The mesh's fields are kept in
-// registers and the planes read through the read-only path, so that several chunks' loads are in
-// flight; with them read again after every store and 64-bit index arithmetic the kernel was bound by
-// its instructions (512^3: 302 us, now 215, 3.2 TB/s).
+// A chunk is 32 words of a mesh's bit planes (up to 1024 voxels, x fastest): state bytes,
+// boundaryPrefixSum, boundaryIndex.  A lane loads a word of each plane and its prefix; then every lane
+// takes four voxels at a time (one where rows or buffers are not aligned) of the words in order, which it
+// gets by shuffles, whatever the row length.  Bound by the writes: 512^3 voxels in 117 us, 5.7 TB/s; a
+// lane loading the words of its own four voxels waited for them (215 us).
 constexpr int kExpandWarps = 8;
-constexpr int kExpandVox = 128;
 struct ExpandMesh {
   const uint32_t *bplane, *iplane, *wp;
   uint8_t *l1;
   int32_t *prefix, *bindex;
   int64_t first;  // its first chunk
-  uint32_t N1, nx, nxw, pbase;
+  uint32_t words, nx, nxw, pbase;
+  uint32_t pw, mul;  // pieces (of four voxels or one) of a full word, ceil(2^20 / pw)
   bool vec;       // rows of a multiple of four voxels and aligned outputs (the batch's arenas are, a
                   // no-alloc caller's buffers may not be)
 };
@@ -870,56 +869,70 @@ __device__ __forceinline__ ExpandMesh expand_mesh(const MeshDesc &d, const uint3
   e.bindex = d.bindex;
   e.first = d.xc_base;
   e.nx = (uint32_t)d.g.n[0];
-  e.N1 = e.nx * (uint32_t)d.g.n[1] * (uint32_t)d.g.n[2];
   e.nxw = (uint32_t)d.g.nxw;
+  e.words = e.nxw * (uint32_t)d.g.n[1] * (uint32_t)d.g.n[2];
   e.pbase = wpre[d.word_base];
   e.vec = (e.nx & 3u) == 0 && (reinterpret_cast<uintptr_t>(d.l1) & 3u) == 0 &&
           (reinterpret_cast<uintptr_t>(d.prefix) & 15u) == 0;
+  e.pw = min(e.nx, 32u) / (e.vec ? 4u : 1u);
+  e.mul = ((1u << 20) + e.pw - 1u) / e.pw;
   return e;
 }
-// One chunk by one warp; returns the lane's inside-voxel count.
-__device__ __forceinline__ uint32_t expand_chunk(const ExpandMesh &e, int64_t gc, uint32_t lane) {
-  const uint32_t v0 = (uint32_t)(gc - e.first) * kExpandVox + lane * 4u;
-  if (v0 >= e.N1) return 0;
-  if (e.vec) {
-    // the lane's four voxels share a row and a plane word (nx, v0 and N1 are multiples of 4)
-    const uint32_t row = v0 / e.nx, x0 = v0 - row * e.nx;
-    const uint32_t w = row * e.nxw + (x0 >> 5), b0 = x0 & 31u;
-    const uint32_t bw = __ldg(e.bplane + w), iw = __ldg(e.iplane + w);
-    const uint32_t p = __ldg(e.wp + w) - e.pbase + __popc(bw & ((1u << b0) - 1u));
-    const uint32_t bb = (bw >> b0) & 0xfu, ib = (iw >> b0) & 0xfu & ~bb;
-    // (4 bits to 4 bytes: bit j to byte j)
-    const uint32_t bytes = ((bb * 0x00204081u) & 0x01010101u) * 254u + ((ib * 0x00204081u) & 0x01010101u) * 127u;
-    const uint32_t p1 = p + (bb & 1u), p2 = p1 + ((bb >> 1) & 1u), p3 = p2 + ((bb >> 2) & 1u);
-    *reinterpret_cast<uint32_t *>(e.l1 + v0) = bytes;
-    *reinterpret_cast<int4 *>(e.prefix + v0) = make_int4((int)p, (int)p1, (int)p2, (int)p3);
-    uint32_t q = p;
-    for (uint32_t k = bb; k; k &= k - 1u) e.bindex[q++] = (int32_t)(v0 + (uint32_t)__ffs(k) - 1u);
-    return (uint32_t)__popc(ib);
+// Words [j0, j1) of a chunk by one warp; returns the lane's inside-voxel count.
+__device__ __forceinline__ uint32_t expand_chunk(const ExpandMesh &e, int64_t gc, uint32_t j0, uint32_t j1,
+                                                 uint32_t lane) {
+  const uint32_t w = (uint32_t)(gc - e.first) * 32u + lane;
+  uint32_t bw = 0, iw = 0, p = 0, v0 = 0, cnt = 0, nin = 0;
+  if (w < e.words) {
+    bw = __ldg(e.bplane + w);
+    iw = __ldg(e.iplane + w) & ~bw;
+    p = __ldg(e.wp + w) - e.pbase;
+    const uint32_t row = w / e.nxw, x0 = (w - row * e.nxw) * 32u;
+    v0 = row * e.nx + x0;
+    cnt = min(32u, e.nx - x0);
+    if (lane >= j0 && lane < j1) {
+      nin = (uint32_t)__popc(iw & (0xffffffffu >> (32u - cnt)));
+      uint32_t q = p;
+      for (uint32_t k = bw; k; k &= k - 1u) e.bindex[q++] = (int32_t)(v0 + (uint32_t)__ffs(k) - 1u);
+    }
   }
-  uint32_t nin = 0;
-  for (uint32_t k = 0; k < 4u && v0 + k < e.N1; ++k) {
-    const uint32_t v = v0 + k, row = v / e.nx, x = v - row * e.nx;
-    const uint32_t w = row * e.nxw + (x >> 5), bit = x & 31u;
-    const uint32_t bw = __ldg(e.bplane + w), iw = __ldg(e.iplane + w);
-    const uint32_t p = __ldg(e.wp + w) - e.pbase + __popc(bw & ((1u << bit) - 1u));
-    const bool isb = (bw >> bit) & 1u, isi = (iw >> bit) & 1u;
-    nin += (!isb && isi);
-    if (isb) e.bindex[p] = (int32_t)v;
-    e.l1[v] = (uint8_t)(isb ? 254u : (isi ? 127u : 0u));
-    e.prefix[v] = (int32_t)p;
+  const uint32_t i1 = j1 * e.pw;
+#pragma unroll 2
+  for (uint32_t i0 = j0 * e.pw; i0 < i1; i0 += 32u) {
+    const uint32_t i = i0 + lane;
+    // i < 1024 and the excess of mul over 2^20 / pw below one: the quotient is exact
+    const uint32_t j = i * e.mul >> 20, b = i - j * e.pw;
+    const uint32_t B = __shfl_sync(FULL, bw, j), I = __shfl_sync(FULL, iw, j), P = __shfl_sync(FULL, p, j),
+                   V = __shfl_sync(FULL, v0, j), n = __shfl_sync(FULL, cnt, j);
+    if (i >= i1) continue;
+    if (e.vec) {
+      const uint32_t b0 = 4u * b;
+      if (b0 >= n) continue;
+      const uint32_t bb = (B >> b0) & 0xfu, ib = (I >> b0) & 0xfu;
+      const uint32_t q = P + __popc(B & ((1u << b0) - 1u));
+      // (4 bits to 4 bytes: bit j to byte j)
+      const uint32_t bytes = ((bb * 0x00204081u) & 0x01010101u) * 254u + ((ib * 0x00204081u) & 0x01010101u) * 127u;
+      const uint32_t q1 = q + (bb & 1u), q2 = q1 + ((bb >> 1) & 1u), q3 = q2 + ((bb >> 2) & 1u);
+      *reinterpret_cast<uint32_t *>(e.l1 + V + b0) = bytes;
+      *reinterpret_cast<int4 *>(e.prefix + V + b0) = make_int4((int)q, (int)q1, (int)q2, (int)q3);
+    } else {
+      if (b >= n) continue;
+      const uint32_t isb = (B >> b) & 1u, isi = (I >> b) & 1u;
+      e.l1[V + b] = (uint8_t)(isb * 254u + isi * 127u);
+      e.prefix[V + b] = (int32_t)(P + __popc(B & ((1u << b) - 1u)));
+    }
   }
   return nin;
 }
 
-// A block takes `iters` x kExpandWarps consecutive chunks; warp w the chunks c0 + w + k x
-// kExpandWarps.  Thread 0 looks up the mesh of the block's first chunk once (a binary search over
+// A block takes `iters` x kExpandWarps consecutive parts of chunks (`split` to a chunk), warp w the
+// parts w + k x kExpandWarps of them.  Thread 0 looks up the mesh of the block's first chunk once (a binary search over
 // the descriptors), and each warp walks forward from it as its chunks pass mesh boundaries, so
 // the search is not repeated per chunk.  A warp adds its inside count to the statistics when it
 // leaves a mesh; the block adds the warps' last runs with one atomic per mesh.
 __global__ void __launch_bounds__(kExpandWarps * 32) k_expand(BatchDev bd,
                                                             const uint32_t *__restrict__ wpre,
-                                                            int iters) {
+                                                            int iters, int split) {
   __shared__ int s_mesh;
   __shared__ int s_m[kExpandWarps];
   __shared__ unsigned long long s_nin[kExpandWarps];
@@ -927,15 +940,16 @@ __global__ void __launch_bounds__(kExpandWarps * 32) k_expand(BatchDev bd,
   if (bd.plan && !bd.plan->ok) return;
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const int64_t c0 = (int64_t)blockIdx.x * kExpandWarps * iters;
-  if (threadIdx.x == 0) s_mesh = find_mesh<&MeshDesc::xc_base>(bd.md, bd.nmesh, c0);
+  if (threadIdx.x == 0) s_mesh = find_mesh<&MeshDesc::xc_base>(bd.md, bd.nmesh, c0 / split);
   __syncthreads();
   int m = s_mesh;
   ExpandMesh em = expand_mesh(bd.md[m], wpre);
   int64_t next = m + 1 < bd.nmesh ? bd.md[m + 1].xc_base : bd.total_xchunks;
   unsigned long long nin = 0;
-#pragma unroll 4
+#pragma unroll 1
   for (int k = 0; k < iters; ++k) {
-    const int64_t gc = c0 + (int64_t)k * kExpandWarps + warp;
+    const int64_t gp = c0 + (int64_t)k * kExpandWarps + warp, gc = gp / split;
+    const uint32_t part = (uint32_t)(gp - gc * split), pn = 32u / (uint32_t)split;
     if (gc >= bd.total_xchunks) break;  // warp-uniform
     if (gc >= next) {
       const unsigned long long t = warp_sum(nin);
@@ -945,7 +959,7 @@ __global__ void __launch_bounds__(kExpandWarps * 32) k_expand(BatchDev bd,
       em = expand_mesh(bd.md[m], wpre);
       next = m + 1 < bd.nmesh ? bd.md[m + 1].xc_base : bd.total_xchunks;
     }
-    nin += expand_chunk(em, gc, lane);
+    nin += expand_chunk(em, gc, part * pn, (part + 1u) * pn, lane);
   }
   // the warps' last mesh runs: one atomic per mesh of the block
   const unsigned long long t = warp_sum(nin);
@@ -1106,13 +1120,14 @@ void launch_boundary_counts(const BatchDev &bd, const uint32_t *wpre, const uint
 
 void launch_expand(const BatchDev &bd, const uint32_t *wpre, cudaStream_t s) {
   if (bd.total_xchunks <= 0) return;
-  // up to 8 chunks per warp where the chunks are many enough to give each of the 152 SMs 64
-  // warps anyway
-  const int64_t spread = bd.total_xchunks / (152 * 64);
-  const int iters = (int)(spread < 1 ? 1 : spread > 8 ? 8 : spread);
+  // few chunks: parts of them, so that each SM has 16 warps (128^3 voxels, 2048 chunks: 9.6 us; 32
+  // warps 12, whose parts each load the chunk's words); many: up to four per warp
+  int split = 1;
+  while (split < 8 && bd.total_xchunks * split < 152 * 16) split *= 2;
+  const int64_t parts = bd.total_xchunks * split, spread = parts / (152 * 64);
+  const int iters = (int)(spread < 1 ? 1 : spread > 4 ? 4 : spread);
   const int64_t per_block = (int64_t)kExpandWarps * iters;
-  k_expand<<<(unsigned)((bd.total_xchunks + per_block - 1) / per_block), kExpandWarps * 32, 0, s>>>(
-      bd, wpre, iters);
+  k_expand<<<(unsigned)((parts + per_block - 1) / per_block), kExpandWarps * 32, 0, s>>>(bd, wpre, iters, split);
   count_launch();
 }
 
