@@ -89,17 +89,6 @@ __device__ __forceinline__ int count_drop_above(const float *oz, int n, float ot
   return i;
 }
 
-// last index tl in [0,31] with pre[tl] <= it (pre nondecreasing, pre[0] = 0)
-__device__ __forceinline__ int batch_search(const uint32_t *pre, uint32_t it) {
-  int lo = 0, hi = 31;
-#pragma unroll 1
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (pre[mid] <= it) lo = mid; else hi = mid - 1;
-  }
-  return lo;
-}
-
 constexpr int kSol = 512;    // solved rows of one batch (a triangle has at most 96); the output stage
                              // keeps 16 layers of 32 lanes there
 constexpr int kCols = 1024;  // its sub-columns (a triangle has at most that many)
@@ -120,13 +109,80 @@ struct __align__(16) WarpScratch {
 };
 static_assert(sizeof(WarpScratch) % 16 == 0, "layout");
 
-struct StScratch {    // stencil fill: the batch's triangles
-  float v[32][9];     // snapped vertices and heights
-  float rA[32];
-  uint32_t rng[32];   // packed sample ranges
-  uint32_t pre[33];   // exclusive prefix of sample counts
+// A triangle of the stencil fill: for each edge the edge function at sample (0, 0) (64 bits), dx and dy;
+// first sample column | columns << 6 | first row << 13 | the edges' top-left flags << 19, 1 / area and
+// the heights of two vertices; the third's, 1 / columns and its first sample of the batch's.
+struct __align__(16) StRec {
+  int4 e[3];
+  float4 a, b;
 };
-static_assert(sizeof(StScratch) <= sizeof(WarpScratch), "the stencil fill's scratch overlays the ray fill's");
+struct StScratch {    // the triangles of a batch that have samples, in order
+  StRec r[32];
+};
+static_assert(sizeof(StScratch) >= 16 * 32 * 4, "the output stage keeps 16 layers of 32 lanes there");
+
+// The samples of a batch of triangles (one per lane, `has`: it has samples), taken one per lane.  An edge
+// function costs two widening multiply-adds from its value at the first sample, the owner of a sample a
+// reduction over the lanes whose triangle starts among the 32, its slice an estimate that the table
+// corrects, and the scratch is 2.5 KB, so that 24 warps fit an SM: the 262k-triangle torus at 128^3 / 8^3
+// took 440 us in the fill and 70 in k_stencil_segment with 64-bit products, searches over the prefix and
+// the slices, and 16 warps; now 215 and 36.  Bound by latency (about half of the issue slots).
+struct StBatch {
+  uint32_t start, cnt, total;  // this lane's triangle's first sample and samples; the batch's
+  __device__ __forceinline__ StBatch(StRec *recs, bool has, const StTri &t) {
+    const unsigned lane = threadIdx.x & 31u;
+    const int nsx = t.sx1 - t.sx0 + 1;
+    cnt = has ? (uint32_t)(nsx * (t.sy1 - t.sy0 + 1)) : 0u;
+    const uint32_t inc = warp_incl_scan(cnt);
+    start = inc - cnt;
+    total = __shfl_sync(FULL, inc, 31);
+    const uint32_t bal = __ballot_sync(FULL, has);
+    if (has) {
+      StRec &r = recs[__popc(bal & ((1u << lane) - 1u))];
+      uint32_t tl = 0;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const int i = (k + 1) % 3, j = (k + 2) % 3;
+        const int32_t dx = t.X[j] - t.X[i], dy = t.Y[j] - t.Y[i];
+        const long long w = (long long)dx * (128 - t.Y[i]) - (long long)dy * (128 - t.X[i]);
+        r.e[k] = make_int4((int)(uint32_t)w, (int)(w >> 32), dx, dy);
+        if (dy < 0 || (dy == 0 && dx > 0)) tl |= 1u << k;
+      }
+      const uint32_t rng = (uint32_t)t.sx0 | ((uint32_t)nsx << 6) | ((uint32_t)t.sy0 << 13) | (tl << 19);
+      r.a = make_float4(__uint_as_float(rng), t.rA, t.z[0], t.z[1]);
+      r.b = make_float4(t.z[2], rcp_fast((float)nsx), __uint_as_float(start), 0.f);
+    }
+  }
+  // The record of sample w0 + lane (all lanes call; w0 a multiple of 32).
+  __device__ __forceinline__ const StRec &owner(const StRec *recs, uint32_t w0) const {
+    const unsigned lane = threadIdx.x & 31u;
+    const uint32_t here = __reduce_or_sync(FULL, cnt && start - w0 < 32u ? 1u << (start - w0) : 0u);
+    const uint32_t before = (uint32_t)__popc(__ballot_sync(FULL, cnt && start < w0));
+    return recs[before + (uint32_t)__popc(here & ((2u << lane) - 1u)) - 1u];
+  }
+};
+
+// Coverage of sample w of the batch (as st_cover), its place and the surface height there.
+__device__ __forceinline__ bool st_sample(const StRec &r, uint32_t w, int &sx, int &sy, float &zs) {
+  const float4 a = r.a, b = r.b;
+  const uint32_t rng = __float_as_uint(a.x), loc = w - __float_as_uint(b.z);
+  const uint32_t nsx = (rng >> 6) & 127u;
+  // (loc + 1/2) / nsx stays at least 1/128 away from an integer, far above the rounding
+  const uint32_t row = (uint32_t)__float2int_rz(((float)loc + 0.5f) * b.y);
+  sx = (int)((rng & 63u) + (loc - row * nsx));
+  sy = (int)(((rng >> 13) & 63u) + row);
+  long long v[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const int4 e = r.e[k];
+    v[k] = (long long)(((unsigned long long)(uint32_t)e.y << 32) | (uint32_t)e.x) + (long long)e.z * (sy * 256) -
+           (long long)e.w * (sx * 256);
+    if (!(v[k] > 0 || (v[k] == 0 && ((rng >> (19 + k)) & 1u)))) return false;
+  }
+  zs = fa(fa(fm(fm(__ll2float_rn(v[0]), a.y), a.z), fm(fm(__ll2float_rn(v[1]), a.y), a.w)),
+          fm(fm(__ll2float_rn(v[2]), a.y), b.x));
+  return true;
+}
 
 // ---- item construction -----------------------------------------------------------------------
 __device__ __forceinline__ int mesh_of_u(const MeshDesc *md, int nmesh, int64_t u) {
@@ -462,8 +518,7 @@ __global__ void __launch_bounds__(kPrefixWarps * 32) k_stencil_segment(
     BatchDev bd, const uint32_t *__restrict__ vals, const uint32_t *__restrict__ useg,
     const Item *__restrict__ items, const uint32_t *__restrict__ nitems) {
   __shared__ uint32_t s_mask[kPrefixWarps][kPrefixMaskWords];
-  __shared__ StTri s_t[kPrefixWarps][32];
-  __shared__ uint32_t s_pre[kPrefixWarps][32];
+  __shared__ StRec s_t[kPrefixWarps][32];
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const int64_t it = (int64_t)blockIdx.x * kPrefixWarps + warp;
   if (it >= (int64_t)*nitems) return;
@@ -487,36 +542,22 @@ __global__ void __launch_bounds__(kPrefixWarps * 32) k_stencil_segment(
   for (uint32_t b0 = e0; b0 < e1; b0 += 32) {
     const uint32_t e = b0 + lane;
     const uint32_t vv = e < e1 ? vals[e] : 0u;
-    uint32_t cnt = 0;
+    StTri st = {};
+    bool has = false;
     if (vv & 0x80000000u) {  // the triangle's topmost record in the column
       const uint32_t t = vv & 0x7fffffffu;
       const float4 a0 = __ldg(ptri + 3 * (size_t)t), a1 = __ldg(ptri + 3 * (size_t)t + 1),
                    a2 = __ldg(ptri + 3 * (size_t)t + 2);
       const float V[9] = {a0.x, a0.y, a0.z, a1.x, a1.y, a1.z, a2.x, a2.y, a2.z};
-      StTri st;
-      if (st_setup(V, lx, hx, ly, hy, SW, SH, st)) {
-        s_t[warp][lane] = st;
-        cnt = (uint32_t)((st.sx1 - st.sx0 + 1) * (st.sy1 - st.sy0 + 1));
-      }
+      has = st_setup(V, lx, hx, ly, hy, SW, SH, st);
     }
-    uint32_t inc = cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t x = __shfl_up_sync(FULL, inc, o);
-      if (lane >= (unsigned)o) inc += x;
-    }
-    s_pre[warp][lane] = inc - cnt;
-    const uint32_t tot = __shfl_sync(FULL, inc, 31);
+    const StBatch batch(s_t[warp], has, st);
     __syncwarp();
-    for (uint32_t w = lane; w < tot; w += 32) {
-      const int tl = batch_search(s_pre[warp], w);
-      const StTri &st = s_t[warp][tl];
-      const uint32_t loc = w - s_pre[warp][tl];
-      const uint32_t nsx = (uint32_t)(st.sx1 - st.sx0 + 1);
-      const uint32_t row = loc / nsx;
-      const int sx = st.sx0 + (int)(loc - row * nsx), sy = st.sy0 + (int)row;
+    for (uint32_t w0 = 0; w0 < batch.total; w0 += 32) {
+      const StRec &r = batch.owner(s_t[warp], w0);
+      int sx, sy;
       float zs;
-      if (st_cover(st, sx, sy, zs)) {
+      if (w0 + lane < batch.total && st_sample(r, w0 + lane, sx, sy, zs)) {
         const int sidx = sy * SW + sx;
         atomicXor(&mask[sidx >> 5], 1u << (sidx & 31));
       }
@@ -969,8 +1010,11 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_fill(
     const uint32_t *__restrict__ ioff, int) {
   extern __shared__ __align__(16) uint32_t sm[];
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  WarpScratch &ws = *reinterpret_cast<WarpScratch *>(sm + (size_t)warp * per_warp);
-  int *const kz = reinterpret_cast<int *>(&ws + 1);
+  uint32_t *const scratch = sm + (size_t)warp * per_warp;
+  WarpScratch &ws = *reinterpret_cast<WarpScratch *>(scratch);  // (ray fill)
+  StScratch &ss = *reinterpret_cast<StScratch *>(scratch);      // (stencil fill)
+  uint32_t *const stage = ST ? scratch : ws.sol;
+  int *const kz = ST ? reinterpret_cast<int *>(&ss + 1) : reinterpret_cast<int *>(&ws + 1);
   uint32_t *const par = reinterpret_cast<uint32_t *>(kz + 32);
   Item it;
   uint32_t part;
@@ -1029,7 +1073,6 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_fill(
     // at the Level2 ray-origin height o2z[k][s] (minZ + (s + 0.5)*gridSizeZ2, :1297), so a
     // covered sample at height zs counts in every slice from the first with o2z >= zs: one
     // toggle bit there, expanded by a prefix XOR below.
-    StScratch &ss = *reinterpret_cast<StScratch *>(&ws);
     // triangles recorded from the chunk's first voxel up (those below are in the prefix)
     const uint32_t g0 = useg[ua], g1 = useg[ucol_end];
     const int SW = 2 * n2x, SH = 2 * n2y;
@@ -1038,11 +1081,17 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_fill(
     const float *ozt = g.o2[2];
     // with increasing clip heights, the chunk's highest one is its top voxel's last slice
     const float top_clip = __ldg(ozt + (size_t)kz[m - 1] * n2z + n2z - 1);
+    const int kz0 = kz[0], span = (kz[m - 1] - kz0 + 1) * n2z;  // clip heights from the chunk's first voxel up
+    const float *clip = ozt + (size_t)kz0 * n2z;
+    const float clip0 = __ldg(clip), inv_n2z = rcp_fast((float)n2z);
+    // bit i: layer kz0 + i belongs to the chunk
+    const uint32_t layers = __reduce_or_sync(FULL, ((int)lane < m && kz[lane] - kz0 < 32) ? 1u << (kz[lane] - kz0) : 0u);
 #pragma unroll 1
     for (uint32_t b0 = g0; b0 < g1; b0 += 32) {
       const uint32_t e = b0 + lane;
       const uint32_t vv = e < g1 ? vals[e] : 0u;
-      uint32_t cnt = 0;
+      StTri st = {};
+      bool has = false;
       if (vv & 0x80000000u) {
         const uint32_t t = vv & 0x7fffffffu;
         const float4 a0 = __ldg(ptri + 3 * (size_t)t), a1 = __ldg(ptri + 3 * (size_t)t + 1),
@@ -1054,52 +1103,39 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_fill(
         const float zmn = fminf(V[2], fminf(V[5], V[8]));
         const float zmag = fmaxf(fabsf(V[2]), fmaxf(fabsf(V[5]), fabsf(V[8])));
         const bool above = g.oz_monotone && zmn - 16.f * EPS24 * zmag > top_clip;
-        StTri st;
-        if (!above && st_setup(V, lx, hx, ly, hy, SW, SH, st)) {
-#pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            ss.v[lane][2 * c] = __int_as_float(st.X[c]);
-            ss.v[lane][2 * c + 1] = __int_as_float(st.Y[c]);
-            ss.v[lane][6 + c] = st.z[c];
-          }
-          ss.rA[lane] = st.rA;
-          const int nsx = st.sx1 - st.sx0 + 1;
-          ss.rng[lane] = (uint32_t)st.sx0 | ((uint32_t)nsx << 7) | ((uint32_t)st.sy0 << 14);
-          cnt = (uint32_t)(nsx * (st.sy1 - st.sy0 + 1));
-        }
+        has = !above && st_setup(V, lx, hx, ly, hy, SW, SH, st);
       }
-      const uint32_t inc = warp_incl_scan(cnt);
-      ss.pre[lane] = inc - cnt;
-      const uint32_t tot = __shfl_sync(FULL, inc, 31);
+      const StBatch batch(ss.r, has, st);
       __syncwarp();
 #pragma unroll 1
-      for (uint32_t w = lane; w < tot; w += 32) {
-        const int tl = batch_search(ss.pre, w);
-        const uint32_t loc = w - ss.pre[tl];
-        const uint32_t rg = ss.rng[tl];
-        const uint32_t nsx = (rg >> 7) & 127u;
-        const uint32_t row = loc / nsx;
-        StTri st;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          st.X[c] = __float_as_int(ss.v[tl][2 * c]);
-          st.Y[c] = __float_as_int(ss.v[tl][2 * c + 1]);
-          st.z[c] = ss.v[tl][6 + c];
-        }
-        st.rA = ss.rA[tl];
-        const int sx = (int)(rg & 127u) + (int)(loc - row * nsx), sy = (int)((rg >> 14) & 127u) + (int)row;
+      for (uint32_t w0 = 0; w0 < batch.total; w0 += 32) {
+        const StRec &r = batch.owner(ss.r, w0);
+        int sx, sy;
         float zs;
-        if (!st_cover(st, sx, sy, zs)) continue;
+        if (!(w0 + lane < batch.total && st_sample(r, w0 + lane, sx, sy, zs))) continue;
         const int sidx = sy * SW + sx, sbit = sidx * n2z;
         if (g.oz_monotone) {
           // clip heights increase through the chunk: the lowest voxel whose top clip keeps zs
           // gets its toggle at the first such slice, and every voxel above it keeps zs in all
-          // slices (one bit in its sample-toggle row, accumulated upwards)
-          int jv = 0;
+          // slices (one bit in its sample-toggle row, accumulated upwards).  The first height from
+          // the chunk's lowest that keeps zs, estimated and corrected by the table:
+          const float f = (zs - clip0) * g.inv_g2[2];
+          int i = !(f > 0.f) ? 0 : f >= (float)span ? span : __float2int_ru(f);
 #pragma unroll 1
-          while (jv < m && !(__ldg(ozt + (size_t)kz[jv] * n2z + n2z - 1) >= zs)) ++jv;
-          if (jv < m) {
-            const int b = sbit + st_first_slice(ozt + (size_t)kz[jv] * n2z, n2z, zs);
+          while (i > 0 && __ldg(clip + i - 1) >= zs) --i;
+#pragma unroll 1
+          while (i < span && !(__ldg(clip + i) >= zs)) ++i;
+          if (i < span) {
+            const int kq = __float2int_rz(((float)i + 0.5f) * inv_n2z);
+            int jv;  // the lowest voxel in or above that layer
+            if (kq < 32) {
+              jv = __popc(layers & ((1u << kq) - 1u));
+            } else {
+              jv = 0;
+#pragma unroll 1
+              while (kz[jv] - kz0 < kq) ++jv;
+            }
+            const int b = sbit + (kz[jv] - kz0 == kq ? i - kq * n2z : 0);
             atomicXor(&stg[jv * SWd + (b >> 5)], 1u << (b & 31));
             if (jv + 1 < m) atomicXor(&sft[(jv + 1) * FWS + (sidx >> 5)], 1u << (sidx & 31));
           }
@@ -1352,8 +1388,8 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_fill(
   const uint32_t pkend = d.l2codes ? bd.pk_end[slab] : 0u;
   const uint32_t vown = (int)lane < m ? (uint32_t)d.prefix[((int64_t)kz[lane] * ny + cj) * nx + ci] : 0u;
   if ((n2z == 8 || n2z == 16) && (ncol2 & 15) == 0 && (reinterpret_cast<uintptr_t>(d.l2) & 15) == 0) {
-    if (n2z == 8) write_chunk<8>(d.l2, d.l2codes, pkend, vown, satm, par, ft, m, ncol2, ws.sol, nbd, nin);
-    else write_chunk<16>(d.l2, d.l2codes, pkend, vown, satm, par, ft, m, ncol2, ws.sol, nbd, nin);
+    if (n2z == 8) write_chunk<8>(d.l2, d.l2codes, pkend, vown, satm, par, ft, m, ncol2, stage, nbd, nin);
+    else write_chunk<16>(d.l2, d.l2codes, pkend, vown, satm, par, ft, m, ncol2, stage, nbd, nin);
     __syncwarp();
   } else {
     // One lane per sub-column of the chunk: its n2z SAT and parity bits are read once and written
@@ -1409,8 +1445,9 @@ Level2Words level2_warp_words(const GridDev &g, int cap, bool stencil) {
   const int CH = level2_chunk(g, cap);
   const int FWS = (4 * g.n2[0] * g.n2[1] + 31) >> 5;
   const int base = (int)(sizeof(WarpScratch) / 4) + 32;
+  const int base_fill = (int)((stencil ? sizeof(StScratch) : sizeof(WarpScratch)) / 4) + 32;
   auto al = [](int words) { return (words + 3) & ~3; };  // a warp's region starts 16-byte aligned
-  return {al(base + 32 + std::max(CH, sat_run_cap(g)) * W), al(base + CH * W + CH * FW + (stencil ? 4 * CH * W + CH * FWS + FWS : 0))};
+  return {al(base + 32 + std::max(CH, sat_run_cap(g)) * W), al(base_fill + CH * W + CH * FW + (stencil ? 4 * CH * W + CH * FWS + FWS : 0))};
 }
 
 int level2_parts(int64_t B, int num_sms) {
