@@ -263,24 +263,33 @@ __device__ __forceinline__ bool sat_z_box_first(const SatCol &s, const float *V,
   return sat_z(s, V, cz, h);
 }
 
-// CUDAClassifyTessellationLevel2Kernel (.cu:403-448), one warp per boundary voxel walking the
-// voxel's list in order.  For each triangle the lanes take the sub-columns of the triangle's
-// Level2 cell range (l2_cell_range: outside it the SAT's own box axes reject, so nothing is
-// skipped that could pass), run the z-invariant axes once per sub-column and the z-dependent part
-// per cell of the range.  Within one triangle every cell has at most one lane; a __syncwarp
-// between triangles orders the updates, so each cell sums the CPU's unit face normals in list
-// order, as a per-cell thread would.  Centres come from `cen` ([b][n2x | n2y | n2z] floats,
-// formed on the host as the CPU does: float(((p+0.5)*gridSize2 + mid) - ext1) in double,
-// src/Object.cpp:2389-2391).  (One thread per (voxel, sub-column), most lanes left each
-// triangle at its box test: 6.4 of 32 lanes active, 1.50 ms on torus262k.)
-__global__ void k_shim_level2_sat(const float *__restrict__ tris, float *__restrict__ l2,
-                                  float *__restrict__ nrm, const float *__restrict__ cen,
-                                  const int *__restrict__ l2index, const int *__restrict__ cnt,
-                                  const int *__restrict__ flatIndex, const int *__restrict__ flat,
-                                  int B, int3 n2, float3 e2) {
+// CUDAClassifyTessellationLevel2Kernel (.cu:403-448), one warp per boundary voxel, its list 32 triangles
+// at a time in order.  A lane each finds a triangle's Level2 cell range (l2_cell_range: outside it the
+// SAT's own box axes reject, so nothing is skipped that could pass) and unit normal; then the lanes take
+// (triangle, sub-column) pairs of the ranges in list order, run the z-invariant axes once and the
+// z-dependent part per cell, and add: lanes with the same sub-column one after the other, so that each
+// cell sums the CPU's unit face normals in list order, as a per-cell thread would.  Centres come from
+// `cen` ([b][n2x | n2y | n2z] floats, formed on the host as the CPU does:
+// float(((p+0.5)*gridSize2 + mid) - ext1) in double, src/Object.cpp:2389-2391).  Bound by latency.  (A
+// triangle at a time, its sub-columns by the lanes: 175 us for 33k triangles at 64^3 / 4^3 against
+// 76.)
+constexpr int kShimWarps = 4;
+struct ShimWarp {
+  float V[32][9], fn[32][3];
+  int p0q0r0r1[32][4];
+  int np[32];
+  uint32_t pre[32];
+};
+__global__ void __launch_bounds__(kShimWarps * 32) k_shim_level2_sat(
+    const float *__restrict__ tris, float *__restrict__ l2, float *__restrict__ nrm, const float *__restrict__ cen,
+    const int *__restrict__ l2index, const int *__restrict__ cnt, const int *__restrict__ flatIndex,
+    const int *__restrict__ flat, int B, int3 n2, float3 e2) {
+  constexpr unsigned FULL = 0xffffffffu;
+  __shared__ ShimWarp s_w[kShimWarps];
   const int64_t b = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (b >= B) return;  // the whole warp
-  const int lane = (int)(threadIdx.x & 31u);
+  ShimWarp &ws = s_w[threadIdx.x >> 5];
+  const unsigned lane = threadIdx.x & 31u;
   const int ncol2 = n2.x * n2.y, cells = ncol2 * n2.z;
   const int v = l2index[b];
   const float *cx = cen + (size_t)b * (n2.x + n2.y + n2.z);
@@ -290,43 +299,90 @@ __global__ void k_shim_level2_sat(const float *__restrict__ tris, float *__restr
   const bool sized = e2.x > 0.f && e2.y > 0.f && e2.z > 0.f && isfinite(ig[0]) &&
                      isfinite(ig[1]) && isfinite(ig[2]);
   const int n = cnt[v], f0 = flatIndex[v];
-  for (int k = 0; k < n; ++k) {
-    const int t = flat[f0 + k];
-    float V[9];
-    for (int j = 0; j < 9; ++j) V[j] = tris[9 * (size_t)t + j];
-    int p0 = 0, p1 = n2.x - 1, q0 = 0, q1 = n2.y - 1, r0 = 0, r1 = n2.z - 1;
-    if (sized) {  // (cells of no size: every cell of the voxel is tested)
-      l2_cell_range(fminf(V[0], fminf(V[3], V[6])), fmaxf(V[0], fmaxf(V[3], V[6])), cx[0], h[0],
-                    ig[0], n2.x, p0, p1);
-      l2_cell_range(fminf(V[1], fminf(V[4], V[7])), fmaxf(V[1], fmaxf(V[4], V[7])), cy[0], h[1],
-                    ig[1], n2.y, q0, q1);
-      l2_cell_range(fminf(V[2], fminf(V[5], V[8])), fmaxf(V[2], fmaxf(V[5], V[8])), cz[0], h[2],
-                    ig[2], n2.z, r0, r1);
-    }
-    if (p0 <= p1 && q0 <= q1 && r0 <= r1) {
-      const int np = p1 - p0 + 1, items = np * (q1 - q0 + 1);
-      for (int it = lane; it < items; it += 32) {
-        const int qq = it / np, p = p0 + (it - qq * np), q = q0 + qq;
-        SatCol sc;
-        if (!sat_col_box_first(V, cx[p], cy[q], h, sc)) continue;
-        bool have_fn = false;
+  for (int k0 = 0; k0 < n; k0 += 32) {
+    // ---- a triangle per lane
+    uint32_t items = 0;
+    if (k0 + (int)lane < n) {
+      const int t = flat[f0 + k0 + (int)lane];
+      float V[9];
+#pragma unroll
+      for (int j = 0; j < 9; ++j) V[j] = tris[9 * (size_t)t + j];
+      int p0 = 0, p1 = n2.x - 1, q0 = 0, q1 = n2.y - 1, r0 = 0, r1 = n2.z - 1;
+      if (sized) {  // (cells of no size: every cell of the voxel is tested)
+        l2_cell_range(fminf(V[0], fminf(V[3], V[6])), fmaxf(V[0], fmaxf(V[3], V[6])), cx[0], h[0],
+                      ig[0], n2.x, p0, p1);
+        l2_cell_range(fminf(V[1], fminf(V[4], V[7])), fmaxf(V[1], fmaxf(V[4], V[7])), cy[0], h[1],
+                      ig[1], n2.y, q0, q1);
+        l2_cell_range(fminf(V[2], fminf(V[5], V[8])), fmaxf(V[2], fmaxf(V[5], V[8])), cz[0], h[2],
+                      ig[2], n2.z, r0, r1);
+      }
+      if (p0 <= p1 && q0 <= q1 && r0 <= r1) {
+        items = (uint32_t)(p1 - p0 + 1) * (uint32_t)(q1 - q0 + 1);
         float fn[3];
-        for (int r = r0; r <= r1; ++r) {
-          if (!sat_z_box_first(sc, V, cz[r], h)) continue;
-          if (!have_fn) {
-            face_normal(V, fn);
-            have_fn = true;
-          }
-          const size_t o = (size_t)b * cells + (size_t)r * ncol2 + (size_t)q * n2.x + p;
-          l2[o] = 2.0f;
-          nrm[4 * o + 0] = fa(nrm[4 * o + 0], fn[0]);
-          nrm[4 * o + 1] = fa(nrm[4 * o + 1], fn[1]);
-          nrm[4 * o + 2] = fa(nrm[4 * o + 2], fn[2]);
-          nrm[4 * o + 3] = fa(nrm[4 * o + 3], 1.0f);
-        }
+        face_normal(V, fn);
+#pragma unroll
+        for (int j = 0; j < 9; ++j) ws.V[lane][j] = V[j];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) ws.fn[lane][j] = fn[j];
+        ws.p0q0r0r1[lane][0] = p0;
+        ws.p0q0r0r1[lane][1] = q0;
+        ws.p0q0r0r1[lane][2] = r0;
+        ws.p0q0r0r1[lane][3] = r1;
+        ws.np[lane] = p1 - p0 + 1;
       }
     }
-    __syncwarp();  // this triangle's updates before the next triangle's
+    uint32_t inc = items;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t x = __shfl_up_sync(FULL, inc, o);
+      if (lane >= (unsigned)o) inc += x;
+    }
+    const uint32_t start = inc - items, total = __shfl_sync(FULL, inc, 31);
+    ws.pre[lane] = start;
+    const uint32_t some = __ballot_sync(FULL, items != 0u);
+    __syncwarp();
+    // ---- a (triangle, sub-column) pair per lane, in order
+    for (uint32_t w0 = 0; w0 < total; w0 += 32) {
+      // the pair's triangle: the last one with items that starts at or before it
+      const uint32_t here = __reduce_or_sync(FULL, items && start - w0 < 32u ? 1u << (start - w0) : 0u);
+      const uint32_t before = __popc(__ballot_sync(FULL, items && start < w0));
+      const int tl = (int)__fns(some, 0, (int)(before + __popc(here & ((2u << lane) - 1u))));
+      uint32_t m = 0, key = 0x80000000u | lane;
+      int col = 0, r0 = 0, r1 = -1;
+      SatCol sc;
+      if (w0 + lane < total) {
+        const int it = (int)(w0 + lane - ws.pre[tl]), np = ws.np[tl], qq = it / np;
+        const int p = ws.p0q0r0r1[tl][0] + (it - qq * np), q = ws.p0q0r0r1[tl][1] + qq;
+        if (sat_col_box_first(ws.V[tl], cx[p], cy[q], h, sc)) {
+          r0 = ws.p0q0r0r1[tl][2];
+          r1 = ws.p0q0r0r1[tl][3];
+          for (int r = r0; r <= min(r1, r0 + 31); ++r)
+            if (sat_z_box_first(sc, ws.V[tl], cz[r], h)) m |= 1u << (r - r0);
+          col = q * n2.x + p;
+          if (m || r1 - r0 > 31) key = (uint32_t)col;
+        }
+      }
+      const uint32_t peers = __match_any_sync(FULL, key);
+      const int rank = __popc(peers & ((1u << lane) - 1u));
+      const int rounds = __reduce_max_sync(FULL, rank);
+      for (int k = 0; k <= rounds; ++k) {
+        if (k == rank && !(key >> 31)) {
+          auto add = [&](int r) {
+            const size_t o = (size_t)b * cells + (size_t)r * ncol2 + (size_t)col;
+            l2[o] = 2.0f;
+            nrm[4 * o + 0] = fa(nrm[4 * o + 0], ws.fn[tl][0]);
+            nrm[4 * o + 1] = fa(nrm[4 * o + 1], ws.fn[tl][1]);
+            nrm[4 * o + 2] = fa(nrm[4 * o + 2], ws.fn[tl][2]);
+            nrm[4 * o + 3] = fa(nrm[4 * o + 3], 1.0f);
+          };
+          for (uint32_t x = m; x; x &= x - 1u) add(r0 + __ffs(x) - 1);
+          for (int r = r0 + 32; r <= r1; ++r)  // (sub-grids of more than 32 layers)
+            if (sat_z_box_first(sc, ws.V[tl], cz[r], h)) add(r);
+        }
+        __syncwarp();  // a sub-column's updates before its next triangle's
+      }
+    }
+    __syncwarp();
   }
 }
 
@@ -596,7 +652,7 @@ int CUDAClassifyTessellationLevel2(float *trianglesCUDAData, float *level2InOutC
   float *d_cen = static_cast<float *>(g_shim.dev);
   cudaMemcpyAsync(d_cen, cen, ncen * sizeof(float), cudaMemcpyHostToDevice, 0);
   const int64_t n = (int64_t)numBoundary * 32;  // a warp per boundary voxel
-  k_shim_level2_sat<<<(unsigned)((n + 127) / 128), 128>>>(
+  k_shim_level2_sat<<<(unsigned)((n + 32 * kShimWarps - 1) / (32 * kShimWarps)), 32 * kShimWarps>>>(
       trianglesCUDAData, level2InOutCUDAData, level2NormalCUDAData, d_cen, level2IndexCUDAData,
       voxelTriCountCUDAData, level1TriFlatIndexCUDAData, level1TriFlatCUDAData, numBoundary,
       numDiv2, boxExtentsLevel2);
