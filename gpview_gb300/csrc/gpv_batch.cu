@@ -559,6 +559,16 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
 
   // ---- one graph for the whole call, when the meshes and grids repeat the previous call's
   const uint64_t key = call_key(n, T, specs);
+  // Records of meshes without a Level2 grid are counted, not written: where their number exceeds this
+  // call's buffer, a later call with Level2 on the context starts with a larger one.
+  auto learn_pairs = [&] {
+    int64_t pairs = 0, need = 0;
+    for (int m = 0; m < n; ++m) {
+      pairs += (int64_t)ctx->h_stats[m].pairs;
+      need += (int64_t)ctx->h_stats[m].sat1;
+    }
+    if (pairs > pair_cap) ctx->pair_hint = std::max(ctx->pair_hint, need + need / 8);
+  };
   const bool og_path = ctx->graphs && ctx->one_graph && !sink && nmode == 0 && !stencil &&
                        res_hier[n] == 0;
   const bool og_skip = ctx->og_skip;  // (one-shot: the re-run of a call that did not fit)
@@ -651,8 +661,9 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
       ctx->og_skip = true;
       fail_all(GPV_OK, "");
       ctx->err.clear();
-      return run_batch(ctx, n, d_tris, T, specs, out, s);
+      return run_batch(ctx, n, d_tris, T, specs, out, s, sink);
     }
+    learn_pairs();
     take_stage_times();
     if (any_l2 && (int64_t)ctx->h_u32[1] != (int64_t)pl.ub)
       return fail_all(GPV_ERR_DEVICE, "boundary plane and pair lists disagree");
@@ -702,9 +713,10 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
       ctx->replans++;
       fail_all(GPV_OK, "");
       ctx->err.clear();
-      return run_batch(ctx, n, d_tris, T, specs, out, s);
+      return run_batch(ctx, n, d_tris, T, specs, out, s, sink);
     }
   }
+  learn_pairs();
   int64_t Btot = 0, l2bytes = 0, P2 = 0, ub = 0;
   std::vector<int64_t> l2off(n + 1, 0), boff(n + 1, 0);
   for (int m = 0; m < n; ++m) {
