@@ -256,7 +256,7 @@ inline int64_t level2_mask_words(int64_t B, int64_t l2bytes) { return l2bytes / 
 // With zslab > 0 and nslab > 1 the Level2 kernel runs once per slab of zslab Level1 layers (one
 // mesh with slab_nz Level1 layers): the outputs of slab k are contiguous and complete after the
 // work after_slab(k, stream) sees on `stream`, so a copy of them can start while the next slab
-// computes.  With aux, slab launches alternate between aux's two streams (joined back into s).
+// computes.  With aux, the slabs' SAT kernels and their fills run on aux's two streams (joined back into s).
 struct SlabStreams {  // two streams and their events for overlapping slab launches
   cudaStream_t st[2];
   cudaEvent_t fork, join[2];

@@ -435,7 +435,8 @@ __device__ __forceinline__ void transpose16(uint32_t (&w)[NZ / 2]) {
 
 // Output of a chunk whose n2z is NZ (8 or 16), with a multiple of 16 sub-columns and 16-byte aligned
 // blocks.  A lane takes 16 sub-columns of one voxel: their SAT and parity bits, transposed to layers,
-// are kept in `stage` (a word per layer, conflict-free) and written layer by layer, 16 bytes each.
+// are kept in `stage` (a word per layer, conflict-free) and written 16 bytes a lane: in output order,
+// 512 bytes of a warp at once, where a voxel's units are a power of two, else layer by layer.
 // With `codes`, the voxels whose output index is below `pkend` go out as 2-bit codes instead, a word
 // per 16 cells (cell k at bits 2k: 0 outside, 1 inside, 2 boundary), for the host to expand.
 template <int NZ>
@@ -444,7 +445,19 @@ __device__ __forceinline__ void write_chunk(uint8_t *l2, uint32_t *codes, uint32
                                             int m, int ncol2, uint32_t *stage, unsigned long long &nbd,
                                             unsigned long long &nin) {
   const int lane = (int)(threadIdx.x & 31u);
+  constexpr int S = NZ == 8 ? 36 : 32;  // (36: eight layers of four units are read without conflicts)
+  constexpr int LZ = NZ == 8 ? 3 : 4;
   const int upv = ncol2 >> 4, W = (ncol2 * NZ) >> 5, FW = (ncol2 + 31) >> 5;
+  // In output order the host link moves 512 bytes of a warp's store at once instead of 64 (8^3 cells,
+  // 192^3 / 8^3 host to host 1076 -> 1001 us) or 256 (16^3, 6.58 -> 6.47 ms for 1.28 GB); in device memory
+  // 8^3 cells take the same time either way, and 16^3 4% more.
+  const bool linear = (upv & (upv - 1)) == 0 && upv <= 32 && (NZ == 8 || codes);
+  const int sh = 31 - __clz(upv);
+  auto put = [&](size_t c, bool packed, uint32_t w) {  // 16-cell group c of the output
+    const uint32_t sb = w & 0xffffu, ib = w >> 16;
+    if (packed) __stcs(codes + c, spread16(sb) * 2u | spread16(ib));
+    else __stcs(reinterpret_cast<uint4 *>(l2) + c, state_bytes(sb, ib));
+  };
   uint32_t nb = 0, ni = 0;
 #pragma unroll 1
   for (int u0 = 0; u0 < m * upv; u0 += 32) {
@@ -469,19 +482,26 @@ __device__ __forceinline__ void write_chunk(uint8_t *l2, uint32_t *codes, uint32
       for (int i = 0; i < NZ / 2; ++i) {
         b[i] = (b[i] ^ f) & ~a[i];
         ni += (uint32_t)__popc(b[i]);
-        stage[(2 * i) * 32 + lane] = __byte_perm(a[i], b[i], 0x5410);
-        stage[(2 * i + 1) * 32 + lane] = __byte_perm(a[i], b[i], 0x7632);
+        stage[(2 * i) * S + lane] = __byte_perm(a[i], b[i], 0x5410);
+        stage[(2 * i + 1) * S + lane] = __byte_perm(a[i], b[i], 0x7632);
       }
-      const size_t c0 = (size_t)vidx * (size_t)(NZ * upv) + (size_t)k;  // 16-cell group of layer 0
-      const bool packed = vidx < pkend;
-      // streaming stores: the output is not read again, so it should not displace the working set
+    }
+    // streaming stores: the output is not read again, so it should not displace the working set
+    if (linear) {
+      __syncwarp();
+      const int total = min(32, m * upv - u0) * NZ;
 #pragma unroll 1
-      for (int r = 0; r < NZ; ++r) {
-        const uint32_t w = stage[r * 32 + lane], sb = w & 0xffffu, ib = w >> 16;
-        const size_t c = c0 + (size_t)(r * upv);
-        if (packed) __stcs(codes + c, spread16(sb) * 2u | spread16(ib));
-        else __stcs(reinterpret_cast<uint4 *>(l2) + c, state_bytes(sb, ib));
+      for (int i0 = 0; i0 < total; i0 += 32) {
+        const int i = i0 + lane, slot = i >> (sh + LZ), rem = i & ((NZ << sh) - 1);
+        const uint32_t v = __shfl_sync(FULL, vown, ((u0 >> sh) + slot) & 31);
+        const uint32_t w = stage[(rem >> sh) * S + (slot << sh) + (rem & (upv - 1))];
+        if (i < total) put((size_t)v * (size_t)(NZ * upv) + (size_t)rem, v < pkend, w);
       }
+      __syncwarp();
+    } else if (live) {
+      const size_t c0 = (size_t)vidx * (size_t)(NZ * upv) + (size_t)k;  // 16-cell group of layer 0
+#pragma unroll 1
+      for (int r = 0; r < NZ; ++r) put(c0 + (size_t)(r * upv), vidx < pkend, stage[r * S + lane]);
     }
   }
   nbd += nb;
@@ -792,8 +812,8 @@ __device__ __forceinline__ uint32_t *sat_words(const BatchDev &bd, const MeshDes
 // 262k-triangle torus, 128^3 / 8^3; 0.2 with two kernels).  The SAT masks go through device memory
 // (one bit per cell).  Both kernels are bound by instruction issue.  Measured against one kernel
 // testing every (triangle, sub-column) and listed cell exactly, both kernels together: the torus
-// 487 -> 197 us, a 1.3M-triangle star at 256^3 / 16^3 3.51 -> 1.27 ms, 256 mixed meshes in one call
-// 19.9 -> 9.9 ms.  A twentieth of the instructions are exact tests (0.4-2.7% of the sub-columns).
+// 487 -> 200 us, a 1.3M-triangle star at 256^3 / 16^3 3.51 -> 1.25 ms, 256 mixed meshes in one call
+// 19.9 -> 8.5 ms.  A twentieth of the instructions are exact tests (0.4-2.7% of the sub-columns).
 // Rows are solved by a lane per triangle looping over them (a lane per row took 190 us for the torus'
 // SAT against 134); the sub-columns they leave are listed and taken a lane each, because lanes that
 // walked their own row had 43-52% of them at work in the SAT and 34% in the fill (the star: SAT
@@ -1521,8 +1541,11 @@ void launch_level2(const BatchDev &bd, const uint32_t *keys, const uint32_t *val
     count_launch(3);
   }
   if (before_kernel) before_kernel();
-  // one launch, or one per z slab over that slab's items; slab launches alternate between two
-  // streams (when given) so that one slab's tail overlaps the next slab's start
+  // one launch of each kernel, or one per z slab over that slab's items; the slabs' SAT kernels run on
+  // one stream and their fills, each after its SAT, on another (when given), so that a slab's SAT
+  // overlaps the writes of the one before, and the slabs finish in order (fills of two slabs side by
+  // side finished together and left their copies or expansion to the end: 192^3 / 8^3 host to host
+  // 1098 against 1076 us)
   const int launches = zslab > 0 ? nslab : 1;
   const bool two = zslab > 0 && launches > 1 && aux;
   if (two) {
@@ -1531,11 +1554,15 @@ void launch_level2(const BatchDev &bd, const uint32_t *keys, const uint32_t *val
     cudaStreamWaitEvent(aux->st[1], aux->fork, 0);
   }
   for (int sl = 0; sl < launches; ++sl) {
-    cudaStream_t ls = two ? aux->st[sl & 1] : s;
     const uint32_t *list = zslab > 0 ? ilist : nullptr;
-    k_level2c_sat<<<grid_sat, kWarps * 32, smem_sat, ls>>>(bd, keys, vals, useg, runs ? runs : items,
+    cudaStream_t ss = two ? aux->st[0] : s, ls = two ? aux->st[1] : s;
+    k_level2c_sat<<<grid_sat, kWarps * 32, smem_sat, ss>>>(bd, keys, vals, useg, runs ? runs : items,
                                                           nitems + (runs ? 1 : 0), words.sat, sl, list, ioff,
                                                           parts);
+    if (two) {
+      cudaEventRecord(aux->join[0], ss);
+      cudaStreamWaitEvent(ls, aux->join[0], 0);
+    }
     fill<<<grid_fill, kWarps * 32, smem_fill, ls>>>(bd, keys, vals, useg, items, nitems, words.fill, sl,
                                                     list, ioff, 1);
     count_launch(2);

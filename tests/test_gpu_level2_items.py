@@ -81,3 +81,36 @@ def test_batch_of_unlike_meshes(ctx, built, normals):
                 ctx.release(r)
     finally:
         ctx.set_normals(gpv.NORMALS_OFF)
+
+
+@pytest.mark.parametrize("n2", [(4, 4, 8), (8, 4, 8), (4, 12, 8), (8, 8, 8), (16, 16, 8), (32, 32, 8), (4, 4, 16),
+                                (8, 8, 16), (12, 8, 16), (16, 32, 16)])
+@pytest.mark.parametrize("where", ["device", "direct", "packed"])
+def test_output_units(ctx, built, n2, where):
+    # one unit of 16 sub-columns a voxel to 64, powers of two and not, in device memory, written to the
+    # host as bytes, and as packed codes for the first half of every slab's voxels
+    import torch
+
+    gpv = built
+    tris = _walls(9)
+    spec = _spec(gpv, (9, 7, 11), n2)
+    want = orc.Run(tris, spec, fill=orc.FILL_CAND).level2_bytes()
+    if where == "device":
+        res = ctx.voxelize_host(tris, spec)
+        np.testing.assert_array_equal(ctx.fetch(res)[3], want)
+        ctx.release(res)
+        return
+    n1 = 9 * 7 * 11
+    pin = [torch.empty(n, dtype=torch.uint8).pin_memory() for n in (n1, 4 * n1, 4 * n1, want.size)]
+    h = torch.from_numpy(tris).pin_memory()
+    if where == "packed":
+        ctx.set_host_expand(2, 0xff, 50, 0)
+    try:
+        for _ in range(2):
+            pin[3].fill_(77)
+            rc, res = ctx.voxelize_to_host(h.data_ptr(), tris.size // 9, spec, *[p.data_ptr() for p in pin], want.size, 0)
+            assert rc == 0
+            np.testing.assert_array_equal(pin[3].numpy(), want)
+            ctx.release(res)
+    finally:
+        ctx.set_host_expand()
