@@ -534,15 +534,16 @@ def run_reference(args):
     print(json.dumps(line))
 
 
-# Warp instructions one launch of the Level2 kernel executes on each single-mesh workload, from
-# a one-launch capture `ncu --metrics smsp__inst_executed.sum,dram__bytes_read.sum,
-# dram__bytes_write.sum -k regex:k_level2c -c 1` of this bench on that workload.  The count is a
-# property of the kernel's code and the input, not of the clock; it is re-captured whenever the
-# kernel changes.
-LEVEL2_INST_PER_LAUNCH = {"star1310k": 3465057518, "torus262k": 330108311, "sphere16k": 24003464}
-# DRAM bytes read + written by one launch of the Level2 kernel (same captures)
-LEVEL2_TRAFFIC = {"star1310k": 128589568 + 1140417024, "torus262k": 30649344 + 4477440,
-                  "sphere16k": 2835456 + 0}
+# Warp instructions one launch of each of the two Level2 kernels (SAT and fill) executes, together, on
+# each single-mesh workload, from a capture `ncu --metrics smsp__inst_executed.sum,dram__bytes_read.sum,
+# dram__bytes_write.sum -k regex:k_level2c -c 2` of this bench on that workload.  The count is a
+# property of the kernels' code and the input, not of the clock; it is re-captured whenever they
+# change.
+LEVEL2_INST_PER_LAUNCH = {"star1310k": 705009388 + 459543690, "torus262k": 89230517 + 52592097,
+                          "sphere16k": 9182402 + 6652508}
+# DRAM bytes read + written by them (same captures)
+LEVEL2_TRAFFIC = {"star1310k": 92091392 + 248506624 + 105511168 + 1144705536,
+                  "torus262k": 20294400 + 37156352 + 1792 + 4806656, "sphere16k": 1637376 + 2857984 + 256}
 
 
 def max_over_ranks(seconds, dist, device):
