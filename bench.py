@@ -539,11 +539,11 @@ def run_reference(args):
 # dram__bytes_write.sum -k regex:k_level2c -c 2` of this bench on that workload.  The count is a
 # property of the kernels' code and the input, not of the clock; it is re-captured whenever they
 # change.
-LEVEL2_INST_PER_LAUNCH = {"star1310k": 705009388 + 459543690, "torus262k": 89230517 + 52592097,
-                          "sphere16k": 9182402 + 6652508}
+LEVEL2_INST_PER_LAUNCH = {"star1310k": 705071604 + 460067112, "torus262k": 89242821 + 51473708,
+                          "sphere16k": 9181381 + 6783604}
 # DRAM bytes read + written by them (same captures)
-LEVEL2_TRAFFIC = {"star1310k": 92091392 + 248506624 + 105511168 + 1144705536,
-                  "torus262k": 20294400 + 37156352 + 1792 + 4806656, "sphere16k": 1637376 + 2857984 + 256}
+LEVEL2_TRAFFIC = {"star1310k": 92170496 + 240988160 + 106115584 + 1140317440,
+                  "torus262k": 20294144 + 36299264 + 3584 + 5583616, "sphere16k": 1637888 + 2834944 + 256}
 
 
 def max_over_ranks(seconds, dist, device):

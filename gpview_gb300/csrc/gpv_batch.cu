@@ -773,6 +773,7 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
   if (l2_direct) {
     set->l2 = sink->l2_dev;
     set->l2_external = true;
+    bd.l2_host = 1;
   } else {
     CK(ctx_malloc_async(ctx, &set->l2, std::max<int64_t>(l2bytes, 16), s));
   }
@@ -881,7 +882,7 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
                      (uint64_t)(uintptr_t)wtot, (uint64_t)(uintptr_t)useg, (uint64_t)any_l2,
                      (uint64_t)ub, (uint64_t)(uintptr_t)l2tmp, (uint64_t)l2_words.sat, (uint64_t)l2_words.fill,
                      (uint64_t)(uintptr_t)bd.smask, (uint64_t)zslab,
-                     (uint64_t)nslab, (uint64_t)gh[0].n[2], (uint64_t)(sink != nullptr),
+                     (uint64_t)nslab, (uint64_t)gh[0].n[2], (uint64_t)(sink != nullptr), (uint64_t)bd.l2_host,
                      (uint64_t)(uintptr_t)(sink ? sink->l1 : nullptr),
                      (uint64_t)(uintptr_t)(sink ? sink->prefix : nullptr),
                      (uint64_t)(uintptr_t)(sink ? sink->bindex : nullptr), (uint64_t)gh[0].N1,

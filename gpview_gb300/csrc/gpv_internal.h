@@ -147,6 +147,7 @@ struct BatchDev {
   // packed Level2 host output: in z slab k of the Level2 launch, the boundary voxels whose output
   // index is below pk_end[k] write MeshDesc::l2codes instead of bytes (the slab's first share)
   uint32_t pk_end[kSlabsMax] = {};
+  int l2_host = 0;  // the Level2 states go to host memory
   // Level2 SAT masks (one bit per cell) between the two Level2 kernels, level2_mask_words() of them
   uint32_t *smask = nullptr;
   // one-graph calls: the device-computed sizes of the second half (nullptr: sizes from the host)

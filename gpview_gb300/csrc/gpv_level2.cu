@@ -435,23 +435,22 @@ __device__ __forceinline__ void transpose16(uint32_t (&w)[NZ / 2]) {
 
 // Output of a chunk whose n2z is NZ (8 or 16), with a multiple of 16 sub-columns and 16-byte aligned
 // blocks.  A lane takes 16 sub-columns of one voxel: their SAT and parity bits, transposed to layers,
-// are kept in `stage` (a word per layer, conflict-free) and written 16 bytes a lane: in output order,
-// 512 bytes of a warp at once, where a voxel's units are a power of two, else layer by layer.
+// are kept in `stage` (a word per layer, conflict-free) and written layer by layer, 16 bytes a lane.  HOST
+// (outputs in host memory, voxels of a power of two of units): in output order, 512 bytes of a warp at
+// once instead of 64 (8^3 cells) or 256, which the link moves faster: 192^3 / 8^3 host to host 1076 ->
+// 1001 us, 1.28 GB of 16^3 cells 6.58 -> 6.47 ms; device memory takes the layers 1-4% faster.
 // With `codes`, the voxels whose output index is below `pkend` go out as 2-bit codes instead, a word
 // per 16 cells (cell k at bits 2k: 0 outside, 1 inside, 2 boundary), for the host to expand.
-template <int NZ>
+template <int NZ, bool HOST>
 __device__ __forceinline__ void write_chunk(uint8_t *l2, uint32_t *codes, uint32_t pkend, uint32_t vown,
                                             const uint32_t *satm, const uint32_t *par, const uint32_t *ft,
                                             int m, int ncol2, uint32_t *stage, unsigned long long &nbd,
                                             unsigned long long &nin) {
   const int lane = (int)(threadIdx.x & 31u);
-  constexpr int S = NZ == 8 ? 36 : 32;  // (36: eight layers of four units are read without conflicts)
+  constexpr int S = HOST && NZ == 8 ? 36 : 32;  // (36: eight layers of four units read without conflicts)
   constexpr int LZ = NZ == 8 ? 3 : 4;
   const int upv = ncol2 >> 4, W = (ncol2 * NZ) >> 5, FW = (ncol2 + 31) >> 5;
-  // In output order the host link moves 512 bytes of a warp's store at once instead of 64 (8^3 cells,
-  // 192^3 / 8^3 host to host 1076 -> 1001 us) or 256 (16^3, 6.58 -> 6.47 ms for 1.28 GB); in device memory
-  // 8^3 cells take the same time either way, and 16^3 4% more.
-  const bool linear = (upv & (upv - 1)) == 0 && upv <= 32 && (NZ == 8 || codes);
+  const bool linear = HOST && (upv & (upv - 1)) == 0 && upv <= 32;
   const int sh = 31 - __clz(upv);
   auto put = [&](size_t c, bool packed, uint32_t w) {  // 16-cell group c of the output
     const uint32_t sb = w & 0xffffu, ib = w >> 16;
@@ -1022,7 +1021,8 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_sat(
 
 // k_level2c_fill: the inside fill, and the Level2 states from it and the SAT masks.
 // ST: the stencil fill (ClassifyInOut2xLevel2) instead of the ray fill.
-template <bool ST>
+// HOST: the states go to host memory (write_chunk).
+template <bool ST, bool HOST>
 __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_fill(
     BatchDev bd, const uint32_t *__restrict__ keys, const uint32_t *__restrict__ vals,
     const uint32_t *__restrict__ useg, const Item *__restrict__ items,
@@ -1408,8 +1408,8 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_fill(
   const uint32_t pkend = d.l2codes ? bd.pk_end[slab] : 0u;
   const uint32_t vown = (int)lane < m ? (uint32_t)d.prefix[((int64_t)kz[lane] * ny + cj) * nx + ci] : 0u;
   if ((n2z == 8 || n2z == 16) && (ncol2 & 15) == 0 && (reinterpret_cast<uintptr_t>(d.l2) & 15) == 0) {
-    if (n2z == 8) write_chunk<8>(d.l2, d.l2codes, pkend, vown, satm, par, ft, m, ncol2, stage, nbd, nin);
-    else write_chunk<16>(d.l2, d.l2codes, pkend, vown, satm, par, ft, m, ncol2, stage, nbd, nin);
+    if (n2z == 8) write_chunk<8, HOST>(d.l2, d.l2codes, pkend, vown, satm, par, ft, m, ncol2, stage, nbd, nin);
+    else write_chunk<16, HOST>(d.l2, d.l2codes, pkend, vown, satm, par, ft, m, ncol2, stage, nbd, nin);
     __syncwarp();
   } else {
     // One lane per sub-column of the chunk: its n2z SAT and parity bits are read once and written
@@ -1511,7 +1511,7 @@ void launch_level2(const BatchDev &bd, const uint32_t *keys, const uint32_t *val
   }
   const bool st = bd.fill == GPV_FILL_STENCIL;
   using Kern = decltype(&k_level2c_sat);
-  static bool attr_set[3] = {false, false, false};
+  static bool attr_set[5] = {};
   // a kernel's persistent grid (one-graph calls: B is a capacity, the queue ends the work)
   auto grid_of = [&](Kern k, int kv, size_t smem, int64_t jobs) {
     if (!attr_set[kv]) {
@@ -1527,10 +1527,12 @@ void launch_level2(const BatchDev &bd, const uint32_t *keys, const uint32_t *val
   // words.  42 voxels of 7k triangles: the SAT kernel 424 -> 17 us.
   const int parts = level2_parts(B, num_sms);
   if (parts > 1) cudaMemsetAsync(bd.smask, 0, (size_t)smask_words * sizeof(uint32_t), s);
-  const Kern fill = st ? k_level2c_fill<true> : k_level2c_fill<false>;
+  const bool host = bd.l2_host;
+  const Kern fill = st ? (host ? k_level2c_fill<true, true> : k_level2c_fill<true, false>)
+                       : (host ? k_level2c_fill<false, true> : k_level2c_fill<false, false>);
   const size_t smem_sat = level2_smem_bytes(words.sat), smem_fill = level2_smem_bytes(words.fill);
   const unsigned grid_sat = grid_of(k_level2c_sat, 0, smem_sat, B * parts);
-  const unsigned grid_fill = grid_of(fill, st ? 2 : 1, smem_fill, B);
+  const unsigned grid_fill = grid_of(fill, 1 + 2 * st + host, smem_fill, B);
   const int nz = slab_nz;
   if (zslab > 0) {
     // single mesh: order the items by slab so that each launch takes only its own
