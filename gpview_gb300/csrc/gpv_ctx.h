@@ -41,9 +41,10 @@ struct gpv_ctx {
   double host_ms[5] = {};
   std::string err;
   int tile = 0;                        // Level1 triangles per ticket (autotuned; 0: by the call's size)
-  // Level2 boundary voxels per chunk, upper bound (autotuned by gpv_autotune; the mask space caps
-  // it at 4 for 16^3 sub-grids).  torus262k at 8^3, Level2 kernel ms: 8 -> 0.626, 16 -> 0.596,
-  // 32 -> 0.712 (fewer chunks per column repeat the fill's u/v work for the triangles above them)
+  // Level2 boundary voxels per fill chunk, upper bound (autotuned by gpv_autotune; the mask space caps
+  // it at 4 for 16^3 sub-grids).  262k-triangle torus at 128^3 / 8^3, us per call: 4 -> 441, 8 -> 407,
+  // 16 -> 398, 32 -> 407; with the stencil fill 639, 609, 620, 733 (shorter chunks repeat the work for the
+  // triangles above them, longer ones leave fewer and less even items)
   int l2_chunk_cap = 16;
   int l2_mode = GPV_LEVEL2_AUTO;       // gpv_set_level2_mode (no effect)
   // failure-detection hooks (gpv_set_debug) and what they caused (gpv_get_debug)

@@ -2,9 +2,9 @@
 // triangle lists (the reference builds them on the host, src/Object.cpp:2146-2180, and
 // compacts boundary voxels there too, :3271-3279).
 //
-// scan_u32:  (of values or bit counts) reduce-then-scan, no inter-block waiting: tile sums, then a down-sweep in which every
-//            block adds up the sums of the tiles before it (up to 1024 tiles; beyond that a
-//            separate single-block scan of the tile sums runs in between).
+// scan_u32:  of values or of words' bit counts, reduce-then-scan, no inter-block waiting: tile sums, then
+//            a down-sweep in which every block adds up the sums of the tiles before it (up to 1024
+//            tiles; beyond that a separate single-block scan of the tile sums runs in between).
 // sort_pairs: stable LSD radix sort of (u32 key, u32 value), 8-bit digits; per pass a tile
 //             histogram, a scan of the digit-major histogram, and a stable scatter whose
 //             in-tile ranks come from __match_any_sync peer masks.
