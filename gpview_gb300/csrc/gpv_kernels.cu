@@ -186,12 +186,14 @@ __global__ void __launch_bounds__(256) k_prep(BatchDev bd) {
     int lo[3], hi[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      // cell_of grows with v but for the step down at v == max, so the cells of the smallest and the
-      // largest coordinate bound the third's (a hi past the last cell is cut to it)
+      // cell_of grows with v but for the step down from n to n - 1 at v == max, so the cells of the
+      // smallest and the largest coordinate bound the third's unless that one is at max, where the
+      // smallest may lie just under it, in cell n (a hi past the last cell is cut to it)
       const float inv = (float)g.n[a] / (g.bmax[a] - g.bmin[a]);
       const int c0 = cell_near(fminf(V[a], fminf(V[3 + a], V[6 + a])), g.bmin[a], g.bmax[a], g.n[a], inv);
       const int c1 = cell_near(fmaxf(V[a], fmaxf(V[3 + a], V[6 + a])), g.bmin[a], g.bmax[a], g.n[a], inv);
-      lo[a] = max(min(c0, c1), 0);
+      const bool at_max = V[a] == g.bmax[a] || V[3 + a] == g.bmax[a] || V[6 + a] == g.bmax[a];
+      lo[a] = max(min(c0, at_max ? min(c1, g.n[a] - 1) : c1), 0);
       hi[a] = min(max(c0, c1), g.n[a] - 1);
     }
     float4 fb = ray_box(V, g);
