@@ -8,8 +8,19 @@
 
 #include "../../include/gpview.h"
 #include "gpv_common.cuh"
+#include "gpv_once.h"
 
 namespace gpv {
+
+// Lets `kernel` use up to `bytes` of dynamic shared memory on the current device.
+template <typename K>
+inline void allow_shared_memory(OncePerDevice &once, K *kernel, size_t bytes) {
+  int device = 0;
+  cudaGetDevice(&device);
+  once(device, [&] {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
+  });
+}
 
 // ---- launch accounting: every kernel launch of the library bumps this counter ----------------
 uint64_t launch_count();

@@ -1511,13 +1511,10 @@ void launch_level2(const BatchDev &bd, const uint32_t *keys, const uint32_t *val
   }
   const bool st = bd.fill == GPV_FILL_STENCIL;
   using Kern = decltype(&k_level2c_sat);
-  static bool attr_set[5] = {};
+  static OncePerDevice once[5];
   // a kernel's persistent grid (one-graph calls: B is a capacity, the queue ends the work)
   auto grid_of = [&](Kern k, int kv, size_t smem, int64_t jobs) {
-    if (!attr_set[kv]) {
-      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-      attr_set[kv] = true;
-    }
+    allow_shared_memory(once[kv], k, 200 * 1024);
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kWarps * 32, smem);
     const int64_t full = (int64_t)num_sms * std::max(per_sm, 1);

@@ -700,11 +700,8 @@ void launch_normals(const BatchDev &bd, const uint32_t *keys, const uint32_t *va
   count_launch();
   if (max_cells <= 0) return;
   const size_t smem = kNWarps * sizeof(NWarp);
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaFuncSetAttribute(k_level2_normals, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    attr_set = true;
-  }
+  static OncePerDevice once;
+  allow_shared_memory(once, k_level2_normals, smem);
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_level2_normals, kNWarps * 32, smem);
   const int64_t warps = (int64_t)num_sms * std::max(per_sm, 1) * kNWarps;
