@@ -439,7 +439,7 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
                        (uint64_t)bd.total_tris, (uint64_t)bd.total_tiles, (uint64_t)bd.total_fblks,
                        (uint64_t)bd.total_rows, (uint64_t)bd.total_words, (uint64_t)bd.total_xchunks,
                        (uint64_t)(uintptr_t)bd.queue, (uint64_t)(uintptr_t)bd.heavy, (uint64_t)bd.normals, (uint64_t)bd.fill,
-                       (uint64_t)(uintptr_t)bd.stp, (uint64_t)bd.stp_words,
+                       (uint64_t)(uintptr_t)bd.stp, (uint64_t)bd.stp_words, (uint64_t)(uintptr_t)bd.kmask,
                        (uint64_t)ctx->timing, (uint64_t)ctx->num_sms, (uint64_t)bd.wait_limit,
                        (uint64_t)bd.fail_wait})
       v.push_back(x);
@@ -881,7 +881,7 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
                      (uint64_t)(uintptr_t)sortmp, (uint64_t)(uintptr_t)flags, (uint64_t)(uintptr_t)uidx,
                      (uint64_t)(uintptr_t)wtot, (uint64_t)(uintptr_t)useg, (uint64_t)any_l2,
                      (uint64_t)ub, (uint64_t)(uintptr_t)l2tmp, (uint64_t)l2_words.sat, (uint64_t)l2_words.fill,
-                     (uint64_t)(uintptr_t)bd.smask, (uint64_t)zslab,
+                     (uint64_t)(uintptr_t)bd.smask, (uint64_t)l2bytes, (uint64_t)zslab,
                      (uint64_t)nslab, (uint64_t)gh[0].n[2], (uint64_t)(sink != nullptr), (uint64_t)bd.l2_host,
                      (uint64_t)(uintptr_t)(sink ? sink->l1 : nullptr),
                      (uint64_t)(uintptr_t)(sink ? sink->prefix : nullptr),
