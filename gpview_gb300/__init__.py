@@ -145,6 +145,7 @@ def lib():
                                               C.c_void_p, C.c_void_p, C.c_void_p,
                                               C.POINTER(C.c_int64), C.c_void_p]
     L.gpv_noalloc_last_error.restype = C.c_char_p
+    L.gpv_noalloc_set_debug.argtypes = [C.c_int, C.c_int64]
     L.gpv_set_level2_chunk.argtypes = [C.c_void_p, C.c_int]
     L.gpv_set_level2_mode.argtypes = [C.c_void_p, C.c_int]
     L.gpv_set_debug.argtypes = [C.c_void_p, C.c_int, C.c_int64]

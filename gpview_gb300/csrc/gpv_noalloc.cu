@@ -41,6 +41,9 @@ constexpr size_t kBytesPerTriangle = 80;
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
 thread_local char g_err[256] = "";
+// failure-detection hooks of this host thread's calls (gpv_noalloc_set_debug)
+thread_local uint32_t g_wait_limit = 0;
+thread_local int g_fail_wait = 0;
 
 void set_err(const char *msg) {
   std::snprintf(g_err, sizeof(g_err), "%s", msg);
@@ -54,6 +57,15 @@ size_t align256(size_t v) { return (v + 255) & ~size_t(255); }
 using namespace gpv;
 
 extern "C" const char *gpv_noalloc_last_error(void) { return g_err; }
+
+extern "C" int gpv_noalloc_set_debug(int what, int64_t value) {
+  if (value < 0 || value > 0xffffffffll) return GPV_ERR_INVALID;
+  switch (what) {
+    case GPV_DEBUG_WAIT_LIMIT: g_wait_limit = (uint32_t)value; return GPV_OK;
+    case GPV_DEBUG_FAIL_WAIT: g_fail_wait = value != 0; return GPV_OK;
+    default: return GPV_ERR_INVALID;
+  }
+}
 
 extern "C" int gpv_voxelize_level1_noalloc(const float *d_tris, int64_t num_triangles,
                                            const gpv_grid_spec *spec, uint8_t *d_level1_inout,
@@ -211,6 +223,8 @@ extern "C" int gpv_voxelize_level1_noalloc(const float *d_tris, int64_t num_tria
   bd.heavy_cap = (uint32_t)std::min<size_t>(std::max(own_cap, rest_cap), kHeavyCap);
   bd.heavy = bd.heavy_cap ? reinterpret_cast<uint4 *>(base + (rest_cap > own_cap ? o : o_hv)) : nullptr;
   bd.heavy_n = d_tot + 2;
+  bd.wait_limit = g_wait_limit;
+  bd.fail_wait = g_fail_wait;
   bd.total_tris = T;
   bd.total_fblks = finish_blocks((int64_t)g.n[1] * g.nxw);
   bd.total_rows = (int64_t)g.n[2] * g.n[1];
@@ -248,6 +262,10 @@ extern "C" int gpv_voxelize_level1_noalloc(const float *d_tris, int64_t num_tria
   if (hs.status & ST_BAD_INPUT) {
     set_err("non-finite vertex");
     return GPV_ERR_INVALID;
+  }
+  if (hs.status) {
+    set_err("device status raised in Level1 (a bounded wait gave up)");
+    return GPV_ERR_DEVICE;
   }
   *num_boundary = (int64_t)nb;
   set_err("");

@@ -313,6 +313,9 @@ int gpv_voxelize_level1_noalloc(const float *d_tris, int64_t num_triangles,
                                 int32_t *d_level1_prefix, int32_t *d_boundary_index,
                                 int64_t *num_boundary, cudaStream_t stream);
 const char *gpv_noalloc_last_error(void);
+/* GPV_DEBUG_WAIT_LIMIT and GPV_DEBUG_FAIL_WAIT (see gpv_set_debug) for the calling host thread's
+ * calls of gpv_voxelize_level1_noalloc, which returns GPV_ERR_DEVICE when a wait gave up. */
+int gpv_noalloc_set_debug(int what, int64_t value);
 
 /* ---- serving: continuous batching (no counterpart in the reference) -------------------------
  * Requests carry host triangles (caller memory, valid until the request completes; pinned memory
