@@ -320,7 +320,7 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
     CK(ws.get(&d_slab, kMaxSlabs + 1));
   }
   // the statistics, then the queue tickets and the heavy list's length: cleared together
-  const size_t stats_bytes = n * sizeof(MeshStats), acc_bytes = stats_bytes + 4 * (kQueueWords + 1);
+  const size_t stats_bytes = n * sizeof(MeshStats), acc_bytes = stats_bytes + 4 * kQueueWords;
   {
     unsigned char *acc;
     CK(ws.get(&acc, acc_bytes));
@@ -389,7 +389,7 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
   bd.total_words = words;
   bd.queue = queue;
   bd.heavy = heavy;
-  bd.heavy_n = queue + kQueueWords;
+  bd.heavy_n = reinterpret_cast<unsigned long long *>(queue + kQueueHeavy);
   bd.heavy_cap = kHeavyCap;
   bd.normals = nmode;
   bd.emit_all = nmode != 0;

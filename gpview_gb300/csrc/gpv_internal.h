@@ -120,7 +120,9 @@ constexpr int kFillNone = -1;
 constexpr int kSlabsMax = 8;
 constexpr int kQueueItems = 1 + 2 * kSlabsMax;
 constexpr int kQueueNormals = kQueueItems + 2;
-constexpr int kQueueWords = kQueueNormals + 1;
+constexpr int kQueueHeavy = kQueueNormals + 1;  // BatchDev::heavy_n, two words
+constexpr int kQueueWords = kQueueHeavy + 2;
+static_assert(kQueueHeavy % 2 == 0, "heavy_n is 8-byte aligned where the queue is");
 constexpr uint32_t kHeavyCap = 1u << 18;  // pieces of a call's heavy list (4 MiB)
 
 constexpr int kFinishGroups = 8;  // plane words of a layer that one fill-finish block takes
@@ -147,9 +149,11 @@ struct BatchDev {
   // grid (the others' are only counted)
   int emit_all = 0;
   // Level1 pieces of triangles with many units, {mesh, triangle, piece, valid}: written by the prep
-  // kernel, heavy_n of them (zeroed before it), room for heavy_cap; nullptr: none are split
+  // kernel, heavy_n of them (zeroed before it), room for heavy_cap; nullptr: none are split.  Triangles
+  // that find the list full still add their pieces to heavy_n (64 bits: 2^31 triangles of up to
+  // heavy_cap pieces do not wrap it)
   uint4 *heavy = nullptr;
-  uint32_t *heavy_n = nullptr;
+  unsigned long long *heavy_n = nullptr;
   uint32_t heavy_cap = 0;
   // Level1's bounded wait for its staged tile: polls before giving up (0: the built-in limit);
   // fail_wait != 0 gives up at once (GPV_DEBUG_FAIL_WAIT, failure-detection tests)

@@ -243,9 +243,10 @@ __global__ void __launch_bounds__(256) k_prep(BatchDev bd) {
     if (bd.heavy && su + fu > (unsigned long long)kHeavyUnits) {
       const unsigned long long pieces = ((su + 31) / 32 + (fu + 31) / 32 + kHeavyChunks - 1) / kHeavyChunks;
       if (pieces <= bd.heavy_cap) {
-        const uint32_t pos = atomicAdd(bd.heavy_n, (uint32_t)pieces);
-        listed = pos < bd.heavy_cap && bd.heavy_cap - pos >= (uint32_t)pieces;
-        for (uint32_t k = 0; k < (uint32_t)pieces && pos < bd.heavy_cap && k < bd.heavy_cap - pos; ++k)
+        const unsigned long long pos = atomicAdd(bd.heavy_n, pieces), cap = bd.heavy_cap;
+        listed = pos < cap && cap - pos >= pieces;
+        const uint32_t room = pos < cap ? (uint32_t)min(cap - pos, pieces) : 0u;
+        for (uint32_t k = 0; k < room; ++k)
           bd.heavy[pos + k] = make_uint4((uint32_t)m, (uint32_t)t, k, (uint32_t)listed);
       }
     }
@@ -518,7 +519,7 @@ __global__ void __launch_bounds__(kL1Warps * 32, 8) k_level1(BatchDev bd, uint32
   }
   __syncwarp();
 
-  const uint32_t nheavy = bd.heavy ? min(*bd.heavy_n, bd.heavy_cap) : 0u;
+  const uint32_t nheavy = bd.heavy ? (uint32_t)min(*bd.heavy_n, (unsigned long long)bd.heavy_cap) : 0u;
   const uint32_t nitems = nheavy + (uint32_t)(bd.total_tiles * S);
   // the group after `it`: the next of its ticket, or the first of a new ticket
   auto advance = [&](L1Item &it) {

@@ -222,7 +222,7 @@ extern "C" int gpv_voxelize_level1_noalloc(const float *d_tris, int64_t num_tria
   const size_t own_cap = (size_t)N1w / 4, rest_cap = (kScratchBytes - o) / sizeof(uint4);
   bd.heavy_cap = (uint32_t)std::min<size_t>(std::max(own_cap, rest_cap), kHeavyCap);
   bd.heavy = bd.heavy_cap ? reinterpret_cast<uint4 *>(base + (rest_cap > own_cap ? o : o_hv)) : nullptr;
-  bd.heavy_n = d_tot + 2;
+  bd.heavy_n = reinterpret_cast<unsigned long long *>(d_tot + 2);
   bd.wait_limit = g_wait_limit;
   bd.fail_wait = g_fail_wait;
   bd.total_tris = T;

@@ -492,7 +492,7 @@ int CUDAClassifyTessellation(float *trianglesCUDAData, int numTriangles, float *
                o_rng = take(16 * (size_t)T), o_fbox = take(16 * (size_t)T),
                o_bp = take(4 * (size_t)N1w), o_ip = take(4 * (size_t)N1w),
                o_tg = take(4 * (size_t)tog), o_st = take(sizeof(MeshStats)),
-               o_md = take(sizeof(MeshDesc)), o_q = take(4 * (kQueueWords + 1)), o_hv = take(16 * (size_t)kHeavyCap);
+               o_md = take(sizeof(MeshDesc)), o_q = take(4 * kQueueWords), o_hv = take(16 * (size_t)kHeavyCap);
   const size_t fixed = off;
   const bool aligned = (reinterpret_cast<uintptr_t>(trianglesCUDAData) & 15u) == 0;
   if (!shim_reserve(fixed) || !shim_tables((size_t)ntab)) return 1;
@@ -537,11 +537,11 @@ int CUDAClassifyTessellation(float *trianglesCUDAData, int numTriangles, float *
   auto set_queue = [&] {
     bd.queue = reinterpret_cast<uint32_t *>(base + o_q);
     bd.heavy = reinterpret_cast<uint4 *>(base + o_hv);
-    bd.heavy_n = bd.queue + kQueueWords;
+    bd.heavy_n = reinterpret_cast<unsigned long long *>(bd.queue + kQueueHeavy);
     bd.heavy_cap = kHeavyCap;
   };
   set_queue();
-  cudaMemsetAsync(bd.queue, 0, 4 * (kQueueWords + 1), 0);
+  cudaMemsetAsync(bd.queue, 0, 4 * kQueueWords, 0);
   bd.emit_all = 1;
   bd.fill = kFillNone;  // SAT units only: ClassifyTessellation marks boundaries, nothing fills
   cudaMemsetAsync(md.stats, 0, sizeof(MeshStats), 0);
