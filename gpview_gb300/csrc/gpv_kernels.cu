@@ -562,25 +562,25 @@ __global__ void __launch_bounds__(kL1Warps * 32, 8) k_level1(BatchDev bd, uint32
 
   uint32_t nbuf = 0;  // collected records of mesh `bm`
   int bm = -1;
-  // room for n records of a mesh in its segment; positions past its capacity raise the status
-  auto take_room = [&](MeshStats *st, uint32_t n) {
+  // Room for n records of a mesh in its segment; positions past its capacity raise the status, once for
+  // all of them (once per record, the atomics of 7.5M records on one word took 5 ms of a first call).
+  auto take_room = [&](const MeshDesc &d, uint32_t n) {
     unsigned long long pos = 0;
-    if (lane == 0) pos = atomicAdd(&st->pairs, (unsigned long long)n);
+    if (lane == 0) {
+      pos = atomicAdd(&d.stats->pairs, (unsigned long long)n);
+      if (pos + n > (unsigned long long)d.pair_cap) atomicOr(&d.stats->status, (unsigned)ST_PAIR_OVERFLOW);
+    }
     return __shfl_sync(FULL, pos, 0);
   };
   auto flush = [&]() {
     if (!nbuf) return;
     const MeshDesc &d = bd.md[bm];
     __syncwarp();
-    const unsigned long long pos = take_room(d.stats, nbuf);
+    const unsigned long long pos = take_room(d, nbuf);
     const uint64_t cap = (uint64_t)d.pair_cap;
-    for (uint32_t i = lane; i < nbuf; i += 32) {
-      if (pos + i < cap) {
-        d.keys[pos + i] = ws.key[i];
-        d.vals[pos + i] = ws.val[i];
-      } else {
-        atomicOr(&d.stats->status, (unsigned)ST_PAIR_OVERFLOW);
-      }
+    for (uint32_t i = lane; i < nbuf && pos + i < cap; i += 32) {
+      d.keys[pos + i] = ws.key[i];
+      d.vals[pos + i] = ws.val[i];
     }
     __syncwarp();
     nbuf = 0;
@@ -689,7 +689,7 @@ __global__ void __launch_bounds__(kL1Warps * 32, 8) k_level1(BatchDev bd, uint32
           if (nbuf + tot > (uint32_t)kL1Pairs) flush();
           pos = nbuf + inc - cnt;
           direct = tot > (uint32_t)kL1Pairs;
-          if (direct) gpos = take_room(d.stats, tot) + inc - cnt;
+          if (direct) gpos = take_room(d, tot) + inc - cnt;
           else nbuf += tot;
         } else {
           counted += cnt;
@@ -704,8 +704,6 @@ __global__ void __launch_bounds__(kL1Warps * 32, 8) k_level1(BatchDev bd, uint32
             if (gpos < (uint64_t)d.pair_cap) {
               d.keys[gpos] = key;
               d.vals[gpos] = val;
-            } else {
-              atomicOr(&d.stats->status, (unsigned)ST_PAIR_OVERFLOW);
             }
             ++gpos;
           } else if (emit) {
