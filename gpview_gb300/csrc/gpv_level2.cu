@@ -507,6 +507,64 @@ __device__ __forceinline__ void write_chunk(uint8_t *l2, uint32_t *codes, uint32
   nin += ni;
 }
 
+// Output of a chunk of any other layout in host memory, for voxels of at least kHostBytes cells: a lane
+// takes 16 bytes at a 16-byte boundary of a voxel's block, in output order, and stores the words of a
+// block's two ends one by one.  (A byte a lane and layer, as in device memory, left the link waiting:
+// 262k-triangle torus at 128^3 host to host, us, by bytes and so: 5^3 722 and 623, 7^3 1215 and 792, 12^3
+// 3007 and 1567; 4^3 479 and 398, but 3^3, whose blocks are mostly ends, 487 and 530.)
+constexpr int kHostBytes = 64;
+__device__ __forceinline__ void write_host_bytes(uint8_t *l2, uint32_t vown, const uint32_t *satm,
+                                                 const uint32_t *par, const uint32_t *ft, int m, int ncol2,
+                                                 int n2z, unsigned long long &nbd, unsigned long long &nin) {
+  const int lane = (int)(threadIdx.x & 31u);
+  const int cells = ncol2 * n2z, W = (cells + 31) >> 5, FW = (ncol2 + 31) >> 5;
+  const int groups = (cells + 30) >> 4;  // 16-byte blocks that a voxel's bytes can touch
+  uint32_t nb = 0, ni = 0;
+#pragma unroll 1
+  for (int u0 = 0; u0 < m * groups; u0 += 32) {
+    const int u = u0 + lane;
+    const bool live = u < m * groups;
+    const int jv = live ? u / groups : 0;
+    uint8_t *const o = l2 + (size_t)__shfl_sync(FULL, vown, jv) * cells;
+    const int c0 = 16 * (u - jv * groups) - (int)(reinterpret_cast<uintptr_t>(o) & 15u);  // cell of byte 0
+    const int b0 = max(-c0, 0), b1 = min(cells - c0, 16);
+    if (!live || b0 >= b1) continue;
+    const uint32_t *sv = satm + jv * W, *pv = par + jv * W, *fv = ft + jv * FW;
+    int r = (c0 + b0) / ncol2, pq = c0 + b0 - r * ncol2;
+    uint32_t w[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+    for (int b = 0; b < 16; ++b) {
+      if (b < b0 || b >= b1) continue;
+      const int off = pq * n2z + r;
+      const uint32_t s = (sv[off >> 5] >> (off & 31)) & 1u;
+      const uint32_t i = ((pv[off >> 5] >> (off & 31)) ^ (fv[pq >> 5] >> (pq & 31))) & 1u & ~s;
+      w[b >> 2] |= (s * 254u + i * 127u) << (8 * (b & 3));
+      nb += s;
+      ni += i;
+      if (++pq == ncol2) {
+        pq = 0;
+        ++r;
+      }
+    }
+    if (b1 - b0 == 16) {
+      __stcs(reinterpret_cast<uint4 *>(o + c0), make_uint4(w[0], w[1], w[2], w[3]));
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (b0 <= 4 * k && b1 >= 4 * k + 4) {
+          __stcs(reinterpret_cast<uint32_t *>(o + c0) + k, w[k]);
+        } else {
+#pragma unroll
+          for (int b = 4 * k; b < 4 * k + 4; ++b)
+            if (b >= b0 && b < b1) __stcs(reinterpret_cast<char *>(o + c0) + b, (char)(w[k] >> (8 * (b & 3))));
+        }
+      }
+    }
+  }
+  nbd += nb;
+  nin += ni;
+}
+
 // n2z bits of a Level2 column starting at bit `off` of a mask.
 __device__ __forceinline__ uint32_t column_bits(const uint32_t *m, int off, int n2z) {
   const int sh = off & 31;
@@ -1021,7 +1079,7 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_sat(
 
 // k_level2c_fill: the inside fill, and the Level2 states from it and the SAT masks.
 // ST: the stencil fill (ClassifyInOut2xLevel2) instead of the ray fill.
-// HOST: the states go to host memory (write_chunk).
+// HOST: the states go to host memory (write_chunk, write_host_bytes).
 template <bool ST, bool HOST>
 __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_fill(
     BatchDev bd, const uint32_t *__restrict__ keys, const uint32_t *__restrict__ vals,
@@ -1410,6 +1468,9 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_fill(
   if ((n2z == 8 || n2z == 16) && (ncol2 & 15) == 0 && (reinterpret_cast<uintptr_t>(d.l2) & 15) == 0) {
     if (n2z == 8) write_chunk<8, HOST>(d.l2, d.l2codes, pkend, vown, satm, par, ft, m, ncol2, stage, nbd, nin);
     else write_chunk<16, HOST>(d.l2, d.l2codes, pkend, vown, satm, par, ft, m, ncol2, stage, nbd, nin);
+    __syncwarp();
+  } else if (HOST && cells >= kHostBytes) {
+    write_host_bytes(d.l2, vown, satm, par, ft, m, ncol2, n2z, nbd, nin);
     __syncwarp();
   } else {
     // One lane per sub-column of the chunk: its n2z SAT and parity bits are read once and written
