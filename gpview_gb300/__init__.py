@@ -318,7 +318,7 @@ class Context:
         SAT has one organisation)."""
         self._check(lib().gpv_set_level2_mode(self._h, int(mode)), "set_level2_mode")
 
-    def set_host_expand(self, threads=-1, slab_mask=0xff, share=45, min_level2_bytes=64 << 20):
+    def set_host_expand(self, threads=-1, slab_mask=0xff, share=52, min_level2_bytes=64 << 20):
         """Packed Level2 transfer of voxelize_to_host (gpv_set_host_expand): host threads (-1 by
         the machine, 0 off), the z slabs (bit mask of 8) that send 2-bit codes for the first
         `share` percent of their boundary voxels, and the Level2 output size from which it

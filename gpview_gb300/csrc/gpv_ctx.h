@@ -58,11 +58,12 @@ struct gpv_ctx {
   int host_threads = -1;               // -1: by the machine (up to 16); 0 or 1: off
   // slab k sends codes for the first packed_share percent of its boundary voxels when bit k is
   // set, and bytes for the rest.  Sharing every slab keeps the link and the host threads busy
-  // together from the first slab to the last (star1310k host to host, ms: all bytes 7.30; the
-  // first four slabs as codes 6.70; every slab 20% codes 6.78, 40% 6.48, 45% 6.41, 50% 6.56,
-  // 60% 6.79, 100% 8.28)
+  // together from the first slab to the last.  1.3M-triangle star at 256^3 / 16^3 host to host, 1.28 GB
+  // out, ms by share (medians of six contexts; in brackets the same on a box whose host threads were
+  // slower): 45% 6.45 [6.57], 48% 6.41 [6.64], 50% 6.35 [6.51], 52% 6.33 [6.47], 55% 6.28 [6.64], 58%
+  // 6.54 [6.73]; all bytes 7.58.  At 192^3 / 8^3, us: 45% 1066, 52% 1059
   uint32_t packed_slabs = 0xff;
-  int packed_share = 45;
+  int packed_share = 52;
   int64_t packed_min_bytes = 64ll << 20;  // smaller Level2 outputs go as bytes
   std::unique_ptr<gpv::ExpandPool> pool;
   uint32_t *h_codes = nullptr;         // page-locked staging of the codes (device-mapped)
