@@ -32,6 +32,11 @@ namespace {
 constexpr unsigned FULL = 0xffffffffu;
 constexpr int kWarps = 4;
 constexpr int kDirectCells = 4;  // a triangle whose box meets at most this many cells is tested exactly
+// Where the centre tables lie further than this many cells from their affine form (coordinates large
+// against the cells), the solved rows leave nearly every cell open: the triangles' sub-columns are
+// tested exactly instead.  262k-triangle torus at 128^3 / 8^3, SAT us, rows and exact, by the distance:
+// 0.5 cells 326 and 445, 1.4 546 and 470, 2.9 784 and 500, 4.8 890 and 535, 14 1715 and 818.
+constexpr float kWide = 1.0f;
 constexpr int kMaskWords = 512;  // words of one mask kind per warp (sets the chunk length)
 
 __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v) {
@@ -725,6 +730,18 @@ __device__ __noinline__ void sat_exact(const MeshDesc &d, WarpScratch &ws, uint3
   __syncwarp();
 }
 
+// The exact x/y tests of a sub-column of the voxel at xy.
+__device__ __noinline__ bool column_passes(const MeshDesc &d, uint32_t t, uint32_t xy, int p, int q) {
+  const GridDev &g = d.g;
+  const float4 a0 = __ldg(d.ptri + 3 * (size_t)t), a1 = __ldg(d.ptri + 3 * (size_t)t + 1),
+               a2 = __ldg(d.ptri + 3 * (size_t)t + 2);
+  const float V[9] = {a0.x, a0.y, a0.z, a1.x, a1.y, a1.z, a2.x, a2.y, a2.z};
+  const float h[3] = {g.e2[0], g.e2[1], g.e2[2]};
+  SatCol sc;
+  return sat_col(V, __ldg(g.c2s[0] + (size_t)(xy & 0xffffu) * g.n2[0] + p),
+                 __ldg(g.c2s[1] + (size_t)(xy >> 16) * g.n2[1] + q), h, sc);
+}
+
 // The exact ray tests of queued (triangle, sub-column) records, one per lane: the toggles of the
 // chunk's voxels at or below the triangle's topmost voxel, top down.
 __device__ __noinline__ void fill_exact(const MeshDesc &d, WarpScratch &ws, uint32_t *par,
@@ -802,6 +819,18 @@ __device__ __noinline__ void fill_exact(const MeshDesc &d, WarpScratch &ws, uint
     }
   }
   __syncwarp();
+}
+
+// The exact u/v test of a sub-column's ray.
+__device__ __noinline__ bool ray_passes(const MeshDesc &d, uint32_t t, int ci, int cj, int p, int q) {
+  const GridDev &g = d.g;
+  const float4 a0 = __ldg(d.ptri + 3 * (size_t)t), a1 = __ldg(d.ptri + 3 * (size_t)t + 1),
+               a2 = __ldg(d.ptri + 3 * (size_t)t + 2);
+  const float V[9] = {a0.x, a0.y, a0.z, a1.x, a1.y, a1.z, a2.x, a2.y, a2.z};
+  RayTri rt;
+  ray_tri_pre(V, a2.w, rt);
+  RayCol rc;
+  return ray_col(rt, __ldg(g.o2[0] + (size_t)ci * g.n2[0] + p), __ldg(g.o2[1] + (size_t)cj * g.n2[1] + q), rc);
 }
 
 // Appends the records of the lanes with `push` to the exact-work queue and returns its length.
@@ -926,7 +955,7 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_sat(
       // ---- one triangle per lane: its cell ranges, its plane and its rows
       const uint32_t e = b0 + lane;
       int p0 = 0, p1 = -1, pi = 0, pe = 0, q0 = 0, q1 = -1, qi = 0, qe = 0, r0 = 0, r1 = -1, ri = 0, re = 0;
-      bool direct = false, on = false;
+      bool direct = false, wide = false, on = false;
       uint32_t nsolve = 0, ncol = 0, t = 0;
       int jv = 0;  // last voxel whose segment starts at or before e
       float4 a0, a1, a2;
@@ -968,7 +997,8 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_sat(
           const int np = p1 - p0 + 1, nq = q1 - q0 + 1;
           // A few cells are tested as fast as they are solved; outside these magnitudes the
           // bounds' own arithmetic could leave the normal range.
-          direct = np * nq * (r1 - r0 + 1) <= kDirectCells || !(R > 1e-9f && R < 1e9f);
+          wide = fmaxf(tx * g.inv_g2[0], fmaxf(ty * g.inv_g2[1], tz * g.inv_g2[2])) > kWide;
+          direct = np * nq * (r1 - r0 + 1) <= kDirectCells || !(R > 1e-9f && R < 1e9f) || wide;
           on = true;
           nsolve = direct ? 0u : (uint32_t)(2 * nq + np);
         }
@@ -979,7 +1009,7 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_sat(
       const uint32_t so0 = is - nsolve;
       if (on) {
         const int np_ = p1 - p0 + 1, nq_ = q1 - q0 + 1;
-        ws.me[lane] = make_uint4(t, (uint32_t)(jv | (direct ? 256 : 0) | (p0 << 16) | (q0 << 24)),
+        ws.me[lane] = make_uint4(t, (uint32_t)(jv | (direct ? 256 : 0) | (wide ? 512 : 0) | (p0 << 16) | (q0 << 24)),
                                  (so0 + (uint32_t)nq_) | ((so0 + 2u * (uint32_t)nq_) << 16),
                                  (uint32_t)(r0 | ((r1 + 1) << 8)));
         ncol = (uint32_t)(np_ * nq_);
@@ -1033,7 +1063,7 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_sat(
           if (me.y & 256u) {
             lo = (int)(me.w & 255u);
             end = (int)(me.w >> 8);
-            amb = true;
+            amb = !(me.y & 512u) || column_passes(d, me.x, xy[j], p, q);
           } else {
             const float4 xa = ws.xa[tl], xb = ws.xb[tl];
             const uint32_t syz = ws.sol[(me.z & 0xffffu) + (uint32_t)dq], sxz = ws.sol[(me.z >> 16) + (uint32_t)dp];
@@ -1397,7 +1427,13 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_fill(
           const int p = (int)((me.y >> 16) & 255u) + dp, q = (int)(me.y >> 24) + dq;
           const int jm = (int)(me.y & 255u);
           amb = !(en & 0x8000u);
-          if (!amb) {
+          // Triangles that no row is solved for list every sub-column of their box, most of which the ray
+          // misses: those stay off the queue, whose lanes then work on heights together (262k-triangle
+          // torus at 128^3 / 8^3, coordinates around 10000, where neighbouring origins can round to one
+          // height: fill 2059 -> 480 us).
+          if (me.y & 256u) {
+            amb = ray_passes(d, me.x, ci, cj, p, q);
+          } else if (!amb) {
             const float4 xa = ws.xa[tl];
             const float x = ff((float)dp, xa.y, ff((float)dq, xa.z, xa.x));
             const int N = min(max(__float2int_ru(x - xa.w), 0), span);
