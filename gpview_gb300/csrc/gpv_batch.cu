@@ -119,7 +119,9 @@ uint64_t call_key(int n, const int64_t *T, const gpv_grid_spec *specs) {
   return h;
 }
 
-// Average triangles a voxel up to which ordering each voxel's list beats the radix sort.
+// Average triangles a voxel up to which each voxel's list is put in order by itself; above, the radix sort of
+// all pairs.  Sort and lists of 131k triangles, us, by the average: 7.5 triangles 49 and 165 (radix), 25 41 and
+// 140, 59 50 and 139; also 84 60 and 139, 176 78 and 142, so the line lies low.
 constexpr int64_t kSegSortAverage = 64;
 
 // Word of the page-locked scratch (gpv_ctx::h_u32) where a one-graph call's DevPlan lands.
@@ -800,9 +802,8 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
   // ---- phase 2: allocations and staging first, then the recorded launch sequence
   const int64_t ntiles = (int64_t)st_host.size();
   const bool do_l2 = (any_l2 || nmode) && ntiles > 0;  // sort + lists (+ Level2, normals)
-  // Lists by the counting sort; with normals each voxel's triangles are then put in order, which pays
-  // while they are few a voxel (430k pairs of 53k voxels: 62 us against the radix sort's 202); lists of
-  // hundreds keep the radix sort, whose passes do not depend on their lengths
+  // Lists by the counting sort; with normals each voxel's triangles are then put in order, or (many a voxel)
+  // all pairs sorted by the radix sort, whose passes do not depend on the lists' lengths
   const bool csort = do_l2 && kmark && (nmode == 0 || P2 <= kSegSortAverage * ub);
   SortTile *d_tiles = nullptr;
   int64_t *d_tb = nullptr;
@@ -927,7 +928,8 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
         // lists in any triangle order: counting sort by voxel rank, segment starts from its scan
         count_sort_pairs(bd, d_tiles, ntiles, keys, vals, wpre + words, ub, P2, flags, useg, kalt,
                          valt, wtot + 1, sortmp, s);
-        if (nmode) launch_seg_sort(valt, useg, ub, uidx, ctx->num_sms, s);
+        // (the records in emission order are done with)
+        if (nmode) launch_seg_sort(bd, valt, useg, ub, uidx, vals, ctx->num_sms, s);
       } else {
         // normals sum in ascending triangle order: radix sort by (voxel, triangle)
         const bool in_alt = sort_pairs_seg(bd, d_tiles, d_tb, ntiles, keys, vals, kalt, valt, P2,

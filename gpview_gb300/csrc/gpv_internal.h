@@ -285,10 +285,11 @@ void launch_level2(const BatchDev &bd, const uint32_t *keys, const uint32_t *val
 
 // ---- normals (gpv_normals.cu) ----------------------------------------------------------------
 void launch_face_normals(const BatchDev &bd, cudaStream_t s);
-// Each voxel's triangles of counting-sorted lists in ascending id; longs: seg_sort_words(U) words.
+// Each voxel's triangles of counting-sorted lists in ascending id; longs: seg_sort_words(U) words; spare:
+// as long as vals.
 int64_t seg_sort_words(int64_t U);
-void launch_seg_sort(uint32_t *vals, const uint32_t *useg, int64_t U, uint32_t *longs, int num_sms,
-                     cudaStream_t s);
+void launch_seg_sort(const BatchDev &bd, uint32_t *vals, const uint32_t *useg, int64_t U, uint32_t *longs,
+                     uint32_t *spare, int num_sms, cudaStream_t s);
 // Level1 normals of the U boundary voxels of the sorted meshes, then Level2 normals of the meshes with
 // a Level2 grid (max_cells cells per voxel at most, 0: none).
 void launch_normals(const BatchDev &bd, const uint32_t *keys, const uint32_t *vals,
