@@ -156,11 +156,11 @@ constexpr int kHeavyChunks = 4;   // ... into pieces of this many 32-unit chunks
 
 // cell_of(v) from its estimate e = (v - mn) * inv, inv = n / (mx - mn).  The float quotient times n is
 // within four roundings of e, an absolute 1e-6 covering inv's denormals: where both ends truncate to one
-// cell that is it, elsewhere (about one in 10^4, and infinities) the quotient itself decides.
+// cell that is it, elsewhere (about one in 10^4, and where inv or e overflow) the quotient itself decides.
 __device__ __forceinline__ int cell_near(float v, float mn, float mx, int n, float inv) {
   const float e = (v - mn) * inv, w = ff(fabsf(e), 8.f * EPS24, 1e-6f), nf = (float)n + 1.0f;
   const int a = __float2int_rz(fminf(fmaxf(e - w, -1.0f), nf)), b = __float2int_rz(fminf(fmaxf(e + w, -1.0f), nf));
-  if (a != b) return cell_of(v, mn, mx, n);
+  if (a != b || !(w < 1e30f)) return cell_of(v, mn, mx, n);  // (NaN too)
   return a == n && v == mx ? a - 1 : a;
 }
 

@@ -1352,11 +1352,11 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_fill(
       const int jm = ws.ujm[lane];
       const float4 fb = __ldg(fbox + t);
       {
-        // sub-columns whose origins can lie in the box
+        // sub-columns whose origins can lie in the box (all of them where the spacing's inverse overflows)
         p0 = max(__float2int_ru((fb.x - ox0) * g.inv_g2[0] - mx), 0);
-        p1 = min(__float2int_rd((fb.z - ox0) * g.inv_g2[0] + mx), n2x - 1);
+        p1 = __float2int_rd(fminf((fb.z - ox0) * g.inv_g2[0] + mx, (float)(n2x - 1)));
         const int q0 = max(__float2int_ru((fb.y - oy0) * g.inv_g2[1] - my), 0);
-        const int q1 = min(__float2int_rd((fb.w - oy0) * g.inv_g2[1] + my), n2y - 1);
+        const int q1 = __float2int_rd(fminf((fb.w - oy0) * g.inv_g2[1] + my, (float)(n2y - 1)));
         if (p0 <= p1 && q0 <= q1) {
           const int np = p1 - p0 + 1;
           nq = q1 - q0 + 1;
@@ -1372,7 +1372,7 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_fill(
           // In units of eps R^2 the float u, v and u + v (times det) are off by less than 48 and
           // solve_rows' sides by less than 42: 90, 96 with the slope's.  An unbounded box marks an
           // ill-conditioned x/y projection, which has no bound on t: exact tests only.
-          direct = !g.oz_monotone || isinf(fb.x) || isinf(fb.z) || !(R > 1e-9f && R < 1e9f);
+          direct = !g.oz_monotone || isinf(fb.x) || isinf(fb.z) || !(R > 1e-9f && R < 1e9f) || isinf(g.inv_g2[2]);
           ncol = (uint32_t)(np * nq);
           if (!direct) {
             nsolve = (uint32_t)nq;

@@ -106,14 +106,16 @@ __device__ __forceinline__ void list_columns(uint16_t *out, const uint32_t *xy, 
 
 // Cells of one axis whose boxes can meet [tmin, tmax] ([lo, hi]) and those that certainly do
 // ([in_lo, in_end)), by the SAT's own box-axis test; `md` (cells) bounds the distance of the centre
-// table from c0 + k * g2 and the roundings.
+// table from c0 + k * g2 and the roundings.  Where inv_g2 overflows (cells under 2^-128) the values are
+// infinite or not numbers: every cell can then meet the box and none does for certain.
 __device__ __forceinline__ void cell_ranges(float tmin, float tmax, float c0, float inv_g2, int n2,
                                             float md, int &lo, int &hi, int &in_lo, int &in_end) {
   const float f0 = ff(tmin - c0, inv_g2, 0.5f), f1 = ff(tmax - c0, inv_g2, 0.5f);
+  const float last = (float)(n2 - 1);
   lo = max(__float2int_rd(f0 - md), 0);
-  hi = min(__float2int_rd(f1 + md), n2 - 1);
-  in_lo = min(max(__float2int_rd(f0 + md), 0), n2);
-  in_end = max(min(__float2int_rd(f1 - md), n2 - 1), -1) + 1;
+  hi = __float2int_rd(fminf(f1 + md, last));
+  in_lo = __float2int_rd(fmaxf(fminf(f0 + md, last + 1.f), 0.f));
+  in_end = __float2int_rd(fminf(fmaxf(f1 - md, -1.f), last)) + 1;
 }
 
 }  // namespace gpv
