@@ -174,7 +174,6 @@ __global__ void __launch_bounds__(256) k_prep(BatchDev bd) {
   const MeshDesc &d = bd.md[m];
   const GridDev &g = d.g;
   unsigned long long sat1 = 0, su = 0, fu = 0, r1 = 0;
-  int4 rng = make_int4(0, 0, 0, 0);
   uint32_t pieces = 0;
   if (live) {
     const int64_t t = gi - d.tri_base;
@@ -238,7 +237,7 @@ __global__ void __launch_bounds__(256) k_prep(BatchDev bd) {
     d.ptri[3 * t + 0] = make_float4(V[0], V[1], V[2], __uint_as_float(pack2(fx0, fx1)));
     d.ptri[3 * t + 1] = make_float4(V[3], V[4], V[5], __uint_as_float(pack2(fy0, fy1)));
     d.ptri[3 * t + 2] = make_float4(V[6], V[7], V[8], __fdiv_rn(1.0f, det));
-    rng = make_int4((int)pack2(lo[0], hi[0]), (int)pack2(lo[1], hi[1]), (int)pack2(lo[2], hi[2]), 0);
+    d.rng[t] = make_int4((int)pack2(lo[0], hi[0]), (int)pack2(lo[1], hi[1]), (int)pack2(lo[2], hi[2]), 0);
     d.fbox[t] = fb;
     if (bd.heavy && su + fu > (unsigned long long)kHeavyUnits) {
       const unsigned long long n = ((su + 31) / 32 + (fu + 31) / 32 + kHeavyChunks - 1) / kHeavyChunks;
@@ -256,13 +255,14 @@ __global__ void __launch_bounds__(256) k_prep(BatchDev bd) {
     pos = __shfl_sync(FULL, pos, 31) + (inc - pieces);
     if (pieces) {
       const unsigned long long cap = bd.heavy_cap;
-      rng.w = pos < cap && cap - pos >= pieces;
+      const int64_t t = gi - d.tri_base;
+      const bool listed = pos < cap && cap - pos >= pieces;
+      if (listed) d.rng[t].w = 1;
       const uint32_t room = pos < cap ? (uint32_t)min(cap - pos, (unsigned long long)pieces) : 0u;
       for (uint32_t k = 0; k < room; ++k)
-        bd.heavy[pos + k] = make_uint4((uint32_t)m, (uint32_t)(gi - d.tri_base), k, (uint32_t)rng.w);
+        bd.heavy[pos + k] = make_uint4((uint32_t)m, (uint32_t)t, k, (uint32_t)listed);
     }
   }
-  if (live) d.rng[gi - d.tri_base] = rng;
   block_add_prep(d.stats, sat1, su, fu, r1);
 }
 
