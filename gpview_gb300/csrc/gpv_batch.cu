@@ -616,7 +616,7 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
       launch_plan(bdp, d_md, static_cast<int32_t *>(set->bindex), static_cast<uint8_t *>(set->l2),
                   cap, d_plan, s);
       mark(5);
-      launch_expand(bdp, wpre, s);
+      launch_expand(bdp, wpre, ctx->num_sms, s);
       mark(6);
       if (any_l2) {
         count_sort_pairs(bdp, nullptr, cap.tiles, keys, vals, wpre + words, cap.U, cap.P, cnt,
@@ -908,7 +908,7 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
     }
     in.launch();
     mark(5);
-    launch_expand(bd, wpre, s);
+    launch_expand(bd, wpre, ctx->num_sms, s);
     if (sink) {
       cudaEventRecord(ctx->cev[0], s);
       cudaStreamWaitEvent(cs, ctx->cev[0], 0);

@@ -230,7 +230,7 @@ void launch_fill_finish(const BatchDev &bd, cudaStream_t s);
 void launch_stencil1(const BatchDev &bd, cudaStream_t s);
 void launch_boundary_counts(const BatchDev &bd, const uint32_t *wpre, const uint32_t *wtotal,
                             cudaStream_t s);
-void launch_expand(const BatchDev &bd, const uint32_t *wpre, cudaStream_t s);
+void launch_expand(const BatchDev &bd, const uint32_t *wpre, int num_sms, cudaStream_t s);
 void launch_heads(const uint32_t *keys, int64_t P, uint32_t *flags, const BatchDev &bd,
                   cudaStream_t s);
 void launch_useg(const uint32_t *flags, const uint32_t *uidx, int64_t P, uint32_t *useg,

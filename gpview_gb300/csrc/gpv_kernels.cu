@@ -1145,13 +1145,13 @@ void launch_boundary_counts(const BatchDev &bd, const uint32_t *wpre, const uint
   count_launch();
 }
 
-void launch_expand(const BatchDev &bd, const uint32_t *wpre, cudaStream_t s) {
+void launch_expand(const BatchDev &bd, const uint32_t *wpre, int num_sms, cudaStream_t s) {
   if (bd.total_xchunks <= 0) return;
   // few chunks: parts of them, so that each SM has 16 warps (128^3 voxels, 2048 chunks: 9.6 us; 32
   // warps 12, whose parts each load the chunk's words); many: up to four per warp
   int split = 1;
-  while (split < 8 && bd.total_xchunks * split < 152 * 16) split *= 2;
-  const int64_t parts = bd.total_xchunks * split, spread = parts / (152 * 64);
+  while (split < 8 && bd.total_xchunks * split < (int64_t)num_sms * 16) split *= 2;
+  const int64_t parts = bd.total_xchunks * split, spread = parts / ((int64_t)num_sms * 64);
   const int iters = (int)(spread < 1 ? 1 : spread > 4 ? 4 : spread);
   const int64_t per_block = (int64_t)kExpandWarps * iters;
   k_expand<<<(unsigned)((parts + per_block - 1) / per_block), kExpandWarps * 32, 0, s>>>(bd, wpre, iters, split);

@@ -248,7 +248,7 @@ extern "C" int gpv_voxelize_level1_noalloc(const float *d_tris, int64_t num_tria
   launch_level1(bd, num_sms, stream);  // (no Level2 grid: the records are counted, not written)
   launch_fill_finish(bd, stream);
   scan_u32(md.bplane, wpre, N1w, d_tot, stmp, stream, true);
-  launch_expand(bd, wpre, stream);
+  launch_expand(bd, wpre, num_sms, stream);
   uint32_t nb = 0;
   MeshStats hs;
   e = cudaGetLastError();
