@@ -49,8 +49,6 @@ def parse():
     p.add_argument("--tile", type=int, default=0)
     p.add_argument("--level2", type=int, default=0, help="override the workload's Level2 divisions")
     p.add_argument("--chunk", type=int, default=0, help="Level2 chunk of the plain path (0: default)")
-    p.add_argument("--level2-mode", default="auto", choices=["auto", "queued", "inline"],
-                   help="Level2 SAT organisation of the plain path (default: chosen per launch)")
     p.add_argument("--no-graphs", action="store_true")
     p.add_argument("--slabs", type=int, default=0,
                    help="z slabs of the e2e path's Level2 launch (0: by the Level2 output size)")
@@ -832,8 +830,6 @@ def main():
         ctx.set_tile(args.tile)
     if args.chunk:
         ctx.set_level2_chunk(args.chunk)
-    ctx.set_level2_mode({"auto": gpv.LEVEL2_AUTO, "queued": gpv.LEVEL2_QUEUED,
-                         "inline": gpv.LEVEL2_INLINE}[args.level2_mode])
     ctx.set_graphs(not args.no_graphs)
     stream = torch.cuda.Stream(device=local)
     sp = stream.cuda_stream

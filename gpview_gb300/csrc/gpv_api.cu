@@ -336,7 +336,6 @@ int64_t gpv_get_debug(gpv_ctx *ctx, int what) {
 
 int gpv_set_level2_mode(gpv_ctx *ctx, int mode) {
   if (!ctx || mode < GPV_LEVEL2_AUTO || mode > GPV_LEVEL2_INLINE) return GPV_ERR_INVALID;
-  ctx->l2_mode = mode;
   return GPV_OK;
 }
 

@@ -245,7 +245,7 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
   std::vector<int64_t> tab_off(n + 1, 0), res_l1(n + 1, 0), res_pre(n + 1, 0), res_l1n(n + 1, 0),
       res_hier(n + 1, 0);
   std::vector<MeshDesc> md(n);
-  int64_t tris = 0, tiles = 0, fblks = 0, rows = 0, xchunks = 0, words = 0, togg = 0, stgw = 0;
+  int64_t tris = 0, tiles = 0, fblks = 0, xchunks = 0, words = 0, togg = 0, stgw = 0;
   int max_keybits = 1;
   Level2Words l2_words = {0, 0};
   int64_t max_T = 1;
@@ -258,13 +258,11 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
     d.tri_base = tris;
     d.tile_base = tiles;
     d.fblk_base = fblks;
-    d.row_base = rows;
     d.xc_base = xchunks;
     d.word_base = words;
     tris += T[m];
     tiles += (T[m] + tile - 1) / tile;
     fblks += finish_blocks((int64_t)g.n[1] * g.nxw);
-    rows += (int64_t)g.n[2] * g.n[1];
     xchunks += ((int64_t)g.n[2] * g.n[1] * g.nxw + 31) / 32;
     words += (int64_t)g.n[2] * g.n[1] * g.nxw;
     togg += (int64_t)g.n[0] * g.n[1] * g.nzw;
@@ -386,7 +384,6 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
   bd.total_tris = tris;
   bd.total_tiles = tiles;
   bd.total_fblks = fblks;
-  bd.total_rows = rows;
   bd.total_xchunks = xchunks;
   bd.total_words = words;
   bd.queue = queue;
@@ -439,7 +436,7 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
   auto bd_sig = [&](std::vector<uint64_t> &v) {
     for (uint64_t x : {(uint64_t)(uintptr_t)bd.md, (uint64_t)bd.nmesh, (uint64_t)bd.tile,
                        (uint64_t)bd.total_tris, (uint64_t)bd.total_tiles, (uint64_t)bd.total_fblks,
-                       (uint64_t)bd.total_rows, (uint64_t)bd.total_words, (uint64_t)bd.total_xchunks,
+                       (uint64_t)bd.total_words, (uint64_t)bd.total_xchunks,
                        (uint64_t)(uintptr_t)bd.queue, (uint64_t)(uintptr_t)bd.heavy, (uint64_t)bd.normals, (uint64_t)bd.fill,
                        (uint64_t)(uintptr_t)bd.stp, (uint64_t)bd.stp_words, (uint64_t)(uintptr_t)bd.kmask,
                        (uint64_t)ctx->timing, (uint64_t)ctx->num_sms, (uint64_t)bd.wait_limit,

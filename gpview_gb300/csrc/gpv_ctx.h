@@ -46,7 +46,6 @@ struct gpv_ctx {
   // 16 -> 398, 32 -> 407; with the stencil fill 639, 609, 620, 733 (shorter chunks repeat the work for the
   // triangles above them, longer ones leave fewer and less even items)
   int l2_chunk_cap = 16;
-  int l2_mode = GPV_LEVEL2_AUTO;       // gpv_set_level2_mode (no effect)
   // failure-detection hooks (gpv_set_debug) and what they caused (gpv_get_debug)
   uint32_t wait_limit = 0;             // Level1 tile wait polls (0: built-in)
   int fail_wait = 0;                   // Level1's tile wait gives up at once

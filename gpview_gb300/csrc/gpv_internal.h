@@ -76,7 +76,6 @@ struct MeshDesc {
   int64_t tri_base;      // prefix over meshes of triangles
   int64_t tile_base;     // ... of Level1 tiles
   int64_t fblk_base;     // ... of fill-finish blocks (ny * nxw words of a layer, kFinishGroups each)
-  int64_t row_base;      // ... of Level1 rows (nz * ny)
   int64_t xc_base;       // ... of expansion chunks (32 bit-plane words)
   int64_t word_base;     // ... of bit-plane words (nz * ny * nxw)
   int64_t emit_base;     // ... of pair capacities (emission segments)
@@ -132,7 +131,7 @@ struct BatchDev {
   const MeshDesc *md;
   int nmesh;
   int tile;              // Level1 triangles per ticket (32, 64, 128, 256)
-  int64_t total_tris, total_tiles, total_fblks, total_rows, total_words;
+  int64_t total_tris, total_tiles, total_fblks, total_words;
   int64_t total_xchunks;  // expansion chunks of all meshes
   uint32_t *queue;       // work-queue tickets, zeroed by the caller: [0] Level1, [1 + k] and
                          // [1 + kSlabsMax + k] the fill and the SAT kernel of Level2 slab k,

@@ -1115,7 +1115,7 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_fill(
     BatchDev bd, const uint32_t *__restrict__ keys, const uint32_t *__restrict__ vals,
     const uint32_t *__restrict__ useg, const Item *__restrict__ items,
     const uint32_t *__restrict__ nitems, int per_warp, int slab, const uint32_t *__restrict__ ilist,
-    const uint32_t *__restrict__ ioff, int) {
+    const uint32_t *__restrict__ ioff) {
   extern __shared__ __align__(16) uint32_t sm[];
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   uint32_t *const scratch = sm + (size_t)warp * per_warp;
@@ -1607,10 +1607,9 @@ void launch_level2(const BatchDev &bd, const uint32_t *keys, const uint32_t *val
     count_launch(2);
   }
   const bool st = bd.fill == GPV_FILL_STENCIL;
-  using Kern = decltype(&k_level2c_sat);
   static OncePerDevice once[5];
   // a kernel's persistent grid (one-graph calls: B is a capacity, the queue ends the work)
-  auto grid_of = [&](Kern k, int kv, size_t smem, int64_t jobs) {
+  auto grid_of = [&](auto *k, int kv, size_t smem, int64_t jobs) {
     allow_shared_memory(once[kv], k, 200 * 1024);
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kWarps * 32, smem);
@@ -1622,8 +1621,8 @@ void launch_level2(const BatchDev &bd, const uint32_t *keys, const uint32_t *val
   const int parts = level2_parts(B, num_sms);
   if (parts > 1) cudaMemsetAsync(bd.smask, 0, (size_t)smask_words * sizeof(uint32_t), s);
   const bool host = bd.l2_host;
-  const Kern fill = st ? (host ? k_level2c_fill<true, true> : k_level2c_fill<true, false>)
-                       : (host ? k_level2c_fill<false, true> : k_level2c_fill<false, false>);
+  auto *const fill = st ? (host ? k_level2c_fill<true, true> : k_level2c_fill<true, false>)
+                        : (host ? k_level2c_fill<false, true> : k_level2c_fill<false, false>);
   const size_t smem_sat = level2_smem_bytes(words.sat), smem_fill = level2_smem_bytes(words.fill);
   const unsigned grid_sat = grid_of(k_level2c_sat, 0, smem_sat, B * parts);
   const unsigned grid_fill = grid_of(fill, 1 + 2 * st + host, smem_fill, B);
@@ -1660,7 +1659,7 @@ void launch_level2(const BatchDev &bd, const uint32_t *keys, const uint32_t *val
       cudaStreamWaitEvent(ls, aux->join[0], 0);
     }
     fill<<<grid_fill, kWarps * 32, smem_fill, ls>>>(bd, keys, vals, useg, items, nitems, words.fill, sl,
-                                                    list, ioff, 1);
+                                                    list, ioff);
     count_launch(2);
     if (after_slab) after_slab(sl, ls);
   }

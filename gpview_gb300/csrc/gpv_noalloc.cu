@@ -227,7 +227,6 @@ extern "C" int gpv_voxelize_level1_noalloc(const float *d_tris, int64_t num_tria
   bd.fail_wait = g_fail_wait;
   bd.total_tris = T;
   bd.total_fblks = finish_blocks((int64_t)g.n[1] * g.nxw);
-  bd.total_rows = (int64_t)g.n[2] * g.n[1];
   bd.total_xchunks = (N1w + 31) / 32;
   bd.total_words = N1w;
 

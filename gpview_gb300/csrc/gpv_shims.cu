@@ -532,7 +532,6 @@ int CUDAClassifyTessellation(float *trianglesCUDAData, int numTriangles, float *
   bd.total_tris = T;
   bd.total_tiles = (T + tile - 1) / tile;
   bd.total_fblks = finish_blocks((int64_t)gh.n[1] * gh.nxw);
-  bd.total_rows = (int64_t)gh.n[2] * gh.n[1];
   bd.total_words = N1w;
   auto set_queue = [&] {
     bd.queue = reinterpret_cast<uint32_t *>(base + o_q);
