@@ -230,7 +230,7 @@ __device__ __forceinline__ uint32_t marked_through(const BatchDev &bd, const Mes
 // average list (a run's pairs vary by about one list around q), nb giving a warp two runs, and a
 // quarter of that for the last eighth of the pairs.  Where a full run's masks hold less than two
 // batches, pairs only bound the longest lists.  Against the fill's items, whose columns are mostly
-// short: a 16k-triangle sphere at 64^3 / 8^3 52 -> 31 us (its longest columns took that long), 7k
+// short: a 16k-triangle sphere at 64^3 / 4^3 52 -> 31 us (its longest columns took that long), 7k
 // triangles at 150x170x130 / 6^3 73 -> 53, 256 mixed meshes 5.4 -> 4.0 ms, the 1.3M-triangle star at
 // 256^3 / 16^3 690 -> 677; a 262k-triangle torus, whose columns are long, 113..119 -> 119.  One run
 // a warp instead of two: torus 135 us, batch 4.1 ms; three: batch 3.9 ms, star 684 us.
@@ -899,7 +899,8 @@ __device__ __forceinline__ uint32_t *sat_words(const BatchDev &bd, const MeshDes
 // (one bit per cell).  Both kernels are bound by instruction issue.  Measured against one kernel
 // testing every (triangle, sub-column) and listed cell exactly, both kernels together: the torus
 // 487 -> 200 us, a 1.3M-triangle star at 256^3 / 16^3 3.51 -> 1.25 ms, 256 mixed meshes in one call
-// 19.9 -> 8.5 ms.  A twentieth of the instructions are exact tests (0.4-2.7% of the sub-columns).
+// 19.9 -> 8.5 ms.  A twentieth of the instructions are exact tests (0.4-2.7% of the sub-columns on these
+// meshes, whose coordinates are of the grid's own size; far from the origin the share grows: see kWide).
 // Rows are solved by a lane per triangle looping over them (a lane per row took 190 us for the torus'
 // SAT against 134); the sub-columns they leave are listed and taken a lane each, because lanes that
 // walked their own row had 43-52% of them at work in the SAT and 34% in the fill (the star: SAT

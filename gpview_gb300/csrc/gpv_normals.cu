@@ -10,8 +10,9 @@
 //                 (AddPointToVoxel, :2715-2719), triangles in list order; sum / count,
 //                 normalised (:2402-2424); cells without a pass 0 (:3309-3310).
 // The list order of the CPU path is ascending triangle id (ClassifyTessellation records the
-// triangles in file order, :2267-2340); with normals on, the pair sort also orders each voxel's
-// triangles by id, so every float sum runs in the reference's order.
+// triangles in file order, :2267-2340); with normals on, each voxel's triangles are put in id order too
+// (by k_seg_sort and k_seg_sort_long, or, with long lists on average, by a radix sort of all pairs by id
+// and voxel), so every float sum runs in the reference's order.
 //
 // Outputs per mode: GPV_NORMALS_BYTES writes the .raw encoding uint8(n * float(256/3) + 127)
 // (src/Object.cpp:2940-2941, :3033-3035), three bytes per voxel / cell; GPV_NORMALS_FLOAT writes
