@@ -823,7 +823,7 @@ int run_batch(gpv_ctx *ctx, int n, const float *const *d_tris, const int64_t *T,
     if (any_l2) CK(ws.get(&bd.smask, (size_t)level2_mask_words(ub, l2bytes)));
     if (stencil && any_l2) {  // per boundary voxel: the column prefix of sample coverage
       for (int m = 0; m < n; ++m)
-        if (gh[m].level2) bd.stp_words = std::max(bd.stp_words, (4 * gh[m].n2[0] * gh[m].n2[1] + 31) / 32);
+        if (gh[m].level2) bd.stp_words = std::max(bd.stp_words, (4 * gh[m].n2[0] * gh[m].n2[1] + 31) / 32 + 1);
       CK(ws.get(&bd.stp, (size_t)std::max<int64_t>(ub, 1) * bd.stp_words));
     }
   }

@@ -140,7 +140,8 @@ struct BatchDev {
   int normals;           // GPV_NORMALS_* of this batch
   int fill;              // GPV_FILL_* of this batch
   uint32_t *stp;         // stencil fill: per boundary voxel, the sample-coverage parity of the
-  int stp_words;         //   column's triangles recorded only below it (stp_words words each)
+  int stp_words;         //   column's triangles recorded only below it (stp_words words each, the last
+                         //   0 or, where they cannot be left to that, 1 + the column's first voxel)
   // Level1 marks the voxel of every pair it emits for a mesh with a Level2 grid here: one
   // column-major bit plane per mesh (bit = pair key) at the mesh's word_base; nullptr: no marks
   uint32_t *kmask = nullptr;

@@ -580,25 +580,29 @@ __device__ __forceinline__ uint32_t column_bits(const uint32_t *m, int off, int 
 
 // ---- stencil fill, column prefix ------------------------------------------------------------------
 // A triangle whose topmost record in a Level1 column lies below voxel v is not recorded in any
-// voxel from v up, so within the column's x/y extent it lies below v's bottom face (up to the
-// SAT's rounding, far less than the half Level2 cell to v's first clip height): every covered
-// sample keeps it in every slice of v and above.  A Level2 chunk therefore starts from the XOR of
+// voxel from v up, so within the column's x/y extent it lies below v's bottom face, up to the
+// SAT's rounding: every covered sample keeps it in every slice of v and above, unless that rounding
+// exceeds the half Level2 cell to v's first clip height (coordinates large against the cells, slivers).
+// The heights show where it does; the column's chunks above then draw all of its triangles.
+// Elsewhere a Level2 chunk starts from the XOR of
 // the sample coverage of the column's triangles whose topmost record lies below its first voxel,
 // and draws only the triangles recorded from that voxel up (otherwise every chunk of a tall
 // column would draw all the triangles below it again).  Two passes, since the XOR is order-free:
 //   k_stencil_segment  one warp per work item: the coverage XOR of the triangles whose topmost
 //                      record lies in the item's own voxels (items that end their column skip it),
-//                      stored at the item's first voxel;
+//                      stored at the item's first voxel, with a last word that says whether one of
+//                      the samples is not below the next item's clip heights;
 //   k_stencil_scan     one warp per column with more than one item: those masks turned in place
-//                      into exclusive XOR prefixes, the mask each item starts from.
+//                      into exclusive XOR prefixes, the mask each item starts from, and the last
+//                      words into 0 or, above such a sample, 1 + the column's first voxel.
 // (One warp per column walking all of its records was latency-bound on the few long columns:
 // 186 us on torus262k at 22% warps active.)
 constexpr int kPrefixWarps = 4;
 constexpr int kPrefixMaskWords = 128;  // 4 * 32 * 32 samples / 32
 
 __global__ void __launch_bounds__(kPrefixWarps * 32) k_stencil_segment(
-    BatchDev bd, const uint32_t *__restrict__ vals, const uint32_t *__restrict__ useg,
-    const Item *__restrict__ items, const uint32_t *__restrict__ nitems) {
+    BatchDev bd, const uint32_t *__restrict__ keys, const uint32_t *__restrict__ vals,
+    const uint32_t *__restrict__ useg, const Item *__restrict__ items, const uint32_t *__restrict__ nitems) {
   __shared__ uint32_t s_mask[kPrefixWarps][kPrefixMaskWords];
   __shared__ StRec s_t[kPrefixWarps][32];
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -619,6 +623,12 @@ __global__ void __launch_bounds__(kPrefixWarps * 32) k_stencil_segment(
   uint32_t *mask = s_mask[warp];
   for (int w = lane; w < FWS; w += 32) mask[w] = 0;
   __syncwarp();
+  // the lowest clip height of the column's voxels from ue up (where the heights do not increase, less
+  // their distance from their affine form)
+  const uint32_t kz = keys[useg[ue]] - col * (uint32_t)g.n[2];
+  float clip = __ldg(g.o2[2] + (size_t)kz * g.n2[2]);
+  if (!g.oz_monotone) clip -= 10.3f * EPS24 * fmaxf(fabsf(g.bmin[2]), fabsf(g.bmax[2]));
+  bool over = false;
   const float4 *__restrict__ ptri = d.ptri;
   const uint32_t e0 = useg[ua], e1 = useg[ue];
   for (uint32_t b0 = e0; b0 < e1; b0 += 32) {
@@ -642,12 +652,15 @@ __global__ void __launch_bounds__(kPrefixWarps * 32) k_stencil_segment(
       if (w0 + lane < batch.total && st_sample(r, w0 + lane, sx, sy, zs)) {
         const int sidx = sy * SW + sx;
         atomicXor(&mask[sidx >> 5], 1u << (sidx & 31));
+        over = over || !(zs <= clip);
       }
     }
     __syncwarp();
   }
   uint32_t *out = bd.stp + (size_t)ua * bd.stp_words;
   for (int w = lane; w < FWS; w += 32) out[w] = mask[w];
+  over = __any_sync(FULL, over);
+  if (lane == 0) out[bd.stp_words - 1] = over ? 1u : 0u;
 }
 
 __global__ void __launch_bounds__(kPrefixWarps * 32) k_stencil_scan(
@@ -662,7 +675,7 @@ __global__ void __launch_bounds__(kPrefixWarps * 32) k_stencil_scan(
   if (!((w0.m_mesh >> 6) & 1u) || u0 + (w0.m_mesh & 63u) >= u1) return;
   const MeshDesc &d = bd.md[w0.m_mesh >> 7];
   const int FWS = (4 * d.g.n2[0] * d.g.n2[1] + 31) >> 5;  // <= kPrefixMaskWords
-  uint32_t acc[kPrefixMaskWords / 32] = {};
+  uint32_t acc[kPrefixMaskWords / 32] = {}, over = 0;
   // the column's item starts 32 voxels at a time (one flag load per lane), then each in order
   for (uint32_t base = u0; base < u1; base += 32) {
     const uint32_t uu = base + lane;
@@ -679,6 +692,11 @@ __global__ void __launch_bounds__(kPrefixWarps * 32) k_stencil_scan(
           m[w] = acc[k];
           acc[k] ^= seg;
         }
+      }
+      if (lane == 0) {
+        const uint32_t o = m[bd.stp_words - 1];
+        m[bd.stp_words - 1] = over ? u0 + 1u : 0u;
+        over |= o;
       }
     }
   }
@@ -1157,16 +1175,20 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_fill(
   for (int w = lane; w < m * W; w += 32) par[w] = 0;
 #pragma unroll 1
   for (int w = lane; w < m * FW; w += 32) ft[w] = 0;
+  uint32_t udraw = ua;  // stencil fill: the first voxel whose triangles are drawn
   if (ST) {
 #pragma unroll 1
     for (int w = lane; w < m * SWd; w += 32) stg[w] = 0;
 #pragma unroll 1
     for (int w = lane; w < m * FWS; w += 32) sft[w] = 0;
     // the coverage parity of the column's triangles recorded only below the chunk (none below a
-    // column's first voxel; the prefix pass writes the masks of the later chunk starts)
-    const bool first = (it.m_mesh >> 6) & 1u;
+    // column's first voxel; the prefix pass writes the masks of the later chunk starts), or none, and
+    // those triangles drawn too
+    const uint32_t *const pre = bd.stp + (size_t)ua * bd.stp_words;
+    const uint32_t head = (it.m_mesh >> 6) & 1u ? ua + 1u : pre[bd.stp_words - 1];
+    if (head) udraw = head - 1u;
 #pragma unroll 1
-    for (int w = lane; w < FWS; w += 32) sftacc[w] = first ? 0u : bd.stp[(size_t)ua * bd.stp_words + w];
+    for (int w = lane; w < FWS; w += 32) sftacc[w] = head ? 0u : pre[w];
   }
   if ((int)lane < m) kz[lane] = (int)(keys[useg[ua + lane]] - col * (uint32_t)nz);
   __syncwarp();
@@ -1182,8 +1204,8 @@ __global__ void __launch_bounds__(kWarps * 32, 6) k_level2c_fill(
     // at the Level2 ray-origin height o2z[k][s] (minZ + (s + 0.5)*gridSizeZ2, :1297), so a
     // covered sample at height zs counts in every slice from the first with o2z >= zs: one
     // toggle bit there, expanded by a prefix XOR below.
-    // triangles recorded from the chunk's first voxel up (those below are in the prefix)
-    const uint32_t g0 = useg[ua], g1 = useg[ucol_end];
+    // triangles recorded from the chunk's first voxel up (those below are in the prefix, where there is one)
+    const uint32_t g0 = useg[udraw], g1 = useg[ucol_end];
     const int SW = 2 * n2x, SH = 2 * n2y;
     const float lx = fa(fm((float)ci, g.g[0]), g.bmin[0]), hx = fa(lx, g.g[0]);
     const float ly = fa(fm((float)cj, g.g[1]), g.bmin[1]), hy = fa(ly, g.g[1]);
@@ -1603,7 +1625,7 @@ void launch_level2(const BatchDev &bd, const uint32_t *keys, const uint32_t *val
   count_launch(1);
   if (stp) {
     const unsigned nbp = (unsigned)((B + kPrefixWarps - 1) / kPrefixWarps);  // items <= B
-    k_stencil_segment<<<nbp, kPrefixWarps * 32, 0, s>>>(bd, vals, useg, items, nitems);
+    k_stencil_segment<<<nbp, kPrefixWarps * 32, 0, s>>>(bd, keys, vals, useg, items, nitems);
     k_stencil_scan<<<nbp, kPrefixWarps * 32, 0, s>>>(bd, iflag, items, nitems);
     count_launch(2);
   }
