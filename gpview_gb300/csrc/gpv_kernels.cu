@@ -429,6 +429,7 @@ struct L1Warp {
 
 // A group of consecutive triangles of one mesh and this warp's share of its chunks of units: every
 // S-th from the part-th, or (a piece of a heavy triangle) kHeavyChunks of them from there.
+constexpr int kNoItemYet = -2;
 struct L1Item {
   int m;           // mesh, -1: none left
   int64_t t0;      // first triangle
@@ -531,14 +532,22 @@ __global__ void __launch_bounds__(kL1Warps * 32, 8) k_level1(BatchDev bd, uint32
   const uint32_t nheavy = bd.heavy ? (uint32_t)min(*bd.heavy_n, (unsigned long long)bd.heavy_cap) : 0u;
   const uint32_t nitems = nheavy + (uint32_t)(bd.total_tiles * S);
   // the group after `it`: the next of its ticket, or the first of a new ticket
+  // (a warp's first ticket is its own place in the grid, the heavy pieces spread over the blocks; one from
+  // the queue, an atomic a warp on one word, and another to learn that none is left, were 8 us of a small call)
+  const uint32_t nwarps = gridDim.x * kL1Warps;
   auto advance = [&](L1Item &it) {
     if (it.m >= 0 && it.t0 + kL1Group < it.tend) {
       it.t0 += kL1Group;
       return;
     }
-    uint32_t tk = 0;
-    if (lane == 0) tk = atomicAdd(&bd.queue[0], 1u);
-    tk = __shfl_sync(FULL, tk, 0);
+    uint32_t tk = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    if (it.m != kNoItemYet) {
+      tk = nwarps;
+      if (nitems > nwarps) {
+        if (lane == 0) tk += atomicAdd(&bd.queue[0], 1u);
+        tk = __shfl_sync(FULL, tk, 0);
+      }
+    }
     if (tk >= nitems) {
       it.m = -1;
       return;
@@ -595,7 +604,7 @@ __global__ void __launch_bounds__(kL1Warps * 32, 8) k_level1(BatchDev bd, uint32
     nbuf = 0;
   };
 
-  L1Item it = {-1, 0, 0, 0, false};
+  L1Item it = {kNoItemYet, 0, 0, 0, false};
   advance(it);
   stage(it);
   for (uint32_t phase = 0; it.m >= 0; phase ^= 1u) {
