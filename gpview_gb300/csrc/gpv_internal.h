@@ -148,10 +148,10 @@ struct BatchDev {
   // Level1 emits the (voxel, triangle) records of every mesh; otherwise only of meshes with a Level2
   // grid (the others' are only counted)
   int emit_all = 0;
-  // Level1 pieces of triangles with many units, {mesh, triangle, piece, valid}: written by the prep
-  // kernel, heavy_n of them (zeroed before it), room for heavy_cap; nullptr: none are split.  Triangles
-  // that find the list full still add their pieces to heavy_n (64 bits: 2^31 triangles of up to
-  // heavy_cap pieces do not wrap it)
+  // Level1 pieces of triangles with many units, {mesh, triangle, piece, chunks of a piece (0: nothing)}:
+  // written by the prep kernel, heavy_n of them (zeroed before it), room for heavy_cap; nullptr: none are
+  // split.  Triangles that find the list full still add their pieces to heavy_n (64 bits: 2^31 triangles of
+  // up to heavy_cap pieces do not wrap it)
   uint4 *heavy = nullptr;
   unsigned long long *heavy_n = nullptr;
   uint32_t heavy_cap = 0;

@@ -152,7 +152,11 @@ __device__ __forceinline__ float4 ray_box(const float *V, const GridDev &g) {
 
 // ---------------------------------------------------------------------------------------------
 constexpr int kHeavyUnits = 64;   // a triangle with more (triangle, column) units is split ...
-constexpr int kHeavyChunks = 4;   // ... into pieces of this many 32-unit chunks
+constexpr int kHeavyChunks = 4;   // ... into pieces of this many 32-unit chunks, or
+// ... or of one in calls of few triangles where its box has more than kLongRun layers: a wall's columns
+// run through all of them (12 triangles of a box on 100x70x88, the no-alloc call: 220 us in pieces of four
+// chunks, 121 of one); with many triangles the other pieces hide it, and the list has room for longer ones
+constexpr int kLongRun = 32, kFewTriangles = 4096;
 
 // cell_of(v) from its estimate e = (v - mn) * inv, inv = n / (mx - mn).  The float quotient times n is
 // within four roundings of e, an absolute 1e-6 covering inv's denormals: where both ends truncate to one
@@ -174,7 +178,7 @@ __global__ void __launch_bounds__(256) k_prep(BatchDev bd) {
   const MeshDesc &d = bd.md[m];
   const GridDev &g = d.g;
   unsigned long long sat1 = 0, su = 0, fu = 0, r1 = 0;
-  uint32_t pieces = 0;
+  uint32_t pieces = 0, chunks = 0;
   if (live) {
     const int64_t t = gi - d.tri_base;
     float V[9];
@@ -240,12 +244,13 @@ __global__ void __launch_bounds__(256) k_prep(BatchDev bd) {
     d.rng[t] = make_int4((int)pack2(lo[0], hi[0]), (int)pack2(lo[1], hi[1]), (int)pack2(lo[2], hi[2]), 0);
     d.fbox[t] = fb;
     if (bd.heavy && su + fu > (unsigned long long)kHeavyUnits) {
-      const unsigned long long n = ((su + 31) / 32 + (fu + 31) / 32 + kHeavyChunks - 1) / kHeavyChunks;
+      chunks = sat_ok && hi[2] - lo[2] >= kLongRun && bd.total_tris <= kFewTriangles ? 1u : (uint32_t)kHeavyChunks;
+      const unsigned long long n = ((su + 31) / 32 + (fu + 31) / 32 + chunks - 1) / chunks;
       if (n <= bd.heavy_cap) pieces = (uint32_t)n;
     }
   }
   // A triangle with many units (large against the cells) goes to the heavy list, in pieces of
-  // kHeavyChunks chunks that any warp of the Level1 kernel takes, and is flagged so that its group
+  // `chunks` chunks that any warp of the Level1 kernel takes, and is flagged so that its group
   // leaves it out; where the list is full it stays with its group.  One atomic a warp: one a triangle
   // took 120 us where 262k triangles were all heavy.
   if (__any_sync(FULL, pieces != 0u)) {
@@ -260,7 +265,7 @@ __global__ void __launch_bounds__(256) k_prep(BatchDev bd) {
       if (listed) d.rng[t].w = 1;
       const uint32_t room = pos < cap ? (uint32_t)min(cap - pos, (unsigned long long)pieces) : 0u;
       for (uint32_t k = 0; k < room; ++k)
-        bd.heavy[pos + k] = make_uint4((uint32_t)m, (uint32_t)t, k, (uint32_t)listed);
+        bd.heavy[pos + k] = make_uint4((uint32_t)m, (uint32_t)t, k, listed ? chunks : 0u);
     }
   }
   block_add_prep(d.stats, sat1, su, fu, r1);
@@ -428,14 +433,14 @@ struct L1Warp {
 };
 
 // A group of consecutive triangles of one mesh and this warp's share of its chunks of units: every
-// S-th from the part-th, or (a piece of a heavy triangle) kHeavyChunks of them from there.
+// S-th from the part-th, or (a piece of a heavy triangle) `piece` of them from there.
 constexpr int kNoItemYet = -2;
 struct L1Item {
   int m;           // mesh, -1: none left
   int64_t t0;      // first triangle
   int64_t tend;    // end of the ticket's triangles
   uint32_t part;
-  bool piece;
+  uint32_t piece;  // 0: no piece
 };
 
 // z interval outside which the SAT's plane test fails for certain in the column at (cx, cy): on
@@ -552,13 +557,14 @@ __global__ void __launch_bounds__(kL1Warps * 32, 8) k_level1(BatchDev bd, uint32
       it.m = -1;
       return;
     }
-    it.piece = tk < nheavy;
-    if (it.piece) {  // the heavy pieces first
+    it.piece = 0u;
+    if (tk < nheavy) {  // the heavy pieces first
       const uint4 h = __ldg(bd.heavy + tk);
       it.m = (int)h.x;
       it.t0 = h.y;
       it.tend = it.t0 + (h.w ? 1 : 0);  // (an entry of a triangle that did not fit the list: nothing)
-      it.part = h.z * kHeavyChunks;
+      it.part = h.z * h.w;
+      it.piece = max(h.w, 1u);
       return;
     }
     tk -= nheavy;
@@ -604,7 +610,7 @@ __global__ void __launch_bounds__(kL1Warps * 32, 8) k_level1(BatchDev bd, uint32
     nbuf = 0;
   };
 
-  L1Item it = {kNoItemYet, 0, 0, 0, false};
+  L1Item it = {kNoItemYet, 0, 0, 0, 0u};
   advance(it);
   stage(it);
   for (uint32_t phase = 0; it.m >= 0; phase ^= 1u) {
@@ -657,7 +663,7 @@ __global__ void __launch_bounds__(kL1Warps * 32, 8) k_level1(BatchDev bd, uint32
     const bool emit = d.has_l2 || bd.emit_all;  // the records are read later (else only counted)
     const uint32_t nsc = (Us + 31u) >> 5;
     const uint32_t step = it.piece ? 1u : S;
-    const uint32_t cend = it.piece ? min(it.part + kHeavyChunks, nsc + ((Uf + 31u) >> 5)) : nsc + ((Uf + 31u) >> 5);
+    const uint32_t cend = it.piece ? min(it.part + it.piece, nsc + ((Uf + 31u) >> 5)) : nsc + ((Uf + 31u) >> 5);
     unsigned long long counted = 0;
     uint32_t chunk = it.part;
 
