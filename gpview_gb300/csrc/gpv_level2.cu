@@ -37,6 +37,7 @@ constexpr int kDirectCells = 4;  // a triangle whose box meets at most this many
 // tested exactly instead.  262k-triangle torus at 128^3 / 8^3, SAT us, rows and exact, by the distance:
 // 0.5 cells 326 and 445, 1.4 546 and 470, 2.9 784 and 500, 4.8 890 and 535, 14 1715 and 818.
 constexpr float kWide = 1.0f;
+constexpr float kFar = 0.125f;  // cells; from there on SAT runs are short (far_grid)
 constexpr int kMaskWords = 512;  // words of one mask kind per warp (sets the chunk length)
 
 __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v) {
@@ -239,9 +240,21 @@ __host__ __device__ __forceinline__ int sat_run_cap(const GridDev &g) {
   const int n = kSatWords / ((g.n2[0] * g.n2[1] * g.n2[2] + 31) >> 5);
   return n < 1 ? 1 : n > 32 ? 32 : n;
 }
+// Far from the origin (the centre tables an eighth of a cell and more off their affine form) a pair can be
+// hundreds of exact tests, so a run has no more pairs than half a warp's share.  Calls of small meshes
+// around 10000, us, with runs of full batches and so (and with the exact kernel before the row solver): 900
+// triangles at 56x65x54 / 8^3, 2 cells off, 665, 339 (418); 484 at 42x82x77 / 9^3 758, 493 (604); 440 at
+// 58x44x53 / 7^3 408, 245 (363); 1.3k at 45x69x41 / 15^3 765, 752 (686); 5.3k at 23x30x31 / 8^3, 0.3 off,
+// 235, 225 (414); where pairs are many nothing changes.
+__device__ __forceinline__ bool far_grid(const GridDev &g) {
+  float w = 0.f;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) w = fmaxf(w, 2.02f * EPS24 * fmaxf(fabsf(g.bmin[a]), fabsf(g.bmax[a])) * g.inv_g2[a]);
+  return w > kFar;
+}
 struct SatRuns {
   uint32_t q, qt, tail, nq;
-  __device__ __forceinline__ SatRuns(uint32_t pairs, uint32_t voxels, int slots, uint32_t cap) {
+  __device__ __forceinline__ SatRuns(uint32_t pairs, uint32_t voxels, int slots, uint32_t cap, bool far) {
     const uint32_t avg = pairs / voxels, nb = max(pairs / (32u * (uint32_t)slots), 1u);
     q = max(32u * nb, avg + 16u) - avg;
     qt = max(32u * max(nb / 4u, 1u), avg + 16u) - avg;
@@ -249,6 +262,7 @@ struct SatRuns {
       q = max(q, 256u);
       qt = q;
     }
+    if (far) q = qt = min(q, max(pairs / (uint32_t)slots, 1u));
     tail = pairs - pairs / 8u;
     nq = tail / q + 1u;
   }
@@ -300,7 +314,7 @@ __global__ void __launch_bounds__(kItemThreads) k_items(
       it.m_mesh = (end - uu) | (uu == head ? 64u : 0u) | ((uint32_t)mesh << 7);
       if (runs) {
         const uint32_t cap = (uint32_t)sat_run_cap(d.g);
-        const SatRuns sr(__ldg(useg + B), (uint32_t)B, slots, cap);
+        const SatRuns sr(__ldg(useg + B), (uint32_t)B, slots, cap, far_grid(d.g));
         const uint32_t r0 = (uu - (uint32_t)d.u_base) % cap, b = sr.bucket(__ldg(useg + u));
         rstart = r0 == 0 || sr.bucket(__ldg(useg + u - 1)) != b;
         if (rstart) {
