@@ -132,7 +132,7 @@ static_assert(sizeof(StScratch) >= 16 * 32 * 4, "the output stage keeps 16 layer
 // reduction over the lanes whose triangle starts among the 32, its slice an estimate that the table
 // corrects, and the scratch is 2.5 KB, so that 24 warps fit an SM: the 262k-triangle torus at 128^3 / 8^3
 // took 440 us in the fill and 70 in k_stencil_segment with 64-bit products, searches over the prefix and
-// the slices, and 16 warps; now 215 and 36.  Bound by latency (about half of the issue slots).
+// the slices, and 16 warps; 215 and 36 so (the heights' comparison added about 10 us to both since).  Bound by latency (about half of the issue slots).
 struct StBatch {
   uint32_t start, cnt, total;  // this lane's triangle's first sample and samples; the batch's
   __device__ __forceinline__ StBatch(StRec *recs, bool has, const StTri &t) {
